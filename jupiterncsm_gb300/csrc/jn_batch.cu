@@ -186,41 +186,42 @@ __global__ void kb_advance(int *d_k) { if (threadIdx.x == 0 && blockIdx.x == 0) 
 /* ------------------------------------------------------------------ */
 /* batched tridiagonal work (n per instance)                            */
 /* ------------------------------------------------------------------ */
-/* one warp per eigenvalue i = blockIdx.x (multisection) */
-__global__ void kb_tri_bisect(const double *__restrict__ alpha, const double *__restrict__ beta, int64_t ldab,
-			      const int *__restrict__ n_arr, int want, double *__restrict__ theta, int ldt,
-			      const int *__restrict__ active)
+/* eigenvalue i = blockIdx.x < want of each instance's T by one warp, and its
+ * eigenvector (rows of Z, its bottom component in zlast when not NULL).
+ * Scratch: shared memory, or `work` (JN_TRI_VECTOR_DOUBLES(ldz) a warp) when
+ * the rows do not fit there.  The first `guesses` entries of theta hold an
+ * earlier check's eigenvalues. */
+__global__ void __launch_bounds__(32) kb_tri_pairs(const double *__restrict__ alpha, const double *__restrict__ beta, int64_t ldab,
+						    const int *__restrict__ n_arr, int want, double *__restrict__ theta, int ldt,
+						    double *__restrict__ Z, int ldz, double *__restrict__ work,
+						    double *__restrict__ zlast, int guesses, const int *__restrict__ active)
 {
 	SKIP_INACTIVE();
+	extern __shared__ double sbuf[];
 	const int i = blockIdx.x;
 	const int n = n_arr[inst];
 	if (i >= want || i >= n) return;
-	const double v = jn_tri_multisect_warp(alpha + inst * ldab, beta + inst * ldab, n, i);
-	if (threadIdx.x == 0) theta[(int64_t)inst * ldt + i] = v;
-}
-
-__global__ void kb_tri_vectors(const double *__restrict__ alpha, const double *__restrict__ beta, int64_t ldab,
-			       const int *__restrict__ n_arr, int want, const double *__restrict__ theta, int ldt,
-			       double *__restrict__ Z, int ldz, double *__restrict__ work, double *__restrict__ zlast,
-			       const int *__restrict__ active)
-{
-	SKIP_INACTIVE();
-	const int i = blockIdx.x * blockDim.x + threadIdx.x;
-	const int n = n_arr[inst];
-	if (i >= want || i >= n) return;
+	const double *a = alpha + inst * ldab, *b = beta + inst * ldab;
+	double *as = work ? work + ((size_t)inst * want + i) * JN_TRI_VECTOR_DOUBLES(ldz) : sbuf, *b2 = as + n;
 	double *z = Z + ((int64_t)inst * want + i) * ldz;
-	jn_tri_vector_one(alpha + inst * ldab, beta + inst * ldab, n, theta[(int64_t)inst * ldt + i], z,
-			  work + ((int64_t)inst * want + i) * 5 * ldz);
-	if (zlast) zlast[(int64_t)inst * ldt + i] = z[n - 1];
+	double lo, hi;
+	const double sc = jn_tri_scale(a, b, n, &lo, &hi);
+	jn_tri_stage(a, b, n, sc, as, b2);
+	const double old = i < guesses ? theta[(int64_t)inst * ldt + i] : 0.0;
+	const double x = jn_tri_multisect_warp(as, b2, n, i, lo, hi, i < guesses, old * sc);
+	jn_tri_vector_warp(as, b2, n, x, z, b2 + n);
+	if (threadIdx.x == 0) {
+		theta[(int64_t)inst * ldt + i] = x / sc;
+		if (zlast) zlast[(int64_t)inst * ldt + i] = z[n - 1];
+	}
 }
 
 __global__ void kb_tri_mgs(double *__restrict__ Z, int ldz, const int *__restrict__ n_arr, int want,
 			   const int *__restrict__ active)
 {
 	SKIP_INACTIVE();
-	__shared__ double sh[BT];
 	const int n = n_arr[inst];
-	jn_tri_mgs(Z + (int64_t)inst * want * ldz, ldz, n, want < n ? want : n, sh);
+	jn_tri_mgs(Z + (int64_t)inst * want * ldz, ldz, n, want < n ? want : n);
 }
 
 /* converged[inst] = every one of the nev lowest Ritz values has
@@ -502,7 +503,11 @@ static jn_status batch_solve(cudaStream_t q, const jn_batch_options *o, const ba
 	BALLOC(s.zlast, (size_t)B * (r + 1));
 	const int zrows = r > want ? r : want;  /* vectors per instance: r at the end, want in checks */
 	BALLOC(s.Z, (size_t)B * zrows * ldz);
-	BALLOC(s.work, (size_t)B * zrows * 5 * ldz);
+	const int tri_smem = ldz <= JN_TRI_SMEM_ROWS;
+	if (!tri_smem) BALLOC(s.work, (size_t)B * zrows * JN_TRI_VECTOR_DOUBLES(ldz));
+	if (!st && cudaFuncSetAttribute(kb_tri_pairs, cudaFuncAttributeMaxDynamicSharedMemorySize,
+					(int)JN_TRI_SMEM(JN_TRI_SMEM_ROWS)) != cudaSuccess)
+		st = jn_fail(JN_ERR_CUDA, "batched Lanczos: shared memory of the tridiagonal kernel");
 	BALLOC(s.dims, B);
 	BALLOC(s.k, 1);
 	BALLOC(s.active, B);
@@ -528,7 +533,7 @@ static jn_status batch_solve(cudaStream_t q, const jn_batch_options *o, const ba
 	for (int i = 0; i < B; i++) { hact[i] = 1; hn[i] = 0; }
 	cudaGraphExec_t gexec = NULL;
 	cudaGraph_t graph = NULL;
-	int k = 0, nactive = B;
+	int k = 0, nactive = B, guesses = 0;
 	const int vg = (int)((Dp + BT - 1) / BT < 64 ? (Dp + BT - 1) / BT : 64);
 	const dim3 gv(vg > 0 ? vg : 1, B), gr(BNB, B), g1(1, B);
 	const int64_t *dims = s.dims;
@@ -586,9 +591,9 @@ static jn_status batch_solve(cudaStream_t q, const jn_batch_options *o, const ba
 		for (int i = 0; i < B; i++) hn[i] = hact[i] ? k : hn[i];
 		cudaMemcpyAsync(s.narr, hn, B * sizeof(int), cudaMemcpyHostToDevice, q);
 		const int wk = want < k ? want : k;
-		kb_tri_bisect<<<dim3(wk, B), 32, 0, q>>>(s.alpha, s.beta, ldab, s.narr, wk, s.theta, r + 1, s.active);
-		kb_tri_vectors<<<dim3((wk + 31) / 32, B), 32, 0, q>>>(s.alpha, s.beta, ldab, s.narr, wk, s.theta, r + 1, s.Z,
-									ldz, s.work, s.zlast, s.active);
+		kb_tri_pairs<<<dim3(wk, B), 32, tri_smem ? JN_TRI_SMEM(k) : 0, q>>>(
+			s.alpha, s.beta, ldab, s.narr, wk, s.theta, r + 1, s.Z, ldz, s.work, s.zlast, guesses, s.active);
+		guesses = wk;
 		kb_converged<<<(B + 127) / 128, 128, 0, q>>>(s.theta, s.zlast, r + 1, s.beta, ldab, s.narr, nev, o->tolerance,
 							     s.flag, s.active, B);
 		if (cudaMemcpyAsync(hflag, s.flag, B * sizeof(int), cudaMemcpyDeviceToHost, q) != cudaSuccess ||
@@ -622,9 +627,8 @@ static jn_status batch_solve(cudaStream_t q, const jn_batch_options *o, const ba
 		for (int i = 0; i < B; i++) hact[i] = 1;
 		cudaMemcpyAsync(s.narr, hn, B * sizeof(int), cudaMemcpyHostToDevice, q);
 		cudaMemcpyAsync(s.active, hact, B * sizeof(int), cudaMemcpyHostToDevice, q);
-		kb_tri_bisect<<<dim3(r, B), 32, 0, q>>>(s.alpha, s.beta, ldab, s.narr, r, s.theta, r + 1, NULL);
-		kb_tri_vectors<<<dim3((r + 31) / 32, B), 32, 0, q>>>(s.alpha, s.beta, ldab, s.narr, r, s.theta, r + 1, s.Z, ldz,
-								     s.work, NULL, NULL);
+		kb_tri_pairs<<<dim3(r, B), 32, tri_smem ? JN_TRI_SMEM(k) : 0, q>>>(
+			s.alpha, s.beta, ldab, s.narr, r, s.theta, r + 1, s.Z, ldz, s.work, NULL, guesses, NULL);
 		kb_tri_mgs<<<g1, BT, 0, q>>>(s.Z, ldz, s.narr, r, NULL);
 		kb_ritz<<<gv, BT, 0, q>>>(s.V, ldV, s.Z, ldz, s.narr, r, Dp, dims, s.X);
 		/* H X in FP64-grade arithmetic, one batched product per Ritz index */

@@ -24,11 +24,13 @@
  *                         residual norm beta_k |s_{k,i}|.
  *
  * The Krylov basis stays in HBM.  Every reduction is a two-pass fixed-order
- * reduction, so two runs give bit-identical alpha/beta.  The tridiagonal
- * eigenvalues are computed on the GPU by Sturm-sequence bisection (one
- * thread per eigenvalue) and the eigenvectors by inverse iteration on the
- * tridiagonal matrix; the final Ritz vectors are refined by FP64 products
- * (Rayleigh quotient and residual norm).
+ * reduction, so two runs give bit-identical alpha/beta.  In full mode one
+ * cooperative kernel (k_orthonormalize) takes w = H v_k to v_{k+1}.  The
+ * convergence check (k_tri_check: eigenvalues of T by multisection and their
+ * eigenvectors, jn_tridiag.cuh) runs on its own stream beside the next
+ * step's product: the host enqueues step k + 1, then reads the check of
+ * step k.  The final Ritz vectors are refined by FP64 products (Rayleigh
+ * quotient and residual norm).
  */
 #include <math.h>
 #include <stdio.h>
@@ -39,6 +41,8 @@
 #include <time.h>
 
 #include <vector>
+
+#include <cooperative_groups.h>
 
 #include "jn_internal.h"
 #include "jn_tridiag.cuh"
@@ -59,10 +63,16 @@ struct jn_lanczos_state {
 	double *d_scalar;       /* 4 scalars */
 	double *d_theta;        /* Ritz values (ascending), mmax */
 	double *d_Z;            /* nev_cap x mmax tridiagonal eigenvectors */
+	double *d_work;         /* scratch of k_tri_check above JN_TRI_SMEM_ROWS rows, else NULL */
+	unsigned int *d_done;   /* finished CTAs of k_tri_check */
+	double *d_pack;         /* a check's results: Ritz values, bottom components, beta */
 	double *d_ritz;         /* nev x D Ritz vectors */
-	double *h_alpha, *h_beta;
-	double *h_theta;
-	double *h_zlast;        /* bottom components */
+	double *d_hritz;        /* and H times them */
+	double *d_rr;           /* Rayleigh quotients, residual norms (2 nev_cap) */
+	double *h_pack[2];      /* pinned copies of d_pack: a check is read while the next one runs */
+	cudaStream_t check;     /* the checks' stream */
+	cudaEvent_t stepped, checked[2];
+	int guesses;            /* entries of d_theta that hold eigenvalues of the last T of this solve */
 	int nev_cap;
 	int have_ritz;
 	double *h_rq, *h_res;   /* refined Rayleigh quotients and residual norms */
@@ -74,7 +84,14 @@ void jn_lanczos_release(jn_ctx *c)
 	if (!s) return;
 	cudaFree(s->d_V); cudaFree(s->d_w); cudaFree(s->d_alpha); cudaFree(s->d_beta); cudaFree(s->d_part);
 	cudaFree(s->d_h); cudaFree(s->d_scalar); cudaFree(s->d_theta); cudaFree(s->d_Z); cudaFree(s->d_ritz);
-	free(s->h_alpha); free(s->h_beta); free(s->h_theta); free(s->h_zlast); free(s->h_rq); free(s->h_res);
+	cudaFree(s->d_work); cudaFree(s->d_done); cudaFree(s->d_pack); cudaFree(s->d_hritz); cudaFree(s->d_rr);
+	for (int i = 0; i < 2; i++) {
+		if (s->h_pack[i]) cudaFreeHost(s->h_pack[i]);
+		if (s->checked[i]) cudaEventDestroy(s->checked[i]);
+	}
+	if (s->stepped) cudaEventDestroy(s->stepped);
+	if (s->check) cudaStreamDestroy(s->check);
+	free(s->h_rq); free(s->h_res);
 	free(s);
 	c->lz = NULL;
 }
@@ -114,28 +131,6 @@ __global__ void k_finish(const double *__restrict__ part, int nblk, int ncol, in
 	if (lane == 0) out[j] = s;
 }
 
-/* w -= sum_j V[j] h[j] (j < nvec) */
-__global__ void k_gemv_n_sub(const double *__restrict__ V, int64_t D, int nvec, const double *__restrict__ h,
-			     double *__restrict__ w)
-{
-	for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < D; i += (int64_t)gridDim.x * blockDim.x) {
-		double s = 0.0;
-		for (int j = 0; j < nvec; j++) s = fma(V[(int64_t)j * D + i], h[j], s);
-		w[i] -= s;
-	}
-}
-
-/* out = sum_j V[j] z[j] */
-__global__ void k_gemv_n(const double *__restrict__ V, int64_t D, int nvec, const double *__restrict__ z,
-			 double *__restrict__ out)
-{
-	for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < D; i += (int64_t)gridDim.x * blockDim.x) {
-		double s = 0.0;
-		for (int j = 0; j < nvec; j++) s = fma(V[(int64_t)j * D + i], z[j], s);
-		out[i] = s;
-	}
-}
-
 /* w -= a*v + b*u (reads a = *pa, b = *pb on the device; u may be NULL) */
 __global__ void k_three_term(double *__restrict__ w, const double *__restrict__ v, const double *__restrict__ u,
 			     const double *pa, const double *pb, int64_t D)
@@ -159,12 +154,6 @@ __global__ void k_normalize(double *__restrict__ dst, const double *__restrict__
 		dst[i] = src[i] * inv;
 }
 
-__global__ void k_scale_copy(double *__restrict__ dst, const double *__restrict__ src, double s, int64_t D)
-{
-	for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < D; i += (int64_t)gridDim.x * blockDim.x)
-		dst[i] = src[i] * s;
-}
-
 __global__ void k_axpy_neg(double *__restrict__ y, const double *__restrict__ x, const double *pa, int64_t D)
 {
 	const double a = *pa;
@@ -173,33 +162,291 @@ __global__ void k_axpy_neg(double *__restrict__ y, const double *__restrict__ x,
 }
 
 /* ------------------------------------------------------------------ */
+/* full reorthogonalisation                                            */
+/* ------------------------------------------------------------------ */
+#define ORTHO_WARPS 8
+#define ORTHO_GROUP 16          /* vectors a warp sums at once in the dot products */
+#define ORTHO_H 1024            /* coefficients staged at a time in the subtraction */
+
+/* part[j G + blockIdx.x] = V_j . w over elements [i0, i1), j < nvec.  A warp
+ * takes 16 vectors, its lanes the elements (coalesced rows of V), 16 sums in
+ * registers; the sums are then folded across the lanes by halves, 16 adds
+ * for the 16 vectors where a butterfly per vector takes 80 (GB300's FP64
+ * pipe charges 64 cycles each).  With few vectors the warps share a group's
+ * elements. */
+__device__ __forceinline__ void ortho_dots(const double *__restrict__ V, int64_t D, int nvec, const double *w, int64_t i0,
+					   int64_t i1, double *__restrict__ part, double (*ps)[ORTHO_WARPS / 2 * ORTHO_GROUP])
+{
+	const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+	const int ng = (nvec + ORTHO_GROUP - 1) / ORTHO_GROUP, split = ng < ORTHO_WARPS ? ORTHO_WARPS / ng : 1;
+	const int64_t sub = ((i1 - i0 + split - 1) / split + 31) & ~31ll;
+	for (int task = warp; task < ng * split; task += ORTHO_WARPS) {
+		const int g = task % ng, sp = task / ng, j0 = g * ORTHO_GROUP;
+		const int64_t e0 = i0 + sp * sub, e1 = min(i1, e0 + sub);
+		double acc[ORTHO_GROUP];
+#pragma unroll
+		for (int u = 0; u < ORTHO_GROUP; u++) acc[u] = 0.0;
+		const double *v = V + (int64_t)j0 * D;
+		if (j0 + ORTHO_GROUP <= nvec) {
+			for (int64_t e = e0 + lane; e < e1; e += 32) {
+				const double we = w[e];
+#pragma unroll
+				for (int u = 0; u < ORTHO_GROUP; u++) acc[u] = fma(v[u * D + e], we, acc[u]);
+			}
+		} else {
+			for (int64_t e = e0 + lane; e < e1; e += 32) {
+				const double we = w[e];
+#pragma unroll
+				for (int u = 0; u < ORTHO_GROUP; u++)
+					if (j0 + u < nvec) acc[u] = fma(v[u * D + e], we, acc[u]);
+			}
+		}
+#pragma unroll
+		for (int h = ORTHO_GROUP / 2; h; h >>= 1) {
+			const bool up = (lane & (2 * h)) != 0;
+#pragma unroll
+			for (int u = 0; u < h; u++) {
+				const double give = up ? acc[u] : acc[u + h], keep = up ? acc[u + h] : acc[u];
+				acc[u] = keep + __shfl_xor_sync(0xffffffffu, give, 2 * h);
+			}
+		}
+		acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], 1);
+		const int j = j0 + (lane >> 1);
+		if (!(lane & 1) && j < nvec) {
+			if (split > 1) ps[sp][j] = acc[0];
+			else part[(int64_t)j * gridDim.x + blockIdx.x] = acc[0];
+		}
+	}
+	if (split > 1) {
+		__syncthreads();
+		for (int j = threadIdx.x; j < nvec; j += blockDim.x) {
+			double s = ps[0][j];
+			for (int sp = 1; sp < split; sp++) s += ps[sp][j];
+			part[(int64_t)j * gridDim.x + blockIdx.x] = s;
+		}
+	}
+}
+
+/* h[j] = sum over the CTAs' partials of vector j, one warp of the grid per j */
+__device__ __forceinline__ void ortho_reduce(const double *part, int nvec, double *h)
+{
+	const int lane = threadIdx.x & 31;
+	for (int j = blockIdx.x * ORTHO_WARPS + (threadIdx.x >> 5); j < nvec; j += gridDim.x * ORTHO_WARPS) {
+		double s = 0.0;
+		for (int b = lane; b < (int)gridDim.x; b += 32) s += __ldcg(part + (int64_t)j * gridDim.x + b);
+		for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+		if (lane == 0) h[j] = s;
+	}
+}
+
+/* w -= sum_j V_j h_j over [i0, i1): a warp's lanes are 32 elements; the warps
+ * share the vectors where the slice has fewer than 8 x 32 elements */
+__device__ __forceinline__ void ortho_subtract(const double *__restrict__ V, int64_t D, int nvec, const double *h, double *w,
+					       int64_t i0, int64_t i1, double *hs, double (*ps)[32])
+{
+	const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+	const int64_t tiles = (i1 - i0 + 31) / 32;
+	const int split = tiles < ORTHO_WARPS ? ORTHO_WARPS / (int)max(tiles, (int64_t)1) : 1;
+	for (int c0 = 0; c0 < nvec; c0 += ORTHO_H) {
+		const int nc = min(ORTHO_H, nvec - c0);
+		__syncthreads();
+		for (int j = threadIdx.x; j < nc; j += blockDim.x) hs[j] = __ldcg(h + c0 + j);
+		__syncthreads();
+		const int sub = (nc + split - 1) / split;
+		for (int64_t task = warp; task < tiles * split; task += ORTHO_WARPS) {
+			const int64_t tile = task % tiles;
+			const int sp = (int)(task / tiles), ja = sp * sub, jb = min(nc, ja + sub);
+			const int64_t e = i0 + tile * 32 + lane;
+			double s = 0.0;
+			if (e < i1) {
+				const double *v = V + (int64_t)(c0 + ja) * D + e;
+#pragma unroll 8
+				for (int j = ja; j < jb; j++, v += D) s = fma(*v, hs[j], s);
+			}
+			if (split > 1) ps[task][lane] = s;
+			else if (e < i1) w[e] -= s;
+		}
+		if (split > 1) {
+			__syncthreads();
+			for (int64_t task = warp; task < tiles; task += ORTHO_WARPS) {
+				const int64_t e = i0 + task * 32 + lane;
+				double s = ps[task][lane];
+				for (int sp = 1; sp < split; sp++) s += ps[task + sp * tiles][lane];
+				if (e < i1) w[e] -= s;
+			}
+		}
+	}
+	__syncthreads();
+}
+
+/* One Lanczos step's vector work: from w = H v_k, with v_0 .. v_k the
+ * orthonormal basis,
+ *     h = V^T w;  w -= V h;  h' = V^T w;  w -= V h';
+ *     alpha_k = h_k;  beta_k = |w|;  v_{k+1} = w / beta_k:
+ * classical Gram-Schmidt twice over the whole basis, of which the first pass
+ * holds the three-term recurrence.  A cooperative launch, one CTA an SM, a
+ * slice of the vectors to each; the CTAs meet at five grid-wide barriers.
+ * Bound by the FP64 pipe (4 multiply-adds per element and vector) and the
+ * barriers: 34 us a step at D = 7 916, k = 25 to 125.  As thirteen kernels in
+ * a row (dots, their sums, recurrence, two passes, norm, scaling) the same
+ * work took 130 us at k = 45, most of it launches and a subtraction on 31
+ * CTAs. */
+__global__ void __launch_bounds__(ORTHO_WARPS * 32)
+	k_orthonormalize(double *__restrict__ V, int64_t D, int64_t chunk, int k, double *w, double *part, double *h,
+			 double *__restrict__ alpha, double *__restrict__ beta)
+{
+	__shared__ double ps[ORTHO_WARPS][ORTHO_WARPS / 2 * ORTHO_GROUP];
+	__shared__ double pt[ORTHO_WARPS][32];
+	__shared__ double hs[ORTHO_H];
+	namespace cg = cooperative_groups;
+	cg::grid_group grid = cg::this_grid();
+	const int nvec = k + 1, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+	const int64_t i0 = (int64_t)blockIdx.x * chunk, i1 = min(D, i0 + chunk);
+	for (int pass = 0; pass < 2; pass++) {
+		ortho_dots(V, D, nvec, w, i0, i1, part, ps);
+		grid.sync();
+		ortho_reduce(part, nvec, h);
+		grid.sync();
+		if (pass == 0 && blockIdx.x == 0 && threadIdx.x == 0) alpha[k] = __ldcg(h + k);
+		ortho_subtract(V, D, nvec, h, w, i0, i1, hs, pt);
+	}
+	/* the norm: every CTA adds the CTAs' partials in the same order */
+	double s = 0.0;
+	for (int64_t e = i0 + threadIdx.x; e < i1; e += blockDim.x) s = fma(w[e], w[e], s);
+	for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+	if (lane == 0) ps[0][warp] = s;
+	__syncthreads();
+	if (threadIdx.x == 0) {
+		s = ps[0][0];
+		for (int i = 1; i < ORTHO_WARPS; i++) s += ps[0][i];
+		part[blockIdx.x] = s;
+	}
+	grid.sync();
+	if (warp == 0) {
+		s = 0.0;
+		for (int b = lane; b < (int)gridDim.x; b += 32) s += __ldcg(part + b);
+		for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+		const double b = sqrt(s);
+		if (lane == 0) {
+			ps[1][0] = b > 0.0 ? 1.0 / b : 0.0;
+			if (blockIdx.x == 0) beta[k] = b;
+		}
+	}
+	__syncthreads();
+	const double inv = ps[1][0];
+	double *v = V + (int64_t)(k + 1) * D;
+	for (int64_t e = i0 + threadIdx.x; e < i1; e += blockDim.x) v[e] = w[e] * inv;
+}
+
+/* X[i] = sum_j Z[i][j] V[j], i < want: an element of each V_j is read once
+ * for 8 Ritz vectors */
+#define RITZ_ROWS 8
+#define RITZ_J 256
+__global__ void __launch_bounds__(128) k_ritz_vectors(const double *__restrict__ V, int64_t D, int n, const double *__restrict__ Z,
+						       int ldz, int want, double *__restrict__ X)
+{
+	__shared__ double zs[RITZ_ROWS][RITZ_J];
+	const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+	const int i0 = blockIdx.y * RITZ_ROWS, ni = min(RITZ_ROWS, want - i0);
+	double acc[RITZ_ROWS];
+#pragma unroll
+	for (int i = 0; i < RITZ_ROWS; i++) acc[i] = 0.0;
+	for (int j0 = 0; j0 < n; j0 += RITZ_J) {
+		const int nj = min(RITZ_J, n - j0);
+		__syncthreads();
+		for (int t = threadIdx.x; t < RITZ_ROWS * nj; t += blockDim.x)
+			zs[t / nj][t % nj] = t / nj < ni ? Z[(int64_t)(i0 + t / nj) * ldz + j0 + t % nj] : 0.0;
+		__syncthreads();
+		if (e < D) {
+			const double *v = V + (int64_t)j0 * D + e;
+#pragma unroll 4
+			for (int j = 0; j < nj; j++, v += D) {
+				const double x = *v;
+#pragma unroll
+				for (int i = 0; i < RITZ_ROWS; i++) acc[i] = fma(x, zs[i][j], acc[i]);
+			}
+		}
+	}
+	if (e < D)
+#pragma unroll
+		for (int i = 0; i < RITZ_ROWS; i++)
+			if (i < ni) X[(int64_t)(i0 + i) * D + e] = acc[i];
+}
+
+/* CTA i: rr[i] = x.w / x.x (the Rayleigh quotient of x = X_i, w = H x), rr[n + i] = |w - rr[i] x| / |x| */
+__global__ void __launch_bounds__(512) k_rayleigh(const double *__restrict__ X, const double *__restrict__ HX, int64_t D, int n,
+						   double *__restrict__ rr)
+{
+	__shared__ double sh[512];
+	const double *x = X + (int64_t)blockIdx.x * D, *w = HX + (int64_t)blockIdx.x * D;
+	double xw = 0.0, xx = 0.0;
+	for (int64_t e = threadIdx.x; e < D; e += blockDim.x) {
+		xw = fma(x[e], w[e], xw);
+		xx = fma(x[e], x[e], xx);
+	}
+	xw = jn_block_sum(xw, sh);
+	xx = jn_block_sum(xx, sh);
+	const double q = xw / xx;
+	double r2 = 0.0;
+	for (int64_t e = threadIdx.x; e < D; e += blockDim.x) {
+		const double r = w[e] - q * x[e];
+		r2 = fma(r, r, r2);
+	}
+	r2 = jn_block_sum(r2, sh);
+	if (threadIdx.x == 0) {
+		rr[blockIdx.x] = q;
+		rr[n + blockIdx.x] = sqrt(r2 / xx);
+	}
+}
+
+/* ------------------------------------------------------------------ */
 /* tridiagonal eigenproblem                                            */
 /* ------------------------------------------------------------------ */
-/* theta[i] for i = blockIdx.x < want: the i-th smallest eigenvalue, by warp multisection */
-__global__ void k_tri_bisect(const double *__restrict__ a, const double *__restrict__ b, int n, int want,
-			     double *__restrict__ theta)
-{
-	const int i = blockIdx.x;
-	if (i >= want) return;
-	const double v = jn_tri_multisect_warp(a, b, n, i);
-	if (threadIdx.x == 0) theta[i] = v;
-}
+#define TRI_THREADS 128
+#define TRI_WAVE 256            /* eigenvalues at a time where the scratch is in global memory */
 
-/* eigenvector of T for theta[i] by inverse iteration; Z row i holds the n components */
-__global__ void k_tri_vectors(const double *__restrict__ a, const double *__restrict__ b, int n, int want,
-			      const double *__restrict__ theta, double *__restrict__ Z, int ldz, double *__restrict__ work,
-			      int ldw)
+/* The `want` lowest eigenvalues of T_n, CTA i the (first + i)-th, and the eigenvectors
+ * of the lowest `nvec` (rows of Z).  The CTA that finishes last makes the
+ * vectors orthogonal among themselves and packs the results for one copy to
+ * the host: theta (want), the vectors' bottom components (nvec), beta_{n-1}.
+ * The first `guesses` entries of theta hold an earlier check's eigenvalues.
+ * Scratch: shared memory, or `work` (JN_TRI_VECTOR_DOUBLES(n) a CTA) above
+ * JN_TRI_SMEM_ROWS rows.  Bound by the FP64 chains of one warp (about five
+ * rounds of 3 n instructions, then 2 n for the vector, 64 cycles each): 125
+ * us for 11 pairs at n = 25 to 125, where bisection, inverse iteration and
+ * Gram-Schmidt as three kernels took 700 us at n = 45. */
+__global__ void __launch_bounds__(TRI_THREADS)
+	k_tri_check(const double *__restrict__ a, const double *__restrict__ b, int n, int want, int nvec,
+		    double *__restrict__ theta, double *Z, int ldz, double *work, unsigned int *__restrict__ done,
+		    double *__restrict__ pack, int first, int guesses)
 {
-	int i = blockIdx.x * blockDim.x + threadIdx.x;
-	if (i >= want) return;
-	jn_tri_vector_one(a, b, n, theta[i], Z + (int64_t)i * ldz, work + (int64_t)i * ldw);
-}
-
-/* modified Gram-Schmidt among the `want` tridiagonal eigenvectors (one CTA) */
-__global__ void k_tri_mgs(double *__restrict__ Z, int ldz, int n, int want)
-{
-	__shared__ double sh[RED_THREADS];
-	jn_tri_mgs(Z, ldz, n, want, sh);
+	extern __shared__ double sbuf[];
+	__shared__ unsigned int last;
+	const int i = first + blockIdx.x;
+	if (threadIdx.x < 32) {
+		double *as = work ? work + (size_t)blockIdx.x * JN_TRI_VECTOR_DOUBLES(n) : sbuf, *b2 = as + n;
+		double lo, hi;
+		const double sc = jn_tri_scale(a, b, n, &lo, &hi);
+		jn_tri_stage(a, b, n, sc, as, b2);
+		const double x = jn_tri_multisect_warp(as, b2, n, i, lo, hi, i < guesses, i < guesses ? theta[i] * sc : 0.0);
+		if (threadIdx.x == 0) theta[i] = x / sc;
+		if (i < nvec) jn_tri_vector_warp(as, b2, n, x, Z + (int64_t)i * ldz, b2 + n);
+	}
+	__syncthreads();
+	if (threadIdx.x == 0) {
+		__threadfence();
+		last = atomicAdd(done, 1u) == gridDim.x - 1;
+	}
+	__syncthreads();
+	if (!last) return;
+	__threadfence();
+	if (nvec > 0) jn_tri_mgs(Z, ldz, n, nvec);
+	for (int j = threadIdx.x; j < want; j += blockDim.x) pack[j] = __ldcg(theta + j);
+	for (int j = threadIdx.x; j < nvec; j += blockDim.x) pack[want + j] = Z[(int64_t)j * ldz + n - 1];
+	if (threadIdx.x == 0) {
+		pack[want + nvec] = b[n - 1];
+		*done = 0;
+	}
 }
 
 /* ------------------------------------------------------------------ */
@@ -222,17 +469,6 @@ static void dot_dev(jn_ctx *c, const double *x, const double *y, double *res)
 	k_finish<<<1, 32, 0, c->stream>>>(s->d_part, RED_BLOCKS, 1, 1, res);
 }
 
-/* w -= V[0..nvec) (V[0..nvec)^T w) */
-static void cgs_pass(jn_ctx *c, int nvec)
-{
-	struct jn_lanczos_state *s = c->lz;
-	if (nvec <= 0) return;
-	int ncol = s->mmax + 2;
-	k_gemv_t<<<RED_BLOCKS, RED_THREADS, 0, c->stream>>>(s->d_V, s->D, nvec, s->d_w, s->d_part, ncol);
-	k_finish<<<(nvec + 3) / 4, 128, 0, c->stream>>>(s->d_part, RED_BLOCKS, ncol, nvec, s->d_h);
-	k_gemv_n_sub<<<grid_for(s->D), 256, 0, c->stream>>>(s->d_V, s->D, nvec, s->d_h, s->d_w);
-}
-
 static jn_status ensure_state(jn_ctx *c, int mmax, int nev)
 {
 	struct jn_lanczos_state *s = c->lz;
@@ -243,8 +479,9 @@ static jn_status ensure_state(jn_ctx *c, int mmax, int nev)
 	c->lz = s;
 	s->D = D; s->mmax = mmax; s->nev_cap = nev;
 	size_t ncol = (size_t)mmax + 2;
+	const size_t packed = (size_t)mmax + nev + 4;
 	cudaError_t e = cudaSuccess;
-#define DALLOC(ptr, n) if (e == cudaSuccess) e = cudaMalloc((void **)&(ptr), (size_t)(n) * sizeof(double))
+#define DALLOC(ptr, n) if (e == cudaSuccess) e = cudaMalloc((void **)&(ptr), (size_t)(n) * sizeof(*(ptr)))
 	DALLOC(s->d_V, (size_t)(mmax + 1) * D);
 	DALLOC(s->d_w, D);
 	DALLOC(s->d_alpha, mmax + 1);
@@ -253,44 +490,77 @@ static jn_status ensure_state(jn_ctx *c, int mmax, int nev)
 	DALLOC(s->d_h, ncol);
 	DALLOC(s->d_scalar, 8);
 	DALLOC(s->d_theta, mmax + 1);
-	DALLOC(s->d_Z, (size_t)nev * (mmax + 1) + (size_t)nev * 5 * (mmax + 1));
+	DALLOC(s->d_Z, (size_t)nev * (mmax + 1));
+	/* one CTA for each of nev + 1 eigenvalues of a check; all the eigenvalues come TRI_WAVE at a time */
+	if (mmax > JN_TRI_SMEM_ROWS)
+		DALLOC(s->d_work, (size_t)(nev + 1 > TRI_WAVE ? nev + 1 : TRI_WAVE) * JN_TRI_VECTOR_DOUBLES(mmax));
+	DALLOC(s->d_done, 1);
+	DALLOC(s->d_pack, packed);
 	DALLOC(s->d_ritz, (size_t)nev * D);
+	DALLOC(s->d_hritz, (size_t)nev * D);
+	DALLOC(s->d_rr, 2 * (size_t)nev);
 #undef DALLOC
+	for (int i = 0; i < 2; i++) {
+		if (e == cudaSuccess) e = cudaMallocHost((void **)&s->h_pack[i], packed * sizeof(double));
+		if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s->checked[i], cudaEventDisableTiming);
+	}
+	if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s->stepped, cudaEventDisableTiming);
+	/* the checks' few CTAs are scheduled before the product's thousands */
+	int least = 0, greatest = 0;
+	if (e == cudaSuccess) e = cudaDeviceGetStreamPriorityRange(&least, &greatest);
+	if (e == cudaSuccess) e = cudaStreamCreateWithPriority(&s->check, cudaStreamNonBlocking, greatest);
+	if (e == cudaSuccess) e = cudaMemsetAsync(s->d_done, 0, sizeof(unsigned int), s->check);
+	if (e == cudaSuccess)
+		e = cudaFuncSetAttribute(k_tri_check, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)JN_TRI_SMEM(JN_TRI_SMEM_ROWS));
 	if (e != cudaSuccess) {
 		jn_lanczos_release(c);
 		return jn_fail(JN_ERR_NOMEM, "Lanczos workspace (%d vectors of %lld): %s", mmax + 1, (long long)D,
 			       cudaGetErrorString(e));
 	}
-	s->h_alpha = (double *)calloc(mmax + 1, sizeof(double));
-	s->h_beta = (double *)calloc(mmax + 1, sizeof(double));
-	s->h_theta = (double *)calloc(mmax + 1, sizeof(double));
-	s->h_zlast = (double *)calloc(nev + 1, sizeof(double));
 	s->h_rq = (double *)calloc(nev + 1, sizeof(double));
 	s->h_res = (double *)calloc(nev + 1, sizeof(double));
 	return JN_OK;
 }
 
-/* Ritz values of T_n (ascending) for the lowest `want`, and the tridiagonal
- * eigenvectors when vectors != 0; results copied to the host arrays. */
-static jn_status tri_eig(jn_ctx *c, int n, int want, int vectors)
+/* Enqueue, behind the work now on the context's stream, the lowest `want`
+ * eigenvalues of T_n and the eigenvectors of the lowest `nvec` (rows of d_Z)
+ * on the checks' stream; h_pack[slot] receives theta (want), the bottom
+ * components (nvec) and beta_{n-1} once checked[slot] has happened. */
+static jn_status tri_enqueue(jn_ctx *c, int n, int want, int nvec, int slot)
 {
 	struct jn_lanczos_state *s = c->lz;
-	if (want > n) want = n;
-	k_tri_bisect<<<want, 32, 0, c->stream>>>(s->d_alpha, s->d_beta, n, want, s->d_theta);
-	if (vectors) {
-		int ldz = s->mmax + 1;
-		double *work = s->d_Z + (size_t)s->nev_cap * ldz;
-		int w2 = want < s->nev_cap ? want : s->nev_cap;
-		k_tri_vectors<<<(w2 + 31) / 32, 32, 0, c->stream>>>(s->d_alpha, s->d_beta, n, w2, s->d_theta, s->d_Z, ldz,
-								    work, 5 * ldz);
-		k_tri_mgs<<<1, RED_THREADS, 0, c->stream>>>(s->d_Z, ldz, n, w2);
-		for (int i = 0; i < w2; i++)
-			CUDA_TRY(cudaMemcpyAsync(s->h_zlast + i, s->d_Z + (size_t)i * ldz + n - 1, sizeof(double),
-						 cudaMemcpyDeviceToHost, c->stream));
+	CUDA_TRY(cudaEventRecord(s->stepped, c->stream));
+	CUDA_TRY(cudaStreamWaitEvent(s->check, s->stepped, 0));
+	const int in_smem = n <= JN_TRI_SMEM_ROWS;
+	if (in_smem || want <= TRI_WAVE) {
+		k_tri_check<<<want, TRI_THREADS, in_smem ? JN_TRI_SMEM(n) : 0, s->check>>>(
+			s->d_alpha, s->d_beta, n, want, nvec, s->d_theta, s->d_Z, s->mmax + 1, in_smem ? NULL : s->d_work, s->d_done,
+			s->d_pack, 0, s->guesses);
+	} else {
+		/* all eigenvalues of a T_n whose rows do not fit shared memory */
+		for (int i = 0; i < want; i += TRI_WAVE)
+			k_tri_check<<<want - i < TRI_WAVE ? want - i : TRI_WAVE, TRI_THREADS, 0, s->check>>>(
+				s->d_alpha, s->d_beta, n, want, nvec, s->d_theta, s->d_Z, s->mmax + 1, s->d_work, s->d_done,
+				s->d_pack, i, s->guesses);
 	}
-	CUDA_TRY(cudaMemcpyAsync(s->h_theta, s->d_theta, want * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-	CUDA_TRY(cudaStreamSynchronize(c->stream));
+	s->guesses = want;
 	CUDA_TRY(cudaGetLastError());
+	CUDA_TRY(cudaMemcpyAsync(s->h_pack[slot], s->d_pack, (size_t)(want + nvec + 1) * sizeof(double), cudaMemcpyDeviceToHost,
+				 s->check));
+	CUDA_TRY(cudaEventRecord(s->checked[slot], s->check));
+	return JN_OK;
+}
+
+/* the same, waited for, into h_pack[0] */
+static jn_status tri_eig(jn_ctx *c, int n, int want, int nvec)
+{
+	struct jn_lanczos_state *s = c->lz;
+	jn_status st = tri_enqueue(c, n, want, nvec, 0);
+	if (st) return st;
+	CUDA_TRY(cudaEventSynchronize(s->checked[0]));
+	/* each eigenvalue is found by itself: those of a cluster may cross by a rounding */
+	for (int i = 1; i < want; i++)
+		if (s->h_pack[0][i] < s->h_pack[0][i - 1]) s->h_pack[0][i] = s->h_pack[0][i - 1];
 	return JN_OK;
 }
 
@@ -310,6 +580,7 @@ extern "C" jn_status jn_lanczos(jn_ctx *c, const jn_lanczos_options *opt, jn_lan
 	struct jn_lanczos_state *s = c->lz;
 	s->nev = nev;
 	s->have_ritz = 0;
+	s->guesses = 0;
 	cudaStream_t q = c->stream;
 	const int g = grid_for(D);
 	double *V = s->d_V;
@@ -326,8 +597,13 @@ extern "C" jn_status jn_lanczos(jn_ctx *c, const jn_lanczos_options *opt, jn_lan
 		CUDA_TRY(cudaStreamSynchronize(q));
 	}
 
+	/* the step's vector work: one CTA an SM, at least 32 elements each */
+	int64_t chunk = (D + c->num_sms - 1) / c->num_sms;
+	chunk = (chunk < 32 ? 32 : chunk + 3) & ~3ll;
+	const int og = (int)((D + chunk - 1) / chunk);
+
 	double prev = 0.0;
-	int k, converged = 0;
+	int k, converged = 0, pending = 0;      /* pending: rows of the check that is still to be read */
 	/* the eigenvector criterion keeps the previous step's vector (and the current one after it) */
 	const int by_vector = reference_mode && opt->criterion == JN_CONVERGE_EIGENVECTORS;
 	std::vector<double> zbuf(by_vector ? 2 * (size_t)(m + 1) : 0, 0.0);
@@ -335,34 +611,55 @@ extern "C" jn_status jn_lanczos(jn_ctx *c, const jn_lanczos_options *opt, jn_lan
 	res->iterations = 0;
 	res->iteration_seconds = res->refinement_seconds = 0.0;
 	const double t_loop = seconds_now();
+	/* the convergence test of T_n from its check's results: 1 converged, 0 not, -1 on an error (in st) */
+	auto test_full = [&](int n) -> int {
+		const int slot = n & 1, wv = nev < n ? nev : n, wt = wv + (wv < n ? 1 : 0);
+		const cudaError_t e = cudaEventSynchronize(s->checked[slot]);
+		if (e != cudaSuccess) {
+			st = jn_fail(JN_ERR_CUDA, "convergence check: %s", cudaGetErrorString(e));
+			return -1;
+		}
+		const double *theta = s->h_pack[slot], *zlast = theta + wt, beta = zlast[wv];
+		int ok = n >= nev;
+		for (int i = 0; i < wv && ok; i++) {
+			double r = fabs(beta * zlast[i]);
+			double gap = 1e300;
+			if (i > 0) gap = fmin(gap, theta[i] - theta[i - 1]);
+			if (i + 1 < wt) gap = fmin(gap, theta[i + 1] - theta[i]);
+			double bound = fmin(r, r * r / fmax(gap, 1e-300));
+			if (!(bound < opt->tolerance)) ok = 0;
+		}
+		if (opt->verbose)
+			printf("Lanczos iteration %d: lowest Ritz value %.17lg, beta %lg\n", n, theta[0], beta);
+		return ok || beta == 0.0;
+	};
 	for (k = 0; k < m; k++) {
 		double *vk = V + (int64_t)k * D, *vk1 = V + (int64_t)(k + 1) * D;
 		st = jn_launch_matvec(c, vk, s->d_w, 0, q);
 		if (st) return st;
-		dot_dev(c, vk, s->d_w, s->d_alpha + k);
-		k_three_term<<<g, 256, 0, q>>>(s->d_w, vk, k ? V + (int64_t)(k - 1) * D : NULL, s->d_alpha + k,
-					       k ? s->d_beta + k - 1 : NULL, D);
 		if (!reference_mode) {
-			cgs_pass(c, k + 1);
-			cgs_pass(c, k + 1);
-		}
-		dot_dev(c, s->d_w, s->d_w, s->d_scalar);
-		k_normalize<<<g, 256, 0, q>>>(vk1, s->d_w, s->d_scalar, s->d_beta + k, D);
-		if (reference_mode && k > 2) {
+			int64_t Dl = D;
+			void *args[] = { &V, &Dl, &chunk, &k, &s->d_w, &s->d_part, &s->d_h, &s->d_alpha, &s->d_beta };
+			CUDA_TRY(cudaLaunchCooperativeKernel((const void *)k_orthonormalize, dim3(og), dim3(ORTHO_WARPS * 32), args, 0, q));
+		} else {
+			dot_dev(c, vk, s->d_w, s->d_alpha + k);
+			k_three_term<<<g, 256, 0, q>>>(s->d_w, vk, k ? V + (int64_t)(k - 1) * D : NULL, s->d_alpha + k,
+						       k ? s->d_beta + k - 1 : NULL, D);
+			dot_dev(c, s->d_w, s->d_w, s->d_scalar);
+			k_normalize<<<g, 256, 0, q>>>(vk1, s->d_w, s->d_scalar, s->d_beta + k, D);
 			/* MGS of v_{k+1} against v_0..v_{k-3}, no renormalisation (vector.c:461-476) */
 			for (int j = 0; j + 2 < k; j++) {
 				dot_dev(c, vk1, V + (int64_t)j * D, s->d_scalar + 1);
 				k_axpy_neg<<<g, 256, 0, q>>>(vk1, V + (int64_t)j * D, s->d_scalar + 1, D);
 			}
+			CUDA_TRY(cudaGetLastError());
 		}
-		CUDA_TRY(cudaGetLastError());
-		const int n = k + 1;
-		if ((n % check_every) && n < m) continue;
-		CUDA_TRY(cudaMemcpyAsync(s->h_alpha, s->d_alpha, n * sizeof(double), cudaMemcpyDeviceToHost, q));
-		CUDA_TRY(cudaMemcpyAsync(s->h_beta, s->d_beta, n * sizeof(double), cudaMemcpyDeviceToHost, q));
+		const int n = k + 1, check = !(n % check_every) || n == m;
 		if (reference_mode) {
+			if (!check) continue;
 			st = tri_eig(c, n, 1, by_vector);
 			if (st) return st;
+			const double theta0 = s->h_pack[0][0];
 			double diff;
 			if (by_vector) {
 				/* the lowest eigenvector of T_n against the previous step's (lanczos.c:210-215, 276-287) */
@@ -375,82 +672,71 @@ extern "C" jn_status jn_lanczos(jn_ctx *c, const jn_lanczos_options *opt, jn_lan
 				diff = sqrt(d2);
 				memcpy(zprev, z, n * sizeof(double));
 			} else {
-				diff = fabs(s->h_theta[0] - prev);
+				diff = fabs(theta0 - prev);
 			}
-			prev = s->h_theta[0];
+			prev = theta0;
 			if (opt->verbose)
-				printf("Lanczos iteration %d: lowest Ritz value %.17lg, difference %lg\n", n, s->h_theta[0], diff);
+				printf("Lanczos iteration %d: lowest Ritz value %.17lg, difference %lg\n", n, theta0, diff);
 			if (diff < opt->tolerance) { converged = 1; k++; break; }
-		} else {
-			int want = nev < n ? nev : n;
-			st = tri_eig(c, n, want + (want < n ? 1 : 0), 1);
-			if (st) return st;
-			int ok = n >= nev;
-			double beta = s->h_beta[n - 1];
-			for (int i = 0; i < want && ok; i++) {
-				double r = fabs(beta * s->h_zlast[i]);
-				double gap = 1e300;
-				if (i > 0) gap = fmin(gap, s->h_theta[i] - s->h_theta[i - 1]);
-				if (i + 1 < want + (want < n ? 1 : 0)) gap = fmin(gap, s->h_theta[i + 1] - s->h_theta[i]);
-				double bound = fmin(r, r * r / fmax(gap, 1e-300));
-				if (!(bound < opt->tolerance)) ok = 0;
-			}
-			if (opt->verbose)
-				printf("Lanczos iteration %d: lowest Ritz value %.17lg, beta %lg\n", n, s->h_theta[0], beta);
-			if (ok || beta == 0.0) { converged = 1; k++; break; }
+			continue;
 		}
+		/* full mode: this step's check is enqueued, then the one before it is
+		   read, so the device always holds work; a solve that has converged
+		   has one step too many in flight, which nothing reads */
+		if (check) {
+			const int wv = nev < n ? nev : n;
+			st = tri_enqueue(c, n, wv + (wv < n ? 1 : 0), wv, n & 1);
+			if (st) return st;
+		}
+		if (pending) {
+			const int t = test_full(pending);
+			if (t < 0) return st;
+			if (t) { converged = 1; k = pending; pending = 0; break; }
+		}
+		pending = check ? n : 0;
+	}
+	if (pending) {
+		const int t = test_full(pending);
+		if (t < 0) return st;
+		converged = t;
+		k = pending;
 	}
 	s->k = k;
 	res->iterations = k;
 	res->converged = converged;
-	const double t_final = seconds_now();      /* the loop ends on a convergence check, which synchronises */
+	const double t_final = seconds_now();      /* the loop ends on a convergence check, which is waited for */
 	res->iteration_seconds = t_final - t_loop;
-	/* final decomposition of T_k: all Ritz values, vectors of the lowest nev */
-	CUDA_TRY(cudaMemcpyAsync(s->h_alpha, s->d_alpha, k * sizeof(double), cudaMemcpyDeviceToHost, q));
-	CUDA_TRY(cudaMemcpyAsync(s->h_beta, s->d_beta, k * sizeof(double), cudaMemcpyDeviceToHost, q));
+	/* final decomposition of T_k: the Ritz values and vectors of the lowest nev */
 	int want = nev < k ? nev : k;
-	st = tri_eig(c, k, k, 0);
-	if (st) return st;
 	res->num_ritz_values = k;
-	st = tri_eig(c, k, want, 1);
+	st = tri_eig(c, k, want, want);
 	if (st) return st;
 	/* Ritz vectors x_i = sum_j z_i[j] v_j and their FP64 refinement */
-	int ldz = s->mmax + 1;
-	for (int i = 0; i < want; i++)
-		k_gemv_n<<<g, 256, 0, q>>>(V, D, k, s->d_Z + (size_t)i * ldz, s->d_ritz + (size_t)i * D);
+	k_ritz_vectors<<<dim3((unsigned int)((D + 127) / 128), (want + RITZ_ROWS - 1) / RITZ_ROWS), 128, 0, q>>>(
+		V, D, k, s->d_Z, s->mmax + 1, want, s->d_ritz);
 	s->have_ritz = 1;
 	/* the refinement's products are FP64-grade whatever the iteration's precision */
 	const int prec0 = c->precision, engine0 = c->engine;
 	c->precision = 64;
 	c->engine = c->engine_of[0];
-	for (int i = 0; i < want; i++) {
-		double *xi = s->d_ritz + (size_t)i * D;
-		st = jn_launch_matvec(c, xi, s->d_w, 0, q);
-		if (st) { c->precision = prec0; c->engine = engine0; return st; }
-		dot_dev(c, xi, s->d_w, s->d_scalar + 0);
-		dot_dev(c, xi, xi, s->d_scalar + 1);
-		double h2[2];
-		CUDA_TRY(cudaMemcpyAsync(h2, s->d_scalar, 2 * sizeof(double), cudaMemcpyDeviceToHost, q));
-		CUDA_TRY(cudaStreamSynchronize(q));
-		double rq = h2[0] / h2[1];
-		s->h_rq[i] = rq;
-		/* r = H x - rq x */
-		CUDA_TRY(cudaMemcpyAsync(s->d_scalar + 2, &rq, sizeof(double), cudaMemcpyHostToDevice, q));
-		k_axpy_neg<<<g, 256, 0, q>>>(s->d_w, xi, s->d_scalar + 2, D);
-		dot_dev(c, s->d_w, s->d_w, s->d_scalar + 3);
-		double r2;
-		CUDA_TRY(cudaMemcpyAsync(&r2, s->d_scalar + 3, sizeof(double), cudaMemcpyDeviceToHost, q));
-		CUDA_TRY(cudaStreamSynchronize(q));
-		s->h_res[i] = sqrt(r2 / h2[1]);
-	}
+	for (int i = 0; i < want && !st; i++)
+		st = jn_launch_matvec(c, s->d_ritz + (size_t)i * D, s->d_hritz + (size_t)i * D, 0, q);
 	c->precision = prec0;
 	c->engine = engine0;
+	if (st) return st;
+	k_rayleigh<<<want, 512, 0, q>>>(s->d_ritz, s->d_hritz, D, want, s->d_rr);
 	CUDA_TRY(cudaGetLastError());
+	CUDA_TRY(cudaMemcpyAsync(s->h_pack[1], s->d_rr, 2 * (size_t)want * sizeof(double), cudaMemcpyDeviceToHost, q));
+	CUDA_TRY(cudaStreamSynchronize(q));
+	for (int i = 0; i < want; i++) {
+		s->h_rq[i] = s->h_pack[1][i];
+		s->h_res[i] = s->h_pack[1][want + i];
+	}
 	res->refinement_seconds = seconds_now() - t_final;
 	res->num_eigenvalues = want;
 	for (int i = 0; i < want && i < JN_MAX_REPORTED; i++) {
 		res->eigenvalues[i] = s->h_rq[i];
-		res->ritz_values[i] = s->h_theta[i];
+		res->ritz_values[i] = s->h_pack[0][i];
 		res->residual_norms[i] = s->h_res[i];
 	}
 	return converged ? JN_OK : (opt->mode == JN_LANCZOS_REFERENCE ? JN_OK : jn_fail(JN_ERR_NOT_CONVERGED,
@@ -461,10 +747,11 @@ extern "C" jn_status jn_lanczos_ritz_values(jn_ctx *c, double *out, int capacity
 {
 	if (!c || !c->lz || !out) return jn_fail(JN_ERR_INVALID, "no Lanczos solve on this context");
 	struct jn_lanczos_state *s = c->lz;
+	s->guesses = 0;         /* the same bits on every call */
 	jn_status st = tri_eig(c, s->k, s->k, 0);
 	if (st) return st;
 	int n = s->k < capacity ? s->k : capacity;
-	memcpy(out, s->h_theta, n * sizeof(double));
+	memcpy(out, s->h_pack[0], n * sizeof(double));
 	if (count) *count = s->k;
 	return JN_OK;
 }

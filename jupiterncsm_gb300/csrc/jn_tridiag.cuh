@@ -4,114 +4,272 @@
  * shared by the single solve (jn_lanczos.cu) and the batched solve
  * (jn_batch.cu).  They replace LAPACK dsteqr in the reference
  * (src/Bacchus/diagonalization/diagonalization.c:16-68).
+ *
+ * What bounds them: GB300's FP64 pipe, one warp instruction in 64 cycles on
+ * an SM sub-partition however few lanes take part (measured; dependent and
+ * independent multiply-adds alike), and one division is about ten of them
+ * (641 cycles measured for a - b/x).  So the serial chains hold no division:
+ * Sturm counts come from the leading principal minors
+ *     p_i = (a_i - x) p_{i-1} - b_{i-1}^2 p_{i-2}
+ * (three FP64 instructions a step; the exponents are kept in range by integer
+ * work every eighth step), and an eigenvector from the leading and trailing
+ * minors at the eigenvalue, joined where their product is largest (the
+ * twisted factorisation, in minors instead of quotients).  The quotient form
+ * of the counts and inverse iteration by an LU factorisation with divisions
+ * in its chain took 380 and 230 us for 11 pairs at n = 45 (SM clock 2.07
+ * GHz).
  */
 #ifndef JN_TRIDIAG_CUH
 #define JN_TRIDIAG_CUH
 
 #include <stdint.h>
 
-/* number of eigenvalues below x (Sturm sequence) */
-__device__ __forceinline__ int jn_sturm_count(const double *a, const double *b, int n, double x)
+/* doubles of scratch one warp needs for n rows: the staged matrix, and with
+ * it the work space of one vector */
+#define JN_TRI_VALUE_DOUBLES(n) (2 * (size_t)(n))
+#define JN_TRI_VECTOR_DOUBLES(n) (8 * (size_t)(n) + 8)
+/* rows up to which that scratch is taken in shared memory (204 KB) */
+#define JN_TRI_SMEM_ROWS 3192
+#define JN_TRI_SMEM(n) (JN_TRI_VECTOR_DOUBLES(n) * sizeof(double))
+
+/* bits of the unbiased exponent field; 0 for zero and subnormals */
+__device__ __forceinline__ int jn_expo(double v) { return (__double2hiint(v) >> 20) & 0x7ff; }
+
+/* v 2^-k by the exponent field, flushed to zero below the normal range */
+__device__ __forceinline__ double jn_shift_expo(double v, int k)
 {
-	int c = 0;
-	double q = a[0] - x;
-	if (q < 0) c++;
-	for (int i = 1; i < n; i++) {
-		double qq = q == 0.0 ? 1e-300 : q;
-		q = a[i] - x - b[i - 1] * b[i - 1] / qq;
-		if (q < 0) c++;
+	const int e = jn_expo(v);
+	if (e == 0 || e - k <= 0) return 0.0;
+	return __hiloint2double(__double2hiint(v) - k * 0x100000, __double2loint(v));
+}
+
+/* bring the larger of p1, p2 to exponent 0 (values in [1, 2)); returns the shift */
+__device__ __forceinline__ int jn_rescale(double &p1, double &p2)
+{
+	const int k = max(jn_expo(p1), jn_expo(p2)) - 1023;
+	if (k == -1023) return 0;
+	p1 = jn_shift_expo(p1, k);
+	p2 = jn_shift_expo(p2, k);
+	return k;
+}
+
+/* the power of two 2^k with |T| 2^k <= 1 (Gershgorin), found by one warp */
+__device__ __forceinline__ double jn_tri_scale(const double *a, const double *b, int n, double *lo, double *hi)
+{
+	const int lane = threadIdx.x & 31;
+	double l = 1e300, h = -1e300;
+	for (int j = lane; j < n; j += 32) {
+		const double r = (j > 0 ? fabs(b[j - 1]) : 0.0) + (j < n - 1 ? fabs(b[j]) : 0.0);
+		l = fmin(l, a[j] - r);
+		h = fmax(h, a[j] + r);
 	}
+	for (int o = 16; o; o >>= 1) {
+		l = fmin(l, __shfl_xor_sync(0xffffffffu, l, o));
+		h = fmax(h, __shfl_xor_sync(0xffffffffu, h, o));
+	}
+	const double span = fmax(fabs(l), fabs(h));
+	const int e = jn_expo(span);
+	const double sc = e > 1 && e < 2045 ? __hiloint2double((2045 - e) << 20, 0) : 1.0;       /* span sc in [1/2, 1) */
+	*lo = l * sc - 1e-12;
+	*hi = h * sc + 1e-12;
+	return sc;
+}
+
+/* one warp: a sc into as, (b sc)^2 into b2; couplings below 2^-53 of the
+ * span are raised to it (a change below the rounding of a), so that the
+ * minors cannot stay at zero */
+__device__ __forceinline__ void jn_tri_stage(const double *a, const double *b, int n, double sc, double *as, double *b2)
+{
+	for (int j = threadIdx.x & 31; j < n; j += 32) {
+		as[j] = a[j] * sc;
+		const double v = j < n - 1 ? fmax(fabs(b[j]) * sc, 0x1p-53) : 0.0;
+		b2[j] = v * v;
+	}
+	__syncwarp();
+}
+
+/* number of eigenvalues below x: sign changes of the leading minors; pm 2^pe
+ * is the last one (det(T - x)) */
+__device__ __forceinline__ int jn_sturm_count(const double *as, const double *b2, int n, double x, double *pm, int *pe)
+{
+	double p2 = 1.0, p1 = as[0] - x;
+	int e = 0, c = 0, s = 0;
+	/* a zero minor takes its predecessor's sign */
+	if (((__double2hiint(p1) << 1) | __double2loint(p1)) != 0) s = __double2hiint(p1) >> 31;
+	c -= s;
+	for (int i = 1; i < n;) {
+		const int stop = min(n, i + 8);
+		for (; i < stop; i++) {
+			const double p = fma(as[i] - x, p1, -(b2[i - 1] * p2));
+			const int sp = ((__double2hiint(p) << 1) | __double2loint(p)) != 0 ? __double2hiint(p) >> 31 : s;
+			c += (sp ^ s) & 1;
+			s = sp;
+			p2 = p1;
+			p1 = p;
+		}
+		e += jn_rescale(p1, p2);
+	}
+	*pm = p1;
+	*pe = e;
 	return c;
 }
 
-/* the i-th smallest eigenvalue by multisection, one warp per eigenvalue:
- * each round the 32 lanes evaluate the Sturm count at 32 points of the
- * bracket, which shrinks 32-fold, so about 11 rounds reach full precision
- * where bisection needs about 52 sequential steps.  Every lane returns the
- * same value. */
-__device__ __forceinline__ double jn_tri_multisect_warp(const double *a, const double *b, int n, int i)
+/* The i-th smallest eigenvalue of the staged matrix (in its units) by
+ * multisection, one warp: each round the 32 lanes count at 32 points of the
+ * bracket [lo, hi].  Points are equidistant until the bracket holds this
+ * eigenvalue alone and det(T - x) is known at both its ends; then they lie
+ * at geometric distances around the secant estimate, whose error shrinks
+ * quadratically: 6 to 8 rounds in all, where equidistant points take 11.
+ * A guess (the same eigenvalue of an earlier, smaller T of the solve) takes
+ * the estimate's place in the first round.  The counts alone decide the
+ * bracket, so a poor estimate costs a round and nothing else.  It ends at
+ * 2^-54 of the span.  Every lane returns the same value. */
+__device__ __forceinline__ double jn_tri_multisect_warp(const double *as, const double *b2, int n, int i, double lo, double hi,
+							 bool guessed, double guess)
 {
 	const int lane = threadIdx.x & 31;
-	double lo = 1e300, hi = -1e300;
-	for (int j = lane; j < n; j += 32) {
-		double r = (j > 0 ? fabs(b[j - 1]) : 0.0) + (j < n - 1 ? fabs(b[j]) : 0.0);
-		lo = fmin(lo, a[j] - r);
-		hi = fmax(hi, a[j] + r);
-	}
-	for (int o = 16; o; o >>= 1) {
-		lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));
-		hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
-	}
-	const double span = fmax(fabs(lo), fabs(hi));
-	lo -= 1e-12 * span + 1e-300;
-	hi += 1e-12 * span + 1e-300;
-	for (int round = 0; round < 64; round++) {
-		const double w = (hi - lo) * (1.0 / 32.0);
-		const double x = lane == 31 ? hi : lo + (double)(lane + 1) * w;
-		const unsigned int above = __ballot_sync(0xffffffffu, jn_sturm_count(a, b, n, x) > i);
-		const int f = above ? __ffs(above) - 1 : 31;
-		const double nlo = f == 0 ? lo : __shfl_sync(0xffffffffu, x, f - 1);
-		const double nhi = __shfl_sync(0xffffffffu, x, f);
-		if (!(nlo > lo || nhi < hi)) break;     /* the bracket no longer shrinks: converged */
-		lo = nlo;
-		hi = nhi;
+	int cl = 0, ch = n, el = 0, eh = 0, known = 0;          /* known: 1 det at lo, 2 det at hi */
+	double pl = 0.0, ph = 0.0;
+	int geo_ok = 1;
+	for (int round = 0; round < 96 && hi - lo > 0x1p-54; round++) {
+		const double w = hi - lo;
+		const int first = guessed && round == 0;
+		const int geo = first || (geo_ok && known == 3 && cl == i && ch == i + 1 && pl != 0.0);
+		double x;
+		if (geo) {
+			double c = guess;
+			if (!first) {
+				const int de = min(max(eh - el, -900), 900);
+				const double q = fabs(ph / pl) * __hiloint2double((1023 + de) << 20, 0);
+				c = lo + w / (1.0 + q);
+			}
+			const int k = lane < 16 ? lane : 31 - lane;
+			double d = w * __hiloint2double((1023 - 1 - k - (k >> 1)) << 20, 0);
+			if (k & 1) d *= 0.70710678118654752;
+			x = fmin(fmax(lane < 16 ? c - d : c + d, lo), hi);
+		} else {
+			x = lane == 31 ? hi : lo + (double)(lane + 1) * (w * (1.0 / 32.0));
+		}
+		double p;
+		int e;
+		const int cnt = jn_sturm_count(as, b2, n, x, &p, &e);
+		const unsigned int above = __ballot_sync(0xffffffffu, cnt > i);
+		const int f = above ? __ffs(above) - 1 : 32, fl = f > 0 ? f - 1 : 0, fh = f < 32 ? f : 31;
+		const double nlo = __shfl_sync(0xffffffffu, x, fl), nhi = __shfl_sync(0xffffffffu, x, fh);
+		const double npl = __shfl_sync(0xffffffffu, p, fl), nph = __shfl_sync(0xffffffffu, p, fh);
+		const int nel = __shfl_sync(0xffffffffu, e, fl), neh = __shfl_sync(0xffffffffu, e, fh);
+		const int ncl = __shfl_sync(0xffffffffu, cnt, fl), nch = __shfl_sync(0xffffffffu, cnt, fh);
+		const double lo0 = lo, hi0 = hi;
+		if (f > 0) { lo = nlo; pl = npl; el = nel; cl = ncl; known |= 1; }
+		if (f < 32) { hi = nhi; ph = nph; eh = neh; ch = nch; known |= 2; }
+		if (!(lo > lo0 || hi < hi0) && !geo) break;     /* the bracket no longer shrinks: converged */
+		geo_ok = !geo || hi - lo < 0.125 * w;
 	}
 	return 0.5 * (lo + hi);
 }
 
-/* eigenvector z[0..n) for the eigenvalue sh by inverse iteration with the
- * LU factorisation (partial pivoting) of T - sh I, as dgttrf/dgtts2 do;
- * normalised, z[0] >= 0 as diagonalization.c:55-58 makes it.
- * work: 5 n doubles. */
-__device__ __forceinline__ void jn_tri_vector_one(const double *a, const double *b, int n, double sh, double *z,
-						  double *work)
+/* The unit eigenvector z[0..n) of the staged matrix for its eigenvalue x,
+ * by one warp, z[0] >= 0 as diagonalization.c:55-58 makes it.  Lanes 0, 1
+ * and 2 run the chains of the leading minors p_t, the trailing minors q_t
+ * and the products c_t of the couplings, one shared instruction stream;
+ * then, with r where |p_r q_{n-1-r}| (the r-th diagonal element of the
+ * adjugate of T - x, so |z_r|^2 up to a factor) is largest,
+ *     z_i / z_r = (-1)^(r-i) (p_i / c_i) / (p_r / c_r)               i <= r
+ *     z_i / z_r = (-1)^(r-i) (q_{n-1-i} c_i) / (q_{n-1-r} c_r)       i >= r.
+ * buf: 5 n doubles and 3 (n/8 + 1) ints: n for d, n for the couplings' roots
+ * and the three chains; as and b2 are read. */
+__device__ __forceinline__ double jn_split(double v, int *e)
 {
-	double *d = work, *u1 = d + n, *u2 = u1 + n, *l = u2 + n, *pv = l + n;
-	double span = 0.0;
-	for (int j = 0; j < n; j++) span = fmax(span, fabs(a[j]) + (j < n - 1 ? fabs(b[j]) : 0.0));
-	const double eps = 2.2e-16 * fmax(span, 1e-300);
-	double dd = a[0] - sh, e = n > 1 ? b[0] : 0.0;
-	for (int j = 0; j < n - 1; j++) {
-		double sub = b[j];
-		double nd = a[j + 1] - sh, ne = (j + 1 < n - 1) ? b[j + 1] : 0.0;
-		if (fabs(dd) >= fabs(sub)) {
-			pv[j] = 0.0;
-			if (dd == 0.0) dd = eps;
-			double m = sub / dd;
-			l[j] = m;
-			d[j] = dd; u1[j] = e; u2[j] = 0.0;
-			dd = nd - m * e;
-			e = ne;
+	const int k = jn_expo(v);
+	if (k == 0) { *e = -100000; return 0.0; }
+	*e = k - 1023;
+	return __hiloint2double((__double2hiint(v) & 0x800fffff) | 0x3ff00000, __double2loint(v));
+}
+
+__device__ __forceinline__ double jn_scale2(double v, int e)
+{
+	if (e < -1000) return 0.0;
+	return v * __hiloint2double((1023 + min(e, 1000)) << 20, 0);
+}
+
+__device__ __forceinline__ void jn_tri_vector_warp(const double *as, const double *b2, int n, double x, double *z, double *buf)
+{
+	const int lane = threadIdx.x & 31, ne = n / 8 + 1;
+	double *d = buf, *bs = d + n, *ch = bs + n;
+	int *ex = (int *)(ch + 3 * (size_t)n);
+	for (int j = lane; j < n; j += 32) {
+		d[j] = as[j] - x;
+		bs[j] = sqrt(b2[j]);
+	}
+	__syncwarp();
+	if (lane < 3) {
+		double *v = ch + (size_t)lane * n;
+		int *ev = ex + lane * ne;
+		double p2 = 0.0, p1 = 1.0;
+		int e = 0;
+		v[0] = 1.0;
+		ev[0] = 0;
+		for (int t = 1; t < n; t++) {
+			if ((t & 7) == 0) {
+				e += jn_rescale(p1, p2);
+				ev[t >> 3] = e;
+			}
+			const double A = lane == 0 ? d[t - 1] : lane == 1 ? d[n - t] : bs[t - 1];
+			const double B = lane == 2 || t < 2 ? 0.0 : lane == 0 ? b2[t - 2] : b2[n - t];
+			const double p = fma(A, p1, -(B * p2));
+			v[t] = p;
+			p2 = p1;
+			p1 = p;
+		}
+	}
+	__syncwarp();
+	const double *P = ch, *Q = ch + n, *C = ch + 2 * (size_t)n;
+	const int *EP = ex, *EQ = ex + ne, *EC = ex + 2 * ne;
+	/* r: the largest |p_r q_{n-1-r}| (lowest index on ties) */
+	float best = -3e38f;
+	int r = 0;
+	for (int i = lane; i < n; i += 32) {
+		int e1, e2;
+		const double m1 = jn_split(P[i], &e1), m2 = jn_split(Q[n - 1 - i], &e2);
+		const float key = (float)(e1 + e2 + EP[i >> 3] + EQ[(n - 1 - i) >> 3]) +
+				  __log2f(fmaxf((float)fabs(m1) * (float)fabs(m2), 1e-30f));
+		if (key > best) { best = key; r = i; }
+	}
+	for (int o = 16; o; o >>= 1) {
+		const float kb = __shfl_xor_sync(0xffffffffu, best, o);
+		const int rb = __shfl_xor_sync(0xffffffffu, r, o);
+		if (kb > best || (kb == best && rb < r)) { best = kb; r = rb; }
+	}
+	int epr, eqr, ecr;
+	const double pr = jn_split(P[r], &epr), qr = jn_split(Q[n - 1 - r], &eqr), cr = jn_split(C[r], &ecr);
+	epr += EP[r >> 3];
+	eqr += EQ[(n - 1 - r) >> 3];
+	ecr += EC[r >> 3];
+	const double fp = cr / pr, fq = 1.0 / (qr * cr);
+	double s = 0.0;
+	for (int i = lane; i < n; i += 32) {
+		int em, ec;
+		const double c = jn_split(C[i], &ec);
+		ec += EC[i >> 3];
+		double v;
+		if (i <= r) {
+			v = jn_split(P[i], &em) * fp / c;
+			v = jn_scale2(v, em + EP[i >> 3] - ec + ecr - epr);
 		} else {
-			pv[j] = 1.0;
-			double m = dd / sub;
-			l[j] = m;
-			d[j] = sub; u1[j] = nd; u2[j] = ne;
-			dd = e - m * nd;
-			e = -m * ne;
+			v = jn_split(Q[n - 1 - i], &em) * fq * c;
+			v = jn_scale2(v, em + EQ[(n - 1 - i) >> 3] + ec - eqr - ecr);
 		}
+		if ((i ^ r) & 1) v = -v;
+		z[i] = v;
+		s = fma(v, v, s);
 	}
-	if (dd == 0.0) dd = eps;
-	d[n - 1] = dd; u1[n - 1] = 0.0; u2[n - 1] = 0.0;
-	for (int j = 0; j < n; j++) z[j] = 1.0;
-	for (int iter = 0; iter < 3; iter++) {
-		for (int j = 0; j < n - 1; j++) {
-			if (pv[j] != 0.0) { double t = z[j]; z[j] = z[j + 1]; z[j + 1] = t - l[j] * z[j]; }
-			else z[j + 1] -= l[j] * z[j];
-		}
-		for (int j = n - 1; j >= 0; j--) {
-			double s = z[j];
-			if (j + 1 < n) s -= u1[j] * z[j + 1];
-			if (j + 2 < n) s -= u2[j] * z[j + 2];
-			z[j] = s / (fabs(d[j]) < eps ? (d[j] < 0 ? -eps : eps) : d[j]);
-		}
-		double nrm = 0.0;
-		for (int j = 0; j < n; j++) nrm = fma(z[j], z[j], nrm);
-		nrm = sqrt(nrm);
-		for (int j = 0; j < n; j++) z[j] /= nrm;
-	}
-	if (z[0] < 0)
-		for (int j = 0; j < n; j++) z[j] = -z[j];
+	for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+	__syncwarp();
+	double inv = 1.0 / sqrt(s);
+	if (z[0] < 0.0) inv = -inv;
+	__syncwarp();
+	for (int i = lane; i < n; i += 32) z[i] *= inv;
+	__syncwarp();
 }
 
 /* fixed-order sum over the CTA (blockDim.x a power of two, sh of blockDim.x) */
@@ -130,30 +288,31 @@ __device__ __forceinline__ double jn_block_sum(double v, double *sh)
 }
 
 /* modified Gram-Schmidt among `want` vectors of length n (rows of Z), by one
- * CTA: repairs inverse-iteration vectors of close eigenvalues */
-__device__ __forceinline__ void jn_tri_mgs(double *Z, int ldz, int n, int want, double *sh)
+ * CTA: repairs the vectors of close eigenvalues.  Each finished vector is
+ * taken out of all later ones at once, a warp per vector, which are the
+ * operations of the vector-by-vector order with one CTA barrier a vector. */
+__device__ __forceinline__ void jn_tri_mgs(double *Z, int ldz, int n, int want)
 {
+	const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
 	for (int i = 0; i < want; i++) {
 		double *zi = Z + (int64_t)i * ldz;
-		for (int j = 0; j < i; j++) {
-			const double *zj = Z + (int64_t)j * ldz;
+		if (warp == 0) {
 			double s = 0.0;
-			for (int t = threadIdx.x; t < n; t += blockDim.x) s = fma(zi[t], zj[t], s);
-			s = jn_block_sum(s, sh);
-			for (int t = threadIdx.x; t < n; t += blockDim.x) zi[t] -= s * zj[t];
-			__syncthreads();
+			for (int t = lane; t < n; t += 32) s = fma(zi[t], zi[t], s);
+			for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+			double inv = 1.0 / sqrt(s);
+			if (zi[0] < 0.0) inv = -inv;
+			__syncwarp();
+			for (int t = lane; t < n; t += 32) zi[t] *= inv;
 		}
-		double s = 0.0;
-		for (int t = threadIdx.x; t < n; t += blockDim.x) s = fma(zi[t], zi[t], s);
-		s = jn_block_sum(s, sh);
-		double inv = 1.0 / sqrt(s);
-		for (int t = threadIdx.x; t < n; t += blockDim.x) zi[t] *= inv;
 		__syncthreads();
-		if (threadIdx.x == 0) sh[0] = zi[0] < 0 ? -1.0 : 1.0;
-		__syncthreads();
-		double sg = sh[0];
-		__syncthreads();
-		for (int t = threadIdx.x; t < n; t += blockDim.x) zi[t] *= sg;
+		for (int j = i + 1 + warp; j < want; j += nwarps) {
+			double *zj = Z + (int64_t)j * ldz;
+			double s = 0.0;
+			for (int t = lane; t < n; t += 32) s = fma(zj[t], zi[t], s);
+			for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+			for (int t = lane; t < n; t += 32) zj[t] -= s * zi[t];
+		}
 		__syncthreads();
 	}
 }
