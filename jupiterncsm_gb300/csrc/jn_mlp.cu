@@ -17,16 +17,24 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include <vector>
+
+#include <cooperative_groups.h>
+
 #include "jn_internal.h"
 #include "jn_tridiag.cuh"
 
 struct jn_mlp {
 	int nin, nh, nout;
+	int num_sms;
 	int64_t np;                     /* parameters */
-	float *d_p, *d_g, *d_m, *d_v;   /* parameters, gradient, Adam moments */
+	float *d_p, *d_g, *d_m, *d_v;   /* parameters (the allocation), gradient, Adam moments */
 	int64_t t;                      /* Adam steps taken */
 	int cap;                        /* samples the activation buffers hold */
+	/* activations, one allocation (d_x): sample by sample, or unit by unit on the fused path */
 	float *d_x, *d_t, *d_a1, *d_h1, *d_a2, *d_h2, *d_y, *d_d1, *d_d2, *d_d3, *d_loss;
+	float *d_corr;                  /* the fused path's bias corrections, then its word for a wait that gave up */
+	float *d_image;                 /* and its image of the weights */
 	cudaStream_t stream;
 };
 
@@ -147,46 +155,489 @@ __global__ void mlp_gradients(int nin, int nh, int nout, int n, const float *__r
 	G[p] = g;
 }
 
-__global__ void mlp_loss_sum(const float *__restrict__ lossp, int n, float *__restrict__ out)
+/* out[n] = the samples' losses summed in order (staged, then one thread adds) */
+__global__ void __launch_bounds__(256) mlp_loss_sum(const float *__restrict__ lossp, int n, float *__restrict__ out)
 {
-	if (threadIdx.x || blockIdx.x) return;
+	__shared__ float buf[1024];
 	float l = 0.0f;
-	for (int s = 0; s < n; s++) l += lossp[s];
-	out[n] = l;
+	for (int s0 = 0; s0 < n; s0 += 1024) {
+		const int ns = min(1024, n - s0);
+		__syncthreads();
+		for (int s = threadIdx.x; s < ns; s += blockDim.x) buf[s] = lossp[s0 + s];
+		__syncthreads();
+		if (threadIdx.x == 0)
+			for (int s = 0; s < ns; s++) l += buf[s];
+	}
+	if (threadIdx.x == 0) out[n] = l;
+}
+
+__device__ __forceinline__ void mlp_adam_one(float &p, float &m, float &v, float g, float lr, float b1, float b2, float eps,
+					     float c1, float c2)
+{
+	/* the contractions are spelt out: both paths round alike */
+	m = fmaf(1.0f - b1, g, b1 * m);
+	v = fmaf((1.0f - b2) * g, g, b2 * v);
+	p -= lr * (m / c1) / (sqrtf(v / c2) + eps);
 }
 
 __global__ void mlp_adam(float *__restrict__ P, const float *__restrict__ G, float *__restrict__ M, float *__restrict__ V,
 			 int64_t np, float lr, float b1, float b2, float eps, float c1, float c2)
 {
 	const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-	if (p >= np) return;
-	const float g = G[p];
-	const float m = M[p] = b1 * M[p] + (1.0f - b1) * g;
-	const float v = V[p] = b2 * V[p] + (1.0f - b2) * g * g;
-	P[p] -= lr * (m / c1) / (sqrtf(v / c2) + eps);
+	if (p < np) mlp_adam_one(P[p], M[p], V[p], G[p], lr, b1, b2, eps, c1, c2);
 }
 
-/* ------------------------------------------------------------------ */
 static int threads_for(const jn_mlp *m)
 {
 	int t = m->nh > m->nout ? m->nh : m->nout;
 	return (t + 31) / 32 * 32;
 }
 
+#define FUSED_SMEM_LIMIT (220 * 1024)
+/* ------------------------------------------------------------------ */
+/* fused path: whole training runs in one launch                        */
+/* ------------------------------------------------------------------ */
+/* Networks whose weights fit an SM's shared memory (hidden widths up to
+ * about 200) run here: one cooperative launch, one CTA an SM, for up to
+ * FUSED_STEPS Adam steps.  Per step, phase A: every CTA loads the weights
+ * (L2 to shared memory, 16-byte asynchronous copies) and takes SP samples
+ * through the forward pass and the deltas, a thread per unit; phase B: every
+ * CTA takes 16 x 16 tiles of (weight matrix | bias), sums their gradient
+ * over the samples and updates its parameters.  Two grid-wide barriers a step.
+ * Every sum runs in the order of the kernel-per-pass path above (bias, then
+ * inputs ascending; samples ascending), so the results are the same bits.
+ * What bounds it: shared-memory reads (a wavefront for every 128 bytes that
+ * a warp's lanes take in, equal or not) and the two barriers (1.1 us each).
+ * 4-128-128-32 on 256 samples: 12.7 us a step (phase A 6.1, of which 1.2 the
+ * weights; phase B 2.9), where the five kernels of the other path take 102
+ * us, 90 of them in strided reads of weights and activations.  With every
+ * CTA fetching the weights by itself the weights alone took 5.0 us: 152 x 85
+ * KB is more than L2 gives in less; as one bulk copy shared by a cluster of
+ * 8 they cost an eighth of that traffic. */
+#define FUSED_STEPS 1024
+#define FUSED_THREADS 512       /* at most: 128 registers a thread */
+#define FUSED_TILE 16
+#define FUSED_CHUNK 256         /* samples staged at a time in phase B */
+#define FUSED_PITCH (FUSED_CHUNK + 4)
+#define FUSED_CLUSTER 8
+
+/* row pitch in floats: a multiple of 4, 4 modulo 32, so that 16-byte reads
+ * of one column group by 8 neighbouring rows touch all 32 banks */
+__host__ __device__ static inline int fused_pitch(int n) { return n <= 4 ? 4 : (n - 4 + 31) / 32 * 32 + 4; }
+__host__ __device__ static inline int round4(int n) { return (n + 3) & ~3; }
+
+struct fused_args {
+	int nin, nh, nout, n, ldn;      /* ldn: samples a unit's row of XT, H1T, ... holds (a multiple of 4) */
+	int steps;                      /* Adam steps */
+	int grad;                       /* after them: the gradient at the parameters (into G) */
+	int eval;                       /* after them: a forward pass; 1 losses per sample, 2 outputs, 0 none */
+	float *P, *G, *M, *V;
+	const float *X, *T;             /* n x nin, n x nout */
+	float *XT, *H1T, *H2T, *D1T, *D2T, *D3T;        /* unit by unit: inputs, activations, deltas */
+	float *Y, *lossp;
+	const float *corr;              /* the steps' bias corrections, c1 and c2 of each */
+	float *image;                   /* the weights in the shared-memory layout */
+	unsigned int *fail;             /* set when a wait gave up */
+	float lr, b1, b2, eps;
+};
+
+/* words of the weights' image: W1, W2 and W3 with padded rows, in equal 16-byte shares for the CTAs of a cluster */
+__host__ __device__ static inline size_t fused_words(int nin, int nh, int nout)
+{
+	const size_t w = (size_t)nh * fused_pitch(nin) + (size_t)(nh + nout) * fused_pitch(nh), unit = 4 * FUSED_CLUSTER;
+	return (w + unit - 1) / unit * unit;
+}
+
+static size_t fused_smem(int nin, int nh, int nout, int sp)
+{
+	const size_t weights = fused_words(nin, nh, nout);
+	const size_t tiles = 2 * FUSED_TILE * FUSED_PITCH;
+	const size_t units = (size_t)sp * (round4(nin) + 3 * round4(nh) + 2 * round4(nout));
+	return ((weights > tiles ? weights : tiles) + units) * sizeof(float);
+}
+
+/* The weights' image (the shared-memory layout, kept in global memory beside
+ * the parameters) to every CTA of the cluster at once: CTA `rank` fetches its
+ * share as one bulk copy that lands at the same place in all CTAs and
+ * completes on each one's barrier.  One thread; every CTA takes part. */
+__device__ __forceinline__ void fused_fetch(const float *image, int words, float *s, unsigned int bar)
+{
+	const int share = words / FUSED_CLUSTER, at = (int)(blockIdx.x % FUSED_CLUSTER) * share;
+	const unsigned int dst = (unsigned int)__cvta_generic_to_shared(s + at);
+	asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(words * 4) : "memory");
+	asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.multicast::cluster [%0], [%1], %2, [%3], %4;"
+		     ::"r"(dst), "l"(image + at), "r"(share * 4), "r"(bar), "h"((unsigned short)((1 << FUSED_CLUSTER) - 1))
+		     : "memory");
+}
+
+/* wait for phase `parity` of the barrier, at most about a second; false if it gave up */
+__device__ __forceinline__ bool fused_wait(unsigned int bar, unsigned int parity)
+{
+	for (int i = 0; i < 1 << 20; i++) {
+		unsigned int done;
+		asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, 1000;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+			     : "=r"(done)
+			     : "r"(bar), "r"(parity)
+			     : "memory");
+		if (done) return true;
+	}
+	return false;
+}
+
+/* acc[s] += sum_k w[k] v[s][k], k ascending (w a padded shared row, v at
+ * pitch ldv); 16 columns' reads are issued before their multiply-adds */
+template <int SP>
+__device__ __forceinline__ void fused_row(float *acc, const float *w, const float *v, int ldv, int n)
+{
+	constexpr int U = SP <= 2 ? 4 : 2;
+	int k = 0;
+	for (; k + 4 * U <= n; k += 4 * U) {
+		float4 a[U], b[U][SP];
+#pragma unroll
+		for (int u = 0; u < U; u++) {
+			a[u] = *(const float4 *)(w + k + 4 * u);
+#pragma unroll
+			for (int s = 0; s < SP; s++) b[u][s] = *(const float4 *)(v + s * ldv + k + 4 * u);
+		}
+#pragma unroll
+		for (int u = 0; u < U; u++)
+#pragma unroll
+			for (int s = 0; s < SP; s++) {
+				acc[s] = fmaf(a[u].x, b[u][s].x, acc[s]);
+				acc[s] = fmaf(a[u].y, b[u][s].y, acc[s]);
+				acc[s] = fmaf(a[u].z, b[u][s].z, acc[s]);
+				acc[s] = fmaf(a[u].w, b[u][s].w, acc[s]);
+			}
+	}
+	for (; k < n; k++)
+#pragma unroll
+		for (int s = 0; s < SP; s++) acc[s] = fmaf(w[k], v[s * ldv + k], acc[s]);
+}
+
+/* acc[s] += sum_k w[k pitch] v[s][k], k ascending */
+template <int SP>
+__device__ __forceinline__ void fused_col(float *acc, const float *w, int pitch, const float *v, int ldv, int n)
+{
+	constexpr int U = SP <= 2 ? 4 : 2;
+	int k = 0;
+	for (; k + 4 * U <= n; k += 4 * U) {
+		float a[4 * U];
+		float4 b[U][SP];
+#pragma unroll
+		for (int u = 0; u < 4 * U; u++) a[u] = w[(k + u) * pitch];
+#pragma unroll
+		for (int u = 0; u < U; u++)
+#pragma unroll
+			for (int s = 0; s < SP; s++) b[u][s] = *(const float4 *)(v + s * ldv + k + 4 * u);
+#pragma unroll
+		for (int u = 0; u < U; u++)
+#pragma unroll
+			for (int s = 0; s < SP; s++) {
+				acc[s] = fmaf(a[4 * u], b[u][s].x, acc[s]);
+				acc[s] = fmaf(a[4 * u + 1], b[u][s].y, acc[s]);
+				acc[s] = fmaf(a[4 * u + 2], b[u][s].z, acc[s]);
+				acc[s] = fmaf(a[4 * u + 3], b[u][s].w, acc[s]);
+			}
+	}
+	for (; k < n; k++)
+#pragma unroll
+		for (int s = 0; s < SP; s++) acc[s] = fmaf(w[k * pitch], v[s * ldv + k], acc[s]);
+}
+
+/* phase A: forward pass of every sample; with deltas, also back-propagation
+ * and the activations that phase B reads.  round: how often the launch has
+ * been here (the barrier's phase).  A CTA without samples takes part in the
+ * cluster's copies. */
+template <int SP>
+__device__ __forceinline__ void fused_samples(const fused_args &a, const mlp_off &o, float *sm, size_t weights, unsigned int bar, unsigned int round,
+					      bool deltas, int eval)
+{
+	const int nin = a.nin, nh = a.nh, nout = a.nout, j = threadIdx.x;
+	const int p1 = fused_pitch(nin), p2 = fused_pitch(nh), lx = round4(nin), lh = round4(nh), lo = round4(nout);
+	float *w1 = sm, *w2 = w1 + (size_t)nh * p1, *w3 = w2 + (size_t)nh * p2;
+	float *x = sm + weights, *h1 = x + SP * lx, *h2 = h1 + SP * lh, *d2 = h2 + SP * lh, *e3 = d2 + SP * lh, *d3 = e3 + SP * lo;
+	const int groups = (a.n + SP - 1) / SP;
+	if (threadIdx.x == 0) fused_fetch(a.image, (int)fused_words(nin, nh, nout), sm, bar);
+	const float *P = a.P;
+	/* the outputs of the CTA's samples, one sample a thread where they fit */
+	const bool spread = SP * nout <= (int)blockDim.x;
+	const int jo = spread ? j % nout : j, so = spread ? j / nout : 0;
+	const float bias1 = j < nh ? __ldcg(P + o.b1 + j) : 0.0f, bias2 = j < nh ? __ldcg(P + o.b2 + j) : 0.0f,
+		    bias3 = jo < nout ? __ldcg(P + o.b3 + jo) : 0.0f;
+	const float inv = 1.0f / (float)a.n;
+	bool landed = false;
+	for (int g = blockIdx.x; g < groups; g += gridDim.x) {
+		const int s0 = g * SP, ns = min(SP, a.n - s0);
+		float target = 0.0f;
+		if (spread && so < ns && (deltas || eval == 1)) target = a.T[(int64_t)(s0 + so) * nout + jo];
+		for (int t = j; t < SP * nin; t += blockDim.x) {
+			const int s = t / nin, i = t - s * nin;
+			x[s * lx + i] = s < ns ? a.X[(int64_t)(s0 + s) * nin + i] : 0.0f;
+		}
+		if (!landed) {
+			landed = true;
+			if (!fused_wait(bar, round & 1)) *a.fail = 1;
+		}
+		__syncthreads();
+		float z1[SP], z2[SP], acc[SP];
+		if (j < nh) {
+#pragma unroll
+			for (int s = 0; s < SP; s++) z1[s] = bias1;
+			fused_row<SP>(z1, w1 + (size_t)j * p1, x, lx, nin);
+#pragma unroll
+			for (int s = 0; s < SP; s++) {
+				const float h = gelu(z1[s]);
+				h1[s * lh + j] = h;
+				if (deltas && s < ns) a.H1T[(int64_t)j * a.ldn + s0 + s] = h;
+			}
+		}
+		__syncthreads();
+		if (j < nh) {
+#pragma unroll
+			for (int s = 0; s < SP; s++) z2[s] = bias2;
+			fused_row<SP>(z2, w2 + (size_t)j * p2, h1, lh, nh);
+#pragma unroll
+			for (int s = 0; s < SP; s++) {
+				const float h = gelu(z2[s]);
+				h2[s * lh + j] = h;
+				if (deltas && s < ns) a.H2T[(int64_t)j * a.ldn + s0 + s] = h;
+			}
+		}
+		__syncthreads();
+		auto output = [&](int s, float y, float t) {
+			float e = 0.0f;
+			if (s < ns) {
+				if (eval == 2) a.Y[(int64_t)(s0 + s) * nout + jo] = y;
+				e = y - t;
+				if (deltas) a.D3T[(int64_t)jo * a.ldn + s0 + s] = e * inv;
+			}
+			e3[s * lo + jo] = e;
+			d3[s * lo + jo] = e * inv;
+		};
+		if (spread) {
+			if (so < SP) {
+				float y = bias3;
+				fused_row<1>(&y, w3 + (size_t)jo * p2, h2 + so * lh, lh, nh);
+				output(so, y, target);
+			}
+		} else if (j < nout) {
+#pragma unroll
+			for (int s = 0; s < SP; s++) acc[s] = bias3;
+			fused_row<SP>(acc, w3 + (size_t)j * p2, h2, lh, nh);
+#pragma unroll
+			for (int s = 0; s < SP; s++)
+				output(s, acc[s], s < ns && (deltas || eval == 1) ? a.T[(int64_t)(s0 + s) * nout + j] : 0.0f);
+		}
+		__syncthreads();
+		if (eval == 1 && j < ns) {
+			float l = 0.0f;
+			for (int q = 0; q < nout; q++) l = fmaf(e3[j * lo + q], e3[j * lo + q], l);
+			a.lossp[s0 + j] = 0.5f * l * inv;
+		}
+		if (deltas) {
+			if (j < nh) {
+#pragma unroll
+				for (int s = 0; s < SP; s++) acc[s] = 0.0f;
+				fused_col<SP>(acc, w3 + j, p2, d3, lo, nout);
+#pragma unroll
+				for (int s = 0; s < SP; s++) {
+					const float d = acc[s] * gelu_grad(z2[s]);
+					d2[s * lh + j] = d;
+					if (s < ns) a.D2T[(int64_t)j * a.ldn + s0 + s] = d;
+				}
+			}
+			__syncthreads();
+			if (j < nh) {
+#pragma unroll
+				for (int s = 0; s < SP; s++) acc[s] = 0.0f;
+				fused_col<SP>(acc, w2 + j, p2, d2, lh, nh);
+#pragma unroll
+				for (int s = 0; s < SP; s++)
+					if (s < ns) a.D1T[(int64_t)j * a.ldn + s0 + s] = acc[s] * gelu_grad(z1[s]);
+			}
+		}
+		__syncthreads();        /* the next samples overwrite x, h1, ... */
+	}
+	/* no CTA goes on with copies in flight */
+	if (!landed && !fused_wait(bar, round & 1)) *a.fail = 1;
+}
+
+/* one parameter's Adam update, or its gradient: p in the parameter array, at
+ * in the image (-1: a bias, which the image does not hold) */
+__device__ __forceinline__ void fused_update(const fused_args &a, int64_t p, int at, float g, bool adam, float c1, float c2, float pv,
+					     float mv, float vv)
+{
+	if (!adam) {
+		a.G[p] = g;
+		return;
+	}
+	mlp_adam_one(pv, mv, vv, g, a.lr, a.b1, a.b2, a.eps, c1, c2);
+	a.P[p] = pv;
+	if (at >= 0) a.image[at] = pv;
+	a.M[p] = mv;
+	a.V[p] = vv;
+}
+
+/* phase B: the gradient of 16 x 16 tiles of W, a parameter a thread, and
+ * with a matrix's first column tile of its bias; with adam the update */
+__device__ __forceinline__ void fused_parameters(const fused_args &a, const mlp_off &o, float *sm, bool adam, float c1, float c2)
+{
+	float *ds = sm, *as = sm + FUSED_TILE * FUSED_PITCH;
+	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, t = threadIdx.x;
+	const int row = (warp >> 1) * 4 + (lane >> 3), col = (warp & 1) * 8 + (lane & 7);
+	const int p1 = fused_pitch(a.nin), p2 = fused_pitch(a.nh);
+	const int rt = (a.nh + FUSED_TILE - 1) / FUSED_TILE, ct1 = (a.nin + FUSED_TILE - 1) / FUSED_TILE;
+	const int n1 = rt * ct1, n2 = n1 + rt * rt, n3 = n2 + (a.nout + FUSED_TILE - 1) / FUSED_TILE * rt;
+	for (int tile = blockIdx.x; tile < n3; tile += gridDim.x) {
+		const float *delta, *act;
+		int rows, cols, k, ct, image, pitch;
+		int64_t w, b;
+		if (tile < n1) {
+			delta = a.D1T; act = a.XT; rows = a.nh; cols = a.nin; w = o.w1; b = o.b1; k = tile; ct = ct1; image = 0; pitch = p1;
+		} else if (tile < n2) {
+			delta = a.D2T; act = a.H1T; rows = a.nh; cols = a.nh; w = o.w2; b = o.b2; k = tile - n1; ct = rt;
+			image = a.nh * p1; pitch = p2;
+		} else {
+			delta = a.D3T; act = a.H2T; rows = a.nout; cols = a.nh; w = o.w3; b = o.b3; k = tile - n2; ct = rt;
+			image = a.nh * (p1 + p2); pitch = p2;
+		}
+		const int r0 = k / ct * FUSED_TILE, c0 = k % ct * FUSED_TILE, r = r0 + row, c = c0 + col;
+		const bool mine = t < FUSED_TILE * FUSED_TILE && r < rows && c < cols, bias = mine && c == 0;
+		const int64_t p = w + (int64_t)r * cols + c, pb = b + r;
+		/* the parameters' state, on its way while the gradient is summed */
+		float pv = 0.0f, mv = 0.0f, vv = 0.0f, pbv = 0.0f, mbv = 0.0f, vbv = 0.0f, g = 0.0f, gb = 0.0f;
+		if (mine && adam) { pv = a.P[p]; mv = a.M[p]; vv = a.V[p]; }
+		if (bias && adam) { pbv = a.P[pb]; mbv = a.M[pb]; vbv = a.V[pb]; }
+		for (int s0 = 0; s0 < a.n; s0 += FUSED_CHUNK) {
+			const int ns = min(FUSED_CHUNK, a.n - s0), n4 = round4(ns) / 4;
+			__syncthreads();
+			/* rows of delta, then of the activations, 4 samples a copy */
+			const int q = t % (FUSED_CHUNK / 4);
+			for (int i = t / (FUSED_CHUNK / 4); i < 2 * FUSED_TILE; i += blockDim.x / (FUSED_CHUNK / 4)) {
+				const bool d = i < FUSED_TILE;
+				const int u = d ? r0 + i : c0 + i - FUSED_TILE;
+				if (q < n4 && u < (d ? rows : cols)) {
+					const float *src = (d ? delta : act) + (int64_t)u * a.ldn + s0 + 4 * q;
+					const unsigned int dst = (unsigned int)__cvta_generic_to_shared(sm + i * FUSED_PITCH + 4 * q);
+					asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+				}
+			}
+			asm volatile("cp.async.wait_all;" ::: "memory");
+			__syncthreads();
+			if (t < FUSED_TILE * FUSED_TILE) {
+				const float *d = ds + row * FUSED_PITCH, *x = as + col * FUSED_PITCH;
+				int s = 0;
+#pragma unroll 4
+				for (; s + 4 <= ns; s += 4) {
+					const float4 u = *(const float4 *)(d + s), v = *(const float4 *)(x + s);
+					g = fmaf(u.x, v.x, g);
+					g = fmaf(u.y, v.y, g);
+					g = fmaf(u.z, v.z, g);
+					g = fmaf(u.w, v.w, g);
+					gb += u.x;
+					gb += u.y;
+					gb += u.z;
+					gb += u.w;
+				}
+				for (; s < ns; s++) {
+					g = fmaf(d[s], x[s], g);
+					gb += d[s];
+				}
+			}
+		}
+		if (mine) fused_update(a, p, image + r * pitch + c, g, adam, c1, c2, pv, mv, vv);
+		if (bias) fused_update(a, pb, -1, gb, adam, c1, c2, pbv, mbv, vbv);
+	}
+	/* the next phase A reads the image and fills this shared memory through the asynchronous proxy */
+	asm volatile("fence.proxy.async;" ::: "memory");
+	__syncthreads();
+}
+
+template <int SP>
+__global__ void __cluster_dims__(FUSED_CLUSTER, 1, 1) __launch_bounds__(FUSED_THREADS) mlp_fused(const fused_args a)
+{
+	extern __shared__ __align__(16) float sm[];
+	__shared__ __align__(8) unsigned long long mbar;
+	namespace cg = cooperative_groups;
+	cg::grid_group grid = cg::this_grid();
+	const mlp_off o = offsets(a.nin, a.nh, a.nout);
+	const size_t w = fused_words(a.nin, a.nh, a.nout), weights = w > 2 * FUSED_TILE * FUSED_PITCH ? w : 2 * FUSED_TILE * FUSED_PITCH;
+	const unsigned int bar = (unsigned int)__cvta_generic_to_shared(&mbar);
+	const int64_t q0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, dq = (int64_t)gridDim.x * blockDim.x;
+	if (threadIdx.x == 0) {
+		asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
+		asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+	}
+	/* the image of the parameters, and the transposed inputs */
+	const int p1 = fused_pitch(a.nin), p2 = fused_pitch(a.nh);
+	for (int64_t q = q0; q < (int64_t)a.nh * a.nin; q += dq) a.image[q / a.nin * p1 + q % a.nin] = a.P[o.w1 + q];
+	for (int64_t q = q0; q < (int64_t)a.nh * a.nh; q += dq) a.image[a.nh * p1 + q / a.nh * p2 + q % a.nh] = a.P[o.w2 + q];
+	for (int64_t q = q0; q < (int64_t)a.nout * a.nh; q += dq) a.image[a.nh * (p1 + p2) + q / a.nh * p2 + q % a.nh] = a.P[o.w3 + q];
+	if (a.steps || a.grad)
+		for (int64_t q = q0; q < (int64_t)a.n * a.nin; q += dq) a.XT[q % a.nin * a.ldn + q / a.nin] = a.X[q];
+	asm volatile("fence.proxy.async;" ::: "memory");
+	grid.sync();
+	unsigned int round = 0;
+	for (int it = 0; it < a.steps + (a.grad ? 1 : 0); it++) {
+		fused_samples<SP>(a, o, sm, weights, bar, round++, true, it == a.steps ? a.eval : 0);
+		grid.sync();
+		const bool adam = it < a.steps;
+		fused_parameters(a, o, sm, adam, adam ? a.corr[2 * it] : 1.0f, adam ? a.corr[2 * it + 1] : 1.0f);
+		grid.sync();
+	}
+	if (!a.grad && a.eval) fused_samples<SP>(a, o, sm, weights, bar, round++, false, a.eval);
+	/* no CTA leaves while another of the cluster may still copy into it */
+	cg::this_cluster().sync();
+}
+
+/* the fused launch for n samples and its grid, or NULL where the network does not fit it */
+typedef void (*fused_kernel)(const fused_args);
+static int fused_threads(const jn_mlp *m) { return threads_for(m) > 256 ? threads_for(m) : 256; }
+static fused_kernel fused_for(const jn_mlp *m, int n, size_t *smem, int *grid)
+{
+	/* the fewest samples a CTA (the shortest phase A) for which one round of CTAs takes them all */
+	int sp = 1;
+	while (sp < 8 && (int64_t)m->num_sms * sp < n) sp *= 2;
+	*smem = fused_smem(m->nin, m->nh, m->nout, sp);
+	if (*smem > FUSED_SMEM_LIMIT || threads_for(m) > FUSED_THREADS) return NULL;
+	fused_kernel f = sp == 1 ? mlp_fused<1> : sp == 2 ? mlp_fused<2> : sp == 4 ? mlp_fused<4> : mlp_fused<8>;
+	/* the grid must be resident at once: at most one CTA an SM, in whole clusters */
+	cudaLaunchConfig_t cfg;
+	memset(&cfg, 0, sizeof cfg);
+	*grid = m->num_sms / FUSED_CLUSTER * FUSED_CLUSTER;
+	cfg.gridDim = dim3(*grid);
+	cfg.blockDim = dim3(fused_threads(m));
+	cfg.dynamicSmemBytes = *smem;
+	int clusters = 0;
+	if (cudaFuncSetAttribute((const void *)f, cudaFuncAttributeMaxDynamicSharedMemorySize, FUSED_SMEM_LIMIT) != cudaSuccess ||
+	    cudaOccupancyMaxActiveClusters(&clusters, (const void *)f, &cfg) != cudaSuccess || clusters < 1) {
+		cudaGetLastError();
+		return NULL;
+	}
+	if (*grid > clusters * FUSED_CLUSTER) *grid = clusters * FUSED_CLUSTER;
+	return f;
+}
+
+static const float ADAM_B1 = 0.9f, ADAM_B2 = 0.999f, ADAM_EPS = 1e-8f;
+
 static jn_status ensure_capacity(jn_mlp *m, int n)
 {
 	if (n <= m->cap) return JN_OK;
 	float **bufs[] = { &m->d_x, &m->d_t, &m->d_a1, &m->d_h1, &m->d_a2, &m->d_h2, &m->d_y, &m->d_d1, &m->d_d2, &m->d_d3,
 			   &m->d_loss };
-	const int64_t w[] = { m->nin, m->nout, m->nh, m->nh, m->nh, m->nh, m->nout, m->nh, m->nh, m->nout, 1 };
-	for (size_t i = 0; i < sizeof bufs / sizeof bufs[0]; i++) {
-		cudaFree(*bufs[i]);
-		*bufs[i] = NULL;
-		if (cudaMalloc((void **)bufs[i], (size_t)(n + 1) * w[i] * sizeof(float)) != cudaSuccess) {
-			m->cap = 0;
-			return jn_fail(JN_ERR_NOMEM, "MLP activations for %d samples", n);
-		}
+	/* d_a1 also takes the transposed inputs of the fused path */
+	const int64_t w[] = { m->nin, m->nout, m->nh > m->nin ? m->nh : m->nin, m->nh, m->nh, m->nh, m->nout, m->nh, m->nh,
+			      m->nout, 1 };
+	const int64_t rows = ((int64_t)n + 4) & ~3ll;
+	int64_t total = 0;
+	for (size_t i = 0; i < sizeof w / sizeof w[0]; i++) total += rows * w[i];
+	cudaFree(m->d_x);
+	m->cap = 0;
+	if (cudaMalloc((void **)&m->d_x, (size_t)total * sizeof(float)) != cudaSuccess) {
+		m->d_x = NULL;
+		return jn_fail(JN_ERR_NOMEM, "MLP activations for %d samples", n);
 	}
+	for (size_t i = 1; i < sizeof w / sizeof w[0]; i++) *bufs[i] = *bufs[i - 1] + rows * w[i - 1];
 	m->cap = n;
 	return JN_OK;
 }
@@ -194,9 +645,8 @@ static jn_status ensure_capacity(jn_mlp *m, int n)
 extern "C" void jn_mlp_destroy(jn_mlp *m)
 {
 	if (!m) return;
-	float *p[] = { m->d_p, m->d_g, m->d_m, m->d_v, m->d_x, m->d_t, m->d_a1, m->d_h1, m->d_a2, m->d_h2, m->d_y,
-		       m->d_d1, m->d_d2, m->d_d3, m->d_loss };
-	for (size_t i = 0; i < sizeof p / sizeof p[0]; i++) cudaFree(p[i]);
+	cudaFree(m->d_p);
+	cudaFree(m->d_x);
 	if (m->stream) cudaStreamDestroy(m->stream);
 	free(m);
 }
@@ -225,11 +675,18 @@ extern "C" jn_status jn_mlp_create(int nin, int nh, int nout, uint64_t seed, jn_
 	for (int64_t i = 0; i < (int64_t)nh * nh; i++) h[o.w2 + i] = (float)(unif() / sqrt((double)nh));
 	for (int64_t i = 0; i < (int64_t)nout * nh; i++) h[o.w3 + i] = (float)(unif() / sqrt((double)nh));
 	jn_status st = JN_OK;
-	float **bufs[] = { &m->d_p, &m->d_g, &m->d_m, &m->d_v };
-	for (int i = 0; i < 4 && !st; i++)
-		if (cudaMalloc((void **)bufs[i], m->np * sizeof(float)) != cudaSuccess ||
-		    cudaMemset(*bufs[i], 0, m->np * sizeof(float)) != cudaSuccess)
-			st = jn_fail(JN_ERR_NOMEM, "MLP parameters");
+	const int64_t np4 = (m->np + 3) & ~3ll;
+	int device = 0;
+	const size_t words = 4 * np4 + 2 * FUSED_STEPS + 4 + fused_words(nin, nh, nout);
+	if (cudaMalloc((void **)&m->d_p, words * sizeof(float)) != cudaSuccess ||
+	    cudaMemset(m->d_p, 0, words * sizeof(float)) != cudaSuccess || cudaGetDevice(&device) != cudaSuccess ||
+	    cudaDeviceGetAttribute(&m->num_sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess)
+		st = jn_fail(JN_ERR_NOMEM, "MLP parameters");
+	m->d_g = m->d_p + np4;
+	m->d_m = m->d_g + np4;
+	m->d_v = m->d_m + np4;
+	m->d_corr = m->d_v + np4;
+	m->d_image = m->d_corr + 2 * FUSED_STEPS + 4;
 	if (!st && cudaMemcpy(m->d_p, h, m->np * sizeof(float), cudaMemcpyHostToDevice) != cudaSuccess)
 		st = jn_fail(JN_ERR_CUDA, "MLP parameter upload");
 	if (!st && cudaStreamCreateWithFlags(&m->stream, cudaStreamNonBlocking) != cudaSuccess)
@@ -270,10 +727,42 @@ static jn_status backward(jn_mlp *m, int n)
 	mlp_deltas<<<n, th, (m->nout + m->nh) * sizeof(float), m->stream>>>(m->d_p, m->nin, m->nh, m->nout, n, m->d_t,
 									      m->d_y, m->d_a1, m->d_a2, m->d_d1, m->d_d2,
 									      m->d_d3, m->d_loss);
-	mlp_loss_sum<<<1, 32, 0, m->stream>>>(m->d_loss, n, m->d_loss);
+	mlp_loss_sum<<<1, 256, 0, m->stream>>>(m->d_loss, n, m->d_loss);
 	mlp_gradients<<<(int)((m->np + 255) / 256), 256, 0, m->stream>>>(m->nin, m->nh, m->nout, n, m->d_x, m->d_h1, m->d_h2,
 									  m->d_d1, m->d_d2, m->d_d3, m->d_g);
 	return cudaGetLastError() == cudaSuccess ? JN_OK : jn_fail(JN_ERR_CUDA, "MLP backward launch");
+}
+
+/* the fused launch over the loaded samples: `steps` Adam steps (the bias
+ * corrections in d_corr), then the gradient (grad) and a pass for the losses
+ * (eval 1) or the outputs (eval 2) */
+static jn_status fused_run(jn_mlp *m, fused_kernel f, size_t smem, int grid, int n, int steps, float lr, int grad, int eval)
+{
+	fused_args a;
+	memset(&a, 0, sizeof a);
+	a.nin = m->nin; a.nh = m->nh; a.nout = m->nout;
+	a.n = n;
+	a.ldn = round4(n);
+	a.steps = steps; a.grad = grad; a.eval = eval;
+	a.P = m->d_p; a.G = m->d_g; a.M = m->d_m; a.V = m->d_v;
+	a.X = m->d_x; a.T = m->d_t;
+	a.XT = m->d_a1; a.H1T = m->d_h1; a.H2T = m->d_h2; a.D1T = m->d_d1; a.D2T = m->d_d2; a.D3T = m->d_d3;
+	a.image = m->d_image;
+	a.fail = (unsigned int *)(m->d_corr + 2 * FUSED_STEPS);
+	a.Y = m->d_y; a.lossp = m->d_loss;
+	a.corr = m->d_corr;
+	a.lr = lr; a.b1 = ADAM_B1; a.b2 = ADAM_B2; a.eps = ADAM_EPS;
+	void *args[] = { &a };
+	CUDA_TRY(cudaLaunchCooperativeKernel((const void *)f, dim3(grid), dim3(fused_threads(m)), args, smem, m->stream));
+	return JN_OK;
+}
+
+/* a copy in the fused path whose wait gave up: the results are not valid */
+static jn_status fused_check(jn_mlp *m, unsigned int failed)
+{
+	if (!failed) return JN_OK;
+	cudaMemset(m->d_corr + 2 * FUSED_STEPS, 0, sizeof(unsigned int));
+	return jn_fail(JN_ERR_TIMEOUT, "MLP: a wait for the weights' copy gave up");
 }
 
 static jn_status load(jn_mlp *m, const float *x, const float *t, int n)
@@ -289,48 +778,83 @@ extern "C" jn_status jn_mlp_loss_and_gradient(jn_mlp *m, const float *x, const f
 {
 	if (!m || !x || !t || n < 1) return jn_fail(JN_ERR_INVALID, "bad argument");
 	jn_status s = load(m, x, t, n);
-	if (!s) s = forward(m, n);
-	if (!s) s = backward(m, n);
+	size_t smem;
+	int grid;
+	unsigned int failed = 0;
+	fused_kernel f = fused_for(m, n, &smem, &grid);
+	if (!s && f) {
+		s = fused_run(m, f, smem, grid, n, 0, 0.0f, 1, 1);
+		if (!s) mlp_loss_sum<<<1, 256, 0, m->stream>>>(m->d_loss, n, m->d_loss);
+	} else {
+		if (!s) s = forward(m, n);
+		if (!s) s = backward(m, n);
+	}
 	if (s) return s;
 	if (loss) CUDA_TRY(cudaMemcpyAsync(loss, m->d_loss + n, sizeof(float), cudaMemcpyDeviceToHost, m->stream));
 	if (grad) CUDA_TRY(cudaMemcpyAsync(grad, m->d_g, m->np * sizeof(float), cudaMemcpyDeviceToHost, m->stream));
+	if (f) CUDA_TRY(cudaMemcpyAsync(&failed, m->d_corr + 2 * FUSED_STEPS, sizeof failed, cudaMemcpyDeviceToHost, m->stream));
 	CUDA_TRY(cudaStreamSynchronize(m->stream));
-	return JN_OK;
+	return fused_check(m, failed);
 }
 
 extern "C" jn_status jn_mlp_train(jn_mlp *m, const float *x, const float *t, int n, int steps, float lr, float *final_loss)
 {
 	if (!m || !x || !t || n < 1 || steps < 0) return jn_fail(JN_ERR_INVALID, "bad argument");
 	jn_status s = load(m, x, t, n);
-	const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
-	for (int it = 0; it < steps && !s; it++) {
-		s = forward(m, n);
+	size_t smem;
+	int grid;
+	unsigned int failed = 0;
+	fused_kernel f = fused_for(m, n, &smem, &grid);
+	if (!s && f) {
+		std::vector<float> corr(2 * FUSED_STEPS);
+		for (int it = 0; (it < steps || it == 0) && !s; it += FUSED_STEPS) {
+			const int run = steps - it < FUSED_STEPS ? steps - it : FUSED_STEPS;
+			for (int i = 0; i < run; i++) {
+				m->t++;
+				corr[2 * i] = 1.0f - powf(ADAM_B1, (float)m->t);
+				corr[2 * i + 1] = 1.0f - powf(ADAM_B2, (float)m->t);
+			}
+			/* pageable memory: the copy has left `corr` when the call returns */
+			if (run) CUDA_TRY(cudaMemcpyAsync(m->d_corr, corr.data(), 2 * run * sizeof(float), cudaMemcpyHostToDevice, m->stream));
+			/* the last launch also takes the loss of the final parameters */
+			s = fused_run(m, f, smem, grid, n, run, lr, 0, it + FUSED_STEPS >= steps);
+		}
+		if (!s) mlp_loss_sum<<<1, 256, 0, m->stream>>>(m->d_loss, n, m->d_loss);
+	} else {
+		for (int it = 0; it < steps && !s; it++) {
+			s = forward(m, n);
+			if (!s) s = backward(m, n);
+			m->t++;
+			const float c1 = 1.0f - powf(ADAM_B1, (float)m->t), c2 = 1.0f - powf(ADAM_B2, (float)m->t);
+			if (!s) mlp_adam<<<(int)((m->np + 255) / 256), 256, 0, m->stream>>>(m->d_p, m->d_g, m->d_m, m->d_v, m->np, lr,
+											       ADAM_B1, ADAM_B2, ADAM_EPS, c1, c2);
+		}
+		/* loss of the final parameters */
+		if (!s) s = forward(m, n);
 		if (!s) s = backward(m, n);
-		m->t++;
-		const float c1 = 1.0f - powf(b1, (float)m->t), c2 = 1.0f - powf(b2, (float)m->t);
-		if (!s) mlp_adam<<<(int)((m->np + 255) / 256), 256, 0, m->stream>>>(m->d_p, m->d_g, m->d_m, m->d_v, m->np, lr, b1,
-										       b2, eps, c1, c2);
 	}
 	if (s) return s;
-	/* loss of the final parameters */
-	s = forward(m, n);
-	if (!s) s = backward(m, n);
-	if (s) return s;
 	if (final_loss) CUDA_TRY(cudaMemcpyAsync(final_loss, m->d_loss + n, sizeof(float), cudaMemcpyDeviceToHost, m->stream));
+	if (f) CUDA_TRY(cudaMemcpyAsync(&failed, m->d_corr + 2 * FUSED_STEPS, sizeof failed, cudaMemcpyDeviceToHost, m->stream));
 	CUDA_TRY(cudaStreamSynchronize(m->stream));
 	CUDA_TRY(cudaGetLastError());
-	return JN_OK;
+	return fused_check(m, failed);
 }
 
 extern "C" jn_status jn_mlp_predict(jn_mlp *m, const float *x, int n, float *y)
 {
 	if (!m || !x || !y || n < 1) return jn_fail(JN_ERR_INVALID, "bad argument");
 	jn_status s = load(m, x, NULL, n);
-	if (!s) s = forward(m, n);
+	size_t smem;
+	int grid;
+	unsigned int failed = 0;
+	fused_kernel f = fused_for(m, n, &smem, &grid);
+	if (!s) s = f ? fused_run(m, f, smem, grid, n, 0, 0.0f, 0, 2) : forward(m, n);
 	if (s) return s;
 	CUDA_TRY(cudaMemcpyAsync(y, m->d_y, (size_t)n * m->nout * sizeof(float), cudaMemcpyDeviceToHost, m->stream));
+	if (f) CUDA_TRY(cudaMemcpyAsync(&failed, m->d_corr + 2 * FUSED_STEPS, sizeof failed, cudaMemcpyDeviceToHost, m->stream));
 	CUDA_TRY(cudaStreamSynchronize(m->stream));
-	return JN_OK;
+	return fused_check(m, failed);
 }
 
 
