@@ -626,6 +626,20 @@ class WarmStart:
         return out
 
 
+def _transform_block(elements, handle, block_id, counts):
+    """A copy of one block of the last run; counts keeps the blocks' lengths (fixed by the plan)."""
+    n = ctypes.c_size_t()
+    count = counts.get(block_id)
+    if count is None:
+        _check(elements(handle, block_id, None, 0, ctypes.byref(n)))
+        count = counts[block_id] = n.value
+    out = np.empty(count)
+    status = elements(handle, block_id, out.ctypes.data, count, ctypes.byref(n))
+    if status:
+        _check(status)
+    return out
+
+
 class Transform:
     """J-scheme -> M-scheme two-body transform on the GPU (Mercury's two-body part)."""
 
@@ -636,6 +650,7 @@ class Transform:
         _check(L.jn_transform_open(comb.encode(), index_list_dir.encode(), Z, N, single_particle_energy,
                                    two_particle_energy, antoine_file.encode(), int(include_kinetic), ctypes.byref(h)))
         self._h = h
+        self._counts = {}
 
     @classmethod
     def from_dir(cls, d, Z, N, single_particle_energy, two_particle_energy, include_kinetic=True):
@@ -652,13 +667,7 @@ class Transform:
         return ms.value
 
     def block(self, block_id):
-        import numpy as np
-        L = gpu_lib()
-        n = ctypes.c_size_t()
-        _check(L.jn_transform_elements(self._h, block_id, None, 0, ctypes.byref(n)))
-        out = np.zeros(n.value)
-        _check(L.jn_transform_elements(self._h, block_id, out.ctypes.data_as(ctypes.c_void_p), n.value, ctypes.byref(n)))
-        return out
+        return _transform_block(gpu_lib().jn_transform_elements, self._h, block_id, self._counts)
 
     def write(self, output_dir):
         _check(gpu_lib().jn_transform_write(self._h, output_dir.encode()))
@@ -697,6 +706,7 @@ class Transform3:
         _check(gpu_lib().jn_transform3_open(comb.encode(), index_list_dir.encode(), Z, N, single_particle_energy,
                                             jscheme_dir.encode(), ctypes.byref(h)))
         self._h = h
+        self._counts = {}
 
     @classmethod
     def from_dir(cls, d, Z, N, single_particle_energy, jscheme_subdir="jjj"):
@@ -713,14 +723,7 @@ class Transform3:
         return ms.value
 
     def block(self, block_id):
-        import numpy as np
-        L = gpu_lib()
-        n = ctypes.c_size_t()
-        _check(L.jn_transform3_elements(self._h, block_id, None, 0, ctypes.byref(n)))
-        out = np.zeros(n.value)
-        _check(L.jn_transform3_elements(self._h, block_id, out.ctypes.data_as(ctypes.c_void_p), n.value,
-                                        ctypes.byref(n)))
-        return out
+        return _transform_block(gpu_lib().jn_transform3_elements, self._h, block_id, self._counts)
 
     def write(self, output_dir):
         _check(gpu_lib().jn_transform3_write(self._h, output_dir.encode()))

@@ -58,6 +58,8 @@ struct jn_transform3 {
 	double *d_out;
 	double *h_out;
 	int have_out;
+	int *slot;                      /* by block id < nslots: i + 1 for three-body block i, else 0 */
+	int nslots;
 	double plan_seconds;
 	int grid;
 };
@@ -180,8 +182,23 @@ extern "C" void jn_transform3_close(jn_transform3 *t)
 	cudaFree(t->d_epair); cudaFree(t->d_pseg); cudaFree(t->d_seg); cudaFree(t->d_T);
 	if (t->stream) cudaStreamDestroy(t->stream);
 	free(t->h_out);
+	free(t->slot);
 	jn_t3plan_free(&t->plan);
 	free(t);
+}
+
+/* the blocks by id (the first of equal ids) */
+static jn_status index_blocks(jn_transform3 *t)
+{
+	const jn_t3plan_t *p = &t->plan;
+	int top = -1;
+	for (int i = 0; i < p->n3; i++) top = p->info[p->tb_info[i]].id > top ? p->info[p->tb_info[i]].id : top;
+	t->nslots = top + 1;
+	t->slot = (int *)calloc((size_t)top + 2, sizeof(int));
+	if (!t->slot) return jn_fail(JN_ERR_NOMEM, "out of memory");
+	for (int i = p->n3 - 1; i >= 0; i--)
+		if (p->info[p->tb_info[i]].id >= 0) t->slot[p->info[p->tb_info[i]].id] = i + 1;
+	return JN_OK;
 }
 
 extern "C" jn_status jn_transform3_open(const char *comb, const char *lists_dir, int Z, int N, int emax,
@@ -214,8 +231,8 @@ extern "C" jn_status jn_transform3_open(const char *comb, const char *lists_dir,
 	cudaGetDevice(&t->device);
 	int sms = 0;
 	cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, t->device);
-	jn_status s = JN_OK;
-	if (cudaStreamCreateWithFlags(&t->stream, cudaStreamNonBlocking) != cudaSuccess) s = jn_fail(JN_ERR_CUDA, "stream");
+	jn_status s = index_blocks(t);
+	if (!s && cudaStreamCreateWithFlags(&t->stream, cudaStreamNonBlocking) != cudaSuccess) s = jn_fail(JN_ERR_CUDA, "stream");
 	if (!s) s = up(&t->d_tb, p->tb, p->n3);
 	if (!s) {
 		const int64_t nch = ((p->nelem ? p->nelem : 1) + (1 << T3_CHUNK_SHIFT) - 1) >> T3_CHUNK_SHIFT;
@@ -313,16 +330,16 @@ extern "C" jn_status jn_transform3_elements(jn_transform3 *t, int block_id, doub
 {
 	if (!t || !count) return jn_fail(JN_ERR_INVALID, "null argument");
 	const jn_t3plan_t *p = &t->plan;
-	for (int i = 0; i < p->n3; i++)
-		if (p->info[p->tb_info[i]].id == block_id) {
-			*count = (size_t)p->tb[i].count;
-			if (!host_out) return JN_OK;
-			if (capacity < *count) return jn_fail(JN_ERR_INVALID, "capacity %zu < %zu", capacity, *count);
-			jn_status s = fetch(t);
-			if (s) return s;
-			memcpy(host_out, t->h_out + p->tb[i].out, *count * sizeof(double));
-			return JN_OK;
-		}
+	const int slot = block_id >= 0 && block_id < t->nslots ? t->slot[block_id] : 0;
+	if (slot) {
+		*count = (size_t)p->tb[slot - 1].count;
+		if (!host_out) return JN_OK;
+		if (capacity < *count) return jn_fail(JN_ERR_INVALID, "capacity %zu < %zu", capacity, *count);
+		jn_status s = fetch(t);
+		if (s) return s;
+		memcpy(host_out, t->h_out + p->tb[slot - 1].out, *count * sizeof(double));
+		return JN_OK;
+	}
 	return jn_fail(JN_ERR_INVALID, "block %d is not a three-body matrix-element block", block_id);
 }
 
