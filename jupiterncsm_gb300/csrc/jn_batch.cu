@@ -12,8 +12,8 @@
  * Arithmetic (precision 32): the products use FP32 copies of the matrix
  * elements and of v_k with exact fixed-point sums (the block-tile engine);
  * the three-term recurrence, full reorthogonalisation (classical
- * Gram-Schmidt, twice), the tridiagonal eigenproblem and the final
- * refinement are FP64.  Refinement: the lowest r Ritz vectors X of each
+ * Gram-Schmidt after the recurrence, again where it cancels), the
+ * tridiagonal eigenproblem and the final refinement are FP64.  Refinement: the lowest r Ritz vectors X of each
  * instance are multiplied by the FP64 Hamiltonian, and the r x r pencil
  * (X^T H X, X^T X) is solved in FP64 (Rayleigh-Ritz), which removes the
  * error of the FP32 operator to second order.  Precision 64 runs the same
@@ -28,15 +28,16 @@
 #include <string.h>
 
 #include "jn_internal.h"
+#include "jn_ortho.cuh"
 #include "jn_tridiag.cuh"
 
 #include <functional>
+#include <vector>
 
 #define BT 256          /* threads of the vector kernels */
-#define BNB 16          /* reduction CTAs per instance */
 
 /* ------------------------------------------------------------------ */
-/* batched vector kernels (instance = blockIdx.y, k = *d_k)            */
+/* batched vector kernels (k = *d_k)                                    */
 /* ------------------------------------------------------------------ */
 #define SKIP_INACTIVE() \
 	const int inst = blockIdx.y; \
@@ -44,160 +45,194 @@
 /* the dimension of an instance: D (the vectors' stride) unless each instance has its own */
 #define DIM_OF(inst) (dims ? dims[inst] : D)
 
-__device__ __forceinline__ void slice(int64_t D, int64_t *i0, int64_t *i1)
-{
-	const int64_t chunk = (D + gridDim.x - 1) / gridDim.x;
-	*i0 = (int64_t)blockIdx.x * chunk;
-	*i1 = min(D, *i0 + chunk);
-}
+/* The vector kernels run on a flat list of CTAs: CTA c works on elements
+ * [blk * chunk, ...) of instance inst, {inst, blk} = cta[c], so that an
+ * instance has CTAs in proportion to its dimension (a grid of the largest
+ * basis's CTAs for every instance leaves half of them empty).  An instance's
+ * CTAs are neighbours, from first[inst] on; partial sums are stored by CTA. */
+#define CTA_SLICE() \
+	const int inst = cta[blockIdx.x].x, blk = cta[blockIdx.x].y; \
+	if (active && !active[inst]) return; \
+	const int64_t n = dims[inst], i0 = (int64_t)blk * chunk, i1 = min(n, i0 + chunk); \
+	const int nblk = (int)((n + chunk - 1) / chunk), cta0 = (int)blockIdx.x - blk
 
-/* part[inst][blk] = x . y over this CTA's slice; x = X + inst*x_ld (+ k*D when xk) */
-__global__ void __launch_bounds__(BT) kb_dot(const double *__restrict__ X, int64_t x_ld, int xk,
-					      const double *__restrict__ Y, int64_t y_ld, int yk, const int *__restrict__ d_k,
-					      int64_t D, const int64_t *__restrict__ dims, double *__restrict__ part,
+static_assert(BT == ORTHO_THREADS, "the sums and dot products share out a CTA of ORTHO_WARPS warps");
+
+/* part[CTA] = x . y over the slice; x = X + inst*x_ld (+ k*D when xk) */
+__global__ void __launch_bounds__(BT) kb_dot(const int2 *__restrict__ cta, int64_t chunk, const double *__restrict__ X, int64_t x_ld,
+					      int xk, const double *__restrict__ Y, int64_t y_ld, const int *__restrict__ d_k, int64_t D,
+					      const int64_t *__restrict__ dims, double *__restrict__ part,
 					      const int *__restrict__ active)
 {
-	SKIP_INACTIVE();
-	const int64_t n = DIM_OF(inst);
 	__shared__ double sh[BT];
-	const int k = *d_k;
-	const double *x = X + inst * x_ld + (xk ? (int64_t)k * D : 0);
-	const double *y = Y + inst * y_ld + (yk ? (int64_t)k * D : 0);
-	int64_t i0, i1;
-	slice(n, &i0, &i1);
+	CTA_SLICE();
+	(void)nblk, (void)cta0;
+	const double *x = X + inst * x_ld + (xk ? (int64_t)*d_k * D : 0), *y = Y + inst * y_ld;
 	double s = 0.0;
-	for (int64_t i = i0 + threadIdx.x; i < i1; i += blockDim.x) s = fma(x[i], y[i], s);
-	s = jn_block_sum(s, sh);
-	if (threadIdx.x == 0) part[(int64_t)inst * gridDim.x + blockIdx.x] = s;
+	for (int64_t i = i0 + threadIdx.x; i < i1; i += BT) s = fma(x[i], y[i], s);
+	s = ortho_cta_sum(s, sh);
+	if (threadIdx.x == 0) part[blockIdx.x] = s;
 }
 
-/* out[inst*out_ld + (k when outk)] = sum of the CTA partials in order */
-__global__ void kb_finish_dot(const double *__restrict__ part, int nblk, double *__restrict__ out, int64_t out_ld,
-			      int outk, const int *__restrict__ d_k, const int *__restrict__ active)
+/* The recurrence and the dot products with the whole basis:
+ *     alpha_k = <v_k|w> (from kb_dot's partials);  w -= alpha_k v_k + beta_{k-1} v_{k-1};
+ *     part = V_j . w over the slice, j <= k (j by j, the instance's CTAs side by side);
+ *     npart[CTA] = w . w over it.
+ * Bound by the FP64 pipe, one multiply-add per element and vector: 79 us a
+ * step for 64 instances on four bases (mean of k = 0 to 189), where one group
+ * of vectors to a warp took 190 us at k = 20 to 97. */
+__global__ void __launch_bounds__(BT) kb_recur_dots(const int2 *__restrict__ cta, int64_t chunk, double *W,
+						     const double *__restrict__ V, int64_t ldV, const double *__restrict__ apart,
+						     double *__restrict__ alpha, const double *__restrict__ beta, int64_t ldab,
+						     const int *__restrict__ d_k, int64_t D, const int64_t *__restrict__ dims,
+						     double *__restrict__ part, int ncol, double *__restrict__ npart,
+						     const int *__restrict__ active)
 {
-	SKIP_INACTIVE();
-	if (threadIdx.x) return;
-	double s = 0.0;
-	for (int b = 0; b < nblk; b++) s += part[(int64_t)inst * nblk + b];
-	out[inst * out_ld + (outk ? *d_k : 0)] = s;
-}
-
-/* w -= alpha_k v_k + beta_{k-1} v_{k-1} */
-__global__ void kb_three_term(double *__restrict__ W, const double *__restrict__ V, int64_t ldV,
-			      const double *__restrict__ alpha, const double *__restrict__ beta, int64_t ldab,
-			      const int *__restrict__ d_k, int64_t D, const int64_t *__restrict__ dims,
-			      const int *__restrict__ active)
-{
-	SKIP_INACTIVE();
-	const int64_t n = DIM_OF(inst);
-	const int k = *d_k;
-	const double a = alpha[inst * ldab + k], b = k > 0 ? beta[inst * ldab + k - 1] : 0.0;
-	const double *v = V + inst * ldV + (int64_t)k * D, *u = k > 0 ? v - D : v;
+	__shared__ double sh[BT];
+	__shared__ double ps[ORTHO_WARPS][ORTHO_SPLIT_VECTORS], word;
+	CTA_SLICE();
+	const int k = *d_k, nvec = k + 1;
+	const double a = ortho_cta_partials(apart + cta0, nblk, &word), b = k > 0 ? beta[inst * ldab + k - 1] : 0.0;
+	if (blk == 0 && threadIdx.x == 0) alpha[inst * ldab + k] = a;
 	double *w = W + inst * D;
-	for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-		double r = w[i] - a * v[i];
+	const double *v0 = V + inst * ldV, *vk = v0 + (int64_t)k * D, *u = k > 0 ? vk - D : vk;
+	double s = 0.0;
+	for (int64_t i = i0 + threadIdx.x; i < i1; i += BT) {
+		double r = w[i] - a * vk[i];
 		if (k > 0) r -= b * u[i];
 		w[i] = r;
+		s = fma(r, r, s);
 	}
+	s = ortho_cta_sum(s, sh);     /* its barriers also publish w to the CTA */
+	if (threadIdx.x == 0) npart[blockIdx.x] = s;
+	ortho_dots(v0, D, nvec, w, i0, i1, part + (int64_t)cta0 * ncol + blk, nblk, ps);
 }
 
-/* part[inst][blk][j] = V_j . w over the slice, j <= k: warp j % 8 owns
- * vector j and reduces it with shuffles in a fixed order, so no CTA-wide
- * barrier is taken per vector */
-__global__ void __launch_bounds__(BT) kb_gemv_t(const double *__restrict__ V, int64_t ldV, const double *__restrict__ W,
-						 const int *__restrict__ d_k, int64_t D, const int64_t *__restrict__ dims,
-						 double *__restrict__ part, int ncol, const int *__restrict__ active)
+/* h[inst][j] = sum of the CTAs' partials of vector j, one warp each; and k
+ * for the kernels after the subtraction: d_k[1] = d_k[0] + 1 */
+__global__ void kb_finish(const double *__restrict__ part, int64_t chunk, const int *__restrict__ first, int ncol, int *__restrict__ d_k,
+			  const int64_t *__restrict__ dims, double *__restrict__ h, const int *__restrict__ active)
 {
+	const int k = d_k[0];
+	if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) d_k[1] = k + 1;
 	SKIP_INACTIVE();
-	const int nvec = *d_k + 1;
-	const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
-	const double *w = W + inst * D;
-	int64_t i0, i1;
-	slice(DIM_OF(inst), &i0, &i1);
-	for (int j = warp; j < nvec; j += nwarps) {
-		const double *v = V + inst * ldV + (int64_t)j * D;
-		double s = 0.0;
-		for (int64_t i = i0 + lane; i < i1; i += 32) s = fma(v[i], w[i], s);
-		for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-		if (lane == 0) part[((int64_t)inst * gridDim.x + blockIdx.x) * ncol + j] = s;
-	}
+	const int j = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+	if (j > k) return;
+	const int nblk = (int)((dims[inst] + chunk - 1) / chunk);
+	const double s = ortho_partials(part + (int64_t)first[inst] * ncol + (int64_t)j * nblk, nblk);
+	if ((threadIdx.x & 31) == 0) h[(int64_t)inst * ncol + j] = s;
 }
 
-__global__ void kb_finish(const double *__restrict__ part, int nblk, int ncol, const int *__restrict__ d_k,
-			  double *__restrict__ h, const int *__restrict__ active)
+/* w -= sum_{j<=k} V_j h_j over the slice; npart[CTA] = w . w over it */
+__global__ void __launch_bounds__(BT) kb_subtract(const int2 *__restrict__ cta, int64_t chunk, const double *__restrict__ V,
+						   int64_t ldV, const double *__restrict__ h, int ncol, const int *__restrict__ d_k,
+						   int64_t D, const int64_t *__restrict__ dims, double *__restrict__ W,
+						   double *__restrict__ npart, const int *__restrict__ active)
 {
-	SKIP_INACTIVE();
-	const int j = blockIdx.x * blockDim.x + threadIdx.x;
-	if (j > *d_k) return;
-	double s = 0.0;
-	for (int b = 0; b < nblk; b++) s += part[((int64_t)inst * nblk + b) * ncol + j];
-	h[(int64_t)inst * ncol + j] = s;
-}
-
-/* w -= sum_{j<=k} V_j h_j */
-__global__ void kb_gemv_n_sub(const double *__restrict__ V, int64_t ldV, const double *__restrict__ h, int ncol,
-			      const int *__restrict__ d_k, int64_t D, const int64_t *__restrict__ dims, double *__restrict__ W,
-			      const int *__restrict__ active)
-{
-	SKIP_INACTIVE();
-	const int64_t n = DIM_OF(inst);
-	const int nvec = *d_k + 1;
-	const double *hh = h + (int64_t)inst * ncol, *v = V + inst * ldV;
+	__shared__ double sh[BT];
+	CTA_SLICE();
+	(void)nblk, (void)cta0;
+	const int nvec = d_k[0] + 1;
+	const double *hh = h + (int64_t)inst * ncol, *v0 = V + inst * ldV;
 	double *w = W + inst * D;
-	for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+	double t = 0.0;
+	for (int64_t i = i0 + threadIdx.x; i < i1; i += BT) {
 		double s = 0.0;
-		for (int j = 0; j < nvec; j++) s = fma(v[(int64_t)j * D + i], hh[j], s);
-		w[i] -= s;
+		const double *v = v0 + i;
+#pragma unroll 8
+		for (int j = 0; j < nvec; j++, v += D) s = fma(*v, hh[j], s);
+		const double r = w[i] - s;
+		w[i] = r;
+		t = fma(r, r, t);
 	}
+	t = ortho_cta_sum(t, sh);
+	if (threadIdx.x == 0) npart[blockIdx.x] = t;
 }
 
-/* v_{k+1} = w / |w|, beta_k = |w| (|w|^2 in nrm2[inst]) */
-__global__ void kb_normalize(double *__restrict__ V, int64_t ldV, const double *__restrict__ W,
-			     const double *__restrict__ nrm2, double *__restrict__ beta, int64_t ldab,
-			     const int *__restrict__ d_k, int64_t D, const int64_t *__restrict__ dims,
-			     const int *__restrict__ active)
+/* After the recurrence w is orthogonal to the basis but for rounding, so one
+ * pass of Gram-Schmidt restores full orthogonality (max |V^T V - 1| 7e-16
+ * over 200 steps, as with two passes) unless the pass itself took most of w
+ * away: |w| fell below 0.7 of what it was, which happens only when the
+ * Krylov space closes.  Then this instance gets another pass, by one CTA.
+ * Also the next step's k: d_k[0] = d_k[1]. */
+__global__ void __launch_bounds__(512) kb_second_pass(const double *__restrict__ V, int64_t ldV, int64_t chunk, double *__restrict__ h,
+						       int ncol, int *__restrict__ d_k, int64_t D, const int64_t *__restrict__ dims,
+						       double *W, const double *__restrict__ before, double *__restrict__ after,
+						       const int *__restrict__ first,
+						       const int *__restrict__ active)
 {
+	const int nvec = d_k[1];
+	if (blockIdx.y == 0 && threadIdx.x == 0) d_k[0] = nvec;
 	SKIP_INACTIVE();
-	const int64_t n = DIM_OF(inst);
-	const int k = *d_k;
-	const double b = sqrt(nrm2[inst]);
-	if (blockIdx.x == 0 && threadIdx.x == 0) beta[inst * ldab + k] = b;
-	const double inv = b > 0.0 ? 1.0 / b : 0.0;
-	double *v = V + inst * ldV + (int64_t)(k + 1) * D;
-	const double *w = W + inst * D;
-	for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-		v[i] = w[i] * inv;
+	__shared__ double sh[512];
+	const int64_t n = dims[inst];
+	const int nblk = (int)((n + chunk - 1) / chunk), warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+	const double n0 = ortho_cta_partials(before + first[inst], nblk, sh), n1 = ortho_cta_partials(after + first[inst], nblk, sh + 1);
+	if (n1 >= 0.49 * n0) return;
+	double *hh = h + (int64_t)inst * ncol, *w = W + inst * D;
+	const double *v0 = V + inst * ldV;
+	for (int j = warp; j < nvec; j += blockDim.x >> 5) {
+		const double *v = v0 + (int64_t)j * D;
+		double s = 0.0;
+		for (int64_t i = lane; i < n; i += 32) s = fma(v[i], w[i], s);
+		for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+		if (lane == 0) hh[j] = s;
+	}
+	__syncthreads();
+	double t = 0.0;
+	for (int64_t i = threadIdx.x; i < n; i += blockDim.x) {
+		double s = 0.0;
+		for (int j = 0; j < nvec; j++) s = fma(v0[(int64_t)j * D + i], hh[j], s);
+		const double r = w[i] - s;
+		w[i] = r;
+		t = fma(r, r, t);
+	}
+	t = jn_block_sum(t, sh);
+	for (int b = threadIdx.x; b < nblk; b += blockDim.x) after[first[inst] + b] = b ? 0.0 : t;
 }
 
-/* v_0 /= |v_0| (|v_0|^2 in nrm2[inst]) */
-__global__ void kb_scale_start(double *__restrict__ V, int64_t ldV, const double *__restrict__ nrm2, int64_t D,
-			       const int64_t *__restrict__ dims)
+/* v_{k+1} = w / |w|, beta_k = |w| from the partials of |w|^2; d_k[1] = k + 1.
+ * The square root and the division are one thread's: FP64 instructions of a
+ * whole CTA's warps, they alone took 20 us */
+__global__ void __launch_bounds__(BT) kb_normalize(const int2 *__restrict__ cta, int64_t chunk, double *V, int64_t ldV,
+						    const double *W, int64_t w_ld, const double *__restrict__ npart,
+						    double *__restrict__ beta, int64_t ldab, const int *__restrict__ d_k, int64_t D,
+						    const int64_t *__restrict__ dims, const int *__restrict__ active)
 {
-	const int inst = blockIdx.y;
-	const int64_t n = DIM_OF(inst);
-	const double inv = 1.0 / sqrt(nrm2[inst]);
-	double *v = V + inst * ldV;
-	for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-		v[i] *= inv;
+	__shared__ double scale;
+	CTA_SLICE();
+	const int k1 = d_k[1];
+	if (threadIdx.x < 32) {
+		const double s = ortho_partials(npart + cta0, nblk);
+		if (threadIdx.x == 0) {
+			const double b = sqrt(s);
+			if (blk == 0 && beta) beta[inst * ldab + k1 - 1] = b;
+			scale = b > 0.0 ? 1.0 / b : 0.0;
+		}
+	}
+	__syncthreads();
+	const double inv = scale;
+	double *v = V + inst * ldV + (int64_t)k1 * D;
+	const double *w = W + inst * w_ld;
+	for (int64_t i = i0 + threadIdx.x; i < i1; i += BT) v[i] = w[i] * inv;
 }
-
-__global__ void kb_advance(int *d_k) { if (threadIdx.x == 0 && blockIdx.x == 0) *d_k += 1; }
 
 /* ------------------------------------------------------------------ */
 /* batched tridiagonal work (n per instance)                            */
 /* ------------------------------------------------------------------ */
-/* eigenvalue i = blockIdx.x < want of each instance's T by one warp, and its
+/* eigenvalue i = blockIdx.x < want of each instance's T by two warps, and its
  * eigenvector (rows of Z, its bottom component in zlast when not NULL).
  * Scratch: shared memory, or `work` (JN_TRI_VECTOR_DOUBLES(ldz) a warp) when
  * the rows do not fit there.  The first `guesses` entries of theta hold an
  * earlier check's eigenvalues. */
-__global__ void __launch_bounds__(32) kb_tri_pairs(const double *__restrict__ alpha, const double *__restrict__ beta, int64_t ldab,
+__global__ void __launch_bounds__(64) kb_tri_pairs(const double *__restrict__ alpha, const double *__restrict__ beta, int64_t ldab,
 						    const int *__restrict__ n_arr, int want, double *__restrict__ theta, int ldt,
 						    double *__restrict__ Z, int ldz, double *__restrict__ work,
 						    double *__restrict__ zlast, int guesses, const int *__restrict__ active)
 {
 	SKIP_INACTIVE();
 	extern __shared__ double sbuf[];
+	__shared__ jn_tri_exchange ex;
 	const int i = blockIdx.x;
 	const int n = n_arr[inst];
 	if (i >= want || i >= n) return;
@@ -206,9 +241,11 @@ __global__ void __launch_bounds__(32) kb_tri_pairs(const double *__restrict__ al
 	double *z = Z + ((int64_t)inst * want + i) * ldz;
 	double lo, hi;
 	const double sc = jn_tri_scale(a, b, n, &lo, &hi);
-	jn_tri_stage(a, b, n, sc, as, b2);
+	if (threadIdx.x < 32) jn_tri_stage(a, b, n, sc, as, b2);
 	const double old = i < guesses ? theta[(int64_t)inst * ldt + i] : 0.0;
-	const double x = jn_tri_multisect_warp(as, b2, n, i, lo, hi, i < guesses, old * sc);
+	__syncthreads();
+	const double x = jn_tri_multisect(as, b2, n, i, lo, hi, i < guesses, old * sc, &ex);
+	if (threadIdx.x >= 32) return;
 	jn_tri_vector_warp(as, b2, n, x, z, b2 + n);
 	if (threadIdx.x == 0) {
 		theta[(int64_t)inst * ldt + i] = x / sc;
@@ -250,24 +287,47 @@ __global__ void kb_converged(const double *__restrict__ theta, const double *__r
 	flag[inst] = ok || b == 0.0;
 }
 
-/* X[inst][j] = sum_{l < n} V[inst][l] Z[inst][j][l], j < r */
-__global__ void kb_ritz(const double *__restrict__ V, int64_t ldV, const double *__restrict__ Z, int ldz,
-			const int *__restrict__ n_arr, int r, int64_t D, const int64_t *__restrict__ dims,
-			double *__restrict__ X)
+/* X[inst][j] = sum_{l < n} V[inst][l] Z[inst][j][l], j < r: CTAs (element
+ * slice, group of RITZ_ROWS vectors, instance); an element of each V_l is read
+ * once for the group (one pass over V a vector took 1.46 ms for 14 vectors of
+ * 64 instances) */
+#define RITZ_ROWS 8
+#define RITZ_L 128
+__global__ void __launch_bounds__(128) kb_ritz(const double *__restrict__ V, int64_t ldV, const double *__restrict__ Z, int ldz,
+						const int *__restrict__ n_arr, int r, int64_t D, const int64_t *__restrict__ dims,
+						double *__restrict__ X)
 {
-	const int inst = blockIdx.y;
-	const int n = n_arr[inst];
-	const int64_t dim = DIM_OF(inst);
-	const double *v = V + inst * ldV;
-	const double *z = Z + (int64_t)inst * r * ldz;
-	double *x = X + (int64_t)inst * r * D;
-	for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < dim; i += (int64_t)gridDim.x * blockDim.x)
-		for (int j = 0; j < r; j++) {
-			double s = 0.0;
-			if (j < n)
-				for (int l = 0; l < n; l++) s = fma(v[(int64_t)l * D + i], z[(int64_t)j * ldz + l], s);
-			x[(int64_t)j * D + i] = s;
+	__shared__ double zs[RITZ_ROWS][RITZ_L];
+	const int inst = blockIdx.z, n = n_arr[inst], j0 = blockIdx.y * RITZ_ROWS, nj = min(RITZ_ROWS, r - j0);
+	const int64_t dim = dims[inst], i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+	if ((int64_t)blockIdx.x * blockDim.x >= dim) return;
+	const double *z = Z + ((int64_t)inst * r + j0) * ldz;
+	double acc[RITZ_ROWS];
+#pragma unroll
+	for (int j = 0; j < RITZ_ROWS; j++) acc[j] = 0.0;
+	for (int l0 = 0; l0 < n; l0 += RITZ_L) {
+		const int nl = min(RITZ_L, n - l0);
+		__syncthreads();
+		for (int t = threadIdx.x; t < RITZ_ROWS * nl; t += blockDim.x) {
+			const int j = t / nl, l = t - j * nl;
+			/* a Krylov space smaller than r has no further vectors */
+			zs[j][l] = j < nj && j0 + j < n ? z[(int64_t)j * ldz + l0 + l] : 0.0;
 		}
+		__syncthreads();
+		if (i < dim) {
+			const double *v = V + inst * ldV + (int64_t)l0 * D + i;
+#pragma unroll 4
+			for (int l = 0; l < nl; l++, v += D) {
+				const double x = *v;
+#pragma unroll
+				for (int j = 0; j < RITZ_ROWS; j++) acc[j] = fma(x, zs[j][l], acc[j]);
+			}
+		}
+	}
+	if (i < dim)
+#pragma unroll
+		for (int j = 0; j < RITZ_ROWS; j++)
+			if (j < nj) X[((int64_t)inst * r + j0 + j) * D + i] = acc[j];
 }
 
 /* G[inst][i][j] = A[inst][i] . Bm[inst][j]; one CTA per (i, j, inst) */
@@ -424,29 +484,34 @@ static int rayleigh_ritz(const double *G1, const double *G2, const double *G3, i
 /* The instances of one batched solve, their layout and their products.
  * Instance i has dimension dims[i] <= Dp; its vectors are stored Dp apart. */
 struct batch_job {
-	int B;
+	int B, num_sms;
 	int64_t Dp;
 	const int64_t *dims;
 	/* W_i = H_i v_k for every active instance, in the solve's arithmetic (k read on the device) */
 	std::function<jn_status(const double *V, int64_t ldV, const int *d_k, double *W, const int *d_active, cudaStream_t)>
 		product;
-	/* HX_i = H_i X_i in FP64-grade arithmetic for every instance (X_i = X + i ld); scratch: B x Dp */
-	std::function<jn_status(const double *X, int64_t ld, double *HX, double *scratch, cudaStream_t)> product64;
+	/* HX = H_i X in FP64-grade arithmetic for the r vectors of every instance (B x r x Dp) */
+	std::function<jn_status(const double *X, int r, double *HX, cudaStream_t)> product64;
+	/* optional, after a convergence check on an idle device: *changed when the products' launches are other
+	   ones for the instances still active (act, host) */
+	std::function<jn_status(const int *act, int *changed)> rebalance;
 	const double *const *start_vectors;     /* B entries, or NULL */
 	double *const *eigenvectors;            /* B entries, or NULL */
 	jn_batch_result **res;                  /* B results */
 };
 
 struct bstate {
-	double *V, *W, *alpha, *beta, *part, *h, *scal, *theta, *zlast, *Z, *work, *X, *HX, *G, *C, *GS;
+	double *V, *W, *alpha, *beta, *part, *h, *apart, *before, *after, *theta, *zlast, *Z, *work, *X, *HX, *G, *C, *GS;
 	int64_t *dims;
-	int *k, *active, *flag, *narr;
+	int2 *cta;
+	int *first;
+	int *k, *active, *flag, *narr;          /* k: the step; from the subtraction on, the step after it */
 };
 
 static void bstate_free(struct bstate *s)
 {
-	void *p[] = { s->V, s->W, s->alpha, s->beta, s->part, s->h, s->scal, s->theta, s->zlast, s->Z, s->work, s->X,
-		      s->HX, s->G, s->C, s->GS, s->dims, s->k, s->active, s->flag, s->narr };
+	void *p[] = { s->V, s->W, s->alpha, s->beta, s->part, s->h, s->apart, s->before, s->after, s->theta, s->zlast, s->Z, s->work, s->X,
+		      s->HX, s->G, s->C, s->GS, s->dims, s->cta, s->first, s->k, s->active, s->flag, s->narr };
 	for (size_t i = 0; i < sizeof p / sizeof p[0]; i++) cudaFree(p[i]);
 }
 
@@ -496,9 +561,25 @@ static jn_status batch_solve(cudaStream_t q, const jn_batch_options *o, const ba
 	BALLOC(s.W, (size_t)B * Dp);
 	BALLOC(s.alpha, (size_t)B * ldab);
 	BALLOC(s.beta, (size_t)B * ldab);
-	BALLOC(s.part, (size_t)B * BNB * ncol);
+	/* the vector kernels' slices: about six CTAs an SM over all instances, at most 304 an instance */
+	int64_t total = 0;
+	for (int i = 0; i < B; i++) total += job.dims[i];
+	int64_t chunk = (total / (6 * job.num_sms) + 31) & ~31ll;
+	if (chunk < (Dp + 303) / 304) chunk = (Dp + 303) / 304;
+	if (chunk < 32) chunk = 32;
+	std::vector<int2> cta;
+	std::vector<int> first(B);
+	for (int i = 0; i < B; i++) {
+		first[i] = (int)cta.size();
+		for (int64_t b = 0; b * chunk < job.dims[i]; b++) cta.push_back(make_int2(i, (int)b));
+	}
+	BALLOC(s.part, cta.size() * ncol);
 	BALLOC(s.h, (size_t)B * ncol);
-	BALLOC(s.scal, (size_t)B);
+	BALLOC(s.apart, cta.size());
+	BALLOC(s.before, cta.size());
+	BALLOC(s.after, cta.size());
+	BALLOC(s.cta, cta.size());
+	BALLOC(s.first, B);
 	BALLOC(s.theta, (size_t)B * (r + 1));
 	BALLOC(s.zlast, (size_t)B * (r + 1));
 	const int zrows = r > want ? r : want;  /* vectors per instance: r at the end, want in checks */
@@ -509,12 +590,14 @@ static jn_status batch_solve(cudaStream_t q, const jn_batch_options *o, const ba
 					(int)JN_TRI_SMEM(JN_TRI_SMEM_ROWS)) != cudaSuccess)
 		st = jn_fail(JN_ERR_CUDA, "batched Lanczos: shared memory of the tridiagonal kernel");
 	BALLOC(s.dims, B);
-	BALLOC(s.k, 1);
+	BALLOC(s.k, 2);
 	BALLOC(s.active, B);
 	BALLOC(s.flag, B);
 	BALLOC(s.narr, B);
 	if (st) { bstate_free(&s); free(lim); return st; }
-	if (cudaMemcpy(s.dims, job.dims, B * sizeof(int64_t), cudaMemcpyHostToDevice) != cudaSuccess)
+	if (cudaMemcpy(s.dims, job.dims, B * sizeof(int64_t), cudaMemcpyHostToDevice) != cudaSuccess ||
+	    cudaMemcpy(s.cta, cta.data(), cta.size() * sizeof(int2), cudaMemcpyHostToDevice) != cudaSuccess ||
+	    cudaMemcpy(s.first, first.data(), B * sizeof(int), cudaMemcpyHostToDevice) != cudaSuccess)
 		st = jn_fail(JN_ERR_CUDA, "upload of the instances' dimensions");
 
 	/* start vectors: given, or one seeded pseudo-random vector of the instance's dimension */
@@ -535,15 +618,15 @@ static jn_status batch_solve(cudaStream_t q, const jn_batch_options *o, const ba
 	cudaGraph_t graph = NULL;
 	int k = 0, nactive = B, guesses = 0;
 	const int vg = (int)((Dp + BT - 1) / BT < 64 ? (Dp + BT - 1) / BT : 64);
-	const dim3 gv(vg > 0 ? vg : 1, B), gr(BNB, B), g1(1, B);
+	const dim3 gv(vg > 0 ? vg : 1, B), g1(1, B);
+	const int gc = (int)cta.size();
 	const int64_t *dims = s.dims;
 	if (!st) {
-		cudaMemsetAsync(s.k, 0, sizeof(int), q);
+		cudaMemsetAsync(s.k, 0, 2 * sizeof(int), q);
 		cudaMemcpyAsync(s.active, hact, B * sizeof(int), cudaMemcpyHostToDevice, q);
 		/* v_0 normalised */
-		kb_dot<<<gr, BT, 0, q>>>(s.V, ldV, 0, s.V, ldV, 0, s.k, Dp, dims, s.part, NULL);
-		kb_finish_dot<<<g1, 32, 0, q>>>(s.part, BNB, s.scal, 1, 0, s.k, NULL);
-		kb_scale_start<<<gv, BT, 0, q>>>(s.V, ldV, s.scal, Dp, dims);
+		kb_dot<<<gc, BT, 0, q>>>(s.cta, chunk, s.V, ldV, 0, s.V, ldV, s.k, Dp, dims, s.after, NULL);
+		kb_normalize<<<gc, BT, 0, q>>>(s.cta, chunk, s.V, ldV, s.V, ldV, s.after, NULL, ldab, s.k, Dp, dims, NULL);
 		if (cudaGetLastError() != cudaSuccess) st = jn_fail(JN_ERR_CUDA, "batched Lanczos start");
 	}
 
@@ -551,30 +634,30 @@ static jn_status batch_solve(cudaStream_t q, const jn_batch_options *o, const ba
 	auto step = [&](cudaStream_t qs) -> jn_status {
 		jn_status e = job.product(s.V, ldV, s.k, s.W, s.active, qs);
 		if (e) return e;
-		kb_dot<<<gr, BT, 0, qs>>>(s.V, ldV, 1, s.W, Dp, 0, s.k, Dp, dims, s.part, s.active);
-		kb_finish_dot<<<g1, 32, 0, qs>>>(s.part, BNB, s.alpha, ldab, 1, s.k, s.active);
-		kb_three_term<<<gv, BT, 0, qs>>>(s.W, s.V, ldV, s.alpha, s.beta, ldab, s.k, Dp, dims, s.active);
-		for (int pass = 0; pass < 2; pass++) {
-			kb_gemv_t<<<gr, BT, 0, qs>>>(s.V, ldV, s.W, s.k, Dp, dims, s.part, ncol, s.active);
-			kb_finish<<<dim3((ncol + 127) / 128, B), 128, 0, qs>>>(s.part, BNB, ncol, s.k, s.h, s.active);
-			kb_gemv_n_sub<<<gv, BT, 0, qs>>>(s.V, ldV, s.h, ncol, s.k, Dp, dims, s.W, s.active);
-		}
-		kb_dot<<<gr, BT, 0, qs>>>(s.W, Dp, 0, s.W, Dp, 0, s.k, Dp, dims, s.part, s.active);
-		kb_finish_dot<<<g1, 32, 0, qs>>>(s.part, BNB, s.scal, 1, 0, s.k, s.active);
-		kb_normalize<<<gv, BT, 0, qs>>>(s.V, ldV, s.W, s.scal, s.beta, ldab, s.k, Dp, dims, s.active);
-		kb_advance<<<1, 32, 0, qs>>>(s.k);
+		kb_dot<<<gc, BT, 0, qs>>>(s.cta, chunk, s.V, ldV, 1, s.W, Dp, s.k, Dp, dims, s.apart, s.active);
+		kb_recur_dots<<<gc, BT, 0, qs>>>(s.cta, chunk, s.W, s.V, ldV, s.apart, s.alpha, s.beta, ldab, s.k, Dp, dims, s.part,
+						 ncol, s.before, s.active);
+		kb_finish<<<dim3((ncol + 7) / 8, B), 256, 0, qs>>>(s.part, chunk, s.first, ncol, s.k, dims, s.h, s.active);
+		kb_subtract<<<gc, BT, 0, qs>>>(s.cta, chunk, s.V, ldV, s.h, ncol, s.k, Dp, dims, s.W, s.after, s.active);
+		kb_second_pass<<<g1, 512, 0, qs>>>(s.V, ldV, chunk, s.h, ncol, s.k, Dp, dims, s.W, s.before, s.after, s.first, s.active);
+		kb_normalize<<<gc, BT, 0, qs>>>(s.cta, chunk, s.V, ldV, s.W, Dp, s.after, s.beta, ldab, s.k, Dp, dims, s.active);
 		return cudaGetLastError() == cudaSuccess ? JN_OK : jn_fail(JN_ERR_CUDA, "batched Lanczos step launch");
 	};
 
-	if (!st && o->use_graph) {
+	auto capture = [&]() -> jn_status {
+		if (gexec) cudaGraphExecDestroy(gexec);
+		if (graph) cudaGraphDestroy(graph);
+		gexec = NULL;
+		graph = NULL;
 		if (cudaStreamBeginCapture(q, cudaStreamCaptureModeThreadLocal) != cudaSuccess)
-			st = jn_fail(JN_ERR_CUDA, "stream capture");
-		jn_status e = st ? st : step(q);
+			return jn_fail(JN_ERR_CUDA, "stream capture");
+		jn_status e = step(q);
 		cudaError_t ce = cudaStreamEndCapture(q, &graph);
-		if (!st && (e || ce != cudaSuccess)) st = e ? e : jn_fail(JN_ERR_CUDA, "end capture: %s", cudaGetErrorString(ce));
-		if (!st && cudaGraphInstantiate(&gexec, graph, 0) != cudaSuccess)
-			st = jn_fail(JN_ERR_CUDA, "graph instantiation");
-	}
+		if (e || ce != cudaSuccess) return e ? e : jn_fail(JN_ERR_CUDA, "end capture: %s", cudaGetErrorString(ce));
+		if (cudaGraphInstantiate(&gexec, graph, 0) != cudaSuccess) return jn_fail(JN_ERR_CUDA, "graph instantiation");
+		return JN_OK;
+	};
+	if (!st && o->use_graph) st = capture();
 
 	while (!st && nactive > 0 && k < m) {
 		if (gexec) {
@@ -591,7 +674,7 @@ static jn_status batch_solve(cudaStream_t q, const jn_batch_options *o, const ba
 		for (int i = 0; i < B; i++) hn[i] = hact[i] ? k : hn[i];
 		cudaMemcpyAsync(s.narr, hn, B * sizeof(int), cudaMemcpyHostToDevice, q);
 		const int wk = want < k ? want : k;
-		kb_tri_pairs<<<dim3(wk, B), 32, tri_smem ? JN_TRI_SMEM(k) : 0, q>>>(
+		kb_tri_pairs<<<dim3(wk, B), 64, tri_smem ? JN_TRI_SMEM(k) : 0, q>>>(
 			s.alpha, s.beta, ldab, s.narr, wk, s.theta, r + 1, s.Z, ldz, s.work, s.zlast, guesses, s.active);
 		guesses = wk;
 		kb_converged<<<(B + 127) / 128, 128, 0, q>>>(s.theta, s.zlast, r + 1, s.beta, ldab, s.narr, nev, o->tolerance,
@@ -610,6 +693,9 @@ static jn_status batch_solve(cudaStream_t q, const jn_batch_options *o, const ba
 				nactive--;
 			}
 		cudaMemcpyAsync(s.active, hact, B * sizeof(int), cudaMemcpyHostToDevice, q);
+		int changed = 0;
+		if (job.rebalance && nactive > 0 && k < m) st = job.rebalance(hact, &changed);
+		if (!st && changed && o->use_graph) st = capture();
 	}
 	if (gexec) cudaGraphExecDestroy(gexec);
 	if (graph) cudaGraphDestroy(graph);
@@ -627,13 +713,15 @@ static jn_status batch_solve(cudaStream_t q, const jn_batch_options *o, const ba
 		for (int i = 0; i < B; i++) hact[i] = 1;
 		cudaMemcpyAsync(s.narr, hn, B * sizeof(int), cudaMemcpyHostToDevice, q);
 		cudaMemcpyAsync(s.active, hact, B * sizeof(int), cudaMemcpyHostToDevice, q);
-		kb_tri_pairs<<<dim3(r, B), 32, tri_smem ? JN_TRI_SMEM(k) : 0, q>>>(
+		kb_tri_pairs<<<dim3(r, B), 64, tri_smem ? JN_TRI_SMEM(k) : 0, q>>>(
 			s.alpha, s.beta, ldab, s.narr, r, s.theta, r + 1, s.Z, ldz, s.work, NULL, guesses, NULL);
 		kb_tri_mgs<<<g1, BT, 0, q>>>(s.Z, ldz, s.narr, r, NULL);
-		kb_ritz<<<gv, BT, 0, q>>>(s.V, ldV, s.Z, ldz, s.narr, r, Dp, dims, s.X);
-		/* H X in FP64-grade arithmetic, one batched product per Ritz index */
-		for (int j = 0; j < r && !st; j++)
-			st = job.product64(s.X + (size_t)j * Dp, (int64_t)r * Dp, s.HX + (size_t)j * Dp, s.W, q);
+		/* instances in waves of the grid's third dimension */
+		for (int i = 0; i < B; i += 65535)
+			kb_ritz<<<dim3((unsigned int)((Dp + 127) / 128), (r + RITZ_ROWS - 1) / RITZ_ROWS, B - i < 65535 ? B - i : 65535), 128, 0,
+				  q>>>(s.V + (size_t)i * ldV, ldV, s.Z + (size_t)i * r * ldz, ldz, s.narr + i, r, Dp, dims + i,
+				       s.X + (size_t)i * r * Dp);
+		st = job.product64(s.X, r, s.HX, q);
 	}
 	if (!st) {
 		kb_gram<<<dim3(r * r, B), BT, 0, q>>>(s.X, s.X, r, Dp, dims, s.G);
@@ -688,6 +776,39 @@ static jn_status batch_solve(cudaStream_t q, const jn_batch_options *o, const ba
 	return st;
 }
 
+/* HX = H_i X for the r vectors of B instances of one basis (X, HX: B x r
+ * vectors Dp apart) on the block-tile engine in FP64: as many vectors at a
+ * time as 512 MB of scratch and the grid take.  (One launch a vector, 56 for
+ * 14 vectors on four bases, took 19 ms, most of it launches too small to fill
+ * the GPU.) */
+static jn_status refine_products(jn_ctx *c, int B, const double *me64, const double *X, int r, int64_t Dp, double *HX,
+				 double abs_bound, cudaStream_t q)
+{
+	const jn_plan_t *p = &c->plan;
+	const int64_t D = p->dim;
+	int64_t per = (512ll << 20) / (16 * B * D);
+	if (per > 65535 / B) per = 65535 / B;
+	if (per > r) per = r;
+	if (per < 1) per = 1;
+	double *x64 = NULL;
+	unsigned long long *gacc = NULL;
+	unsigned int *ctrl = NULL;
+	jn_status st = JN_OK;
+	BALLOC(x64, (size_t)B * per * D);
+	BALLOC(gacc, (size_t)B * per * D);
+	BALLOC(ctrl, (size_t)2 * B * per);
+	if (!st && cudaMemsetAsync(gacc, 0, (size_t)B * per * D * sizeof(unsigned long long), q) != cudaSuccess)
+		st = jn_fail(JN_ERR_CUDA, "accumulator clear");
+	for (int j = 0; j < r && !st; j += (int)per) {
+		const int nv = r - j < per ? r - j : (int)per;
+		st = jn_enqueue_batched(c, B * nv, nv, 0, me64, p->n_me, X + (size_t)j * Dp, (int64_t)r * Dp, Dp, NULL, 0,
+					HX + (size_t)j * Dp, (int64_t)r * Dp, x64, NULL, gacc, ctrl, NULL, abs_bound, q);
+	}
+	if (cudaStreamSynchronize(q) != cudaSuccess && !st) st = jn_fail(JN_ERR_CUDA, "refinement products");
+	cudaFree(x64); cudaFree(gacc); cudaFree(ctrl);
+	return st;
+}
+
 extern "C" jn_status jn_lanczos_batch(jn_ctx *c, const jn_batch_options *o, jn_batch_result *res)
 {
 	if (!c || !o || !res || !o->matrix_elements) return jn_fail(JN_ERR_INVALID, "null argument");
@@ -707,20 +828,17 @@ extern "C" jn_status jn_lanczos_batch(jn_ctx *c, const jn_batch_options *o, jn_b
 	/* the products' state: matrix elements, converted x, accumulators */
 	double *me64 = NULL, *x64 = NULL;
 	float *me32 = NULL, *x32 = NULL;
-	unsigned long long *gacc = NULL, *pcmax = NULL;
+	unsigned long long *gacc = NULL;
 	unsigned int *ctrl = NULL;
-	int *pcoef = NULL, *pxbuf = NULL;
+	struct jn_panel_batch *pb = NULL;
 	BALLOC(me64, (size_t)B * nme);
 	/* 32-bit products on the panel engine where it is this context's engine */
-	const int panels = f32 && c->engine_of[1] == 4 && jn_panels_setup(c) == JN_OK && jn_panels_fit(c, 1);
-	if (f32 && !panels) { BALLOC(me32, (size_t)B * nme); BALLOC(x32, (size_t)B * D); }
-	else BALLOC(x64, (size_t)B * D);
-	BALLOC(gacc, (size_t)B * D);
-	BALLOC(ctrl, (size_t)2 * B);
-	if (panels) {
-		BALLOC(pcoef, (size_t)B * (p->n_coef ? p->n_coef : 1));
-		BALLOC(pxbuf, (size_t)B * 2 * D);
-		BALLOC(pcmax, B);
+	const int panels = f32 && jn_panel_batch_possible(&c, 1);
+	if (!panels) {
+		if (f32) { BALLOC(me32, (size_t)B * nme); BALLOC(x32, (size_t)B * D); }
+		else BALLOC(x64, (size_t)B * D);
+		BALLOC(gacc, (size_t)B * D);
+		BALLOC(ctrl, (size_t)2 * B);
 	}
 	/* matrix elements: FP64 for refinement, FP32 copies with the reference's
 	   |M| < 1e-12 skip of single-species blocks (matrix_vector_multiplication.c:52-53) */
@@ -745,17 +863,13 @@ extern "C" jn_status jn_lanczos_batch(jn_ctx *c, const jn_batch_options *o, jn_b
 		}
 	}
 	free(h32);
-	if (!st) st = cudaMemsetAsync(gacc, 0, (size_t)B * D * sizeof(unsigned long long), q) == cudaSuccess
-			      ? JN_OK : jn_fail(JN_ERR_CUDA, "accumulator clear");
+	if (!st && gacc && cudaMemsetAsync(gacc, 0, (size_t)B * D * sizeof(unsigned long long), q) != cudaSuccess)
+		st = jn_fail(JN_ERR_CUDA, "accumulator clear");
 	/* fixed-point scale bound valid for every instance */
 	const double abs_bound = jn_plan_abs_bound(p, NULL) * maxme;
-	if (!st && panels) st = jn_panels_batched_coefficients(c, B, me64, nme, pcoef, pcmax, q);
-	/* each instance gets about (resident CTAs) / B persistent CTAs */
-	jn_panel_partition part;
-	memset(&part, 0, sizeof part);
 	if (!st && panels) {
-		int g = c->num_sms * c->panel_per_sm[1] / B;
-		st = jn_panels_partition_upload(c, g < 8 ? 8 : g, &part);
+		if (cudaStreamSynchronize(q) != cudaSuccess) st = jn_fail(JN_ERR_CUDA, "upload of matrix elements");
+		if (!st) st = jn_panel_batch_create(&c, 1, &B, &me64, &pb);
 	}
 	int64_t *dims = (int64_t *)malloc(B * sizeof(int64_t));
 	jn_batch_result **rp = (jn_batch_result **)malloc(B * sizeof(jn_batch_result *));
@@ -763,27 +877,27 @@ extern "C" jn_status jn_lanczos_batch(jn_ctx *c, const jn_batch_options *o, jn_b
 	if (!st) {
 		batch_job job;
 		job.B = B;
+		job.num_sms = c->num_sms;
 		job.Dp = D;
 		job.dims = dims;
 		job.product = [&](const double *V, int64_t ldV, const int *d_k, double *W, const int *act, cudaStream_t qs) {
-			return panels ? jn_enqueue_panels_batched(c, B, pcoef, pcmax, V, ldV, d_k, D, W, D, pxbuf, gacc, ctrl, act,
-								  &part, qs)
-				      : jn_enqueue_batched(c, B, f32, f32 ? (const void *)me32 : (const void *)me64, nme, V, ldV,
-							   d_k, D, W, D, x64, x32, gacc, ctrl, act, abs_bound, qs);
+			return pb ? jn_panel_batch_enqueue(pb, V, ldV, d_k, D, W, D, act, D, qs)
+				  : jn_enqueue_batched(c, B, 1, f32, f32 ? (const void *)me32 : (const void *)me64, nme, V, ldV, 0, d_k, D, W,
+						       D, x64, x32, gacc, ctrl, act, abs_bound, qs);
 		};
-		job.product64 = [&](const double *X, int64_t ld, double *HX, double *scratch, cudaStream_t qs) {
-			return jn_enqueue_batched(c, B, 0, me64, nme, X, ld, NULL, 0, HX, ld, scratch, NULL, gacc, ctrl, NULL,
-						  abs_bound, qs);
+		job.product64 = [&](const double *X, int r, double *HX, cudaStream_t qs) {
+			return refine_products(c, B, me64, X, r, D, HX, abs_bound, qs);
 		};
+		if (pb) job.rebalance = [&](const int *act, int *changed) { return jn_panel_batch_rebalance(pb, act, changed); };
 		job.start_vectors = o->start_vectors;
 		job.eigenvectors = o->eigenvectors;
 		job.res = rp;
 		st = batch_solve(q, o, job);
 	}
 	free(dims); free(rp);
-	void *bufs[] = { me64, x64, me32, x32, gacc, pcmax, ctrl, pcoef, pxbuf };
+	jn_panel_batch_free(pb);
+	void *bufs[] = { me64, x64, me32, x32, gacc, ctrl };
 	for (size_t i = 0; i < sizeof bufs / sizeof bufs[0]; i++) cudaFree(bufs[i]);
-	jn_panels_partition_free(&part);
 	return st;
 }
 
@@ -838,17 +952,13 @@ extern "C" jn_status jn_lanczos_batch_bases(jn_ctx *const *ctxs, int num_bases, 
 			rp[i] = results[b] + j;
 		}
 	}
-	/* per basis: FP64 matrix elements on the device, the refinement's accumulators, the scale bound */
+	/* per basis: FP64 matrix elements on the device, the scale bound */
 	double **me64 = (double **)calloc(num_bases, sizeof(double *));
-	unsigned long long **gacc = (unsigned long long **)calloc(num_bases, sizeof(void *));
-	unsigned int **ctrl = (unsigned int **)calloc(num_bases, sizeof(void *));
 	double *bound = (double *)calloc(num_bases, sizeof(double));
 	for (int b = 0; b < num_bases && !st; b++) {
 		const jn_plan_t *p = &ctxs[b]->plan;
 		const int64_t nme = p->n_me;
 		BALLOC(me64[b], (size_t)count[b] * nme);
-		BALLOC(gacc[b], (size_t)count[b] * p->dim);
-		BALLOC(ctrl[b], (size_t)2 * count[b]);
 		double maxme = 0.0;
 		for (int j = 0; j < count[b] && !st; j++) {
 			const double *m = me[first[b] + j];
@@ -856,8 +966,6 @@ extern "C" jn_status jn_lanczos_batch_bases(jn_ctx *const *ctxs, int num_bases, 
 			if (cudaMemcpy(me64[b] + (size_t)j * nme, m, nme * sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess)
 				st = jn_fail(JN_ERR_CUDA, "upload of matrix elements");
 		}
-		if (!st && cudaMemset(gacc[b], 0, (size_t)count[b] * p->dim * sizeof(unsigned long long)) != cudaSuccess)
-			st = jn_fail(JN_ERR_CUDA, "accumulator clear");
 		bound[b] = jn_plan_abs_bound(p, NULL) * maxme;
 	}
 	/* the iteration products: one launch for every instance of every basis, on
@@ -875,6 +983,7 @@ extern "C" jn_status jn_lanczos_batch_bases(jn_ctx *const *ctxs, int num_bases, 
 		const int mode = o->precision == 32 ? 32 : 64;
 		batch_job job;
 		job.B = B;
+		job.num_sms = ctxs[0]->num_sms;
 		job.Dp = Dp;
 		job.dims = dims;
 		job.product = [&](const double *V, int64_t ldV, const int *d_k, double *W, const int *act, cudaStream_t qs) {
@@ -882,17 +991,15 @@ extern "C" jn_status jn_lanczos_batch_bases(jn_ctx *const *ctxs, int num_bases, 
 				  : jn_walk_batch_enqueue(wb, mode, V, ldV, d_k, Dp, W, Dp, act, Dp, qs);
 		};
 		/* refinement, basis by basis, on the block-tile engine in FP64 */
-		job.product64 = [&](const double *X, int64_t ld, double *HX, double *scratch, cudaStream_t qs) {
+		job.product64 = [&](const double *X, int r, double *HX, cudaStream_t qs) {
 			for (int b = 0; b < num_bases; b++) {
-				jn_ctx *c = ctxs[b];
-				const size_t i0 = (size_t)first[b];
-				jn_status e = jn_enqueue_batched(c, count[b], 0, me64[b], c->plan.n_me, X + i0 * ld, ld, NULL, 0,
-								 HX + i0 * ld, ld, scratch + i0 * Dp, NULL, gacc[b], ctrl[b], NULL,
-								 bound[b], qs);
+				const size_t at = (size_t)first[b] * r * Dp;
+				jn_status e = refine_products(ctxs[b], count[b], me64[b], X + at, r, Dp, HX + at, bound[b], qs);
 				if (e) return e;
 			}
 			return JN_OK;
 		};
+		if (pb) job.rebalance = [&](const int *act, int *changed) { return jn_panel_batch_rebalance(pb, act, changed); };
 		job.start_vectors = sv;
 		job.eigenvectors = ev;
 		job.res = rp;
@@ -900,12 +1007,8 @@ extern "C" jn_status jn_lanczos_batch_bases(jn_ctx *const *ctxs, int num_bases, 
 	}
 	jn_panel_batch_free(pb);
 	jn_walk_batch_free(wb);
-	for (int b = 0; b < num_bases; b++) {
-		cudaFree(me64[b]);
-		cudaFree(gacc[b]);
-		cudaFree(ctrl[b]);
-	}
-	free(me64); free(gacc); free(ctrl); free(bound);
+	for (int b = 0; b < num_bases; b++) cudaFree(me64[b]);
+	free(me64); free(bound);
 	free(ictx); free(count); free(first); free(dims); free(me); free(sv); free(ev); free(rp);
 	return st;
 }

@@ -102,16 +102,18 @@ jn_status jn_enqueue_tiles(jn_ctx *c, const double *d_x, double *d_y, int accumu
 			   cudaEvent_t pre, cudaEvent_t mid, unsigned long long *gacc, unsigned int *ctrl, float *x32,
 			   int clear_acc);
 
-/* B products at once, instance i = blockIdx.y: y[i] = H_i x_i with the
- * context's lists and the matrix elements me + i * me_ld (FP32 when f32),
- * x_i = src + i * src_ld + (*d_sel) * sel_ld (d_sel may be NULL).
+/* B products at once, product i = blockIdx.y: y_i = H x_i with the context's
+ * lists and the matrix elements me + (i / per) * me_ld (FP32 when f32): `per`
+ * products in a row share a Hamiltonian.  With h = i / per, v = i % per:
+ * x_i = src + h * src_ld + v * vec_ld + (*d_sel) * sel_ld (d_sel may be NULL)
+ * and y_i = y + h * y_ld + v * vec_ld.
  * Scratch: x64 or x32 (B x dim), gacc (B x dim, zero on entry, left zero),
- * ctrl (2 B words).  Instances with d_active[i] == 0 are skipped.  abs_bound
- * must bound every instance's matrix elements (jn_plan_abs_bound). */
-jn_status jn_enqueue_batched(jn_ctx *c, int B, int f32, const void *me, int64_t me_ld, const double *src,
-			     int64_t src_ld, const int *d_sel, int64_t sel_ld, double *y, int64_t y_ld, double *x64,
-			     float *x32, unsigned long long *gacc, unsigned int *ctrl, const int *d_active, double abs_bound,
-			     cudaStream_t st);
+ * ctrl (2 B words).  Products with d_active[i] == 0 are skipped.  abs_bound
+ * must bound every Hamiltonian's matrix elements (jn_plan_abs_bound). */
+jn_status jn_enqueue_batched(jn_ctx *c, int B, int per, int f32, const void *me, int64_t me_ld, const double *src,
+			     int64_t src_ld, int64_t vec_ld, const int *d_sel, int64_t sel_ld, double *y, int64_t y_ld,
+			     double *x64, float *x32, unsigned long long *gacc, unsigned int *ctrl, const int *d_active,
+			     double abs_bound, cudaStream_t st);
 
 /* max|x| into ctrl[0] (zeroed before) and the optional FP32 copy of x */
 void jn_launch_prep(const double *d_x, float *x32, int64_t n, unsigned int *ctrl, cudaStream_t st);
@@ -127,29 +129,6 @@ void jn_panels_invalidate(jn_ctx *c);
 void jn_panels_release(jn_ctx *c);
 jn_status jn_enqueue_panels(jn_ctx *c, const double *d_x, double *d_y, int accumulate, cudaStream_t st, cudaEvent_t pre,
 			    cudaEvent_t mid);
-
-/* batched panel products (jn_panel.cu): the 32-bit coefficients of B
- * instances' matrix elements (device, me + i me_ld, the context's layout)
- * into d_coef (B x n_coef) with their max|c| bits in d_cmax (B words); then
- * per step y_i = H_i x_i with x_i = src + i src_ld + (*d_sel) sel_ld.
- * Scratch: xbuf (B x 2 dim ints), gacc (B x dim, zero on entry, left zero),
- * ctrl (2 B words). */
-typedef struct {
-	int grid;               /* persistent CTAs per instance */
-	int words;              /* the largest CTA accumulator of the partition */
-	uint32_t *cta, *flush_ptr, *flush;      /* device copies of the partition */
-} jn_panel_partition;
-jn_status jn_panels_partition_upload(jn_ctx *c, int grid, jn_panel_partition *pp);
-void jn_panels_partition_free(jn_panel_partition *pp);
-jn_status jn_panels_batched_coefficients(jn_ctx *c, int B, const double *d_me, int64_t me_ld, int *d_coef,
-					 unsigned long long *d_cmax, cudaStream_t st);
-/* pp: the CTA partition of each instance (a batch gives each instance fewer,
- * larger chunks than a single product, so fewer blocks are cleared and
- * flushed); NULL for the context's own */
-jn_status jn_enqueue_panels_batched(jn_ctx *c, int B, const int *d_coef, const unsigned long long *d_cmax,
-				    const double *src, int64_t src_ld, const int *d_sel, int64_t sel_ld, double *y,
-				    int64_t y_ld, int *xbuf, unsigned long long *gacc, unsigned int *ctrl,
-				    const int *d_active, const jn_panel_partition *pp, cudaStream_t st);
 
 /* walk engine (jn_walk.cu): plan upload (built on first use), coefficient
  * reset after new matrix elements, release, and the product */
@@ -185,6 +164,11 @@ jn_status jn_panel_batch_create(jn_ctx *const *ctxs, int nbases, const int *coun
 jn_status jn_panel_batch_enqueue(struct jn_panel_batch *pb, const double *src, int64_t src_ld, const int *d_sel,
 				 int64_t sel_ld, double *y, int64_t y_ld, const int *d_active, int64_t max_dim,
 				 cudaStream_t st);
+/* After instances have converged: where the active ones (act, host) hold less
+ * than 0.6 of the work that the CTAs were shared out for, share them out
+ * anew; *changed: the next enqueue launches another grid.  The device must be
+ * idle. */
+jn_status jn_panel_batch_rebalance(struct jn_panel_batch *pb, const int *act, int *changed);
 void jn_panel_batch_free(struct jn_panel_batch *pb);
 
 /* release the Lanczos state of a context */

@@ -17,8 +17,9 @@
  *                         vector.c:461-476), convergence when the target
  *                         (ground-state) Ritz value moves by less than the
  *                         tolerance (lanczos.c:199-235).
- *   JN_LANCZOS_FULL       full reorthogonalisation (classical Gram-Schmidt,
- *                         applied twice) and convergence when the error
+ *   JN_LANCZOS_FULL       full reorthogonalisation (classical Gram-Schmidt
+ *                         after the recurrence, again where it cancels) and
+ *                         convergence when the error
  *                         bound min(r, r^2/gap) of each of the lowest `nev`
  *                         Ritz values is below the tolerance, r being the
  *                         residual norm beta_k |s_{k,i}|.
@@ -45,6 +46,7 @@
 #include <cooperative_groups.h>
 
 #include "jn_internal.h"
+#include "jn_ortho.cuh"
 #include "jn_tridiag.cuh"
 
 #define RED_BLOCKS 304      /* 2 x 152 SMs */
@@ -164,77 +166,14 @@ __global__ void k_axpy_neg(double *__restrict__ y, const double *__restrict__ x,
 /* ------------------------------------------------------------------ */
 /* full reorthogonalisation                                            */
 /* ------------------------------------------------------------------ */
-#define ORTHO_WARPS 8
-#define ORTHO_GROUP 16          /* vectors a warp sums at once in the dot products */
 #define ORTHO_H 1024            /* coefficients staged at a time in the subtraction */
-
-/* part[j G + blockIdx.x] = V_j . w over elements [i0, i1), j < nvec.  A warp
- * takes 16 vectors, its lanes the elements (coalesced rows of V), 16 sums in
- * registers; the sums are then folded across the lanes by halves, 16 adds
- * for the 16 vectors where a butterfly per vector takes 80 (GB300's FP64
- * pipe charges 64 cycles each).  With few vectors the warps share a group's
- * elements. */
-__device__ __forceinline__ void ortho_dots(const double *__restrict__ V, int64_t D, int nvec, const double *w, int64_t i0,
-					   int64_t i1, double *__restrict__ part, double (*ps)[ORTHO_WARPS / 2 * ORTHO_GROUP])
-{
-	const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-	const int ng = (nvec + ORTHO_GROUP - 1) / ORTHO_GROUP, split = ng < ORTHO_WARPS ? ORTHO_WARPS / ng : 1;
-	const int64_t sub = ((i1 - i0 + split - 1) / split + 31) & ~31ll;
-	for (int task = warp; task < ng * split; task += ORTHO_WARPS) {
-		const int g = task % ng, sp = task / ng, j0 = g * ORTHO_GROUP;
-		const int64_t e0 = i0 + sp * sub, e1 = min(i1, e0 + sub);
-		double acc[ORTHO_GROUP];
-#pragma unroll
-		for (int u = 0; u < ORTHO_GROUP; u++) acc[u] = 0.0;
-		const double *v = V + (int64_t)j0 * D;
-		if (j0 + ORTHO_GROUP <= nvec) {
-			for (int64_t e = e0 + lane; e < e1; e += 32) {
-				const double we = w[e];
-#pragma unroll
-				for (int u = 0; u < ORTHO_GROUP; u++) acc[u] = fma(v[u * D + e], we, acc[u]);
-			}
-		} else {
-			for (int64_t e = e0 + lane; e < e1; e += 32) {
-				const double we = w[e];
-#pragma unroll
-				for (int u = 0; u < ORTHO_GROUP; u++)
-					if (j0 + u < nvec) acc[u] = fma(v[u * D + e], we, acc[u]);
-			}
-		}
-#pragma unroll
-		for (int h = ORTHO_GROUP / 2; h; h >>= 1) {
-			const bool up = (lane & (2 * h)) != 0;
-#pragma unroll
-			for (int u = 0; u < h; u++) {
-				const double give = up ? acc[u] : acc[u + h], keep = up ? acc[u + h] : acc[u];
-				acc[u] = keep + __shfl_xor_sync(0xffffffffu, give, 2 * h);
-			}
-		}
-		acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], 1);
-		const int j = j0 + (lane >> 1);
-		if (!(lane & 1) && j < nvec) {
-			if (split > 1) ps[sp][j] = acc[0];
-			else part[(int64_t)j * gridDim.x + blockIdx.x] = acc[0];
-		}
-	}
-	if (split > 1) {
-		__syncthreads();
-		for (int j = threadIdx.x; j < nvec; j += blockDim.x) {
-			double s = ps[0][j];
-			for (int sp = 1; sp < split; sp++) s += ps[sp][j];
-			part[(int64_t)j * gridDim.x + blockIdx.x] = s;
-		}
-	}
-}
 
 /* h[j] = sum over the CTAs' partials of vector j, one warp of the grid per j */
 __device__ __forceinline__ void ortho_reduce(const double *part, int nvec, double *h)
 {
 	const int lane = threadIdx.x & 31;
 	for (int j = blockIdx.x * ORTHO_WARPS + (threadIdx.x >> 5); j < nvec; j += gridDim.x * ORTHO_WARPS) {
-		double s = 0.0;
-		for (int b = lane; b < (int)gridDim.x; b += 32) s += __ldcg(part + (int64_t)j * gridDim.x + b);
-		for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+		const double s = ortho_partials(part + (int64_t)j * gridDim.x, gridDim.x);
 		if (lane == 0) h[j] = s;
 	}
 }
@@ -281,59 +220,75 @@ __device__ __forceinline__ void ortho_subtract(const double *__restrict__ V, int
 
 /* One Lanczos step's vector work: from w = H v_k, with v_0 .. v_k the
  * orthonormal basis,
- *     h = V^T w;  w -= V h;  h' = V^T w;  w -= V h';
- *     alpha_k = h_k;  beta_k = |w|;  v_{k+1} = w / beta_k:
- * classical Gram-Schmidt twice over the whole basis, of which the first pass
- * holds the three-term recurrence.  A cooperative launch, one CTA an SM, a
- * slice of the vectors to each; the CTAs meet at five grid-wide barriers.
- * Bound by the FP64 pipe (4 multiply-adds per element and vector) and the
- * barriers: 34 us a step at D = 7 916, k = 25 to 125.  As thirteen kernels in
- * a row (dots, their sums, recurrence, two passes, norm, scaling) the same
- * work took 130 us at k = 45, most of it launches and a subtraction on 31
- * CTAs. */
+ *     alpha_k = <v_k|w>;  w -= alpha_k v_k + beta_{k-1} v_{k-1};
+ *     w -= V (V^T w);  beta_k = |w|;  v_{k+1} = w / beta_k.
+ * After the recurrence w is orthogonal to the basis but for rounding, so one
+ * Gram-Schmidt pass restores full orthogonality (max |V^T V - 1| 7e-16 over
+ * 200 steps, as with two passes) unless the pass took most of w away: |w|
+ * below 0.7 of what it was, which happens only when the Krylov space closes;
+ * then there is a second pass.  A cooperative launch, one CTA an SM, a slice
+ * of the vectors to each; the CTAs meet at four grid-wide barriers.  Bound by
+ * the barriers (1.1 us each) and the FP64 pipe (2 multiply-adds per element
+ * and vector): 31 us a step at D = 7 916, k = 25 to 125.  As thirteen
+ * kernels in a row, with two passes, the same work took 130 us at k = 45,
+ * most of it launches and a subtraction on 31 CTAs; with two passes in one
+ * launch, 34 us. */
 __global__ void __launch_bounds__(ORTHO_WARPS * 32)
 	k_orthonormalize(double *__restrict__ V, int64_t D, int64_t chunk, int k, double *w, double *part, double *h,
 			 double *__restrict__ alpha, double *__restrict__ beta)
 {
-	__shared__ double ps[ORTHO_WARPS][ORTHO_WARPS / 2 * ORTHO_GROUP];
+	__shared__ double ps[ORTHO_WARPS][ORTHO_SPLIT_VECTORS];
 	__shared__ double pt[ORTHO_WARPS][32];
 	__shared__ double hs[ORTHO_H];
+	__shared__ double sh[ORTHO_THREADS], word[4];
 	namespace cg = cooperative_groups;
 	cg::grid_group grid = cg::this_grid();
-	const int nvec = k + 1, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+	const int nvec = k + 1;
 	const int64_t i0 = (int64_t)blockIdx.x * chunk, i1 = min(D, i0 + chunk);
-	for (int pass = 0; pass < 2; pass++) {
-		ortho_dots(V, D, nvec, w, i0, i1, part, ps);
+	/* partial sums of alpha and, later, of |w|^2 after a pass; of |w|^2 before it */
+	double *pa = part + (int64_t)nvec * gridDim.x, *pb = pa + gridDim.x;
+	const double *vk = V + (int64_t)k * D, *u = k > 0 ? vk - D : vk;
+	double s = 0.0;
+	for (int64_t e = i0 + threadIdx.x; e < i1; e += blockDim.x) s = fma(vk[e], w[e], s);
+	s = ortho_cta_sum(s, sh);
+	if (threadIdx.x == 0) pa[blockIdx.x] = s;
+	grid.sync();
+	const double a = ortho_cta_partials(pa, gridDim.x, word), b0 = k > 0 ? beta[k - 1] : 0.0;
+	if (blockIdx.x == 0 && threadIdx.x == 0) alpha[k] = a;
+	s = 0.0;
+	for (int64_t e = i0 + threadIdx.x; e < i1; e += blockDim.x) {
+		double r = w[e] - a * vk[e];
+		if (k > 0) r -= b0 * u[e];
+		w[e] = r;
+		s = fma(r, r, s);
+	}
+	s = ortho_cta_sum(s, sh);       /* its barriers also publish w to the CTA */
+	if (threadIdx.x == 0) pb[blockIdx.x] = s;
+	double n2, n0 = 0.0;
+	for (int pass = 0;; pass++) {
+		ortho_dots(V, D, nvec, w, i0, i1, part + blockIdx.x, gridDim.x, ps);
 		grid.sync();
 		ortho_reduce(part, nvec, h);
+		if (pass == 0) n0 = ortho_cta_partials(pb, gridDim.x, word + 2);
 		grid.sync();
-		if (pass == 0 && blockIdx.x == 0 && threadIdx.x == 0) alpha[k] = __ldcg(h + k);
 		ortho_subtract(V, D, nvec, h, w, i0, i1, hs, pt);
-	}
-	/* the norm: every CTA adds the CTAs' partials in the same order */
-	double s = 0.0;
-	for (int64_t e = i0 + threadIdx.x; e < i1; e += blockDim.x) s = fma(w[e], w[e], s);
-	for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-	if (lane == 0) ps[0][warp] = s;
-	__syncthreads();
-	if (threadIdx.x == 0) {
-		s = ps[0][0];
-		for (int i = 1; i < ORTHO_WARPS; i++) s += ps[0][i];
-		part[blockIdx.x] = s;
-	}
-	grid.sync();
-	if (warp == 0) {
 		s = 0.0;
-		for (int b = lane; b < (int)gridDim.x; b += 32) s += __ldcg(part + b);
-		for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-		const double b = sqrt(s);
-		if (lane == 0) {
-			ps[1][0] = b > 0.0 ? 1.0 / b : 0.0;
-			if (blockIdx.x == 0) beta[k] = b;
-		}
+		for (int64_t e = i0 + threadIdx.x; e < i1; e += blockDim.x) s = fma(w[e], w[e], s);
+		s = ortho_cta_sum(s, sh);
+		if (threadIdx.x == 0) pa[blockIdx.x] = s;
+		grid.sync();
+		n2 = ortho_cta_partials(pa, gridDim.x, word + 1);
+		/* every CTA decides alike */
+		if (pass == 1 || n2 >= 0.49 * n0) break;
+		__syncthreads();
+	}
+	if (threadIdx.x == 0) {
+		const double b = sqrt(n2);
+		word[3] = b > 0.0 ? 1.0 / b : 0.0;
+		if (blockIdx.x == 0) beta[k] = b;
 	}
 	__syncthreads();
-	const double inv = ps[1][0];
+	const double inv = word[3];
 	double *v = V + (int64_t)(k + 1) * D;
 	for (int64_t e = i0 + threadIdx.x; e < i1; e += blockDim.x) v[e] = w[e] * inv;
 }
@@ -411,9 +366,9 @@ __global__ void __launch_bounds__(512) k_rayleigh(const double *__restrict__ X, 
  * the host: theta (want), the vectors' bottom components (nvec), beta_{n-1}.
  * The first `guesses` entries of theta hold an earlier check's eigenvalues.
  * Scratch: shared memory, or `work` (JN_TRI_VECTOR_DOUBLES(n) a CTA) above
- * JN_TRI_SMEM_ROWS rows.  Bound by the FP64 chains of one warp (about five
- * rounds of 3 n instructions, then 2 n for the vector, 64 cycles each): 125
- * us for 11 pairs at n = 25 to 125, where bisection, inverse iteration and
+ * JN_TRI_SMEM_ROWS rows.  Bound by the FP64 chains of a warp (about five
+ * rounds of 1.5 n instructions, then 2 n for the vector, 64 cycles each): 100
+ * us for 11 pairs at n = 25 to 125 (125 us with one warp to a count), where bisection, inverse iteration and
  * Gram-Schmidt as three kernels took 700 us at n = 45. */
 __global__ void __launch_bounds__(TRI_THREADS)
 	k_tri_check(const double *__restrict__ a, const double *__restrict__ b, int n, int want, int nvec,
@@ -421,16 +376,21 @@ __global__ void __launch_bounds__(TRI_THREADS)
 		    double *__restrict__ pack, int first, int guesses)
 {
 	extern __shared__ double sbuf[];
+	__shared__ jn_tri_exchange ex;
 	__shared__ unsigned int last;
 	const int i = first + blockIdx.x;
-	if (threadIdx.x < 32) {
-		double *as = work ? work + (size_t)blockIdx.x * JN_TRI_VECTOR_DOUBLES(n) : sbuf, *b2 = as + n;
-		double lo, hi;
-		const double sc = jn_tri_scale(a, b, n, &lo, &hi);
-		jn_tri_stage(a, b, n, sc, as, b2);
-		const double x = jn_tri_multisect_warp(as, b2, n, i, lo, hi, i < guesses, i < guesses ? theta[i] * sc : 0.0);
+	double *as = work ? work + (size_t)blockIdx.x * JN_TRI_VECTOR_DOUBLES(n) : sbuf, *b2 = as + n;
+	double lo, hi, sc = 0.0, guess = 0.0;
+	if (threadIdx.x < 64) {
+		sc = jn_tri_scale(a, b, n, &lo, &hi);
+		if (threadIdx.x < 32) jn_tri_stage(a, b, n, sc, as, b2);
+		if (i < guesses) guess = theta[i] * sc;
+	}
+	__syncthreads();
+	if (threadIdx.x < 64) {
+		const double x = jn_tri_multisect(as, b2, n, i, lo, hi, i < guesses, guess, &ex);
 		if (threadIdx.x == 0) theta[i] = x / sc;
-		if (i < nvec) jn_tri_vector_warp(as, b2, n, x, Z + (int64_t)i * ldz, b2 + n);
+		if (i < nvec && threadIdx.x < 32) jn_tri_vector_warp(as, b2, n, x, Z + (int64_t)i * ldz, b2 + n);
 	}
 	__syncthreads();
 	if (threadIdx.x == 0) {

@@ -250,18 +250,19 @@ __global__ void __launch_bounds__(TILE_THREADS) jn_tile_kernel(DevPlan P, const 
 							       const T *__restrict__ x, const T *__restrict__ me,
 							       unsigned long long *__restrict__ gacc,
 							       const unsigned int *__restrict__ xmax_bits, double abs_bound,
-							       int64_t inst_stride, int64_t me_stride,
+							       int64_t inst_stride, int64_t me_stride, int per,
 							       const int *__restrict__ active)
 {
 	extern __shared__ unsigned int sacc[];
 	__shared__ int next_item, cur_tile;
-	/* batched products: instance blockIdx.y owns x, me and gacc at its strides
+	/* batched products: product blockIdx.y owns x and gacc at their stride, `per`
+	   products in a row share matrix elements, and it has
 	   and the control words (max|x| bits, tile counter) at 2 * instance */
 	if (gridDim.y > 1 || active) {
 		const int inst = blockIdx.y;
 		if (active && !active[inst]) return;
 		x += inst * inst_stride;
-		me += inst * me_stride;
+		me += inst / per * me_stride;
 		gacc += inst * inst_stride;
 		tile_counter += 2 * inst;
 		xmax_bits += 2 * inst;
@@ -459,18 +460,20 @@ void jn_launch_finalize(unsigned long long *gacc, double *d_y, int64_t n, const 
 	if (n > 0) jn_finalize_kernel<<<g, 256, 0, st>>>(gacc, d_y, n, ctrl, abs_bound, accumulate);
 }
 
-/* Batched products (instance = blockIdx.y).  The source vector of instance
- * i is src + i * src_ld + (*sel) * sel_ld: the Lanczos vector v_k of a batched
- * solve, with k read on the device so that a captured graph can be replayed
- * at every step.  It is copied to x64 (FP64 products) or converted to x32
+/* Batched products (product i = blockIdx.y, `per` of them to a Hamiltonian).
+ * The source vector is src + (i / per) * src_ld + (i % per) * vec_ld +
+ * (*sel) * sel_ld: the Lanczos vector v_k of a batched solve (per = 1), with k
+ * read on the device so that a captured graph can be replayed at every step,
+ * or the Ritz vectors of its refinement.  It is copied to x64 (FP64 products) or converted to x32
  * (FP32 products); max|x| goes to ctrl[2 i]. */
-__global__ void jn_prep_batched_kernel(const double *__restrict__ src, int64_t src_ld, const int *__restrict__ sel,
+__global__ void jn_prep_batched_kernel(const double *__restrict__ src, int64_t src_ld, int64_t vec_ld, int per,
+				       const int *__restrict__ sel,
 				       int64_t sel_ld, double *__restrict__ x64, float *__restrict__ x32, int64_t n,
 				       unsigned int *__restrict__ ctrl, const int *__restrict__ active)
 {
 	const int inst = blockIdx.y;
 	if (active && !active[inst]) return;
-	const double *x = src + inst * src_ld + (sel ? (int64_t)(*sel) * sel_ld : 0);
+	const double *x = src + inst / per * src_ld + inst % per * vec_ld + (sel ? (int64_t)(*sel) * sel_ld : 0);
 	float m = 0.0f;
 	for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
 		const double v = x[i];
@@ -483,7 +486,8 @@ __global__ void jn_prep_batched_kernel(const double *__restrict__ src, int64_t s
 }
 
 __global__ void jn_finalize_batched_kernel(unsigned long long *__restrict__ gacc, double *__restrict__ y,
-					   int64_t y_ld, int64_t n, const unsigned int *__restrict__ ctrl, double abs_bound,
+					   int64_t y_ld, int64_t vec_ld, int per, int64_t n,
+					   const unsigned int *__restrict__ ctrl, double abs_bound,
 					   const int *__restrict__ active)
 {
 	const int inst = blockIdx.y;
@@ -491,7 +495,7 @@ __global__ void jn_finalize_batched_kernel(unsigned long long *__restrict__ gacc
 	const int S = fixed_exponent(ctrl[2 * inst], abs_bound);
 	const double unit = ldexp(1.0, -S);
 	unsigned long long *g = gacc + inst * n;
-	double *yy = y + inst * y_ld;
+	double *yy = y + inst / per * y_ld + inst % per * vec_ld;
 	for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
 		yy[i] = (double)(long long)g[i] * unit;
 		g[i] = 0ull;
@@ -677,11 +681,11 @@ jn_status jn_enqueue_tiles(jn_ctx *c, const double *d_x, double *d_y, int accumu
 		if (f32)
 			jn_tile_kernel<float><<<c->tile_grid, TILE_THREADS, smem, st>>>(
 				P, c->d_btiles, p->nbtiles, ctrl + 1, (const uint2 *)c->d_items, c->d_pieces, c->d_tterms,
-				c->d_walks, x32, c->d_me32, gacc, ctrl, p->abs_bound, 0, 0, NULL);
+				c->d_walks, x32, c->d_me32, gacc, ctrl, p->abs_bound, 0, 0, 1, NULL);
 		else
 			jn_tile_kernel<double><<<c->tile_grid, TILE_THREADS, smem, st>>>(
 				P, c->d_btiles, p->nbtiles, ctrl + 1, (const uint2 *)c->d_items, c->d_pieces, c->d_tterms,
-				c->d_walks, d_x, c->d_me, gacc, ctrl, p->abs_bound, 0, 0, NULL);
+				c->d_walks, d_x, c->d_me, gacc, ctrl, p->abs_bound, 0, 0, 1, NULL);
 	}
 	if (mid) cudaEventRecord(mid, st);
 	if (p->dim) jn_finalize_kernel<<<g, 256, 0, st>>>(gacc, d_y, p->dim, ctrl, p->abs_bound, accumulate);
@@ -690,10 +694,10 @@ jn_status jn_enqueue_tiles(jn_ctx *c, const double *d_x, double *d_y, int accumu
 	return JN_OK;
 }
 
-jn_status jn_enqueue_batched(jn_ctx *c, int B, int f32, const void *me, int64_t me_ld, const double *src,
-			     int64_t src_ld, const int *d_sel, int64_t sel_ld, double *y, int64_t y_ld, double *x64,
-			     float *x32, unsigned long long *gacc, unsigned int *ctrl, const int *d_active, double abs_bound,
-			     cudaStream_t st)
+jn_status jn_enqueue_batched(jn_ctx *c, int B, int per, int f32, const void *me, int64_t me_ld, const double *src,
+			     int64_t src_ld, int64_t vec_ld, const int *d_sel, int64_t sel_ld, double *y, int64_t y_ld,
+			     double *x64, float *x32, unsigned long long *gacc, unsigned int *ctrl, const int *d_active,
+			     double abs_bound, cudaStream_t st)
 {
 	const jn_plan_t *p = &c->plan;
 	if (B < 1 || B > 65535) return fail(JN_ERR_INVALID, "batch of %d instances", B);
@@ -709,19 +713,19 @@ jn_status jn_enqueue_batched(jn_ctx *c, int B, int f32, const void *me, int64_t 
 	cudaError_t e = cudaMemsetAsync(ctrl, 0, (size_t)2 * B * sizeof(unsigned int), st);
 	if (e != cudaSuccess) return fail(JN_ERR_CUDA, "cudaMemsetAsync: %s", cudaGetErrorString(e));
 	if (!p->dim) return JN_OK;
-	jn_prep_batched_kernel<<<dim3(g, B), 256, 0, st>>>(src, src_ld, d_sel, sel_ld, x64, f32 ? x32 : NULL, p->dim, ctrl,
+	jn_prep_batched_kernel<<<dim3(g, B), 256, 0, st>>>(src, src_ld, vec_ld, per, d_sel, sel_ld, x64, f32 ? x32 : NULL, p->dim, ctrl,
 							     d_active);
 	if (p->nbtiles) {
 		if (f32)
 			jn_tile_kernel<float><<<dim3(gx, B), TILE_THREADS, smem, st>>>(
 				P, c->d_btiles, p->nbtiles, ctrl + 1, (const uint2 *)c->d_items, c->d_pieces, c->d_tterms,
-				c->d_walks, x32, (const float *)me, gacc, ctrl, abs_bound, p->dim, me_ld, d_active);
+				c->d_walks, x32, (const float *)me, gacc, ctrl, abs_bound, p->dim, me_ld, per, d_active);
 		else
 			jn_tile_kernel<double><<<dim3(gx, B), TILE_THREADS, smem, st>>>(
 				P, c->d_btiles, p->nbtiles, ctrl + 1, (const uint2 *)c->d_items, c->d_pieces, c->d_tterms,
-				c->d_walks, x64, (const double *)me, gacc, ctrl, abs_bound, p->dim, me_ld, d_active);
+				c->d_walks, x64, (const double *)me, gacc, ctrl, abs_bound, p->dim, me_ld, per, d_active);
 	}
-	jn_finalize_batched_kernel<<<dim3(g, B), 256, 0, st>>>(gacc, y, y_ld, p->dim, ctrl, abs_bound, d_active);
+	jn_finalize_batched_kernel<<<dim3(g, B), 256, 0, st>>>(gacc, y, y_ld, vec_ld, per, p->dim, ctrl, abs_bound, d_active);
 	e = cudaGetLastError();
 	if (e != cudaSuccess) return fail(JN_ERR_CUDA, "batched product launch: %s", cudaGetErrorString(e));
 	return JN_OK;

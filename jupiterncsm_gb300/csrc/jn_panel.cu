@@ -27,6 +27,10 @@
  * touch few blocks, and at the end add only the touched ranges into the
  * global accumulator.
  */
+#include <algorithm>
+#include <utility>
+#include <vector>
+
 #include <cooperative_groups.h>
 
 #include "jn_internal.h"
@@ -164,6 +168,7 @@ __device__ __forceinline__ void panel_task(const uint4 pa, const uint4 pb, const
 	}
 }
 
+/* one CTA's run: cta_ptr and flush_ptr point at its own entries */
 template <typename T, typename Fix, bool XS>
 __device__ __forceinline__ void jn_panel_body(const uint4 *__restrict__ panels, const uint4 *__restrict__ tasks,
 					      const uint32_t *__restrict__ cta_ptr, const uint32_t *__restrict__ flush,
@@ -181,7 +186,7 @@ __device__ __forceinline__ void jn_panel_body(const uint4 *__restrict__ panels, 
 	unsigned int *lo = sacc, *hi = sacc + words, *bmap = sacc + (XS ? 3 : 2) * words;
 	T *xs = XS ? (T *)(sacc + 2 * words) : NULL;
 	const int lane = threadIdx.x & 31;
-	const uint32_t f0 = flush_ptr[blockIdx.x], f1 = flush_ptr[blockIdx.x + 1];
+	const uint32_t f0 = flush_ptr[0], f1 = flush_ptr[1];
 	/* clear the blocks this CTA touches (padded rows) */
 	for (uint32_t f = f0; f < f1; f++) {
 		const uint32_t b = __ldg(flush + 2 * f), so = __ldg(flush + 2 * f + 1);
@@ -199,7 +204,7 @@ __device__ __forceinline__ void jn_panel_body(const uint4 *__restrict__ panels, 
 	}
 	if (threadIdx.x == 0) next_task = 0;
 	__syncthreads();
-	const uint32_t t0 = cta_ptr[blockIdx.x], nt = cta_ptr[blockIdx.x + 1] - t0;
+	const uint32_t t0 = cta_ptr[0], nt = cta_ptr[1] - t0;
 	for (;;) {
 		uint32_t k = 0;
 		if (lane == 0) k = atomicAdd(&next_task, 1u);
@@ -241,10 +246,8 @@ __device__ __forceinline__ void jn_panel_body(const uint4 *__restrict__ panels, 
 }
 
 /* the 32-bit product: coefficients and x are 32-bit fixed-point integers.
- * Batched products (many Hamiltonians on one set of lists) run instance
- * blockIdx.y with its own coefficients, x and accumulator at the given
- * strides; instances with active[i] == 0 are skipped.  XS: x staged in
- * shared memory (one more word per state) instead of gathered through L1. */
+ * XS: x staged in shared memory (one more word per state) instead of
+ * gathered through L1. */
 template <bool XS>
 __global__ void __launch_bounds__(PANEL_THREADS, 3) jn_panel_kernel_i32(const uint4 *__restrict__ panels,
 								     const uint4 *__restrict__ tasks,
@@ -254,14 +257,10 @@ __global__ void __launch_bounds__(PANEL_THREADS, 3) jn_panel_kernel_i32(const ui
 								     const uint4 *__restrict__ blocks,
 								     const uint32_t *__restrict__ meta, const int *__restrict__ coef,
 								     const int *__restrict__ x, const int *__restrict__ xt,
-								     unsigned long long *__restrict__ gacc, const FixInt32 fix, int words,
-								     int64_t coef_ld, int64_t x_ld, int64_t acc_ld,
-								     const int *__restrict__ active)
+								     unsigned long long *__restrict__ gacc, const FixInt32 fix, int words)
 {
-	const int inst = blockIdx.y;
-	if (active && !active[inst]) return;
-	jn_panel_body<int, FixInt32, XS>(panels, tasks, cta_ptr, flush, flush_ptr, blocks, meta, coef + inst * coef_ld,
-					 x + inst * x_ld, xt + inst * x_ld, gacc + inst * acc_ld, fix, words);
+	jn_panel_body<int, FixInt32, XS>(panels, tasks, cta_ptr + blockIdx.x, flush, flush_ptr + blockIdx.x, blocks, meta, coef, x,
+					 xt, gacc, fix, words);
 }
 
 /* the FP64 product: the fixed-point scale 2^S comes from max|x| on the device */
@@ -278,7 +277,7 @@ __global__ void __launch_bounds__(PANEL_THREADS) jn_panel_kernel_fp64(const uint
 								      int words)
 {
 	const FixFp64 fix = { ldexp(1.0, fixed_exponent(*xmax_bits, abs_bound)) };
-	jn_panel_body<double, FixFp64, false>(panels, tasks, cta_ptr, flush, flush_ptr, blocks, meta, coef, x, xt, gacc, fix,
+	jn_panel_body<double, FixFp64, false>(panels, tasks, cta_ptr + blockIdx.x, flush, flush_ptr + blockIdx.x, blocks, meta, coef, x, xt, gacc, fix,
 					      words);
 }
 
@@ -630,7 +629,7 @@ static void panel_launch(const panel_sig_t *g, int has_tasks, int capturing)
 			(g->xs ? jn_panel_kernel_i32<true> : jn_panel_kernel_i32<false>)<<<g->grid, PANEL_THREADS, g->smem, st>>>(
 				(const uint4 *)g->panels, (const uint4 *)g->tasks, (const uint32_t *)g->cta, (const uint32_t *)g->flush,
 				(const uint32_t *)g->flush_ptr, blocks, (const uint32_t *)g->meta, (const int *)g->coef,
-				(const int *)g->xi, (const int *)g->xt, (unsigned long long *)g->gacc, fix, g->words, 0, 0, 0, NULL);
+				(const int *)g->xi, (const int *)g->xt, (unsigned long long *)g->gacc, fix, g->words);
 		} else {
 			jn_panel_kernel_fp64<<<g->grid, PANEL_THREADS, g->smem, st>>>(
 				(const uint4 *)g->panels, (const uint4 *)g->tasks, (const uint32_t *)g->cta, (const uint32_t *)g->flush,
@@ -969,7 +968,7 @@ __global__ void jn_coef_build_kernel(const uint32_t *__restrict__ gather, int64_
 	}
 }
 
-jn_status jn_panels_batched_coefficients(jn_ctx *c, int B, const double *d_me, int64_t me_ld, int *d_coef,
+static jn_status batched_coefficients(jn_ctx *c, int B, const double *d_me, int64_t me_ld, int *d_coef,
 					 unsigned long long *d_cmax, cudaStream_t st)
 {
 	const jn_plan_t *p = &c->plan;
@@ -982,113 +981,6 @@ jn_status jn_panels_batched_coefficients(jn_ctx *c, int B, const double *d_me, i
 		jn_coef_build_kernel<<<dim3(g, B), 256, 0, st>>>(c->d_pgather, p->n_coef, d_me, me_ld, d_cmax, d_coef,
 								   p->n_coef);
 	}
-	CUDA_TRY(cudaGetLastError());
-	return JN_OK;
-}
-
-/* instance blockIdx.y: max|x| of x_i = src + i src_ld + (*sel) sel_ld into ctrl[2 i] */
-__global__ void jn_xmax_batched_kernel(const double *__restrict__ src, int64_t src_ld, const int *__restrict__ sel,
-				       int64_t sel_ld, int64_t n, unsigned int *__restrict__ ctrl,
-				       const int *__restrict__ active)
-{
-	const int inst = blockIdx.y;
-	if (active && !active[inst]) return;
-	const double *x = src + inst * src_ld + (sel ? (int64_t)(*sel) * sel_ld : 0);
-	float m = 0.0f;
-	for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-		m = fmaxf(m, (float)fabs(x[i]) * 1.0000002f);
-	for (int o = 16; o; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-	if ((threadIdx.x & 31) == 0 && m > 0.0f) atomicMax(ctrl + 2 * inst, __float_as_uint(m));
-}
-
-/* block blockIdx.x of instance blockIdx.y: x_i as 32-bit fixed point, [p][n] and transposed [n][p] */
-__global__ void jn_panel_x_batched_kernel(const double *__restrict__ src, int64_t src_ld, const int *__restrict__ sel,
-					  int64_t sel_ld, int *__restrict__ xi, int64_t dim, const uint4 *__restrict__ blocks,
-					  const unsigned int *__restrict__ ctrl, const int *__restrict__ active)
-{
-	const int inst = blockIdx.y;
-	if (active && !active[inst]) return;
-	const double *x = src + inst * src_ld + (sel ? (int64_t)(*sel) * sel_ld : 0);
-	int *xn = xi + inst * 2 * dim, *xt = xn + dim;
-	const uint4 bk = blocks[blockIdx.x];
-	const uint32_t Np = bk.z, Nn = bk.w, n = Np * Nn;
-	const double s = ldexp(1.0, x_exponent(ctrl[2 * inst]));
-	for (uint32_t e = threadIdx.x; e < n; e += blockDim.x) {
-		const int t = __double2int_rn(x[bk.x + e] * s);
-		xn[bk.x + e] = t;
-		xt[bk.x + (e % Nn) * Np + e / Nn] = t;
-	}
-}
-
-/* y_i (=) acc_i 2^(30 - Sc_i - Sx_i); the accumulator is cleared */
-__global__ void jn_int_finalize_batched_kernel(unsigned long long *__restrict__ gacc, double *__restrict__ y, int64_t y_ld,
-					       int64_t n, const unsigned int *__restrict__ ctrl,
-					       const unsigned long long *__restrict__ cmax, const int *__restrict__ active)
-{
-	const int inst = blockIdx.y;
-	if (active && !active[inst]) return;
-	const double unit = ldexp(1.0, PANEL_INT_SHIFT - coef_exponent(cmax[inst]) - x_exponent(ctrl[2 * inst]));
-	unsigned long long *g = gacc + inst * n;
-	double *yy = y + inst * y_ld;
-	for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-		yy[i] = (double)(long long)g[i] * unit;
-		g[i] = 0ull;
-	}
-}
-
-jn_status jn_panels_partition_upload(jn_ctx *c, int grid, jn_panel_partition *pp)
-{
-	memset(pp, 0, sizeof *pp);
-	jn_status s = jn_panels_setup(c);
-	if (s) return s;
-	uint32_t *cta = NULL, *fptr = NULL, *flush = NULL;
-	int64_t nf = 0, words = 0;
-	if (jn_panels_partition(&c->plan, grid, &cta, &fptr, &flush, &nf, &words))
-		return jn_fail(JN_ERR_NOMEM, "out of host memory");
-	pp->words = (int)words;
-	if ((s = upload_n(&pp->cta, cta, (size_t)grid + 1)) || (s = upload_n(&pp->flush_ptr, fptr, (size_t)grid + 1)) ||
-	    (s = upload_n(&pp->flush, flush, (size_t)nf * 2)))
-		jn_panels_partition_free(pp);
-	else
-		pp->grid = grid;
-	free(cta); free(fptr); free(flush);
-	return s;
-}
-
-void jn_panels_partition_free(jn_panel_partition *pp)
-{
-	cudaFree(pp->cta); cudaFree(pp->flush_ptr); cudaFree(pp->flush);
-	memset(pp, 0, sizeof *pp);
-}
-
-jn_status jn_enqueue_panels_batched(jn_ctx *c, int B, const int *d_coef, const unsigned long long *d_cmax,
-				    const double *src, int64_t src_ld, const int *d_sel, int64_t sel_ld, double *y,
-				    int64_t y_ld, int *xbuf, unsigned long long *gacc, unsigned int *ctrl,
-				    const int *d_active, const jn_panel_partition *pp, cudaStream_t st)
-{
-	const jn_plan_t *p = &c->plan;
-	if (!jn_panels_fit(c, 1)) return jn_fail(JN_ERR_INVALID, "the panel engine is not set up for this context");
-	if (B < 1 || B > 65535) return jn_fail(JN_ERR_INVALID, "batch of %d instances", B);
-	if (!p->dim) return JN_OK;
-	int g = (int)((p->dim + 255) / 256);
-	if (g > 256) g = 256;
-	CUDA_TRY(cudaMemsetAsync(ctrl, 0, (size_t)2 * B * sizeof(unsigned int), st));
-	jn_xmax_batched_kernel<<<dim3(g, B), 256, 0, st>>>(src, src_ld, d_sel, sel_ld, p->dim, ctrl, d_active);
-	jn_panel_x_batched_kernel<<<dim3(p->nblocks, B), 256, 0, st>>>(src, src_ld, d_sel, sel_ld, xbuf, p->dim,
-									 (const uint4 *)c->d_pblocks, ctrl, d_active);
-	if (p->nptasks) {
-		const FixInt32 fix = {};
-		const int grid = pp ? pp->grid : c->panel_grid;
-		const int64_t words = pp ? pp->words : p->pcta_words;
-		const int xs = panel_use_xs(c, words, panel_per_sm_of(c, grid));
-		(xs ? jn_panel_kernel_i32<true> : jn_panel_kernel_i32<false>)<<<dim3(grid, B), PANEL_THREADS,
-									      panel_smem_words(p, words, xs), st>>>(
-			(const uint4 *)c->d_panels, (const uint4 *)c->d_ptasks, pp ? pp->cta : c->d_pcta,
-			pp ? pp->flush : c->d_pflush, pp ? pp->flush_ptr : c->d_pflush_ptr,
-			(const uint4 *)c->d_pblocks, c->d_pmeta, d_coef, xbuf, xbuf + p->dim, gacc, fix, (int)words,
-			p->n_coef, 2 * p->dim, p->dim, d_active);
-	}
-	jn_int_finalize_batched_kernel<<<dim3(g, B), 256, 0, st>>>(gacc, y, y_ld, p->dim, ctrl, d_cmax, d_active);
 	CUDA_TRY(cudaGetLastError());
 	return JN_OK;
 }
@@ -1114,27 +1006,39 @@ struct jn_panel_inst {
 };
 static_assert(sizeof(jn_panel_inst) == 112, "one descriptor is 112 bytes");
 
-struct jn_panel_batch {
-	int B;
-	jn_panel_inst *h, *d;
-	unsigned int *d_ctrl;           /* max|x| bits of instance i at 2 i */
-	int max_grid, max_blocks;
-	size_t smem;
-	jn_panel_partition *parts;      /* one per basis */
-	int nbases;
+/* the device copies of a basis's CTA partition */
+struct panel_part {
+	uint32_t *cta, *flush_ptr, *flush;
 };
 
-/* instance blockIdx.y; CTAs beyond the instance's grid have no work */
-__global__ void __launch_bounds__(PANEL_THREADS, 3)
-	jn_panel_multi_kernel(const jn_panel_inst *__restrict__ I, const int *__restrict__ active)
+typedef void (*panel_multi_t)(const jn_panel_inst *, const int2 *, const int *);
+
+struct jn_panel_batch {
+	int B, nbases;
+	jn_ctx **ctxs;                  /* per basis */
+	int *basis;                     /* per instance: its basis */
+	jn_panel_inst *h, *d;
+	panel_part *parts;              /* one per basis */
+	int2 *d_list;                   /* the product's CTAs {instance, chunk}, most work first */
+	int nlist, threads;
+	size_t smem;
+	panel_multi_t kernel;
+	double work;                    /* coefficients of the instances the partition was made for */
+	unsigned int *d_ctrl;           /* max|x| bits of instance i at 2 i */
+	int max_blocks;
+};
+
+/* CTA c of the launch runs chunk list[c].y of instance list[c].x */
+template <int THREADS, int PER_SM, bool XS>
+__global__ void __launch_bounds__(THREADS, PER_SM)
+	jn_panel_multi_kernel(const jn_panel_inst *__restrict__ I, const int2 *__restrict__ list, const int *__restrict__ active)
 {
-	const int inst = blockIdx.y;
+	const int inst = list[blockIdx.x].x, chunk = list[blockIdx.x].y;
 	if (active && !active[inst]) return;
 	const jn_panel_inst d = I[inst];
-	if ((int)blockIdx.x >= d.grid) return;
 	const FixInt32 fix = {};
-	jn_panel_body<int, FixInt32, false>(d.panels, d.tasks, d.cta, d.flush, d.flush_ptr, d.blocks, d.meta, d.coef, d.xi,
-					    d.xi + d.dim, d.gacc, fix, d.words);
+	jn_panel_body<int, FixInt32, XS>(d.panels, d.tasks, d.cta + chunk, d.flush, d.flush_ptr + chunk, d.blocks, d.meta, d.coef,
+					 d.xi, d.xi + d.dim, d.gacc, fix, d.words);
 }
 
 __global__ void jn_panel_multi_xmax_kernel(const jn_panel_inst *__restrict__ I, const double *__restrict__ src,
@@ -1188,6 +1092,12 @@ __global__ void jn_panel_multi_finalize_kernel(const jn_panel_inst *__restrict__
 	}
 }
 
+static void panel_part_free(panel_part *pp)
+{
+	cudaFree(pp->cta); cudaFree(pp->flush_ptr); cudaFree(pp->flush);
+	memset(pp, 0, sizeof *pp);
+}
+
 void jn_panel_batch_free(jn_panel_batch *pb)
 {
 	if (!pb) return;
@@ -1201,10 +1111,13 @@ void jn_panel_batch_free(jn_panel_batch *pb)
 			cudaFree(pb->h[i].gacc);
 		}
 	if (pb->parts)
-		for (int b = 0; b < pb->nbases; b++) jn_panels_partition_free(&pb->parts[b]);
+		for (int b = 0; b < pb->nbases; b++) panel_part_free(&pb->parts[b]);
 	free(pb->parts);
+	free(pb->ctxs);
+	free(pb->basis);
 	free(pb->h);
 	cudaFree(pb->d);
+	cudaFree(pb->d_list);
 	cudaFree(pb->d_ctrl);
 	free(pb);
 }
@@ -1219,6 +1132,117 @@ int jn_panel_batch_possible(jn_ctx *const *ctxs, int nbases)
 	return 1;
 }
 
+/* Share the GPU's CTAs out among the active instances (NULL: all) by their
+ * coefficients: the product's CTA list, the kernel that runs it, and the
+ * descriptors.  Two shapes of CTA.  512 threads, three to an SM, where three
+ * accumulators with x staged beside them fit an SM (small bases); else 1 024
+ * threads, one to an SM, x staged where that fits.  With 512 threads and a
+ * large accumulator an SM holds one CTA of 16 warps: 64 Hamiltonians on
+ * 4He Nmax 2, 4, 6 and 6Li Nmax 4 take 690 us a product that way, 410 us with
+ * 1 024 threads.  One round of CTAs: two rounds clear and flush every
+ * accumulator twice as often (+1.5 % of the whole solve, three +6 %).  The
+ * result does not depend on the partition. */
+static jn_status panel_batch_partition(jn_panel_batch *pb, const int *act)
+{
+	const int sms = pb->ctxs[0]->num_sms;
+	std::vector<int> count(pb->nbases, 0), g(pb->nbases, 0);
+	double work = 0.0;
+	for (int i = 0; i < pb->B; i++)
+		if (!act || act[i]) {
+			const int64_t nc = pb->ctxs[pb->basis[i]]->plan.n_coef;
+			count[pb->basis[i]]++;
+			work += (double)(nc ? nc : 1);
+		}
+	int optin = 0, xs = 0;
+	CUDA_TRY(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, pb->ctxs[0]->device));
+	struct host_part {
+		uint32_t *cta, *fptr, *flush;
+		int64_t nf, words;
+	};
+	std::vector<host_part> hp(pb->nbases);
+	auto release = [&]() {
+		for (auto &q : hp) {
+			free(q.cta); free(q.fptr); free(q.flush);
+			memset(&q, 0, sizeof q);
+		}
+	};
+	size_t smem = 0;
+	for (int shape = 0; shape < 2; shape++) {
+		const int per = shape == 0 ? 3 : 1;
+		size_t with = 0, without = 0;
+		release();
+		for (int b = 0; b < pb->nbases; b++) {
+			if (!count[b]) continue;
+			const jn_plan_t *p = &pb->ctxs[b]->plan;
+			g[b] = (int)(per * sms * (double)(p->n_coef ? p->n_coef : 1) / work);
+			if (g[b] < 1) g[b] = 1;
+			if (jn_panels_partition(p, g[b], &hp[b].cta, &hp[b].fptr, &hp[b].flush, &hp[b].nf, &hp[b].words)) {
+				release();
+				return jn_fail(JN_ERR_NOMEM, "out of host memory");
+			}
+			with = std::max(with, panel_smem_words(p, hp[b].words, 1));
+			without = std::max(without, panel_smem_words(p, hp[b].words, 0));
+		}
+		pb->threads = shape == 0 ? 512 : 1024;
+		xs = shape == 0 || with + 1024 <= (size_t)optin;
+		smem = xs ? with : without;
+		pb->kernel = shape == 0 ? jn_panel_multi_kernel<512, 3, true> : xs ? jn_panel_multi_kernel<1024, 1, true>
+										      : jn_panel_multi_kernel<1024, 1, false>;
+		if (shape == 0 && 3 * (with + 1024) <= (size_t)pb->ctxs[0]->smem_per_sm) break;
+	}
+	jn_status s = JN_OK;
+	for (int b = 0; b < pb->nbases && !s; b++) {
+		panel_part_free(&pb->parts[b]);
+		if (!count[b]) continue;
+		if ((s = upload_n(&pb->parts[b].cta, hp[b].cta, (size_t)g[b] + 1)) ||
+		    (s = upload_n(&pb->parts[b].flush_ptr, hp[b].fptr, (size_t)g[b] + 1)) ||
+		    (s = upload_n(&pb->parts[b].flush, hp[b].flush, (size_t)hp[b].nf * 2)))
+			break;
+	}
+	std::vector<std::pair<double, int2>> cl;
+	for (int i = 0; i < pb->B && !s; i++) {
+		const int b = pb->basis[i];
+		if (act && !act[i]) continue;
+		pb->h[i].cta = pb->parts[b].cta;
+		pb->h[i].flush_ptr = pb->parts[b].flush_ptr;
+		pb->h[i].flush = pb->parts[b].flush;
+		pb->h[i].grid = g[b];
+		pb->h[i].words = (int)hp[b].words;
+		for (int k = 0; k < g[b]; k++) cl.push_back({ (double)pb->ctxs[b]->plan.n_coef / g[b], make_int2(i, k) });
+	}
+	release();
+	if (s) return s;
+	std::stable_sort(cl.begin(), cl.end(), [](const std::pair<double, int2> &x, const std::pair<double, int2> &y) { return x.first > y.first; });
+	std::vector<int2> list;
+	for (auto &e : cl) list.push_back(e.second);
+	cudaFree(pb->d_list);
+	pb->d_list = NULL;
+	if ((s = upload_n(&pb->d_list, list.data(), list.size()))) return s;
+	pb->nlist = (int)list.size();
+	pb->smem = smem;
+	pb->work = work;
+	CUDA_TRY(cudaMemcpy(pb->d, pb->h, (size_t)pb->B * sizeof(jn_panel_inst), cudaMemcpyHostToDevice));
+	/* the attribute is the kernel's, shared by every batch of the process: at least what an SM gives beside the
+	   kernel's own few words */
+	CUDA_TRY(cudaFuncSetAttribute((const void *)pb->kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+				      (int)std::max(smem, (size_t)optin - 1024)));
+	CUDA_TRY(cudaDeviceSynchronize());
+	return JN_OK;
+}
+
+jn_status jn_panel_batch_rebalance(jn_panel_batch *pb, const int *act, int *changed)
+{
+	*changed = 0;
+	double work = 0.0;
+	for (int i = 0; i < pb->B; i++) {
+		const int64_t nc = pb->ctxs[pb->basis[i]]->plan.n_coef;
+		if (act[i]) work += (double)(nc ? nc : 1);
+	}
+	if (!(work > 0.0) || work > 0.6 * pb->work) return JN_OK;
+	*changed = 1;
+	return panel_batch_partition(pb, act);
+}
+
 jn_status jn_panel_batch_create(jn_ctx *const *ctxs, int nbases, const int *count, const double *const *d_me64,
 				jn_panel_batch **out)
 {
@@ -1231,22 +1255,15 @@ jn_status jn_panel_batch_create(jn_ctx *const *ctxs, int nbases, const int *coun
 	pb->B = B;
 	pb->nbases = nbases;
 	pb->h = (jn_panel_inst *)calloc((size_t)B, sizeof(jn_panel_inst));
-	pb->parts = (jn_panel_partition *)calloc((size_t)nbases, sizeof(jn_panel_partition));
-	jn_status s = (!pb->h || !pb->parts) ? jn_fail(JN_ERR_NOMEM, "out of host memory") : JN_OK;
-	/* CTAs: the resident CTAs of the 32-bit kernel shared out by each instance's coefficients */
-	double work = 0.0;
-	for (int b = 0; b < nbases && !s; b++) {
-		if ((s = jn_panels_setup(ctxs[b]))) break;
-		work += (double)count[b] * (double)(ctxs[b]->plan.n_coef ? ctxs[b]->plan.n_coef : 1);
-	}
-	const int resident = !s ? ctxs[0]->num_sms * ctxs[0]->panel_per_sm[1] : 0;
+	pb->parts = (panel_part *)calloc((size_t)nbases, sizeof(panel_part));
+	pb->ctxs = (jn_ctx **)calloc((size_t)nbases, sizeof(jn_ctx *));
+	pb->basis = (int *)calloc((size_t)B, sizeof(int));
+	jn_status s = (!pb->h || !pb->parts || !pb->ctxs || !pb->basis) ? jn_fail(JN_ERR_NOMEM, "out of host memory") : JN_OK;
 	for (int b = 0, i0 = 0; b < nbases && !s; i0 += count[b], b++) {
 		jn_ctx *c = ctxs[b];
+		pb->ctxs[b] = c;
+		if ((s = jn_panels_setup(c))) break;
 		const jn_plan_t *p = &c->plan;
-		int g = (int)(resident * (double)(p->n_coef ? p->n_coef : 1) / work);
-		if (g < 8) g = 8;
-		if ((s = jn_panels_partition_upload(c, g, &pb->parts[b]))) break;
-		const jn_panel_partition *pp = &pb->parts[b];
 		int *coef = NULL;
 		unsigned long long *cmax = NULL;
 		const int64_t nc = p->n_coef ? p->n_coef : 1;
@@ -1257,21 +1274,17 @@ jn_status jn_panel_batch_create(jn_ctx *const *ctxs, int nbases, const int *coun
 			break;
 		}
 		pb->h[i0].owner = 1;
-		s = jn_panels_batched_coefficients(c, count[b], d_me64[b], p->n_me, coef, cmax, c->stream);
+		s = batched_coefficients(c, count[b], d_me64[b], p->n_me, coef, cmax, c->stream);
 		for (int j = 0; j < count[b]; j++) {
 			jn_panel_inst *d = &pb->h[i0 + j];
+			pb->basis[i0 + j] = b;
 			d->coef = coef + (size_t)j * nc;
 			d->cmax = cmax + j;
 			d->panels = (const uint4 *)c->d_panels;
 			d->tasks = (const uint4 *)c->d_ptasks;
-			d->cta = pp->cta;
-			d->flush = pp->flush;
-			d->flush_ptr = pp->flush_ptr;
 			d->blocks = (const uint4 *)c->d_pblocks;
 			d->meta = c->d_pmeta;
 			d->dim = p->dim;
-			d->grid = pp->grid;
-			d->words = pp->words;
 			d->nblocks = p->nblocks;
 		}
 		if (s) break;
@@ -1282,21 +1295,12 @@ jn_status jn_panel_batch_create(jn_ctx *const *ctxs, int nbases, const int *coun
 			    cudaMemset(d->gacc, 0, (size_t)(p->dim ? p->dim : 1) * sizeof(unsigned long long)) != cudaSuccess)
 				s = jn_fail(JN_ERR_NOMEM, "cudaMalloc of batched panel buffers failed");
 		}
-		const size_t sm = panel_smem_words(p, pp->words, 0);
-		if (sm > pb->smem) pb->smem = sm;
-		if (pp->grid > pb->max_grid) pb->max_grid = pp->grid;
 		if (p->nblocks > pb->max_blocks) pb->max_blocks = p->nblocks;
 	}
 	if (!s && (cudaMalloc((void **)&pb->d, (size_t)B * sizeof(jn_panel_inst)) != cudaSuccess ||
 		   cudaMalloc((void **)&pb->d_ctrl, (size_t)2 * B * sizeof(unsigned int)) != cudaSuccess))
 		s = jn_fail(JN_ERR_NOMEM, "cudaMalloc of the batch descriptors failed");
-	if (!s && cudaMemcpy(pb->d, pb->h, (size_t)B * sizeof(jn_panel_inst), cudaMemcpyHostToDevice) != cudaSuccess)
-		s = jn_fail(JN_ERR_CUDA, "upload of the batch descriptors failed");
-	if (!s) {
-		cudaError_t e = cudaFuncSetAttribute(jn_panel_multi_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pb->smem);
-		if (e == cudaSuccess) e = cudaDeviceSynchronize();
-		if (e != cudaSuccess) s = jn_fail(JN_ERR_CUDA, "batched panel set-up: %s", cudaGetErrorString(e));
-	}
+	if (!s) s = panel_batch_partition(pb, NULL);
 	if (s) {
 		jn_panel_batch_free(pb);
 		return s;
@@ -1316,7 +1320,7 @@ jn_status jn_panel_batch_enqueue(jn_panel_batch *pb, const double *src, int64_t 
 	jn_panel_multi_xmax_kernel<<<dim3(g, B), 256, 0, st>>>(pb->d, src, src_ld, d_sel, sel_ld, pb->d_ctrl, d_active);
 	jn_panel_multi_x_kernel<<<dim3(pb->max_blocks > 0 ? pb->max_blocks : 1, B), 256, 0, st>>>(pb->d, src, src_ld, d_sel,
 												      sel_ld, pb->d_ctrl, d_active);
-	jn_panel_multi_kernel<<<dim3(pb->max_grid, B), PANEL_THREADS, pb->smem, st>>>(pb->d, d_active);
+	pb->kernel<<<pb->nlist, pb->threads, pb->smem, st>>>(pb->d, pb->d_list, d_active);
 	jn_panel_multi_finalize_kernel<<<dim3(g, B), 256, 0, st>>>(pb->d, y, y_ld, pb->d_ctrl, d_active);
 	CUDA_TRY(cudaGetLastError());
 	return JN_OK;

@@ -12,7 +12,8 @@
  * Sturm counts come from the leading principal minors
  *     p_i = (a_i - x) p_{i-1} - b_{i-1}^2 p_{i-2}
  * (three FP64 instructions a step; the exponents are kept in range by integer
- * work every eighth step), and an eigenvector from the leading and trailing
+ * work every eighth step), taken from both ends of the matrix at once by two
+ * warps, and an eigenvector from the leading and trailing
  * minors at the eigenvalue, joined where their product is largest (the
  * twisted factorisation, in minors instead of quotients).  The quotient form
  * of the counts and inverse iteration by an LU factorisation with divisions
@@ -88,35 +89,73 @@ __device__ __forceinline__ void jn_tri_stage(const double *a, const double *b, i
 	__syncwarp();
 }
 
-/* number of eigenvalues below x: sign changes of the leading minors; pm 2^pe
- * is the last one (det(T - x)) */
-__device__ __forceinline__ int jn_sturm_count(const double *as, const double *b2, int n, double x, double *pm, int *pe)
+/* one end's minors of T - x: the last two (times 2^e), the sign changes up to
+ * the last, and the signs of the last two (bit 0 and 1; a zero minor takes
+ * its predecessor's sign) */
+struct jn_minors {
+	double last, prev;
+	int e, changes, signs;
+};
+
+/* what the two warps of a pair exchange in a round */
+struct jn_tri_exchange {
+	jn_minors m[2][2][32];          /* [round parity][warp][lane] */
+};
+
+__device__ __forceinline__ int jn_sign_or(double v, int s) { return ((__double2hiint(v) << 1) | __double2loint(v)) != 0 ? (__double2hiint(v) >> 31) & 1 : s; }
+
+/* `steps` minors from row `row` in direction dir (1: leading, -1: trailing) */
+__device__ __forceinline__ jn_minors jn_minor_chain(const double *as, const double *b2, int row, int dir, int steps, double x)
 {
-	double p2 = 1.0, p1 = as[0] - x;
-	int e = 0, c = 0, s = 0;
-	/* a zero minor takes its predecessor's sign */
-	if (((__double2hiint(p1) << 1) | __double2loint(p1)) != 0) s = __double2hiint(p1) >> 31;
-	c -= s;
-	for (int i = 1; i < n;) {
-		const int stop = min(n, i + 8);
+	jn_minors r = { 1.0, 0.0, 0, 0, 0 };
+	int s = 0, sp = 0;
+	double p2 = 0.0, p1 = 1.0;
+	/* the coupling to the row before: b2[row - 1] going down, b2[row] going up */
+	const double *a = as + row, *c = b2 + (dir > 0 ? row - 1 : row);
+	for (int i = 0; i < steps;) {
+		const int stop = min(steps, i + 8);
 		for (; i < stop; i++) {
-			const double p = fma(as[i] - x, p1, -(b2[i - 1] * p2));
-			const int sp = ((__double2hiint(p) << 1) | __double2loint(p)) != 0 ? __double2hiint(p) >> 31 : s;
-			c += (sp ^ s) & 1;
-			s = sp;
+			const double p = fma(a[i * dir] - x, p1, i > 0 ? -(c[i * dir] * p2) : 0.0);
+			sp = s;
+			s = jn_sign_or(p, s);
+			r.changes += s ^ sp;
 			p2 = p1;
 			p1 = p;
 		}
-		e += jn_rescale(p1, p2);
+		r.e += jn_rescale(p1, p2);
 	}
-	*pm = p1;
-	*pe = e;
-	return c;
+	r.last = p1;
+	r.prev = p2;
+	r.signs = s | (sp << 1);
+	return r;
+}
+
+/* Number of eigenvalues below x, by two warps w = 0, 1 (the same x on lane l
+ * of both): warp 0 takes the leading minors of rows 0 .. m-1, warp 1 the
+ * trailing ones of rows n-1 .. m, half of the chain each, and both put them
+ * together: eliminating rows 0 .. m-2 from the top and n-1 .. m from the
+ * bottom leaves the pivot det / (p_{m-1} q_m) in row m-1.  pm 2^pe is
+ * det(T - x). */
+__device__ __forceinline__ int jn_sturm_count(const double *as, const double *b2, int n, double x, jn_tri_exchange *ex, int round,
+					      double *pm, int *pe)
+{
+	const int w = (threadIdx.x >> 5) & 1, lane = threadIdx.x & 31, m = (n + 1) / 2;
+	const jn_minors mine = w == 0 ? jn_minor_chain(as, b2, 0, 1, m, x) : jn_minor_chain(as, b2, n - 1, -1, n - m, x);
+	ex->m[round & 1][w][lane] = mine;
+	asm volatile("bar.sync 1, 64;" ::: "memory");
+	const jn_minors p = ex->m[round & 1][0][lane], q = ex->m[round & 1][1][lane];
+	/* b2[m-1] couples the halves (0 when there is one row); q.prev is 0 when the lower half is empty */
+	const double det = fma(p.last, q.last, -(b2[m - 1] * (p.prev * q.prev)));
+	const int sp = p.signs >> 1, sq = q.signs & 1, sd = jn_sign_or(det, sp ^ sq);
+	*pm = det;
+	*pe = p.e + q.e;
+	return p.changes - ((p.signs ^ (p.signs >> 1)) & 1) + q.changes + (sd ^ sp ^ sq);
 }
 
 /* The i-th smallest eigenvalue of the staged matrix (in its units) by
- * multisection, one warp: each round the 32 lanes count at 32 points of the
- * bracket [lo, hi].  Points are equidistant until the bracket holds this
+ * multisection, two warps (see jn_sturm_count; both must call): each round
+ * the lanes count at 32 points of the bracket [lo, hi].  Points are
+ * equidistant until the bracket holds this
  * eigenvalue alone and det(T - x) is known at both its ends; then they lie
  * at geometric distances around the secant estimate, whose error shrinks
  * quadratically: 6 to 8 rounds in all, where equidistant points take 11.
@@ -124,8 +163,8 @@ __device__ __forceinline__ int jn_sturm_count(const double *as, const double *b2
  * the estimate's place in the first round.  The counts alone decide the
  * bracket, so a poor estimate costs a round and nothing else.  It ends at
  * 2^-54 of the span.  Every lane returns the same value. */
-__device__ __forceinline__ double jn_tri_multisect_warp(const double *as, const double *b2, int n, int i, double lo, double hi,
-							 bool guessed, double guess)
+__device__ __forceinline__ double jn_tri_multisect(const double *as, const double *b2, int n, int i, double lo, double hi,
+						    bool guessed, double guess, jn_tri_exchange *ex)
 {
 	const int lane = threadIdx.x & 31;
 	int cl = 0, ch = n, el = 0, eh = 0, known = 0;          /* known: 1 det at lo, 2 det at hi */
@@ -152,7 +191,7 @@ __device__ __forceinline__ double jn_tri_multisect_warp(const double *as, const 
 		}
 		double p;
 		int e;
-		const int cnt = jn_sturm_count(as, b2, n, x, &p, &e);
+		const int cnt = jn_sturm_count(as, b2, n, x, ex, round, &p, &e);
 		const unsigned int above = __ballot_sync(0xffffffffu, cnt > i);
 		const int f = above ? __ffs(above) - 1 : 32, fl = f > 0 ? f - 1 : 0, fh = f < 32 ? f : 31;
 		const double nlo = __shfl_sync(0xffffffffu, x, fl), nhi = __shfl_sync(0xffffffffu, x, fh);
