@@ -45,6 +45,7 @@
  */
 #include "jn_internal.h"
 #include "jn_fixed.cuh"
+#include "jn_pdl.cuh"
 
 #include <type_traits>
 
@@ -246,6 +247,12 @@ __global__ void __launch_bounds__(WALK_THREADS, MODE == 32 ? 32 : 28)
 	unsigned long long *slots = wslots + warp * WALK_SLOTS;
 	for (int i = lane; i < WALK_SLOTS; i += 32) slots[i] = 0ull;
 	__syncwarp();
+	/* from here on the kernel reads what the x view kernel wrote */
+	pdl_wait();
+	pdl_trigger();
+	ctrl = pdl_after(ctrl);
+	x = pdl_after(x);
+	xt = pdl_after(xt);
 	int S, sh;
 	walk_scales(ctrl[0], abs_bound, Sc, MODE, &S, &sh);
 	const float scalef = MODE == 32 ? __int_as_float((127 + (S < -126 ? -126 : (S > 127 ? 127 : S))) << 23) : 0.0f;
@@ -291,6 +298,9 @@ __global__ void jn_walk_xview_kernel(const double *__restrict__ x, const int32_t
 				     typename WalkT<MODE>::X *__restrict__ xv, typename WalkT<MODE>::X *__restrict__ xt, int64_t n,
 				     const unsigned int *__restrict__ ctrl)
 {
+	pdl_wait();
+	pdl_trigger();
+	ctrl = pdl_after(ctrl);
 	const double s = MODE == 1 ? ldexp(1.0, walk_x_exponent(ctrl[0])) : 1.0;
 	for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
 		if constexpr (MODE == 1) {
@@ -302,11 +312,67 @@ __global__ void jn_walk_xview_kernel(const double *__restrict__ x, const int32_t
 	}
 }
 
+/* Everything before the walk kernel in one launch, for a small basis: every
+ * CTA takes max|x| over the whole of x (largest bit pattern of |x|, NaN left
+ * out; the FP32 bound, monotone in |x|, is taken once of it) and converts its
+ * own states; the first CTA sets ctrl[0] and the task counter ctrl[1].
+ * Bound by latency; it stands for a memset and two kernels.  Up to 12 288
+ * states reading x once per CTA costs less than those launches: products back
+ * to back at D = 59 / 952 / 7916 / 10 817 / 15 764 take 12.4 / 21.3 / 128.3 /
+ * 117.0 / 49.6 us with it and 15.4 / 23.0 / 129.4 / 118.3 / 49.6 us without
+ * (a cluster of eight CTAs that meets over the maximum: 16.4 / 26.6 / 132.4 /
+ * 121.3 / 52.8 us). */
+#define WALK_SMALL_THREADS 256
+#define WALK_SMALL_DIM 12288
+template <int MODE>
+__global__ void __launch_bounds__(WALK_SMALL_THREADS)
+	jn_walk_small_x_kernel(const double *__restrict__ x, const int32_t *__restrict__ perm,
+			       typename WalkT<MODE>::X *__restrict__ xv, typename WalkT<MODE>::X *__restrict__ xt, int n,
+			       unsigned int *__restrict__ ctrl)
+{
+	typedef typename WalkT<MODE>::X X;
+	__shared__ unsigned long long wmax[WALK_SMALL_THREADS / 32];
+	pdl_trigger();
+	const int i = blockIdx.x * WALK_SMALL_THREADS + threadIdx.x;
+	const double v = i < n ? x[i] : 0.0, t = perm && i < n ? x[__ldg(perm + i)] : 0.0;
+	unsigned long long m = 0;
+#pragma unroll 8
+	for (int k = threadIdx.x; k < n; k += WALK_SMALL_THREADS) {
+		const unsigned long long a = (unsigned long long)__double_as_longlong(x[k]) & 0x7fffffffffffffffull;
+		if (a <= 0x7ff0000000000000ull && a > m) m = a;
+	}
+	for (int o = 16; o; o >>= 1) {
+		const unsigned long long w = __shfl_xor_sync(0xffffffffu, m, o);
+		m = w > m ? w : m;
+	}
+	if ((threadIdx.x & 31) == 0) wmax[threadIdx.x >> 5] = m;
+	__syncthreads();
+#pragma unroll
+	for (int w = 0; w < WALK_SMALL_THREADS / 32; w++) m = wmax[w] > m ? wmax[w] : m;
+	const unsigned int bound = __float_as_uint((float)__longlong_as_double((long long)m) * 1.0000002f);
+	if (i == 0) {
+		ctrl[0] = bound;
+		ctrl[1] = 0u;
+	}
+	if (i >= n) return;
+	if constexpr (MODE == 1) {
+		const double s = ldexp(1.0, walk_x_exponent(bound));
+		xv[i] = walk_xsplit(v, s);
+		if (perm) xt[i] = walk_xsplit(t, s);
+	} else {
+		if (MODE == 32) xv[i] = (X)v;
+		if (perm) xt[i] = (X)t;
+	}
+}
+
 /* y (+)= acc 2^-S with the integer path's unit; the accumulator is cleared */
 __global__ void jn_walk_finalize_kernel(unsigned long long *__restrict__ gacc, double *__restrict__ y, int64_t n,
 					const unsigned int *__restrict__ ctrl, double abs_bound, int Sc, int mode,
 					int accumulate)
 {
+	pdl_wait();
+	ctrl = pdl_after(ctrl);
+	gacc = pdl_after(gacc);
 	int S, sh;
 	walk_scales(ctrl[0], abs_bound, Sc, mode, &S, &sh);
 	const double unit = ldexp(1.0, -S);
@@ -478,7 +544,9 @@ static jn_status walk_elements(jn_ctx *c, int mode)
 }
 
 /* y (+)= H x on the walk engine: max|x| (and the converted copy of x), the
- * walk kernel, the conversion of the accumulator into y */
+ * walk kernel, the conversion of the accumulator into y.  Each kernel is set
+ * up while the one before it still runs (jn_pdl.cuh): without that overlap the
+ * gaps and launches cost 6 us more a product at any size. */
 jn_status jn_enqueue_walk(jn_ctx *c, const double *d_x, double *d_y, int accumulate, cudaStream_t st, cudaEvent_t pre,
 			  cudaEvent_t mid)
 {
@@ -490,37 +558,63 @@ jn_status jn_enqueue_walk(jn_ctx *c, const double *d_x, double *d_y, int accumul
 	int g = (int)((p->dim + 255) / 256);
 	if (g > 1024) g = 1024;
 	if (g < 1) g = 1;
-	CUDA_TRY(cudaMemsetAsync(c->d_xmax, 0, 2 * sizeof(unsigned int), st));
-	if (p->dim) {
-		jn_launch_prep(d_x, mode == 32 ? (float *)c->d_wx : NULL, p->dim, c->d_xmax, st);
-		const int32_t *perm = p->wxt ? c->d_wxperm : NULL;
-		if (mode == 1)
-			jn_walk_xview_kernel<1><<<g, 256, 0, st>>>(d_x, perm, c->d_wx, c->d_wxt, p->dim, c->d_xmax);
-		else if (perm && mode == 32)
-			jn_walk_xview_kernel<32><<<g, 256, 0, st>>>(d_x, perm, NULL, (float *)c->d_wxt, p->dim, c->d_xmax);
-		else if (perm)
-			jn_walk_xview_kernel<64><<<g, 256, 0, st>>>(d_x, perm, NULL, (double *)c->d_wxt, p->dim, c->d_xmax);
+	if (!p->dim) {
+		if (pre) cudaEventRecord(pre, st);
+		if (mid) cudaEventRecord(mid, st);
+		return JN_OK;
 	}
-	if (pre) cudaEventRecord(pre, st);
+	const int32_t *perm = p->wxt ? c->d_wxperm : NULL;
+	/* what precedes the walk kernel on the stream is a kernel of this product
+	   unless an event was recorded in between */
+	int overlap = 1;
+	if (p->dim <= WALK_SMALL_DIM) {
+		const int sg = (int)((p->dim + WALK_SMALL_THREADS - 1) / WALK_SMALL_THREADS), n = (int)p->dim;
+		if (mode == 1)
+			jn_walk_small_x_kernel<1><<<sg, WALK_SMALL_THREADS, 0, st>>>(d_x, perm, c->d_wx, c->d_wxt, n, c->d_xmax);
+		else if (mode == 32)
+			jn_walk_small_x_kernel<32><<<sg, WALK_SMALL_THREADS, 0, st>>>(d_x, perm, (float *)c->d_wx, (float *)c->d_wxt, n,
+										      c->d_xmax);
+		else
+			jn_walk_small_x_kernel<64><<<sg, WALK_SMALL_THREADS, 0, st>>>(d_x, perm, NULL, (double *)c->d_wxt, n, c->d_xmax);
+	} else {
+		CUDA_TRY(cudaMemsetAsync(c->d_xmax, 0, 2 * sizeof(unsigned int), st));
+		jn_launch_prep(d_x, mode == 32 ? (float *)c->d_wx : NULL, p->dim, c->d_xmax, st);
+		if (mode == 1)
+			pdl_launch(1, jn_walk_xview_kernel<1>, g, 256, 0, st, d_x, perm, c->d_wx, c->d_wxt, p->dim, c->d_xmax);
+		else if (perm && mode == 32)
+			pdl_launch(1, jn_walk_xview_kernel<32>, g, 256, 0, st, d_x, perm, (float *)NULL, (float *)c->d_wxt, p->dim, c->d_xmax);
+		else if (perm)
+			pdl_launch(1, jn_walk_xview_kernel<64>, g, 256, 0, st, d_x, perm, (double *)NULL, (double *)c->d_wxt, p->dim,
+				   c->d_xmax);
+	}
+	if (pre) {
+		cudaEventRecord(pre, st);
+		overlap = 0;
+	}
 	if (p->nwtasks) {
-		const int grid = c->num_sms * c->walk_per_sm[walk_slot(mode)];
+		int grid = c->num_sms * c->walk_per_sm[walk_slot(mode)];
+		if (grid > p->nwtasks) grid = (int)p->nwtasks;
 		const uint4 *T = (const uint4 *)c->d_wtasks, *P = (const uint4 *)c->d_wpieces;
 		if (mode == 32)
-			jn_walk_kernel<32><<<grid, WALK_THREADS, WALK_SMEM, st>>>(
-				T, P, c->d_wlanes, c->d_wwalks, c->d_wrows, c->d_wrdst, c->d_wgroups, NULL, (const float *)c->d_welem[0],
-				(const float *)c->d_wx, (const float *)c->d_wxt, c->d_gacc, c->d_xmax, p->nwtasks, p->abs_bound, 0);
+			pdl_launch(overlap, jn_walk_kernel<32>, grid, WALK_THREADS, WALK_SMEM, st, T, P, c->d_wlanes, c->d_wwalks, c->d_wrows,
+				   c->d_wrdst, c->d_wgroups, (const uint8_t *)NULL, (const float *)c->d_welem[0], (const float *)c->d_wx,
+				   (const float *)c->d_wxt, c->d_gacc, c->d_xmax, p->nwtasks, p->abs_bound, 0);
 		else if (mode == 64)
-			jn_walk_kernel<64><<<grid, WALK_THREADS, WALK_SMEM, st>>>(
-				T, P, c->d_wlanes, c->d_wwalks, c->d_wrows, c->d_wrdst, c->d_wgroups, NULL, (const double *)c->d_welem[1],
-				d_x, (const double *)c->d_wxt, c->d_gacc, c->d_xmax, p->nwtasks, p->abs_bound, 0);
+			pdl_launch(overlap, jn_walk_kernel<64>, grid, WALK_THREADS, WALK_SMEM, st, T, P, c->d_wlanes, c->d_wwalks, c->d_wrows,
+				   c->d_wrdst, c->d_wgroups, (const uint8_t *)NULL, (const double *)c->d_welem[1], d_x,
+				   (const double *)c->d_wxt, c->d_gacc, c->d_xmax, p->nwtasks, p->abs_bound, 0);
 		else
-			jn_walk_kernel<1><<<grid, WALK_THREADS, WALK_SMEM, st>>>(
-				T, P, c->d_wlanes, c->d_wwalks, c->d_wrows, c->d_wrdst, c->d_wgroups, c->d_wgshift, (const int2 *)c->d_welem[2],
-				c->d_wx, c->d_wxt, c->d_gacc, c->d_xmax, p->nwtasks, p->abs_bound, c->walk_sc);
+			pdl_launch(overlap, jn_walk_kernel<1>, grid, WALK_THREADS, WALK_SMEM, st, T, P, c->d_wlanes, c->d_wwalks, c->d_wrows,
+				   c->d_wrdst, c->d_wgroups, c->d_wgshift, (const int2 *)c->d_welem[2], c->d_wx, c->d_wxt, c->d_gacc,
+				   c->d_xmax, p->nwtasks, p->abs_bound, c->walk_sc);
+		overlap = 1;
 	}
-	if (mid) cudaEventRecord(mid, st);
-	if (p->dim) jn_walk_finalize_kernel<<<g, 256, 0, st>>>(c->d_gacc, d_y, p->dim, c->d_xmax, p->abs_bound, c->walk_sc, mode,
-								accumulate);
+	if (mid) {
+		cudaEventRecord(mid, st);
+		overlap = 0;
+	}
+	pdl_launch(overlap, jn_walk_finalize_kernel, g, 256, 0, st, c->d_gacc, d_y, p->dim, c->d_xmax, p->abs_bound, c->walk_sc, mode,
+		   accumulate);
 	cudaError_t e = cudaGetLastError();
 	if (e != cudaSuccess) return jn_fail(JN_ERR_CUDA, "walk product launch: %s", cudaGetErrorString(e));
 	return JN_OK;

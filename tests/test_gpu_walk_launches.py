@@ -1,0 +1,63 @@
+"""The walk product's launches at the sizes where they change: up to 12 288 states one kernel takes max|x| and makes the
+views of x (one CTA, a last CTA that is nearly empty, many CTAs), above it two do; and products that follow one another
+on a stream, each reading what the one before it wrote while its own kernels are already resident.  Results are the
+CPU model's, bit for bit."""
+import numpy as np
+import pytest
+
+import jupiterncsm_gb300 as jn
+from .test_gpu_walk import emu5, set_mode
+
+pytestmark = pytest.mark.gpu
+
+SYSTEMS = {             # Z, N, Nmax, 2M, dimension
+    "li6_n0": (3, 3, 0, 2, 8),
+    "he4_n4": (2, 2, 4, 0, 952),
+    "li7_n4": (3, 4, 4, 1, 10817),
+    "li6_n4": (3, 3, 4, 2, 15764),
+}
+_dirs = {}
+
+
+@pytest.fixture(scope="module")
+def system(tmp_path_factory):
+    def get(name):
+        if name not in _dirs:
+            Z, N, nmax, M2, _ = SYSTEMS[name]
+            d = str(tmp_path_factory.mktemp(name))
+            jn.generate(d, Z=Z, N=N, nmax=nmax, M2=M2, nbody=2, basis_files=False)
+            _dirs[name] = (d, Z, N)
+        return _dirs[name]
+    return get
+
+
+@pytest.mark.parametrize("name", list(SYSTEMS))
+@pytest.mark.parametrize("mode", [1, 64, 32])
+def test_walk_launches(system, name, mode):
+    import torch
+    d, Z, N = system(name)
+    H = jn.Hamiltonian.from_dir(d, Z, N)
+    H.set_engine(5)
+    set_mode(H, mode)
+    D = H.dimension
+    x = np.random.default_rng(5).standard_normal(D)
+    for at in (0, D // 2, D - 1):           # the largest state in the first, a middle and the last CTA
+        v = x.copy()
+        v[at] = -77.0
+        assert np.array_equal(H.matvec(v).view(np.uint64), emu5(d, Z, N, v, mode).view(np.uint64))
+    assert not H.matvec(np.zeros(D)).any()
+    # a chain on one stream: every product reads the previous one's result, scaled back into range
+    st = torch.cuda.Stream()
+    a, b = torch.from_numpy(x).cuda(), torch.zeros(D, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    with torch.cuda.stream(st):
+        for _ in range(6):
+            H.matvec_device(a.data_ptr(), b.data_ptr(), False, st.cuda_stream)
+            H.matvec_device(b.data_ptr(), a.data_ptr(), False, st.cuda_stream)
+            a.mul_(2.0 ** -12)
+    st.synchronize()
+    want = x
+    for _ in range(6):
+        want = emu5(d, Z, N, emu5(d, Z, N, want, mode), mode) * 2.0 ** -12
+    assert np.array_equal(a.cpu().numpy().view(np.uint64), want.view(np.uint64))
+    H.close()
