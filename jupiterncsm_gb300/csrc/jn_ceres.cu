@@ -54,8 +54,7 @@ extern "C" jn_status jn_subspace_matrices(jn_ctx *c, int n, const double *const 
 	for (int i = 0; i < n && !st; i++)
 		if (cudaMemcpyAsync(dV + (size_t)i * D, vectors[i], D * sizeof(double), cudaMemcpyHostToDevice, q) != cudaSuccess)
 			st = jn_fail(JN_ERR_CUDA, "upload of training vector %d", i);
-	for (int i = 0; i < n && !st && op; i++)
-		st = jn_launch_matvec(c, dV + (size_t)i * D, dHV + (size_t)i * D, 0, q);
+	if (!st && op) st = jn_enqueue_many(c, dV, dHV, n, q);
 	if (!st) {
 		if (norm) jn_subspace_gram<<<dim3(n, n), CT, 0, q>>>(dV, dV, D, n, dM);
 		if (op) jn_subspace_gram<<<dim3(n, n), CT, 0, q>>>(dHV, dV, D, n, dM + (size_t)n * n);

@@ -84,6 +84,8 @@ struct jn_ctx {
 	void *d_welem[3];               /* walk element arrays: FP32, FP64, split integers (built on first use) */
 	int2 *d_wx;                     /* x converted for the product (FP32 or split 52-bit integers) */
 	int2 *d_wxt;                    /* the transposed view of x that proton walks read, in the product's type */
+	void *d_wmany;                  /* accumulators, views of x and control words of several products at once */
+	int walk_many;                  /* vectors it holds */
 	int32_t *d_wxperm;              /* position in x of each element of that view */
 };
 
@@ -115,8 +117,6 @@ jn_status jn_enqueue_batched(jn_ctx *c, int B, int per, int f32, const void *me,
 			     double *x64, float *x32, unsigned long long *gacc, unsigned int *ctrl, const int *d_active,
 			     double abs_bound, cudaStream_t st);
 
-/* max|x| into ctrl[0] (zeroed before) and the optional FP32 copy of x */
-void jn_launch_prep(const double *d_x, float *x32, int64_t n, unsigned int *ctrl, cudaStream_t st);
 /* y (+)= gacc * 2^-S with S from ctrl[0]; gacc is cleared */
 void jn_launch_finalize(unsigned long long *gacc, double *d_y, int64_t n, const unsigned int *ctrl, double abs_bound,
 			int accumulate, cudaStream_t st);
@@ -135,6 +135,7 @@ jn_status jn_enqueue_panels(jn_ctx *c, const double *d_x, double *d_y, int accum
 jn_status jn_walk_setup(jn_ctx *c);
 void jn_walk_invalidate(jn_ctx *c);
 void jn_walk_release(jn_ctx *c);
+jn_status jn_enqueue_many(jn_ctx *c, const double *d_x, double *d_y, int n, cudaStream_t st);  /* Y = H X, any engine */
 jn_status jn_enqueue_walk(jn_ctx *c, const double *d_x, double *d_y, int accumulate, cudaStream_t st, cudaEvent_t pre,
 			  cudaEvent_t mid);
 

@@ -679,8 +679,7 @@ extern "C" jn_status jn_lanczos(jn_ctx *c, const jn_lanczos_options *opt, jn_lan
 	const int prec0 = c->precision, engine0 = c->engine;
 	c->precision = 64;
 	c->engine = c->engine_of[0];
-	for (int i = 0; i < want && !st; i++)
-		st = jn_launch_matvec(c, s->d_ritz + (size_t)i * D, s->d_hritz + (size_t)i * D, 0, q);
+	st = jn_enqueue_many(c, s->d_ritz, s->d_hritz, want, q);
 	c->precision = prec0;
 	c->engine = engine0;
 	if (st) return st;

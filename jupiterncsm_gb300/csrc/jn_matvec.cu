@@ -445,13 +445,6 @@ __global__ void jn_finalize_kernel(unsigned long long *__restrict__ gacc, double
 	}
 }
 
-void jn_launch_prep(const double *d_x, float *x32, int64_t n, unsigned int *ctrl, cudaStream_t st)
-{
-	int g = (int)((n + 255) / 256);
-	if (g > 1024) g = 1024;
-	if (n > 0) jn_prep_kernel<<<g, 256, 0, st>>>(d_x, x32, n, ctrl);
-}
-
 void jn_launch_finalize(unsigned long long *gacc, double *d_y, int64_t n, const unsigned int *ctrl, double abs_bound,
 			int accumulate, cudaStream_t st)
 {

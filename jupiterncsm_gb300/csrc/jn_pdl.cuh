@@ -32,10 +32,10 @@ template <typename T> __device__ __forceinline__ T *pdl_after(T *p)
  * preceding kernel when `overlap` (the operation before it on the stream is
  * then a kernel of the same product) */
 template <typename... P, typename... A>
-static inline void pdl_launch(int overlap, void (*kernel)(P...), int grid, int block, size_t smem, cudaStream_t st, A... args)
+static inline void pdl_launch(int overlap, void (*kernel)(P...), dim3 grid, int block, size_t smem, cudaStream_t st, A... args)
 {
 	cudaLaunchConfig_t cfg = {};
-	cfg.gridDim = dim3((unsigned int)grid);
+	cfg.gridDim = grid;
 	cfg.blockDim = dim3((unsigned int)block);
 	cfg.dynamicSmemBytes = smem;
 	cfg.stream = st;

@@ -61,3 +61,25 @@ def test_walk_launches(system, name, mode):
         want = emu5(d, Z, N, emu5(d, Z, N, want, mode), mode) * 2.0 ** -12
     assert np.array_equal(a.cpu().numpy().view(np.uint64), want.view(np.uint64))
     H.close()
+
+
+@pytest.mark.parametrize("name", list(SYSTEMS))
+@pytest.mark.parametrize("mode,n", [(1, 2), (1, 32), (1, 33), (64, 9), (32, 9), (1, 1)])
+def test_many_vectors(system, name, mode, n):
+    """The products of one subspace call share launches (32 vectors at most): rows and columns of unit vectors show the
+    components of H v, which are the single products', bit for bit."""
+    d, Z, N = system(name)
+    H = jn.Hamiltonian.from_dir(d, Z, N)
+    H.set_engine(5)
+    set_mode(H, mode)
+    D = H.dimension
+    rng = np.random.default_rng(n)
+    at = sorted({0, D // 3, D - 1})
+    vs = [rng.standard_normal(D) * 10.0 ** rng.uniform(-4, 4) for _ in range(max(n - len(at), 0))]
+    units = [np.eye(1, D, k)[0] for k in at][:n]
+    _, op = H.subspace_matrices(vs + units)
+    for i, v in enumerate(vs + units):
+        hv = H.matvec(v)
+        for j in range(max(i, len(vs)), len(vs) + len(units)):
+            assert op[i, j] == hv[at[j - len(vs)]]
+    H.close()
