@@ -306,6 +306,7 @@ typedef struct {
 	wview_t *views;
 	wdir_t *dirs;
 	uint32_t *lanes;
+	int64_t cap;                    /* rows of a piece */
 } wjob_t;
 
 /* the walk list, the row list and element-row addressing of instruction q */
@@ -411,8 +412,9 @@ static void view_lanes(int64_t vi, void *v)
 }
 
 /* rows of one directed instruction, checked and cut into pieces: runs of
-   whole row groups with at most JN_WALK_RS distinct destination rows (a
-   group with more is split, and its element row read once per part) */
+   whole row groups with at most JN_WALK_RS distinct destination rows and
+   `cap` rows (a group with more is split, and its element row read once per
+   part) */
 static void dir_pieces(int64_t di, void *v)
 {
 	const wjob_t *J = (const wjob_t *)v;
@@ -477,7 +479,7 @@ static void dir_pieces(int64_t di, void *v)
 		int64_t r1 = r0;
 		const int64_t rdst0 = D->nrdst, row0 = D->nrows, group0 = D->ngroups;
 		uint32_t *slot = D->rdst + rdst0;       /* the piece's destination rows */
-		while (r1 < nr) {
+		while (r1 < nr && r1 - r0 < J->cap) {
 			/* the next group [r1, g1) and the destinations it would add */
 			int64_t g1 = r1;
 			while (g1 < nr && R[g1].k == R[r1].k) g1++;
@@ -488,10 +490,10 @@ static void dir_pieces(int64_t di, void *v)
 				for (int i = 0; i < rs; i++) in |= slot[i] == R[e].dst;
 				add += !in;
 			}
-			if (rs > 0 && rs + add > JN_WALK_RS) break;
+			if (rs > 0 && (rs + add > JN_WALK_RS || g1 - r0 > J->cap)) break;
 			/* take the group, or as much of it as fits */
 			int64_t e = r1;
-			for (; e < g1; e++) {
+			for (; e < g1 && e - r0 < J->cap; e++) {
 				int in = 0;
 				for (int i = 0; i < rs; i++) in |= slot[i] == R[e].dst;
 				if (!in) {
@@ -537,6 +539,63 @@ static void wdir_free(wdir_t *D)
 	D->pieces = NULL;
 	D->prows = NULL;
 }
+
+/*
+ * Tasks differ by two orders of magnitude, and a long one taken last keeps
+ * one warp busy while the others have nothing left.  So the last
+ * WALK_TAIL_TASKS of the list (all of them for most bases) go by falling
+ * cost, in classes of powers of two that keep the order inside a class; their
+ * matrix elements fit L2 together, which the list's order otherwise serves.
+ * Products back to back, list order -> by cost: 6Li Nmax 4 2NF (18 659 tasks)
+ * 50.2 -> 42.3 us; with 3NF 7Li Nmax 4 (44 758) 117 -> 92, 4He Nmax 6 (51 432)
+ * 129 -> 99, 6Li Nmax 4 (82 282) 174 -> 148 us (157 with the last 65 536 by
+ * cost); 6Li Nmax 6 (1.4 million) 3498 -> 3488 us, but 3606 us with all of
+ * them by cost.
+ */
+#define WALK_TAIL_TASKS 131072
+
+static int order_tail(jn_wtask_t *t, int64_t n, const jn_wpiece_t *pieces, int64_t npieces, int64_t nrows)
+{
+	int64_t at[33] = { 0 };
+	unsigned char *cls = malloc((size_t)(n ? n : 1));
+	jn_wtask_t *to = malloc((size_t)(n ? n : 1) * sizeof *to);
+	if (!cls || !to) {
+		free(cls);
+		free(to);
+		return 1;
+	}
+	for (int64_t i = 0; i < n; i++) {
+		const jn_wpiece_t *P = pieces + t[i].piece;
+		const int64_t rows = (t[i].piece + 1 < npieces ? P[1].row0 : nrows) - P->row0;
+		/* a row's fixed cost counts as two entries, as does a group's */
+		const int64_t cost = (rows + (int64_t)(P->meta >> 9)) * ((t[i].meta >> 8 & 0xff) + 2);
+		int b = 0;
+		while (b < 31 && (int64_t)1 << b < cost) b++;
+		cls[i] = (unsigned char)(31 - b);
+		at[cls[i] + 1]++;
+	}
+	for (int b = 0; b < 32; b++) at[b + 1] += at[b];
+	for (int64_t i = 0; i < n; i++) to[at[cls[i]]++] = t[i];
+	memcpy(t, to, (size_t)n * sizeof *t);
+	free(cls);
+	free(to);
+	return 0;
+}
+
+/*
+ * Rows of a piece.  A task's fixed cost (its records, its sums) asks for long
+ * pieces, the end of the product for short ones: at most WALK_CAP rows, and
+ * WALK_CAP_FEW where that leaves at most WALK_FEW_TASKS tasks, about as many
+ * as the chip holds warps twice over, so that the longest task sets the time.
+ * Products back to back with 64, 16, 8, 4 and 2 rows: 4He Nmax 2 (145 tasks)
+ * 12.4, 12.4, 12.3, 10.3, 10.3 us; 6Li Nmax 2 (about 2000) 18.5, 18.5, 15.0,
+ * 14.4, 14.4; 4He Nmax 4 (2396) 19.3, 19.3, 16.8, 16.4, 17.4; 6Li Nmax 4
+ * (18 659) 42.0, 42.2, 41.9, 48.0, 63.5; 7Li Nmax 4 with 3NF (44 758) 88.8,
+ * 92.2, 99.6, 116, 168.
+ */
+#define WALK_CAP 64
+#define WALK_CAP_FEW 4
+#define WALK_FEW_TASKS 8192
 
 int jn_walk_build(jn_plan_t *p, char *err, size_t errlen)
 {
@@ -622,9 +681,20 @@ int jn_walk_build(jn_plan_t *p, char *err, size_t errlen)
 	lanes = malloc((size_t)(nlanes ? nlanes : 1) * sizeof(uint32_t));
 	if (!lanes) ERR("out of host memory");
 	{
-		wjob_t job = { p, views, dirs, lanes };
+		wjob_t job = { p, views, dirs, lanes, WALK_CAP };
 		jn_par_for(nviews, view_lanes, &job);
 		jn_par_for(ndirs, dir_pieces, &job);
+		int64_t n = 0;
+		for (int64_t d = 0; d < ndirs; d++) n += dirs[d].npieces * views[dirs[d].view].nsets;
+		if (n <= WALK_FEW_TASKS) {
+			job.cap = WALK_CAP_FEW;
+			for (int64_t d = 0; d < ndirs; d++) {
+				wdir_free(&dirs[d]);
+				dirs[d].nrows = dirs[d].nrdst = dirs[d].ngroups = dirs[d].npieces = 0;
+				dirs[d].status = 0;
+				dir_pieces(d, &job);    /* too little work to start threads for */
+			}
+		}
 	}
 	for (int64_t v = 0; v < nviews; v++)
 		if (views[v].status) ERR("out of host memory");
@@ -680,7 +750,12 @@ int jn_walk_build(jn_plan_t *p, char *err, size_t errlen)
 	}
 	/* tasks stay in this order: warps take the next one from a counter, so
 	   warps that run at the same time work on neighbouring instructions and
-	   share their matrix elements in L2 */
+	   share their matrix elements in L2; all but the last of them */
+	{
+		const int64_t n = tasks.n < WALK_TAIL_TASKS ? tasks.n : WALK_TAIL_TASKS;
+		if (order_tail((jn_wtask_t *)tasks.a + tasks.n - n, n, (const jn_wpiece_t *)pieces.a, pieces.n, rows.n))
+			ERR("out of host memory");
+	}
 	/* the transposed view of x that proton walks read: block [n][p] */
 	if (p->wxt) {
 		p->wxperm = malloc((size_t)(p->dim ? p->dim : 1) * sizeof(int32_t));
