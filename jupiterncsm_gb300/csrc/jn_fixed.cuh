@@ -47,4 +47,27 @@ __device__ __forceinline__ void add_fixed32(unsigned int *lo, unsigned int *hi, 
 	if (h) atomicAdd(hi + i, (unsigned int)h);
 }
 
+/* The FP32 bound of max|x| over the whole of x (n values), taken by every CTA
+ * for itself: the largest bit pattern of |x| (NaN left out), the bound, which
+ * is monotone in |x|, once of it.  `wmax`: THREADS / 32 words of shared memory. */
+template <int THREADS>
+__device__ __forceinline__ unsigned int x_bound_of_all(const double *__restrict__ x, int n, unsigned long long *wmax)
+{
+	unsigned long long m = 0;
+#pragma unroll 8
+	for (int k = threadIdx.x; k < n; k += THREADS) {
+		const unsigned long long a = (unsigned long long)__double_as_longlong(x[k]) & 0x7fffffffffffffffull;
+		if (a <= 0x7ff0000000000000ull && a > m) m = a;
+	}
+	for (int o = 16; o; o >>= 1) {
+		const unsigned long long w = __shfl_xor_sync(0xffffffffu, m, o);
+		m = w > m ? w : m;
+	}
+	if ((threadIdx.x & 31) == 0) wmax[threadIdx.x >> 5] = m;
+	__syncthreads();
+#pragma unroll
+	for (int w = 0; w < THREADS / 32; w++) m = wmax[w] > m ? wmax[w] : m;
+	return __float_as_uint((float)__longlong_as_double((long long)m) * 1.0000002f);
+}
+
 #endif

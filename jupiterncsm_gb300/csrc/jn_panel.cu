@@ -370,6 +370,40 @@ __global__ void __cluster_dims__(PREP_CTAS, 1, 1) __launch_bounds__(PREP_THREADS
 	cluster.sync();
 }
 
+/* The same for a small basis without a cluster: every CTA takes max|x| over
+ * the whole of x and converts its own states.  Bound by latency, where the
+ * cluster pays for its launch and two barriers; reading x once per CTA costs
+ * less up to 12 288 states.  32-bit products back to back, cluster -> this:
+ * D = 59 12.3 -> 10.3 us, 952 17.0 -> 14.4, 7916 (2NF) 32.8 -> 30.8, 8294 63.4
+ * -> 61.4, 10 817 80.5 -> 79.9, 15 764 49.2 -> 49.2. */
+#define SMALL_THREADS 256
+#define SMALL_DIM 12288
+template <typename T>
+__global__ void __launch_bounds__(SMALL_THREADS)
+	jn_panel_small_prep_kernel(const double *__restrict__ x, T *__restrict__ xn, T *__restrict__ xt,
+				   const uint4 *__restrict__ blocks, const uint16_t *__restrict__ elem, int dim,
+				   unsigned int *__restrict__ ctrl)
+{
+	__shared__ unsigned long long wmax[SMALL_THREADS / 32];
+	const int i = blockIdx.x * SMALL_THREADS + threadIdx.x;
+	const double v = i < dim ? x[i] : 0.0;
+	const unsigned int bound = x_bound_of_all<SMALL_THREADS>(x, dim, wmax);
+	if (i == 0) {
+		ctrl[0] = bound;
+		ctrl[1] = 0u;
+	}
+	if (i >= dim) return;
+	T t;
+	if (sizeof(T) == 4) t = (T)fixed32_bits(v, x_exponent(bound));
+	else t = (T)v;
+	if (xn) xn[i] = t;
+	if (xt) {
+		const uint4 bk = __ldg(blocks + __ldg(elem + i));
+		const uint32_t e = (uint32_t)i - bk.x, Nn = bk.w, Np = bk.z;
+		xt[bk.x + (e % Nn) * Np + e / Nn] = t;
+	}
+}
+
 /* y (+)= acc 2^(k - Sc - Sx); the accumulator is cleared for the next product */
 __global__ void jn_int_finalize_kernel(unsigned long long *__restrict__ gacc, double *__restrict__ y, int64_t n,
 				       const unsigned int *__restrict__ xmax_bits, int k_minus_sc, int accumulate)
@@ -614,14 +648,20 @@ static void panel_launch(const panel_sig_t *g, int has_tasks, int capturing)
 	const uint4 *blocks = (const uint4 *)g->blocks;
 	unsigned int *ctrl = (unsigned int *)g->ctrl;
 	if (g->start) cudaEventRecordWithFlags((cudaEvent_t)g->start, st, evflags);
-	if (g->f32)
-		/* the kernel that stages x in shared memory reads only the [p][n] copy */
-		jn_panel_prep_kernel<int><<<PREP_CTAS, PREP_THREADS, 0, st>>>((const double *)g->x, (int *)g->xi,
-									 g->xs && has_tasks ? NULL : (int *)g->xt, blocks,
-									 (const uint16_t *)g->elem, g->dim, ctrl);
+	const double *x = (const double *)g->x;
+	const uint16_t *elem = (const uint16_t *)g->elem;
+	/* the kernel that stages x in shared memory reads only the [p][n] copy */
+	int *xi = (int *)g->xi, *xti = g->xs && has_tasks ? NULL : (int *)g->xt;
+	const int sg = (int)((g->dim + SMALL_THREADS - 1) / SMALL_THREADS);
+	if (g->dim <= SMALL_DIM && g->f32)
+		jn_panel_small_prep_kernel<int><<<sg, SMALL_THREADS, 0, st>>>(x, xi, xti, blocks, elem, (int)g->dim, ctrl);
+	else if (g->dim <= SMALL_DIM)
+		jn_panel_small_prep_kernel<double><<<sg, SMALL_THREADS, 0, st>>>(x, NULL, (double *)g->xt, blocks, elem, (int)g->dim,
+										  ctrl);
+	else if (g->f32)
+		jn_panel_prep_kernel<int><<<PREP_CTAS, PREP_THREADS, 0, st>>>(x, xi, xti, blocks, elem, g->dim, ctrl);
 	else
-		jn_panel_prep_kernel<double><<<PREP_CTAS, PREP_THREADS, 0, st>>>((const double *)g->x, NULL, (double *)g->xt, blocks,
-									    (const uint16_t *)g->elem, g->dim, ctrl);
+		jn_panel_prep_kernel<double><<<PREP_CTAS, PREP_THREADS, 0, st>>>(x, NULL, (double *)g->xt, blocks, elem, g->dim, ctrl);
 	if (g->pre) cudaEventRecordWithFlags((cudaEvent_t)g->pre, st, evflags);
 	if (has_tasks) {
 		if (g->f32) {

@@ -343,8 +343,7 @@ __global__ void jn_walk_xview_kernel(const double *__restrict__ x, const int32_t
 }
 
 /* Everything before the walk kernel in one launch, for a small basis: every
- * CTA takes max|x| over the whole of x (largest bit pattern of |x|, NaN left
- * out; the FP32 bound, monotone in |x|, is taken once of it) and converts its
+ * CTA takes max|x| over the whole of x and converts its
  * own states (of vector blockIdx.y); its first CTA sets ctrl[0], and the task
  * counter ctrl[1] to zero.
  * Bound by latency; it stands for a memset and two kernels.  Up to 12 288
@@ -370,21 +369,7 @@ __global__ void __launch_bounds__(WALK_SMALL_THREADS)
 	ctrl += 2 * blockIdx.y;
 	const int i = blockIdx.x * WALK_SMALL_THREADS + threadIdx.x;
 	const double v = i < n ? x[i] : 0.0, t = perm && i < n ? x[__ldg(perm + i)] : 0.0;
-	unsigned long long m = 0;
-#pragma unroll 8
-	for (int k = threadIdx.x; k < n; k += WALK_SMALL_THREADS) {
-		const unsigned long long a = (unsigned long long)__double_as_longlong(x[k]) & 0x7fffffffffffffffull;
-		if (a <= 0x7ff0000000000000ull && a > m) m = a;
-	}
-	for (int o = 16; o; o >>= 1) {
-		const unsigned long long w = __shfl_xor_sync(0xffffffffu, m, o);
-		m = w > m ? w : m;
-	}
-	if ((threadIdx.x & 31) == 0) wmax[threadIdx.x >> 5] = m;
-	__syncthreads();
-#pragma unroll
-	for (int w = 0; w < WALK_SMALL_THREADS / 32; w++) m = wmax[w] > m ? wmax[w] : m;
-	const unsigned int bound = __float_as_uint((float)__longlong_as_double((long long)m) * 1.0000002f);
+	const unsigned int bound = x_bound_of_all<WALK_SMALL_THREADS>(x, n, wmax);
 	if (i == 0) {
 		ctrl[0] = bound;
 		ctrl[1] = 0u;

@@ -1,4 +1,4 @@
-"""The walk product's launches at the sizes where they change: up to 12 288 states one kernel takes max|x| and makes the
+"""The products' launches at the sizes where they change: up to 12 288 states one kernel takes max|x| and makes the
 views of x (one CTA, a last CTA that is nearly empty, many CTAs), above it two do; and products that follow one another
 on a stream, each reading what the one before it wrote while its own kernels are already resident.  Results are the
 CPU model's, bit for bit."""
@@ -6,6 +6,7 @@ import numpy as np
 import pytest
 
 import jupiterncsm_gb300 as jn
+from .test_gpu_matvec import emu4
 from .test_gpu_walk import emu5, set_mode
 
 pytestmark = pytest.mark.gpu
@@ -82,4 +83,24 @@ def test_many_vectors(system, name, mode, n):
         hv = H.matvec(v)
         for j in range(max(i, len(vs)), len(vs) + len(units)):
             assert op[i, j] == hv[at[j - len(vs)]]
+    H.close()
+
+
+@pytest.mark.parametrize("name", list(SYSTEMS))
+@pytest.mark.parametrize("bits", [32, 64])
+def test_panel_launches(system, name, bits):
+    """The panel product changes at the same dimension: every CTA takes the maximum below it, one cluster above."""
+    d, Z, N = system(name)
+    H = jn.Hamiltonian.from_dir(d, Z, N)
+    H.set_engine(4)
+    H.set_precision(bits)
+    if H.active_engine() != 4:
+        pytest.skip("the FP64 accumulators do not fit")
+    D = H.dimension
+    x = np.random.default_rng(6).standard_normal(D)
+    for at in (0, D // 2, D - 1):
+        v = x.copy()
+        v[at] = 77.0
+        assert np.array_equal(H.matvec(v).view(np.uint64), emu4(d, Z, N, v, bits == 32).view(np.uint64))
+    assert not H.matvec(np.zeros(D)).any()
     H.close()
