@@ -168,6 +168,62 @@ __device__ __forceinline__ void panel_task(const uint4 pa, const uint4 pb, const
 	}
 }
 
+/* one block of a CTA's accumulator: its words [so, end), first state and row length (rows are Nn | 1 words) */
+struct PanelBlock {
+	uint32_t so, end, at, Nn;
+};
+
+/* the block of flush pair f (past the last pair: one that no word reaches) */
+__device__ __forceinline__ PanelBlock panel_block(const uint32_t *__restrict__ flush, const uint4 *__restrict__ blocks, uint32_t f,
+						  uint32_t f1)
+{
+	PanelBlock b = { 0xffffffffu, 0xffffffffu, 0u, 0u };
+	if (f < f1) {
+		const uint4 bk = __ldg(blocks + __ldg(flush + 2 * f));
+		b.so = __ldg(flush + 2 * f + 1);
+		b.at = bk.x;
+		b.Nn = bk.w;
+		b.end = b.so + bk.z * (bk.w | 1u);
+	}
+	return b;
+}
+
+/* body(word, first state of its row, column, row length) for each word of a
+ * CTA's accumulator, the words dealt to the threads across block boundaries:
+ * lane l of every warp holds block l of 32 (b: the first 32, loaded before),
+ * and a word's block is found among them by shuffles.  The blocks' records
+ * are so two dependent loads for 32 blocks; block by block, with the whole
+ * CTA on each, a CTA paid about 830 cycles a block (4He Nmax 6: 6 blocks a
+ * CTA on average, up to 44; the 32-bit product went from 76.5 to 65.5 us;
+ * 3H Nmax 8 60.3 to 39.5 us). */
+template <typename Body>
+__device__ __forceinline__ void panel_words(const uint32_t *__restrict__ flush, const uint4 *__restrict__ blocks, uint32_t f0,
+					    uint32_t f1, PanelBlock b, Body body)
+{
+	const uint32_t lane = threadIdx.x & 31;
+	for (uint32_t fb = f0; fb < f1;) {
+		const uint32_t start = __shfl_sync(0xffffffffu, b.so, 0);
+		const uint32_t stop = __shfl_sync(0xffffffffu, b.end, f1 - fb < 32 ? f1 - fb - 1 : 31);
+		for (uint32_t base = start + (threadIdx.x & ~31u); base < stop; base += blockDim.x) {
+			const uint32_t e = base + lane;
+			uint32_t i = 0;         /* blocks that end at or before e */
+#pragma unroll
+			for (uint32_t s = 16; s; s >>= 1) {
+				const uint32_t end = __shfl_sync(0xffffffffu, b.end, i + s - 1);
+				if (end <= e) i += s;
+			}
+			const uint32_t so = __shfl_sync(0xffffffffu, b.so, i), at = __shfl_sync(0xffffffffu, b.at, i);
+			const uint32_t Nn = __shfl_sync(0xffffffffu, b.Nn, i);
+			if (e < stop) {
+				const uint32_t k = e - so, row = k / (Nn | 1u), col = k - row * (Nn | 1u);
+				body(e, at + row * Nn, col, Nn);
+			}
+		}
+		fb += 32;
+		if (fb < f1) b = panel_block(flush, blocks, fb + lane, f1);
+	}
+}
+
 /* one CTA's run: cta_ptr and flush_ptr point at its own entries */
 template <typename T, typename Fix, bool XS>
 __device__ __forceinline__ void jn_panel_body(const uint4 *__restrict__ panels, const uint4 *__restrict__ tasks,
@@ -187,21 +243,13 @@ __device__ __forceinline__ void jn_panel_body(const uint4 *__restrict__ panels, 
 	T *xs = XS ? (T *)(sacc + 2 * words) : NULL;
 	const int lane = threadIdx.x & 31;
 	const uint32_t f0 = flush_ptr[0], f1 = flush_ptr[1];
-	/* clear the blocks this CTA touches (padded rows) */
-	for (uint32_t f = f0; f < f1; f++) {
-		const uint32_t b = __ldg(flush + 2 * f), so = __ldg(flush + 2 * f + 1);
-		const uint4 bk = __ldg(blocks + b);
-		const uint32_t n = bk.z * (bk.w | 1u);
-		if (threadIdx.x == 0) bmap[b] = so;
-		for (uint32_t e = threadIdx.x; e < n; e += blockDim.x) {
-			lo[so + e] = 0u;
-			hi[so + e] = 0u;
-			if (XS) {
-				const uint32_t Ns = bk.w | 1u, row = e / Ns, col = e - row * Ns;
-				xs[so + e] = col < bk.w ? __ldg(x + bk.x + row * bk.w + col) : (T)0;
-			}
-		}
-	}
+	for (uint32_t f = f0 + threadIdx.x; f < f1; f += blockDim.x) bmap[__ldg(flush + 2 * f)] = __ldg(flush + 2 * f + 1);
+	panel_words(flush, blocks, f0, f1, panel_block(flush, blocks, f0 + lane, f1),
+		    [&](uint32_t e, uint32_t at, uint32_t col, uint32_t Nn) {
+			    lo[e] = 0u;
+			    hi[e] = 0u;
+			    if (XS) xs[e] = col < Nn ? __ldg(x + at + col) : (T)0;
+		    });
 	if (threadIdx.x == 0) next_task = 0;
 	__syncthreads();
 	const uint32_t t0 = cta_ptr[0], nt = cta_ptr[1] - t0;
@@ -231,18 +279,13 @@ __device__ __forceinline__ void jn_panel_body(const uint4 *__restrict__ panels, 
 			else panel_task<T, Fix, JN_KIND_P, false, XS>(pa, pb, pc, pd, tk.y, tk.z, R, r, i, lo, hi, x, xt, coef, meta, fix, so, si, xs);
 		}
 	}
-	__syncthreads();
 	/* add the touched blocks into the global accumulator (unpadded layout) */
-	for (uint32_t f = f0; f < f1; f++) {
-		const uint32_t so = __ldg(flush + 2 * f + 1);
-		const uint4 bk = __ldg(blocks + __ldg(flush + 2 * f));
-		const uint32_t Nn = bk.w, Ns = bk.w | 1u, n = bk.z * Nn;
-		for (uint32_t e = threadIdx.x; e < n; e += blockDim.x) {
-			const uint32_t s = so + (e / Nn) * Ns + e % Nn;
-			const unsigned long long v = (unsigned long long)lo[s] | ((unsigned long long)hi[s] << 32);
-			if (v) atomicAdd(gacc + bk.x + e, v);
-		}
-	}
+	const PanelBlock b = panel_block(flush, blocks, f0 + lane, f1);
+	__syncthreads();
+	panel_words(flush, blocks, f0, f1, b, [&](uint32_t e, uint32_t at, uint32_t col, uint32_t) {
+		const unsigned long long v = (unsigned long long)lo[e] | ((unsigned long long)hi[e] << 32);
+		if (v) atomicAdd(gacc + at + col, v);
+	});
 }
 
 /* the 32-bit product: coefficients and x are 32-bit fixed-point integers.
@@ -264,7 +307,7 @@ __global__ void __launch_bounds__(PANEL_THREADS, 3) jn_panel_kernel_i32(const ui
 }
 
 /* the FP64 product: the fixed-point scale 2^S comes from max|x| on the device */
-__global__ void __launch_bounds__(PANEL_THREADS) jn_panel_kernel_fp64(const uint4 *__restrict__ panels,
+__global__ void __launch_bounds__(PANEL_THREADS, 3) jn_panel_kernel_fp64(const uint4 *__restrict__ panels,
 								      const uint4 *__restrict__ tasks,
 								      const uint32_t *__restrict__ cta_ptr,
 								      const uint32_t *__restrict__ flush,
