@@ -38,6 +38,7 @@
 
 #define PANEL_THREADS 512
 #define PANEL_UNROLL 4
+#define PANEL_MOST 3        /* CTAs an SM: what the kernels' registers allow */
 
 template <typename T> __device__ __forceinline__ T load_stream(const T *p) { return __ldcs(p); }
 
@@ -292,7 +293,7 @@ __device__ __forceinline__ void jn_panel_body(const uint4 *__restrict__ panels, 
  * XS: x staged in shared memory (one more word per state) instead of
  * gathered through L1. */
 template <bool XS>
-__global__ void __launch_bounds__(PANEL_THREADS, 3) jn_panel_kernel_i32(const uint4 *__restrict__ panels,
+__global__ void __launch_bounds__(PANEL_THREADS, PANEL_MOST) jn_panel_kernel_i32(const uint4 *__restrict__ panels,
 								     const uint4 *__restrict__ tasks,
 								     const uint32_t *__restrict__ cta_ptr,
 								     const uint32_t *__restrict__ flush,
@@ -307,7 +308,7 @@ __global__ void __launch_bounds__(PANEL_THREADS, 3) jn_panel_kernel_i32(const ui
 }
 
 /* the FP64 product: the fixed-point scale 2^S comes from max|x| on the device */
-__global__ void __launch_bounds__(PANEL_THREADS, 3) jn_panel_kernel_fp64(const uint4 *__restrict__ panels,
+__global__ void __launch_bounds__(PANEL_THREADS, PANEL_MOST) jn_panel_kernel_fp64(const uint4 *__restrict__ panels,
 								      const uint4 *__restrict__ tasks,
 								      const uint32_t *__restrict__ cta_ptr,
 								      const uint32_t *__restrict__ flush,
@@ -589,9 +590,22 @@ jn_status jn_panels_setup(jn_ctx *c)
 			c->panel_xs_limit = (int)g_xs_limit;
 		cudaGetLastError();
 	}
-	/* the task split is the same for every grid; CTAs take contiguous runs of the FP32 grid */
-	if (jn_panels_build(p, c->num_sms * per[1], JN_PANEL_ITER, err, sizeof err))
-		return jn_fail(JN_ERR_NOMEM, "panel plan: %s", err);
+	/* The task split is the same for every grid; CTAs take contiguous runs of
+	   the FP32 grid.  Where accumulators of the whole vector would leave an SM
+	   one CTA (16 warps), take as many as the accumulators of the runs
+	   themselves allow, which hold only the blocks that a run touches.  32-bit
+	   products with 1, 2, 3 CTAs an SM: 6Li Nmax 4 (D = 15 764) 2NF 43.1, 33.2,
+	   33.7 us, with 3NF 228, 165, 133 us.  Where the whole vector fits twice
+	   there is no clear gain in a third (7Li Nmax 4 with 3NF 77.9, 80.0 us;
+	   5He Nmax 6 35.0, 33.0 us: x no longer fits beside the accumulator). */
+	for (int k = per[1] == 1 ? PANEL_MOST : per[1];; k--) {
+		if (jn_panels_build(p, c->num_sms * k, JN_PANEL_ITER, err, sizeof err))
+			return jn_fail(JN_ERR_NOMEM, "panel plan: %s", err);
+		if (k == per[1] || (size_t)k * (panel_smem_words(p, p->pcta_words, 0) + 1024) <= (size_t)c->smem_per_sm) {
+			if (k > per[1]) c->panel_per_sm[0] = c->panel_per_sm[1] = k;
+			break;
+		}
+	}
 	c->panel_iter = JN_PANEL_ITER;
 	jn_status s;
 	if ((s = upload_n(&c->d_panels, p->panels, (size_t)p->npanels)) ||
