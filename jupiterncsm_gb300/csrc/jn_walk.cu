@@ -21,7 +21,7 @@
  * values, sums the U products in registers, rounds the sum once to the
  * 64-bit fixed-point unit and adds it into its own slot (destination row,
  * lane) in shared memory: no atomics, no bank conflicts.  After the task a
- * segmented sum over the lanes of each walk gives one global add per
+ * lane sums the slots of one walk and gives one global add per
  * (destination row, walk).  A CTA is one warp, so the register file alone
  * sets how many warps an SM holds.
  *
@@ -51,8 +51,9 @@
 
 #define WALK_WARPS 1     /* one warp a CTA: 32 resident CTAs an SM, the most the integer path's 63 registers allow too */
 #define WALK_THREADS (WALK_WARPS * 32)
-#define WALK_SLOTS (JN_WALK_RS * 32)    /* per warp: one 64-bit slot per (destination row, lane) */
-#define WALK_SMEM ((size_t)WALK_WARPS * WALK_SLOTS * sizeof(unsigned long long))
+#define WALK_PITCH 33    /* words of a slot row: lanes on different rows of one column hit different banks */
+#define WALK_SLOTS (JN_WALK_RS * WALK_PITCH)    /* per warp: one 64-bit slot per (destination row, lane) */
+#define WALK_SMEM ((size_t)WALK_WARPS * (WALK_SLOTS * sizeof(unsigned long long) + 32 * sizeof(uint32_t)))
 
 static_assert(sizeof(jn_wtask_t) == 16 && sizeof(jn_wpiece_t) == 32, "tasks are read as one uint4, pieces as two");
 
@@ -144,7 +145,7 @@ __device__ __forceinline__ void walk_task(const uint4 ta, const uint4 pa, const 
 					  const uint32_t *__restrict__ rdst, const uint32_t *__restrict__ groups,
 					  const uint8_t *__restrict__ gshift, const typename WalkT<MODE>::C *__restrict__ elem,
 					  const typename WalkT<MODE>::X *__restrict__ x, const typename WalkT<MODE>::X *__restrict__ xt,
-					  unsigned long long *__restrict__ gacc, unsigned long long *__restrict__ slots, int lane,
+					  unsigned long long *__restrict__ gacc, unsigned long long *__restrict__ slots, uint32_t *__restrict__ tab, int lane,
 					  int sh, float scalef, double scale)
 {
 	typedef typename WalkT<MODE>::C C;
@@ -194,9 +195,9 @@ __device__ __forceinline__ void walk_task(const uint4 ta, const uint4 pa, const 
 #pragma unroll
 				for (int u = 0; u < U; u++) c[u] = walk_coef<MODE>(c[u], mul, u);
 			}
-			slots[(int)((row >> 16) & 31u) * 32 + lane] += (unsigned long long)walk_row<MODE, U>(c, xv, row, shg, scalef, scale);
+			slots[(int)((row >> 16) & 31u) * WALK_PITCH + lane] += (unsigned long long)walk_row<MODE, U>(c, xv, row, shg, scalef, scale);
 			if (two)
-				slots[(int)((row2 >> 16) & 31u) * 32 + lane] +=
+				slots[(int)((row2 >> 16) & 31u) * WALK_PITCH + lane] +=
 					(unsigned long long)walk_row<MODE, U>(c, xv2, row2, shg, scalef, scale);
 			const bool end = !two || (row2 & JN_WALK_GROUP_END);
 			j += two ? 2 : 1;
@@ -205,27 +206,39 @@ __device__ __forceinline__ void walk_task(const uint4 ta, const uint4 pa, const 
 		}
 	}
 	__syncwarp();
-	/* the task's slots into the global accumulator; slots are left zero.  The
-	   lanes of one walk are a run of neighbouring lanes: a segmented sum over
-	   each run (shuffles down, log2 of the longest run steps) leaves the
-	   walk's total in the run's first lane, which adds it */
+	/* The task's slots into the global accumulator; slots are left zero.  The
+	   lanes of one walk are a run of neighbouring lanes: a lane takes a
+	   (destination row, walk) pair and sums its run's slots, so the pairs of
+	   all rows share a warp's instructions (a segmented shuffle sum, row by
+	   row, takes about three times as many, and as many passes of the
+	   shared-memory pipe, which bounds the large products: 6Li Nmax 6 3492 ->
+	   3419 us, FP32 2794 -> 2657; 7Li Nmax 4 with 3NF 88.2 -> 84.2; 4He Nmax 4
+	   16.4 -> 14.4).  Lanes past the view's chunks carry walk slot 0 after a
+	   higher one and hold zeros. */
 	const int ws_prev = __shfl_up_sync(0xffffffffu, ws, 1);     /* every lane takes part */
 	const unsigned int starts = __ballot_sync(0xffffffffu, lane == 0 || ws != ws_prev);
 	const unsigned int after = lane == 31 ? 0u : starts >> (lane + 1);
 	const int end = after ? lane + __ffs(after) : 32;
-	const bool first = (starts >> lane) & 1u;
-	const int longest = __reduce_max_sync(0xffffffffu, first ? (unsigned int)(end - lane) : 0u);
-	const int dw = (int)__ldg(walks + ta.z + ws);
-	for (int r = 0; r < rs; r++) {
-		unsigned long long v = slots[r * 32 + lane];
-		slots[r * 32 + lane] = 0ull;
-		for (int d = 1; d < longest; d <<= 1) {
-			const unsigned long long t = __shfl_down_sync(0xffffffffu, v, d);
-			if (lane + d < end) v += t;
-		}
-		if (first && v) {
-			const int dr = (int)__ldg(rdst + (int)pb.y + r);
-			atomicAdd(gacc + dst_off + (wp ? dw * Nn_dst + dr : dr * Nn_dst + dw), v);
+	if (lane == 0 || ws > ws_prev) tab[ws] = __ldg(walks + ta.z + ws) | ((uint32_t)lane << 16) | ((uint32_t)end << 21);
+	const uint32_t dr_of = lane < rs ? __ldg(rdst + (int)pb.y + lane) : 0u;
+	__syncwarp();
+	const int nw = (int)(ta.w & 0xffu), total = rs * nw;
+	const float per = __frcp_rn((float)nw);
+	for (int p0 = 0; p0 < total; p0 += 32) {
+		const int p = p0 + lane;
+		int r = (int)(((float)p + 0.5f) * per);         /* p / nw: p < 512 */
+		const int w = p - r * nw;
+		const uint32_t dr = __shfl_sync(0xffffffffu, dr_of, r & 31);
+		if (p < total) {
+			const uint32_t t = tab[w];
+			unsigned long long v = 0ull, *slot = slots + r * WALK_PITCH;
+			const int last = (int)(t >> 21);
+			for (int q = (int)((t >> 16) & 31u); q < last; q++) {
+				v += slot[q];
+				slot[q] = 0ull;
+			}
+			const int dw = (int)(t & 0xffffu);
+			if (v) atomicAdd(gacc + dst_off + (wp ? dw * Nn_dst + (int)dr : (int)dr * Nn_dst + dw), v);
 		}
 	}
 	__syncwarp();
@@ -245,6 +258,7 @@ __global__ void __launch_bounds__(WALK_THREADS, MODE == 32 ? 32 : 28)
 	extern __shared__ unsigned long long wslots[];
 	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 	unsigned long long *slots = wslots + warp * WALK_SLOTS;
+	uint32_t *tab = (uint32_t *)(wslots + WALK_WARPS * WALK_SLOTS) + warp * 32;
 	for (int i = lane; i < WALK_SLOTS; i += 32) slots[i] = 0ull;
 	__syncwarp();
 	/* from here on the kernel reads what the x view kernel wrote */
@@ -286,14 +300,14 @@ __global__ void __launch_bounds__(WALK_THREADS, MODE == 32 ? 32 : 28)
 		const uint4 pa = __ldg(pieces + 2 * ta.x), pb = __ldg(pieces + 2 * ta.x + 1);
 		const uint32_t U = (ta.w >> 8) & 0xffu;
 		if (U == 8)
-			walk_task<MODE, 8>(ta, pa, pb, lanes, walks, rows, rdst, groups, gshift, elem, x, xt, gacc, slots, lane, sh, scalef,
-					       scale);
+			walk_task<MODE, 8>(ta, pa, pb, lanes, walks, rows, rdst, groups, gshift, elem, x, xt, gacc, slots, tab, lane, sh,
+					       scalef, scale);
 		else if (U == 4)
-			walk_task<MODE, 4>(ta, pa, pb, lanes, walks, rows, rdst, groups, gshift, elem, x, xt, gacc, slots, lane, sh, scalef,
-					       scale);
+			walk_task<MODE, 4>(ta, pa, pb, lanes, walks, rows, rdst, groups, gshift, elem, x, xt, gacc, slots, tab, lane, sh,
+					       scalef, scale);
 		else
-			walk_task<MODE, 2>(ta, pa, pb, lanes, walks, rows, rdst, groups, gshift, elem, x, xt, gacc, slots, lane, sh, scalef,
-					       scale);
+			walk_task<MODE, 2>(ta, pa, pb, lanes, walks, rows, rdst, groups, gshift, elem, x, xt, gacc, slots, tab, lane, sh,
+					       scalef, scale);
 	}
 }
 
@@ -764,6 +778,7 @@ __global__ void __launch_bounds__(WALK_THREADS, MODE == 32 ? 32 : 28)
 	extern __shared__ unsigned long long wslots[];
 	const int lane = threadIdx.x & 31;
 	unsigned long long *slots = wslots;
+	uint32_t *tab = (uint32_t *)(wslots + WALK_SLOTS);
 	for (int i = lane; i < WALK_SLOTS; i += 32) slots[i] = 0ull;
 	__syncwarp();
 	const int64_t k = sel ? (int64_t)(*sel) : 0;
@@ -801,13 +816,13 @@ __global__ void __launch_bounds__(WALK_THREADS, MODE == 32 ? 32 : 28)
 		const uint32_t U = (ta.w >> 8) & 0xffu;
 		if (U == 8)
 			walk_task<MODE, 8>(ta, pa, pb, d->lanes, d->walks, d->rows, d->rdst, d->groups, NULL, elem, x, xt, d->gacc,
-					   slots, lane, sh, scalef, scale);
+					   slots, tab, lane, sh, scalef, scale);
 		else if (U == 4)
 			walk_task<MODE, 4>(ta, pa, pb, d->lanes, d->walks, d->rows, d->rdst, d->groups, NULL, elem, x, xt, d->gacc,
-					   slots, lane, sh, scalef, scale);
+					   slots, tab, lane, sh, scalef, scale);
 		else
 			walk_task<MODE, 2>(ta, pa, pb, d->lanes, d->walks, d->rows, d->rdst, d->groups, NULL, elem, x, xt, d->gacc,
-					   slots, lane, sh, scalef, scale);
+					   slots, tab, lane, sh, scalef, scale);
 	}
 }
 
