@@ -134,6 +134,13 @@ static double task_cost(const jn_plan_t *p, const uint32_t *T)
 	return (double)((T[2] - T[1] + R - 1) / R) * (diag ? 1.0 : 2.0) + 4.0;
 }
 
+double jn_panels_cost(const jn_plan_t *p)
+{
+	double c = 0.0;
+	for (int64_t k = 0; k < p->nptasks; k++) c += task_cost(p, p->ptasks + 4 * k);
+	return c;
+}
+
 /* qsort_r comparators: the plan comes with the call, so concurrent panel
  * builds share no state */
 static int cmp_task_cost(const void *a, const void *b, void *plan)

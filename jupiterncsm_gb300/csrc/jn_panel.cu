@@ -28,6 +28,7 @@
  * global accumulator.
  */
 #include <algorithm>
+#include <queue>
 #include <utility>
 #include <vector>
 
@@ -1120,7 +1121,8 @@ struct jn_panel_batch {
 	int nlist, threads;
 	size_t smem;
 	panel_multi_t kernel;
-	double work;                    /* coefficients of the instances the partition was made for */
+	double *cost;                   /* per basis: its tasks (jn_panels_cost) */
+	double work;                    /* cost of the instances the partition was made for */
 	unsigned int *d_ctrl;           /* max|x| bits of instance i at 2 i */
 	int max_blocks;
 };
@@ -1212,6 +1214,7 @@ void jn_panel_batch_free(jn_panel_batch *pb)
 	free(pb->parts);
 	free(pb->ctxs);
 	free(pb->basis);
+	free(pb->cost);
 	free(pb->h);
 	cudaFree(pb->d);
 	cudaFree(pb->d_list);
@@ -1229,8 +1232,54 @@ int jn_panel_batch_possible(jn_ctx *const *ctxs, int nbases)
 	return 1;
 }
 
+/* CTAs of each basis's instances: of the splits into CTAs of at most a target
+ * cost, the one with the earliest end when `slots` CTAs run at once and the
+ * next largest takes the first free slot.  `per_cta`: what a CTA of the basis
+ * pays beside its tasks.  (Shares by coefficients, rounded down, left 24 of
+ * 152 SMs without a large CTA and gave 4He Nmax 6 CTAs 1.3 times the cost of
+ * 6Li Nmax 4's: 315 us a product of those 64 Hamiltonians, 275 us like this.) */
+static void panel_batch_split(const std::vector<double> &cost, const std::vector<double> &per_cta, const std::vector<int> &count,
+			      int slots, std::vector<int> &g)
+{
+	double work = 0.0;
+	int64_t instances = 0;
+	for (size_t b = 0; b < cost.size(); b++) {
+		work += cost[b] * count[b];
+		instances += count[b];
+		g[b] = 1;
+	}
+	if (instances > 4 * (int64_t)slots || !(work > 0.0)) return;
+	double best = 0.0;
+	for (int k = 0; k <= 32; k++) {
+		const double target = work / slots * (1.0 + 0.03125 * k);
+		std::vector<int> t(cost.size(), 1);
+		std::vector<std::pair<double, int>> cta;        /* cost, how many */
+		for (size_t b = 0; b < cost.size(); b++) {
+			if (!count[b]) continue;
+			t[b] = (int)ceil(cost[b] / target);
+			if (t[b] < 1) t[b] = 1;
+			cta.push_back({ cost[b] / t[b] + per_cta[b], t[b] * count[b] });
+		}
+		std::sort(cta.begin(), cta.end(), [](const std::pair<double, int> &x, const std::pair<double, int> &y) { return x.first > y.first; });
+		std::priority_queue<double, std::vector<double>, std::greater<double>> busy;
+		for (int i = 0; i < slots; i++) busy.push(0.0);
+		double end = 0.0;
+		for (auto &c : cta)
+			for (int i = 0; i < c.second; i++) {
+				const double e = busy.top() + c.first;
+				busy.pop();
+				busy.push(e);
+				end = std::max(end, e);
+			}
+		if (k == 0 || end < best) {
+			best = end;
+			g = t;
+		}
+	}
+}
+
 /* Share the GPU's CTAs out among the active instances (NULL: all) by their
- * coefficients: the product's CTA list, the kernel that runs it, and the
+ * tasks' cost: the product's CTA list, the kernel that runs it, and the
  * descriptors.  Two shapes of CTA.  512 threads, three to an SM, where three
  * accumulators with x staged beside them fit an SM (small bases); else 1 024
  * threads, one to an SM, x staged where that fits.  With 512 threads and a
@@ -1243,12 +1292,19 @@ static jn_status panel_batch_partition(jn_panel_batch *pb, const int *act)
 {
 	const int sms = pb->ctxs[0]->num_sms;
 	std::vector<int> count(pb->nbases, 0), g(pb->nbases, 0);
+	const std::vector<double> cost(pb->cost, pb->cost + pb->nbases);
+	std::vector<double> per_cta(pb->nbases, 0.0);
 	double work = 0.0;
+	for (int b = 0; b < pb->nbases; b++) {
+		const jn_plan_t *p = &pb->ctxs[b]->plan;
+		/* clearing, staging and adding an accumulator of the whole vector, about 100 instructions a warp's words
+		   where a contribution takes 45, and the latencies at both ends */
+		per_cta[b] = 300.0 + 2.2 / 32 * (double)p->psmem_words;
+	}
 	for (int i = 0; i < pb->B; i++)
 		if (!act || act[i]) {
-			const int64_t nc = pb->ctxs[pb->basis[i]]->plan.n_coef;
 			count[pb->basis[i]]++;
-			work += (double)(nc ? nc : 1);
+			work += cost[pb->basis[i]];
 		}
 	int optin = 0, xs = 0;
 	CUDA_TRY(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, pb->ctxs[0]->device));
@@ -1268,11 +1324,10 @@ static jn_status panel_batch_partition(jn_panel_batch *pb, const int *act)
 		const int per = shape == 0 ? 3 : 1;
 		size_t with = 0, without = 0;
 		release();
+		panel_batch_split(cost, per_cta, count, per * sms, g);
 		for (int b = 0; b < pb->nbases; b++) {
 			if (!count[b]) continue;
 			const jn_plan_t *p = &pb->ctxs[b]->plan;
-			g[b] = (int)(per * sms * (double)(p->n_coef ? p->n_coef : 1) / work);
-			if (g[b] < 1) g[b] = 1;
 			if (jn_panels_partition(p, g[b], &hp[b].cta, &hp[b].fptr, &hp[b].flush, &hp[b].nf, &hp[b].words)) {
 				release();
 				return jn_fail(JN_ERR_NOMEM, "out of host memory");
@@ -1305,7 +1360,7 @@ static jn_status panel_batch_partition(jn_panel_batch *pb, const int *act)
 		pb->h[i].flush = pb->parts[b].flush;
 		pb->h[i].grid = g[b];
 		pb->h[i].words = (int)hp[b].words;
-		for (int k = 0; k < g[b]; k++) cl.push_back({ (double)pb->ctxs[b]->plan.n_coef / g[b], make_int2(i, k) });
+		for (int k = 0; k < g[b]; k++) cl.push_back({ cost[b] / g[b] + per_cta[b], make_int2(i, k) });
 	}
 	release();
 	if (s) return s;
@@ -1331,10 +1386,8 @@ jn_status jn_panel_batch_rebalance(jn_panel_batch *pb, const int *act, int *chan
 {
 	*changed = 0;
 	double work = 0.0;
-	for (int i = 0; i < pb->B; i++) {
-		const int64_t nc = pb->ctxs[pb->basis[i]]->plan.n_coef;
-		if (act[i]) work += (double)(nc ? nc : 1);
-	}
+	for (int i = 0; i < pb->B; i++)
+		if (act[i]) work += pb->cost[pb->basis[i]];
 	if (!(work > 0.0) || work > 0.6 * pb->work) return JN_OK;
 	*changed = 1;
 	return panel_batch_partition(pb, act);
@@ -1355,12 +1408,14 @@ jn_status jn_panel_batch_create(jn_ctx *const *ctxs, int nbases, const int *coun
 	pb->parts = (panel_part *)calloc((size_t)nbases, sizeof(panel_part));
 	pb->ctxs = (jn_ctx **)calloc((size_t)nbases, sizeof(jn_ctx *));
 	pb->basis = (int *)calloc((size_t)B, sizeof(int));
-	jn_status s = (!pb->h || !pb->parts || !pb->ctxs || !pb->basis) ? jn_fail(JN_ERR_NOMEM, "out of host memory") : JN_OK;
+	pb->cost = (double *)calloc((size_t)nbases, sizeof(double));
+	jn_status s = (!pb->cost || !pb->h || !pb->parts || !pb->ctxs || !pb->basis) ? jn_fail(JN_ERR_NOMEM, "out of host memory") : JN_OK;
 	for (int b = 0, i0 = 0; b < nbases && !s; i0 += count[b], b++) {
 		jn_ctx *c = ctxs[b];
 		pb->ctxs[b] = c;
 		if ((s = jn_panels_setup(c))) break;
 		const jn_plan_t *p = &c->plan;
+		pb->cost[b] = jn_panels_cost(p) + 1.0;
 		int *coef = NULL;
 		unsigned long long *cmax = NULL;
 		const int64_t nc = p->n_coef ? p->n_coef : 1;

@@ -357,6 +357,8 @@ int jn_plan_read_me(const jn_plan_t *plan, const char *dir, double *out, char *e
  * schedule gives bit-identical products. */
 int jn_panels_build(jn_plan_t *plan, int grid, int iter, char *err, size_t errlen);
 void jn_panels_free(jn_plan_t *plan);
+/* Total cost of the panel plan's tasks, in warp-wide contributions. */
+double jn_panels_cost(const jn_plan_t *plan);
 /* the CTA ranges and flush lists of the plan's tasks for a grid of `grid`
  * persistent CTAs (malloc'ed; the plan's own are those of plan->pgrid) */
 int jn_panels_partition(const jn_plan_t *plan, int grid, uint32_t **cta, uint32_t **flush_ptr, uint32_t **flush,
