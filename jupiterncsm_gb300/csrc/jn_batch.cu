@@ -776,6 +776,47 @@ static jn_status batch_solve(cudaStream_t q, const jn_batch_options *o, const ba
 	return st;
 }
 
+/* the largest |me| of n matrix elements (NaN left out) as its bits, which
+ * order as the values do; *out is zero before */
+__global__ void __launch_bounds__(BT) kb_max_abs(const double *__restrict__ me, int64_t n, unsigned long long *__restrict__ out)
+{
+	unsigned long long m = 0;
+	for (int64_t e = (int64_t)blockIdx.x * BT + threadIdx.x; e < n; e += (int64_t)gridDim.x * BT) {
+		const unsigned long long a = (unsigned long long)__double_as_longlong(me[e]) & 0x7fffffffffffffffull;
+		if (a <= 0x7ff0000000000000ull && a > m) m = a;
+	}
+	for (int o = 16; o; o >>= 1) {
+		const unsigned long long w = __shfl_xor_sync(0xffffffffu, m, o);
+		m = w > m ? w : m;
+	}
+	if ((threadIdx.x & 31) == 0 && m) atomicMax(out, m);
+}
+
+/* The fixed-point scale bound valid for every instance of a basis: the
+ * plan's bound for unit elements (kept with the plan: it depends on the lists
+ * alone) times max|M| of the uploaded elements me[0, n).  The maximum is a
+ * pass over device memory: on the host it read 160 MB element by element for
+ * 64 Hamiltonians (13 ms of their solves, with the unit bounds).  BALLOC
+ * leaves the 8 bytes after the elements. */
+static jn_status elements_bound(jn_ctx *c, double *me, int64_t n, double *bound, cudaStream_t q)
+{
+	jn_plan_t *p = &c->plan;
+	const double unit = p->unit_bound > 0.0 ? p->unit_bound : jn_plan_abs_bound(p, NULL);
+	if (isfinite(unit)) p->unit_bound = unit;       /* infinite: out of host memory */
+	unsigned long long *out = (unsigned long long *)(me + n);
+	double m = 0.0;
+	cudaError_t e = cudaMemsetAsync(out, 0, sizeof *out, q);
+	if (e == cudaSuccess && n > 0) {
+		kb_max_abs<<<(int)std::min<int64_t>((n + 4 * BT - 1) / (4 * BT), 2048), BT, 0, q>>>(me, n, out);
+		e = cudaGetLastError();
+	}
+	if (e == cudaSuccess) e = cudaMemcpyAsync(&m, out, sizeof m, cudaMemcpyDeviceToHost, q);
+	if (e == cudaSuccess) e = cudaStreamSynchronize(q);
+	if (e != cudaSuccess) return jn_fail(JN_ERR_CUDA, "matrix elements: %s", cudaGetErrorString(e));
+	*bound = unit * m;
+	return JN_OK;
+}
+
 /* HX = H_i X for the r vectors of B instances of one basis (X, HX: B x r
  * vectors Dp apart) on the block-tile engine in FP64: as many vectors at a
  * time as 512 MB of scratch and the grid take.  (One launch a vector, 56 for
@@ -842,12 +883,10 @@ extern "C" jn_status jn_lanczos_batch(jn_ctx *c, const jn_batch_options *o, jn_b
 	}
 	/* matrix elements: FP64 for refinement, FP32 copies with the reference's
 	   |M| < 1e-12 skip of single-species blocks (matrix_vector_multiplication.c:52-53) */
-	double maxme = 0.0;
 	float *h32 = !st && f32 && !panels ? (float *)malloc(nme * sizeof(float)) : NULL;
 	for (int i = 0; i < B && !st; i++) {
 		const double *me = o->matrix_elements[i];
 		if (!me) { st = jn_fail(JN_ERR_INVALID, "matrix_elements[%d] is NULL", i); break; }
-		for (int64_t e = 0; e < nme; e++) maxme = fmax(maxme, fabs(me[e]));
 		if (cudaMemcpyAsync(me64 + (size_t)i * nme, me, nme * sizeof(double), cudaMemcpyHostToDevice, q) != cudaSuccess)
 			st = jn_fail(JN_ERR_CUDA, "upload of matrix elements");
 		if (h32 && !st) {
@@ -866,10 +905,10 @@ extern "C" jn_status jn_lanczos_batch(jn_ctx *c, const jn_batch_options *o, jn_b
 	if (!st && gacc && cudaMemsetAsync(gacc, 0, (size_t)B * D * sizeof(unsigned long long), q) != cudaSuccess)
 		st = jn_fail(JN_ERR_CUDA, "accumulator clear");
 	/* fixed-point scale bound valid for every instance */
-	const double abs_bound = jn_plan_abs_bound(p, NULL) * maxme;
+	double abs_bound = 0.0;
+	if (!st) st = elements_bound(c, me64, (int64_t)B * nme, &abs_bound, q);
 	if (!st && panels) {
-		if (cudaStreamSynchronize(q) != cudaSuccess) st = jn_fail(JN_ERR_CUDA, "upload of matrix elements");
-		if (!st) st = jn_panel_batch_create(&c, 1, &B, &me64, &pb);
+		st = jn_panel_batch_create(&c, 1, &B, &me64, &pb);
 	}
 	int64_t *dims = (int64_t *)malloc(B * sizeof(int64_t));
 	jn_batch_result **rp = (jn_batch_result **)malloc(B * sizeof(jn_batch_result *));
@@ -959,14 +998,12 @@ extern "C" jn_status jn_lanczos_batch_bases(jn_ctx *const *ctxs, int num_bases, 
 		const jn_plan_t *p = &ctxs[b]->plan;
 		const int64_t nme = p->n_me;
 		BALLOC(me64[b], (size_t)count[b] * nme);
-		double maxme = 0.0;
 		for (int j = 0; j < count[b] && !st; j++) {
 			const double *m = me[first[b] + j];
-			for (int64_t e = 0; e < nme; e++) maxme = fmax(maxme, fabs(m[e]));
-			if (cudaMemcpy(me64[b] + (size_t)j * nme, m, nme * sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess)
+			if (cudaMemcpyAsync(me64[b] + (size_t)j * nme, m, nme * sizeof(double), cudaMemcpyHostToDevice, q) != cudaSuccess)
 				st = jn_fail(JN_ERR_CUDA, "upload of matrix elements");
 		}
-		bound[b] = jn_plan_abs_bound(p, NULL) * maxme;
+		if (!st) st = elements_bound(ctxs[b], me64[b], (int64_t)count[b] * nme, &bound[b], q);
 	}
 	/* the iteration products: one launch for every instance of every basis, on
 	   the panel engine where every basis runs it (32-bit products), else on the

@@ -1205,9 +1205,8 @@ void jn_panel_batch_free(jn_panel_batch *pb)
 			if (pb->h[i].owner) {
 				cudaFree((void *)pb->h[i].coef);
 				cudaFree((void *)pb->h[i].cmax);
+				cudaFree(pb->h[i].gacc);
 			}
-			cudaFree(pb->h[i].xi);
-			cudaFree(pb->h[i].gacc);
 		}
 	if (pb->parts)
 		for (int b = 0; b < pb->nbases; b++) panel_part_free(&pb->parts[b]);
@@ -1440,12 +1439,18 @@ jn_status jn_panel_batch_create(jn_ctx *const *ctxs, int nbases, const int *coun
 			d->nblocks = p->nblocks;
 		}
 		if (s) break;
-		for (int j = 0; j < count[b] && !s; j++) {
-			jn_panel_inst *d = &pb->h[i0 + j];
-			if (cudaMalloc((void **)&d->xi, (size_t)2 * (p->dim ? p->dim : 1) * sizeof(int)) != cudaSuccess ||
-			    cudaMalloc((void **)&d->gacc, (size_t)(p->dim ? p->dim : 1) * sizeof(unsigned long long)) != cudaSuccess ||
-			    cudaMemset(d->gacc, 0, (size_t)(p->dim ? p->dim : 1) * sizeof(unsigned long long)) != cudaSuccess)
-				s = jn_fail(JN_ERR_NOMEM, "cudaMalloc of batched panel buffers failed");
+		/* one allocation for the basis's instances: accumulators, then x views */
+		const size_t dim = (size_t)(p->dim ? p->dim : 1), n = (size_t)count[b];
+		unsigned long long *gacc = NULL;
+		if (cudaMalloc((void **)&gacc, n * dim * (sizeof *gacc + 2 * sizeof(int))) != cudaSuccess ||
+		    cudaMemset(gacc, 0, n * dim * sizeof *gacc) != cudaSuccess) {
+			cudaFree(gacc);
+			s = jn_fail(JN_ERR_NOMEM, "cudaMalloc of batched panel buffers failed");
+			break;
+		}
+		for (int j = 0; j < count[b]; j++) {
+			pb->h[i0 + j].gacc = gacc + (size_t)j * dim;
+			pb->h[i0 + j].xi = (int *)(gacc + n * dim) + (size_t)j * 2 * dim;
 		}
 		if (p->nblocks > pb->max_blocks) pb->max_blocks = p->nblocks;
 	}

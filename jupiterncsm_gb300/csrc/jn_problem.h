@@ -283,6 +283,7 @@ typedef struct {
 	int64_t nitems;    uint32_t *items;    /* warp items {first task, width | ntasks << 8} */
 	int max_tile_elems;             /* shared-memory accumulator size needed */
 	double abs_bound;               /* max over y elements of sum |M| over its contributions */
+	double unit_bound;              /* the same for matrix elements of 1 (jn_plan_abs_bound); 0 until asked for */
 	int *term_dst;                  /* destination basis block of each term */
 	/* accounting */
 	int64_t list_entries;           /* sum of distinct list lengths */
