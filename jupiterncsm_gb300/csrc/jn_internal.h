@@ -86,6 +86,8 @@ struct jn_ctx {
 	int2 *d_wxt;                    /* the transposed view of x that proton walks read, in the product's type */
 	void *d_wmany;                  /* accumulators, views of x and control words of several products at once */
 	int walk_many;                  /* vectors it holds */
+	double *d_subspace;             /* the subspace matrices' workspace, while it is small */
+	size_t subspace_bytes;
 	int32_t *d_wxperm;              /* position in x of each element of that view */
 };
 

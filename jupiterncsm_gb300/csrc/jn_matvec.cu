@@ -524,6 +524,7 @@ extern "C" void jn_close(jn_ctx *c)
 		if (c->prof_ev[i]) cudaEventDestroy(c->prof_ev[i]);
 	jn_panels_release(c);
 	jn_walk_release(c);
+	cudaFree(c->d_subspace);
 	jn_lanczos_release(c);
 	if (c->stream) cudaStreamDestroy(c->stream);
 	jn_plan_free(&c->plan);

@@ -86,6 +86,19 @@ def test_many_vectors(system, name, mode, n):
     H.close()
 
 
+def test_subspace_workspace(system):
+    """The workspace that stays between calls: calls that fit it, outgrow it, and are too large to be kept (68 MB)."""
+    d, Z, N = system("li6_n4")
+    H = jn.Hamiltonian.from_dir(d, Z, N)
+    v = np.random.default_rng(8).standard_normal((270, H.dimension))
+    norm, op = H.subspace_matrices(list(v[:5]))
+    for n in (40, 5, 270, 3, 5):
+        more = H.subspace_matrices(list(v[:n]))
+        m = min(n, 5)
+        assert np.array_equal(more[0][:m, :m], norm[:m, :m]) and np.array_equal(more[1][:m, :m], op[:m, :m])
+    H.close()
+
+
 @pytest.mark.parametrize("name", list(SYSTEMS))
 @pytest.mark.parametrize("bits", [32, 64])
 def test_panel_launches(system, name, bits):
