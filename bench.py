@@ -544,7 +544,7 @@ def solves_leg(workdir, seed=20261203):
             "plain_fp64_per_step_sync_solves_per_s": SOLVE_INSTANCES / sync_s,
             "max_eigenvalue_diff_vs_plain_fp64_MeV": worst,
             "mean_iterations": {"plain": float(np.mean(iters_plain)), "batched": float(np.mean(iters_batch))},
-            "batched": "one call for all 64 instances of the four bases: FP32 products (one persistent walk-engine "
+            "batched": "one call for all 64 instances of the four bases: FP32 products (one product "
                        "launch per step for every instance), FP64 recurrence + full reorthogonalisation + "
                        "Rayleigh-Ritz refinement, CUDA graph per step, convergence checked every 10 steps",
             "plain": "FP64 products and recurrence, one Hamiltonian at a time, CUDA graph per step, convergence "
