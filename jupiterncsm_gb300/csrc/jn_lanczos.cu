@@ -52,6 +52,14 @@
 #define RED_BLOCKS 304      /* 2 x 152 SMs */
 #define RED_THREADS 256
 
+/* Checks in flight, one more than the steps by which the host reads them
+ * behind: it enqueues steps k + 1 and k + 2, then reads check k.  A check
+ * takes about as long as a small basis's product (83 against 96 us for 4He
+ * Nmax 6), and one step behind left the host no time to enqueue the next
+ * before the device ran out: 165 steps with a check each 23.1 -> 21.1 ms, where
+ * a check every tenth takes 20.7. */
+#define CHECKS 3
+
 struct jn_lanczos_state {
 	int64_t D;
 	int mmax;               /* allocated Krylov dimension (vectors mmax+1) */
@@ -71,9 +79,9 @@ struct jn_lanczos_state {
 	double *d_ritz;         /* nev x D Ritz vectors */
 	double *d_hritz;        /* and H times them */
 	double *d_rr;           /* Rayleigh quotients, residual norms (2 nev_cap) */
-	double *h_pack[2];      /* pinned copies of d_pack: a check is read while the next one runs */
+	double *h_pack[CHECKS]; /* pinned copies of d_pack: a check is read while the next ones run */
 	cudaStream_t check;     /* the checks' stream */
-	cudaEvent_t stepped, checked[2];
+	cudaEvent_t stepped, checked[CHECKS];
 	int guesses;            /* entries of d_theta that hold eigenvalues of the last T of this solve */
 	int nev_cap;
 	int have_ritz;
@@ -87,7 +95,7 @@ void jn_lanczos_release(jn_ctx *c)
 	cudaFree(s->d_V); cudaFree(s->d_w); cudaFree(s->d_alpha); cudaFree(s->d_beta); cudaFree(s->d_part);
 	cudaFree(s->d_h); cudaFree(s->d_scalar); cudaFree(s->d_theta); cudaFree(s->d_Z); cudaFree(s->d_ritz);
 	cudaFree(s->d_work); cudaFree(s->d_done); cudaFree(s->d_pack); cudaFree(s->d_hritz); cudaFree(s->d_rr);
-	for (int i = 0; i < 2; i++) {
+	for (int i = 0; i < CHECKS; i++) {
 		if (s->h_pack[i]) cudaFreeHost(s->h_pack[i]);
 		if (s->checked[i]) cudaEventDestroy(s->checked[i]);
 	}
@@ -460,7 +468,7 @@ static jn_status ensure_state(jn_ctx *c, int mmax, int nev)
 	DALLOC(s->d_hritz, (size_t)nev * D);
 	DALLOC(s->d_rr, 2 * (size_t)nev);
 #undef DALLOC
-	for (int i = 0; i < 2; i++) {
+	for (int i = 0; i < CHECKS; i++) {
 		if (e == cudaSuccess) e = cudaMallocHost((void **)&s->h_pack[i], packed * sizeof(double));
 		if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s->checked[i], cudaEventDisableTiming);
 	}
@@ -563,7 +571,8 @@ extern "C" jn_status jn_lanczos(jn_ctx *c, const jn_lanczos_options *opt, jn_lan
 	const int og = (int)((D + chunk - 1) / chunk);
 
 	double prev = 0.0;
-	int k, converged = 0, pending = 0;      /* pending: rows of the check that is still to be read */
+	int k, converged = 0;
+	int pending[CHECKS], npending = 0;      /* rows of the checks that are still to be read, oldest first */
 	/* the eigenvector criterion keeps the previous step's vector (and the current one after it) */
 	const int by_vector = reference_mode && opt->criterion == JN_CONVERGE_EIGENVECTORS;
 	std::vector<double> zbuf(by_vector ? 2 * (size_t)(m + 1) : 0, 0.0);
@@ -573,7 +582,7 @@ extern "C" jn_status jn_lanczos(jn_ctx *c, const jn_lanczos_options *opt, jn_lan
 	const double t_loop = seconds_now();
 	/* the convergence test of T_n from its check's results: 1 converged, 0 not, -1 on an error (in st) */
 	auto test_full = [&](int n) -> int {
-		const int slot = n & 1, wv = nev < n ? nev : n, wt = wv + (wv < n ? 1 : 0);
+		const int slot = n % CHECKS, wv = nev < n ? nev : n, wt = wv + (wv < n ? 1 : 0);
 		const cudaError_t e = cudaEventSynchronize(s->checked[slot]);
 		if (e != cudaSuccess) {
 			st = jn_fail(JN_ERR_CUDA, "convergence check: %s", cudaGetErrorString(e));
@@ -640,26 +649,28 @@ extern "C" jn_status jn_lanczos(jn_ctx *c, const jn_lanczos_options *opt, jn_lan
 			if (diff < opt->tolerance) { converged = 1; k++; break; }
 			continue;
 		}
-		/* full mode: this step's check is enqueued, then the one before it is
-		   read, so the device always holds work; a solve that has converged
-		   has one step too many in flight, which nothing reads */
+		/* full mode: this step's check is enqueued, then the one two steps
+		   before it is read, so the device always holds work; a solve that has
+		   converged has two steps too many in flight, which nothing reads */
 		if (check) {
 			const int wv = nev < n ? nev : n;
-			st = tri_enqueue(c, n, wv + (wv < n ? 1 : 0), wv, n & 1);
+			st = tri_enqueue(c, n, wv + (wv < n ? 1 : 0), wv, n % CHECKS);
 			if (st) return st;
+			pending[npending++] = n;
 		}
-		if (pending) {
-			const int t = test_full(pending);
+		if (npending && pending[0] <= n - (CHECKS - 1)) {
+			const int t = test_full(pending[0]);
 			if (t < 0) return st;
-			if (t) { converged = 1; k = pending; pending = 0; break; }
+			if (t) { converged = 1; k = pending[0]; npending = 0; break; }
+			npending--;
+			for (int i = 0; i < npending; i++) pending[i] = pending[i + 1];
 		}
-		pending = check ? n : 0;
 	}
-	if (pending) {
-		const int t = test_full(pending);
+	for (int i = 0; i < npending && !converged; i++) {
+		const int t = test_full(pending[i]);
 		if (t < 0) return st;
 		converged = t;
-		k = pending;
+		k = pending[i];
 	}
 	s->k = k;
 	res->iterations = k;
