@@ -537,6 +537,20 @@ static void set_carveout(jn_ctx *c)
 	cudaGetLastError();
 }
 
+/* Rows a lane walks per task, from the tasks that JN_PANEL_ITER rows make and
+ * the warps that run them.  A task is a chain of shared-memory adds, so where
+ * the warps outnumber the tasks its length is the product's time: 4 rows;
+ * where a warp gets about one or two, 16; else the fixed cost of a task asks
+ * for JN_PANEL_ITER.  32-bit products with 32, 16, 8, 4, 2 rows, us with a
+ * synchronisation each: 4He Nmax 4 2NF (1510 tasks at 32 rows) 23.5, 22.0,
+ * 20.5, 19.3, 19.6, with 3NF 26.5, 22.3, 20.9, 20.2, 21.7; 4He Nmax 6 2NF
+ * (13 240) 33.0, 31.2, 32.3, 33.2, 36.7; 6Li Nmax 4 2NF (12 102) 41.3, 38.2,
+ * 39.1, 41.9, 47.1; 4He Nmax 6 2NF + 3NF (28 591) 73.1, 73.2, 78.4, 87.8, 116. */
+static int panel_iter(int64_t tasks, int warps)
+{
+	return tasks <= warps ? 4 : tasks <= 2 * (int64_t)warps ? 16 : JN_PANEL_ITER;
+}
+
 jn_status jn_panels_setup(jn_ctx *c)
 {
 	jn_plan_t *p = &c->plan;
@@ -599,15 +613,17 @@ jn_status jn_panels_setup(jn_ctx *c)
 	   33.7 us, with 3NF 228, 165, 133 us.  Where the whole vector fits twice
 	   there is no clear gain in a third (7Li Nmax 4 with 3NF 77.9, 80.0 us;
 	   5He Nmax 6 35.0, 33.0 us: x no longer fits beside the accumulator). */
-	for (int k = per[1] == 1 ? PANEL_MOST : per[1];; k--) {
-		if (jn_panels_build(p, c->num_sms * k, JN_PANEL_ITER, err, sizeof err))
+	const int most = per[1] == 1 ? PANEL_MOST : per[1];
+	const int iter = panel_iter(p->nptasks, c->num_sms * most * (PANEL_THREADS / 32));
+	for (int k = most;; k--) {
+		if (jn_panels_build(p, c->num_sms * k, iter, err, sizeof err))
 			return jn_fail(JN_ERR_NOMEM, "panel plan: %s", err);
 		if (k == per[1] || (size_t)k * (panel_smem_words(p, p->pcta_words, 0) + 1024) <= (size_t)c->smem_per_sm) {
 			if (k > per[1]) c->panel_per_sm[0] = c->panel_per_sm[1] = k;
 			break;
 		}
 	}
-	c->panel_iter = JN_PANEL_ITER;
+	c->panel_iter = iter;
 	jn_status s;
 	if ((s = upload_n(&c->d_panels, p->panels, (size_t)p->npanels)) ||
 	    (s = upload_n(&c->d_ptasks, p->ptasks, (size_t)p->nptasks * 4)) ||
@@ -966,7 +982,7 @@ static jn_status autotune(jn_ctx *c, int trials, int tune_engine, jn_tuning *out
 	float best = 3.4e38f;
 	int best_engine = engine0, best_iter = c->panel_iter, best_per = c->panel_grid / (c->num_sms ? c->num_sms : 1);
 	if (jn_panels_setup(c) == JN_OK && jn_panels_fit(c, f32) && (engine0 == 4 || tune_engine)) {
-		const int iters[] = { 8, 16, 32, 64, 128 };
+		const int iters[] = { 4, 8, 16, 32, 64, 128 };
 		const int maxper = c->panel_per_sm[0] && c->panel_per_sm[0] < c->panel_per_sm[1] ? c->panel_per_sm[0]
 												    : c->panel_per_sm[1];
 		c->engine = 4;

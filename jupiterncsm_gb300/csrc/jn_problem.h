@@ -171,7 +171,7 @@ typedef struct {
  */
 #define JN_PANEL_DIAG 8          /* input block == output block: no transpose */
 #define JN_PANEL_ROWS_N 16       /* NP panel stored transposed: rows are neutron entries, columns proton entries */
-#define JN_PANEL_ITER 32         /* rows a lane walks per task (default; the autotuner may choose another) */
+#define JN_PANEL_ITER 32         /* rows a lane walks per task (fewer for small plans; the autotuner may choose another) */
 #define JN_PANEL_MAX_DIM 26624   /* the accumulator (8 B per state, rows padded to an odd length) in shared memory */
 
 typedef struct {
