@@ -884,13 +884,17 @@ static jn_status check_x_range(const jn_ctx *c, const double *x)
 extern "C" jn_status jn_matvec(jn_ctx *c, const double *x, double *y)
 {
 	if (!c || !x || !y) return fail(JN_ERR_INVALID, "null argument");
-	jn_status rs = check_x_range(c, x);
-	if (rs) return rs;
 	const size_t bytes = (size_t)c->plan.dim * sizeof(double);
 	CUDA_TRY(cudaMemcpyAsync(c->d_x, x, bytes, cudaMemcpyHostToDevice, c->stream));
 	CUDA_TRY(cudaMemcpyAsync(c->d_y, y, bytes, cudaMemcpyHostToDevice, c->stream));
 	jn_status s = jn_launch_matvec(c, c->d_x, c->d_y, 1, c->stream);
-	if (s) return s;
+	/* x is checked while the product runs; out of range, its result is not
+	   copied back and y stays as it was */
+	jn_status rs = check_x_range(c, x);
+	if (rs || s) {
+		cudaStreamSynchronize(c->stream);
+		return rs ? rs : s;
+	}
 	CUDA_TRY(cudaMemcpyAsync(y, c->d_y, bytes, cudaMemcpyDeviceToHost, c->stream));
 	CUDA_TRY(cudaStreamSynchronize(c->stream));
 	return JN_OK;

@@ -117,3 +117,21 @@ def test_panel_launches(system, name, bits):
         assert np.array_equal(H.matvec(v).view(np.uint64), emu4(d, Z, N, v, bits == 32).view(np.uint64))
     assert not H.matvec(np.zeros(D)).any()
     H.close()
+
+
+@pytest.mark.parametrize("engine,bits", [(5, 64), (5, 32), (4, 32), (3, 64)])
+def test_refused_x_leaves_y(system, engine, bits):
+    """x is checked while the product already runs: out of range, y is untouched and the next product is right."""
+    d, Z, N = system("he4_n4")
+    H = jn.Hamiltonian.from_dir(d, Z, N)
+    H.set_engine(engine)
+    H.set_precision(bits)
+    x = np.random.default_rng(9).standard_normal(H.dimension)
+    want = H.matvec(x)
+    for bad in (1e300, np.inf, np.nan, 1e-200):
+        y = np.arange(H.dimension, dtype=np.float64)
+        with pytest.raises(jn.JnError):
+            H.matvec(np.full(H.dimension, bad), y)
+        assert np.array_equal(y, np.arange(H.dimension))
+        assert np.array_equal(H.matvec(x).view(np.uint64), want.view(np.uint64))
+    H.close()
