@@ -49,7 +49,7 @@
 
 #include <type_traits>
 
-#define WALK_WARPS 1     /* one warp a CTA: 32 resident CTAs an SM, the most the integer path's 63 registers allow too */
+#define WALK_WARPS 1     /* one warp a CTA: the register file alone sets how many an SM holds */
 #define WALK_THREADS (WALK_WARPS * 32)
 #define WALK_PITCH 33    /* words of a slot row: lanes on different rows of one column hit different banks */
 #define WALK_SLOTS (JN_WALK_RS * WALK_PITCH)    /* per warp: one 64-bit slot per (destination row, lane) */
@@ -244,7 +244,9 @@ __device__ __forceinline__ void walk_task(const uint4 ta, const uint4 pa, const 
 	__syncwarp();
 }
 
-/* FP32: 32 warps an SM (64 registers); the 64-bit paths need more registers: 28 (72) */
+/* FP32: 32 warps an SM (64 registers); the 64-bit paths 28 (the integer path
+ * uses 68).  With 64 registers and 32 warps the integer path's warps have less
+ * L1 each: 6Li Nmax 6 takes 3524 us, not 3420; with 20 warps 3726. */
 template <int MODE, bool MANY>
 __global__ void __launch_bounds__(WALK_THREADS, MODE == 32 ? 32 : 28)
 	jn_walk_kernel(const uint4 *__restrict__ tasks, const uint4 *__restrict__ pieces, const uint32_t *__restrict__ lanes,
@@ -376,7 +378,10 @@ __global__ void __launch_bounds__(WALK_SMALL_THREADS)
 {
 	typedef typename WalkT<MODE>::X X;
 	__shared__ unsigned long long wmax[WALK_SMALL_THREADS / 32];
+	/* x, and the product before this one, which reads the views and ctrl */
+	pdl_wait();
 	pdl_trigger();
+	x = pdl_after(x);
 	x += (int64_t)blockIdx.y * n;
 	if (MODE != 64) xv += (int64_t)blockIdx.y * n;
 	if (perm) xt += (int64_t)blockIdx.y * n;
@@ -405,6 +410,7 @@ __global__ void jn_walk_finalize_kernel(unsigned long long *__restrict__ gacc, d
 					int accumulate)
 {
 	pdl_wait();
+	pdl_trigger();
 	ctrl = pdl_after(ctrl) + 2 * blockIdx.y;
 	gacc = pdl_after(gacc) + blockIdx.y * n;
 	y += blockIdx.y * n;
@@ -585,7 +591,10 @@ static jn_status walk_elements(jn_ctx *c, int mode)
  * walk engine: max|x| and the converted copies of x, the walk kernel, the
  * conversion of the accumulators into Y.  Each kernel is set up while the one
  * before it still runs (jn_pdl.cuh): without that overlap the gaps and
- * launches cost 6 us more at any size.  xv, xt, gacc and ctrl hold nvec
+ * launches cost 6 us more at any size, and where the first kernel overlaps the
+ * product before it as well (up to WALK_SMALL_DIM states), 2 us more: products
+ * back to back at D = 59 / 952 / 10 817 / 7916 10.3 / 14.4 / 84.1 / 96.6 -> 8.1 /
+ * 13.1 / 82.1 / 93.9 us.  xv, xt, gacc and ctrl hold nvec
  * vectors (control words 2 v). */
 template <int MODE>
 static jn_status walk_launch(jn_ctx *c, const double *d_x, double *d_y, int nvec, int accumulate, int2 *wx, int2 *wxt,
@@ -603,8 +612,14 @@ static jn_status walk_launch(jn_ctx *c, const double *d_x, double *d_y, int nvec
 	   unless an event was recorded in between */
 	int overlap = 1;
 	if (p->dim <= WALK_SMALL_DIM) {
-		jn_walk_small_x_kernel<MODE><<<dim3((unsigned int)((p->dim + WALK_SMALL_THREADS - 1) / WALK_SMALL_THREADS), nvec),
-					       WALK_SMALL_THREADS, 0, st>>>(d_x, perm, xv, xt, (int)p->dim, ctrl);
+		/* overlaps whatever kernel precedes it on the stream (back to back that
+		   is the last product's conversion), except in a capture, where what
+		   precedes it may be no kernel */
+		cudaStreamCaptureStatus cs = cudaStreamCaptureStatusActive;
+		const int first = !pre && cudaStreamIsCapturing(st, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone;
+		pdl_launch(first, jn_walk_small_x_kernel<MODE>,
+			   dim3((unsigned int)((p->dim + WALK_SMALL_THREADS - 1) / WALK_SMALL_THREADS), nvec), WALK_SMALL_THREADS, 0, st,
+			   d_x, perm, xv, xt, (int)p->dim, ctrl);
 	} else {
 		CUDA_TRY(cudaMemsetAsync(ctrl, 0, (size_t)nvec * 2 * sizeof(unsigned int), st));
 		jn_walk_max_kernel<<<dim3(g, nvec), 256, 0, st>>>(d_x, p->dim, ctrl);
