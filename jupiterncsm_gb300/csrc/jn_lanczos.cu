@@ -29,7 +29,7 @@
  * cooperative kernel (k_orthonormalize) takes w = H v_k to v_{k+1}.  The
  * convergence check (k_tri_check: eigenvalues of T by multisection and their
  * eigenvectors, jn_tridiag.cuh) runs on its own stream beside the next
- * step's product: the host enqueues step k + 1, then reads the check of
+ * steps' products: the host enqueues steps k + 1 and k + 2, then reads the check of
  * step k.  The final Ritz vectors are refined by FP64 products (Rayleigh
  * quotient and residual norm).
  */

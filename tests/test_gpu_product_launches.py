@@ -135,3 +135,41 @@ def test_refused_x_leaves_y(system, engine, bits):
         assert np.array_equal(y, np.arange(H.dimension))
         assert np.array_equal(H.matvec(x).view(np.uint64), want.view(np.uint64))
     H.close()
+
+
+@pytest.mark.parametrize("name", ["he4_n4", "li6_n4"])
+@pytest.mark.parametrize("engine,bits", [(5, 64), (5, 32), (4, 32)])
+def test_products_in_a_caller_graph(system, name, engine, bits):
+    """A caller's graph of a copy, two products and a scaling: the products' own overlapped launches join the capture."""
+    import torch
+    d, Z, N = system(name)
+    H = jn.Hamiltonian.from_dir(d, Z, N)
+    H.set_engine(engine)
+    H.set_precision(bits)
+    D = H.dimension
+    src = torch.from_numpy(np.random.default_rng(10).standard_normal(D)).cuda()
+    a, b, c = (torch.zeros_like(src) for _ in range(3))
+    st = torch.cuda.Stream()
+
+    def work():
+        a.copy_(src)
+        H.matvec_device(a.data_ptr(), b.data_ptr(), False, st.cuda_stream)
+        b.mul_(2.0 ** -6)
+        H.matvec_device(b.data_ptr(), c.data_ptr(), False, st.cuda_stream)
+
+    torch.cuda.synchronize()
+    with torch.cuda.stream(st):
+        work()
+    st.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=st):
+        work()
+    for k in range(3):
+        src.copy_(torch.from_numpy(np.random.default_rng(11 + k).standard_normal(D)))
+        torch.cuda.synchronize()
+        g.replay()
+        torch.cuda.synchronize()
+        want = H.matvec(H.matvec(src.cpu().numpy()) * 2.0 ** -6)
+        assert np.array_equal(c.cpu().numpy().view(np.uint64), want.view(np.uint64))
+    del g
+    H.close()
