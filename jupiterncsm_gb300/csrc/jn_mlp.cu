@@ -200,7 +200,7 @@ static int threads_for(const jn_mlp *m)
 /* Networks whose weights fit an SM's shared memory (hidden widths up to
  * about 200) run here: one cooperative launch, one CTA an SM, for up to
  * FUSED_STEPS Adam steps.  Per step, phase A: every CTA loads the weights
- * (L2 to shared memory, 16-byte asynchronous copies) and takes SP samples
+ * (L2 to shared memory, bulk copies) and takes SP samples
  * through the forward pass and the deltas, a thread per unit; phase B: every
  * CTA takes 16 x 16 tiles of (weight matrix | bias), sums their gradient
  * over the samples and updates its parameters.  Two grid-wide barriers a step.
@@ -208,18 +208,18 @@ static int threads_for(const jn_mlp *m)
  * inputs ascending; samples ascending), so the results are the same bits.
  * What bounds it: shared-memory reads (a wavefront for every 128 bytes that
  * a warp's lanes take in, equal or not) and the two barriers (1.1 us each).
- * 4-128-128-32 on 256 samples: 12.7 us a step (phase A 6.1, of which 1.2 the
- * weights; phase B 2.9), where the five kernels of the other path take 102
- * us, 90 of them in strided reads of weights and activations.  With every
- * CTA fetching the weights by itself the weights alone took 5.0 us: 152 x 85
- * KB is more than L2 gives in less; as one bulk copy shared by a cluster of
- * 8 they cost an eighth of that traffic. */
+ * 4-128-128-32 on 256 samples: 10.8 us a step, where the five kernels of the
+ * other path take 102 us, 90 of them in strided reads of weights and
+ * activations.  The weights as 8 bulk copies a CTA; measured with the CTAs in
+ * clusters of 8, which do not fill all SMs, that takes 12.9 us a step, 32 copies 13.3, 16-byte
+ * asynchronous copies by all threads 14.0, and an eighth from L2 with the rest
+ * from the shared memory of seven neighbours 17.6 to 17.9. */
 #define FUSED_STEPS 1024
 #define FUSED_THREADS 512       /* at most: 128 registers a thread */
 #define FUSED_TILE 16
 #define FUSED_CHUNK 256         /* samples staged at a time in phase B */
 #define FUSED_PITCH (FUSED_CHUNK + 4)
-#define FUSED_CLUSTER 8
+#define FUSED_PARTS 8           /* copies of a fetch of the weights */
 
 /* row pitch in floats: a multiple of 4, 4 modulo 32, so that 16-byte reads
  * of one column group by 8 neighbouring rows touch all 32 banks */
@@ -241,10 +241,10 @@ struct fused_args {
 	float lr, b1, b2, eps;
 };
 
-/* words of the weights' image: W1, W2 and W3 with padded rows, in equal 16-byte shares for the CTAs of a cluster */
+/* words of the weights' image: W1, W2 and W3 with padded rows, in FUSED_PARTS equal parts of 16-byte units */
 __host__ __device__ static inline size_t fused_words(int nin, int nh, int nout)
 {
-	const size_t w = (size_t)nh * fused_pitch(nin) + (size_t)(nh + nout) * fused_pitch(nh), unit = 4 * FUSED_CLUSTER;
+	const size_t w = (size_t)nh * fused_pitch(nin) + (size_t)(nh + nout) * fused_pitch(nh), unit = 4 * FUSED_PARTS;
 	return (w + unit - 1) / unit * unit;
 }
 
@@ -257,17 +257,20 @@ static size_t fused_smem(int nin, int nh, int nout, int sp)
 }
 
 /* The weights' image (the shared-memory layout, kept in global memory beside
- * the parameters) to every CTA of the cluster at once: CTA `rank` fetches its
- * share as one bulk copy that lands at the same place in all CTAs and
- * completes on each one's barrier.  One thread; every CTA takes part. */
+ * the parameters) into the CTA's shared memory: FUSED_PARTS bulk copies that
+ * complete on its barrier, by its first warp.  Each CTA starts at another
+ * part, so that the CTAs do not all ask L2 for the same lines at once. */
 __device__ __forceinline__ void fused_fetch(const float *image, int words, float *s, unsigned int bar)
 {
-	const int share = words / FUSED_CLUSTER, at = (int)(blockIdx.x % FUSED_CLUSTER) * share;
-	const unsigned int dst = (unsigned int)__cvta_generic_to_shared(s + at);
-	asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(words * 4) : "memory");
-	asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.multicast::cluster [%0], [%1], %2, [%3], %4;"
-		     ::"r"(dst), "l"(image + at), "r"(share * 4), "r"(bar), "h"((unsigned short)((1 << FUSED_CLUSTER) - 1))
-		     : "memory");
+	if (threadIdx.x == 0) asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(words * 4) : "memory");
+	__syncwarp();
+	if (threadIdx.x < FUSED_PARTS) {
+		const int part = words / FUSED_PARTS, at = (int)((threadIdx.x + blockIdx.x) % FUSED_PARTS) * part;
+		const unsigned int dst = (unsigned int)__cvta_generic_to_shared(s + at);
+		asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+			     ::"r"(dst), "l"(image + at), "r"(part * 4), "r"(bar)
+			     : "memory");
+	}
 }
 
 /* wait for phase `parity` of the barrier, at most about a second; false if it gave up */
@@ -346,8 +349,8 @@ __device__ __forceinline__ void fused_col(float *acc, const float *w, int pitch,
 
 /* phase A: forward pass of every sample; with deltas, also back-propagation
  * and the activations that phase B reads.  round: how often the launch has
- * been here (the barrier's phase).  A CTA without samples takes part in the
- * cluster's copies. */
+ * been here (the barrier's phase).  A CTA without samples fetches the
+ * weights as well, so that all barriers keep the same phase. */
 template <int SP>
 __device__ __forceinline__ void fused_samples(const fused_args &a, const mlp_off &o, float *sm, size_t weights, unsigned int bar, unsigned int round,
 					      bool deltas, int eval)
@@ -357,7 +360,7 @@ __device__ __forceinline__ void fused_samples(const fused_args &a, const mlp_off
 	float *w1 = sm, *w2 = w1 + (size_t)nh * p1, *w3 = w2 + (size_t)nh * p2;
 	float *x = sm + weights, *h1 = x + SP * lx, *h2 = h1 + SP * lh, *d2 = h2 + SP * lh, *e3 = d2 + SP * lh, *d3 = e3 + SP * lo;
 	const int groups = (a.n + SP - 1) / SP;
-	if (threadIdx.x == 0) fused_fetch(a.image, (int)fused_words(nin, nh, nout), sm, bar);
+	if (threadIdx.x < 32) fused_fetch(a.image, (int)fused_words(nin, nh, nout), sm, bar);
 	const float *P = a.P;
 	/* the outputs of the CTA's samples, one sample a thread where they fit */
 	const bool spread = SP * nout <= (int)blockDim.x;
@@ -554,7 +557,7 @@ __device__ __forceinline__ void fused_parameters(const fused_args &a, const mlp_
 }
 
 template <int SP>
-__global__ void __cluster_dims__(FUSED_CLUSTER, 1, 1) __launch_bounds__(FUSED_THREADS) mlp_fused(const fused_args a)
+__global__ void __launch_bounds__(FUSED_THREADS) mlp_fused(const fused_args a)
 {
 	extern __shared__ __align__(16) float sm[];
 	__shared__ __align__(8) unsigned long long mbar;
@@ -586,8 +589,6 @@ __global__ void __cluster_dims__(FUSED_CLUSTER, 1, 1) __launch_bounds__(FUSED_TH
 		grid.sync();
 	}
 	if (!a.grad && a.eval) fused_samples<SP>(a, o, sm, weights, bar, round++, false, a.eval);
-	/* no CTA leaves while another of the cluster may still copy into it */
-	cg::this_cluster().sync();
 }
 
 /* the fused launch for n samples and its grid, or NULL where the network does not fit it */
@@ -601,20 +602,14 @@ static fused_kernel fused_for(const jn_mlp *m, int n, size_t *smem, int *grid)
 	*smem = fused_smem(m->nin, m->nh, m->nout, sp);
 	if (*smem > FUSED_SMEM_LIMIT || threads_for(m) > FUSED_THREADS) return NULL;
 	fused_kernel f = sp == 1 ? mlp_fused<1> : sp == 2 ? mlp_fused<2> : sp == 4 ? mlp_fused<4> : mlp_fused<8>;
-	/* the grid must be resident at once: at most one CTA an SM, in whole clusters */
-	cudaLaunchConfig_t cfg;
-	memset(&cfg, 0, sizeof cfg);
-	*grid = m->num_sms / FUSED_CLUSTER * FUSED_CLUSTER;
-	cfg.gridDim = dim3(*grid);
-	cfg.blockDim = dim3(fused_threads(m));
-	cfg.dynamicSmemBytes = *smem;
-	int clusters = 0;
+	/* the grid must be resident at once: one CTA an SM */
+	int per_sm = 0;
 	if (cudaFuncSetAttribute((const void *)f, cudaFuncAttributeMaxDynamicSharedMemorySize, FUSED_SMEM_LIMIT) != cudaSuccess ||
-	    cudaOccupancyMaxActiveClusters(&clusters, (const void *)f, &cfg) != cudaSuccess || clusters < 1) {
+	    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void *)f, fused_threads(m), *smem) != cudaSuccess || per_sm < 1) {
 		cudaGetLastError();
 		return NULL;
 	}
-	if (*grid > clusters * FUSED_CLUSTER) *grid = clusters * FUSED_CLUSTER;
+	*grid = m->num_sms;
 	return f;
 }
 
