@@ -573,6 +573,10 @@ jn_status jn_mlp_loss_and_gradient(jn_mlp *mlp, const float *x, const float *t, 
 jn_status jn_mlp_train(jn_mlp *mlp, const float *x, const float *t, int n, int steps, float learning_rate,
 		       float *final_loss);
 jn_status jn_mlp_predict(jn_mlp *mlp, const float *x, int n, float *y);
+/* Polls of up to a microsecond after which a kernel's wait for its copy of the
+ * weights gives up (default 2^20).  The call then fails with JN_ERR_TIMEOUT;
+ * a training run stops before the step's parameters are changed. */
+jn_status jn_mlp_set_wait_limit(jn_mlp *mlp, int polls);
 
 /*
  * The warm start for jn_lanczos_batch.  Fitting takes solutions that the

@@ -191,6 +191,7 @@ def gpu_lib():
     L.jn_mlp_loss_and_gradient.argtypes = [vp, vp, vp, ci, fp, vp]
     L.jn_mlp_train.argtypes = [vp, vp, vp, ci, ci, ctypes.c_float, fp]
     L.jn_mlp_predict.argtypes = [vp, vp, ci, vp]
+    L.jn_mlp_set_wait_limit.argtypes = [vp, ci]
     L.jn_warm_start_fit.argtypes = [ctypes.POINTER(WarmStartOptions), ctypes.c_int64, ci, ci, vp, ci, vp,
                                     ctypes.POINTER(vp), fp]
     L.jn_warm_start_vectors.argtypes = [vp, ci, vp, vp]
@@ -201,7 +202,7 @@ def gpu_lib():
     L.jn_default_start_vector.argtypes = [ctypes.c_int64, vp]
     L.jn_default_start_vector.restype = None
     for name in ("jn_mlp_create", "jn_mlp_get_params", "jn_mlp_set_params", "jn_mlp_loss_and_gradient",
-                 "jn_mlp_train", "jn_mlp_predict", "jn_warm_start_fit", "jn_warm_start_vectors",
+                 "jn_mlp_train", "jn_mlp_predict", "jn_mlp_set_wait_limit", "jn_warm_start_fit", "jn_warm_start_vectors",
                  "jn_warm_start_basis"):
         getattr(L, name).restype = ci
     L.jn_subspace_matrices.argtypes = [vp, ci, vp, vp, vp]
@@ -543,6 +544,10 @@ class MLP:
         y = np.zeros((len(x), self.shape[2]), dtype=np.float32)
         _check(gpu_lib().jn_mlp_predict(self._h, x.ctypes.data, len(x), y.ctypes.data))
         return y
+
+    def set_wait_limit(self, polls):
+        """Polls after which a kernel's wait for its copy of the weights gives up (JN_ERR_TIMEOUT)."""
+        _check(gpu_lib().jn_mlp_set_wait_limit(self._h, int(polls)))
 
 
 def aurora(comb, anicre_dir, output_dir, Z, N, human_readable=False, skip_three_body=False):

@@ -33,8 +33,9 @@ struct jn_mlp {
 	int cap;                        /* samples the activation buffers hold */
 	/* activations, one allocation (d_x): sample by sample, or unit by unit on the fused path */
 	float *d_x, *d_t, *d_a1, *d_h1, *d_a2, *d_h2, *d_y, *d_d1, *d_d2, *d_d3, *d_loss;
-	float *d_corr;                  /* the fused path's bias corrections, then its word for a wait that gave up */
+	float *d_corr;                  /* the fused path's bias corrections, then its two status words */
 	float *d_image;                 /* and its image of the weights */
+	int polls;                      /* limit of a wait for a copy of it */
 	cudaStream_t stream;
 };
 
@@ -208,7 +209,7 @@ static int threads_for(const jn_mlp *m)
  * inputs ascending; samples ascending), so the results are the same bits.
  * What bounds it: shared-memory reads (a wavefront for every 128 bytes that
  * a warp's lanes take in, equal or not) and the two barriers (1.1 us each).
- * 4-128-128-32 on 256 samples: 10.8 us a step, where the five kernels of the
+ * 4-128-128-32 on 256 samples: 11.7 us a step, where the five kernels of the
  * other path take 102 us, 90 of them in strided reads of weights and
  * activations.  The weights as 8 bulk copies a CTA; measured with the CTAs in
  * clusters of 8, which do not fill all SMs, that takes 12.9 us a step, 32 copies 13.3, 16-byte
@@ -237,7 +238,9 @@ struct fused_args {
 	float *Y, *lossp;
 	const float *corr;              /* the steps' bias corrections, c1 and c2 of each */
 	float *image;                   /* the weights in the shared-memory layout */
-	unsigned int *fail;             /* set when a wait gave up */
+	unsigned int *status;           /* set when a wait gave up; Adam steps taken, `before` and this launch's */
+	int before;
+	int polls;
 	float lr, b1, b2, eps;
 };
 
@@ -273,10 +276,11 @@ __device__ __forceinline__ void fused_fetch(const float *image, int words, float
 	}
 }
 
-/* wait for phase `parity` of the barrier, at most about a second; false if it gave up */
-__device__ __forceinline__ bool fused_wait(unsigned int bar, unsigned int parity)
+/* wait for phase `parity` of the barrier, at most `polls` times up to a microsecond; false if it gave up */
+#define FUSED_POLLS (1 << 20)
+__device__ __forceinline__ bool fused_wait(unsigned int bar, unsigned int parity, int polls)
 {
-	for (int i = 0; i < 1 << 20; i++) {
+	for (int i = 0; i < polls; i++) {
 		unsigned int done;
 		asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, 1000;\n\tselp.u32 %0, 1, 0, p;\n\t}"
 			     : "=r"(done)
@@ -285,6 +289,17 @@ __device__ __forceinline__ bool fused_wait(unsigned int bar, unsigned int parity
 		if (done) return true;
 	}
 	return false;
+}
+
+/* The wait for the weights.  If it gives up, the status word is set and the
+ * copies are waited for once more, so that none lands after the CTA has gone
+ * on; the grid leaves the step loop in the phase B that follows, before any
+ * parameter is changed. */
+__device__ __forceinline__ void fused_land(const fused_args &a, unsigned int bar, unsigned int parity)
+{
+	if (fused_wait(bar, parity, a.polls)) return;
+	*a.status = 1;
+	fused_wait(bar, parity, FUSED_POLLS);
 }
 
 /* acc[s] += sum_k w[k] v[s][k], k ascending (w a padded shared row, v at
@@ -379,7 +394,7 @@ __device__ __forceinline__ void fused_samples(const fused_args &a, const mlp_off
 		}
 		if (!landed) {
 			landed = true;
-			if (!fused_wait(bar, round & 1)) *a.fail = 1;
+			fused_land(a, bar, round & 1);
 		}
 		__syncthreads();
 		float z1[SP], z2[SP], acc[SP];
@@ -462,7 +477,8 @@ __device__ __forceinline__ void fused_samples(const fused_args &a, const mlp_off
 		__syncthreads();        /* the next samples overwrite x, h1, ... */
 	}
 	/* no CTA goes on with copies in flight */
-	if (!landed && !fused_wait(bar, round & 1)) *a.fail = 1;
+	/* no CTA goes on with copies in flight */
+	if (!landed) fused_land(a, bar, round & 1);
 }
 
 /* one parameter's Adam update, or its gradient: p in the parameter array, at
@@ -482,8 +498,9 @@ __device__ __forceinline__ void fused_update(const fused_args &a, int64_t p, int
 }
 
 /* phase B: the gradient of 16 x 16 tiles of W, a parameter a thread, and
- * with a matrix's first column tile of its bias; with adam the update */
-__device__ __forceinline__ void fused_parameters(const fused_args &a, const mlp_off &o, float *sm, bool adam, float c1, float c2)
+ * with a matrix's first column tile of its bias; with adam the update.  Nothing
+ * is written if a wait gave up. */
+__device__ __forceinline__ void fused_parameters(const fused_args &a, const mlp_off &o, float *sm, bool adam, float c1, float c2, unsigned int gave_up)
 {
 	float *ds = sm, *as = sm + FUSED_TILE * FUSED_PITCH;
 	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, t = threadIdx.x;
@@ -548,6 +565,7 @@ __device__ __forceinline__ void fused_parameters(const fused_args &a, const mlp_
 				}
 			}
 		}
+		if (gave_up) break;
 		if (mine) fused_update(a, p, image + r * pitch + c, g, adam, c1, c2, pv, mv, vv);
 		if (bias) fused_update(a, pb, -1, gb, adam, c1, c2, pbv, mbv, vbv);
 	}
@@ -563,6 +581,7 @@ __global__ void __launch_bounds__(FUSED_THREADS) mlp_fused(const fused_args a)
 	__shared__ __align__(8) unsigned long long mbar;
 	namespace cg = cooperative_groups;
 	cg::grid_group grid = cg::this_grid();
+	if (__ldcg(a.status)) return;   /* an earlier launch of the call gave up */
 	const mlp_off o = offsets(a.nin, a.nh, a.nout);
 	const size_t w = fused_words(a.nin, a.nh, a.nout), weights = w > 2 * FUSED_TILE * FUSED_PITCH ? w : 2 * FUSED_TILE * FUSED_PITCH;
 	const unsigned int bar = (unsigned int)__cvta_generic_to_shared(&mbar);
@@ -581,14 +600,20 @@ __global__ void __launch_bounds__(FUSED_THREADS) mlp_fused(const fused_args a)
 	asm volatile("fence.proxy.async;" ::: "memory");
 	grid.sync();
 	unsigned int round = 0;
-	for (int it = 0; it < a.steps + (a.grad ? 1 : 0); it++) {
+	int it = 0;
+	unsigned int gave_up = 0;
+	for (; it < a.steps + (a.grad ? 1 : 0); it++) {
 		fused_samples<SP>(a, o, sm, weights, bar, round++, true, it == a.steps ? a.eval : 0);
 		grid.sync();
+		/* all CTAs alike: the word is set in phase A only.  It is on its way while the gradients are summed */
+		gave_up = __ldcg(a.status);
 		const bool adam = it < a.steps;
-		fused_parameters(a, o, sm, adam, adam ? a.corr[2 * it] : 1.0f, adam ? a.corr[2 * it + 1] : 1.0f);
+		fused_parameters(a, o, sm, adam, adam ? a.corr[2 * it] : 1.0f, adam ? a.corr[2 * it + 1] : 1.0f, gave_up);
+		if (gave_up) break;
 		grid.sync();
 	}
-	if (!a.grad && a.eval) fused_samples<SP>(a, o, sm, weights, bar, round++, false, a.eval);
+	if (blockIdx.x == 0 && threadIdx.x == 0) a.status[1] = a.before + min(it, a.steps);
+	if (!a.grad && a.eval && !gave_up) fused_samples<SP>(a, o, sm, weights, bar, round++, false, a.eval);
 }
 
 /* the fused launch for n samples and its grid, or NULL where the network does not fit it */
@@ -637,6 +662,13 @@ static jn_status ensure_capacity(jn_mlp *m, int n)
 	return JN_OK;
 }
 
+extern "C" jn_status jn_mlp_set_wait_limit(jn_mlp *m, int polls)
+{
+	if (!m || polls < 0) return jn_fail(JN_ERR_INVALID, "bad argument");
+	m->polls = polls;
+	return JN_OK;
+}
+
 extern "C" void jn_mlp_destroy(jn_mlp *m)
 {
 	if (!m) return;
@@ -655,6 +687,7 @@ extern "C" jn_status jn_mlp_create(int nin, int nh, int nout, uint64_t seed, jn_
 	m->nin = nin; m->nh = nh; m->nout = nout;
 	const mlp_off o = offsets(nin, nh, nout);
 	m->np = o.b3 + nout;
+	m->polls = FUSED_POLLS;
 	float *h = (float *)calloc(m->np, sizeof(float));
 	/* seeded uniform(-1/sqrt(fan_in), 1/sqrt(fan_in)) weights, zero biases */
 	uint64_t z = seed;
@@ -729,9 +762,9 @@ static jn_status backward(jn_mlp *m, int n)
 }
 
 /* the fused launch over the loaded samples: `steps` Adam steps (the bias
- * corrections in d_corr), then the gradient (grad) and a pass for the losses
+ * corrections in d_corr; the call's `before` are behind it), then the gradient (grad) and a pass for the losses
  * (eval 1) or the outputs (eval 2) */
-static jn_status fused_run(jn_mlp *m, fused_kernel f, size_t smem, int grid, int n, int steps, float lr, int grad, int eval)
+static jn_status fused_run(jn_mlp *m, fused_kernel f, size_t smem, int grid, int n, int before, int steps, float lr, int grad, int eval)
 {
 	fused_args a;
 	memset(&a, 0, sizeof a);
@@ -743,7 +776,9 @@ static jn_status fused_run(jn_mlp *m, fused_kernel f, size_t smem, int grid, int
 	a.X = m->d_x; a.T = m->d_t;
 	a.XT = m->d_a1; a.H1T = m->d_h1; a.H2T = m->d_h2; a.D1T = m->d_d1; a.D2T = m->d_d2; a.D3T = m->d_d3;
 	a.image = m->d_image;
-	a.fail = (unsigned int *)(m->d_corr + 2 * FUSED_STEPS);
+	a.status = (unsigned int *)(m->d_corr + 2 * FUSED_STEPS);
+	a.before = before;
+	a.polls = m->polls;
 	a.Y = m->d_y; a.lossp = m->d_loss;
 	a.corr = m->d_corr;
 	a.lr = lr; a.b1 = ADAM_B1; a.b2 = ADAM_B2; a.eps = ADAM_EPS;
@@ -752,11 +787,14 @@ static jn_status fused_run(jn_mlp *m, fused_kernel f, size_t smem, int grid, int
 	return JN_OK;
 }
 
-/* a copy in the fused path whose wait gave up: the results are not valid */
-static jn_status fused_check(jn_mlp *m, unsigned int failed)
+/* A wait of the call's launches gave up: the parameters and moments are those
+ * after status[1] of its steps, t0 + status[1] in all; the call's other results
+ * are not valid. */
+static jn_status fused_check(jn_mlp *m, const unsigned int *status, int64_t t0)
 {
-	if (!failed) return JN_OK;
-	cudaMemset(m->d_corr + 2 * FUSED_STEPS, 0, sizeof(unsigned int));
+	if (!status[0]) return JN_OK;
+	m->t = t0 + status[1];
+	CUDA_TRY(cudaMemset(m->d_corr + 2 * FUSED_STEPS, 0, sizeof(unsigned int)));
 	return jn_fail(JN_ERR_TIMEOUT, "MLP: a wait for the weights' copy gave up");
 }
 
@@ -775,10 +813,11 @@ extern "C" jn_status jn_mlp_loss_and_gradient(jn_mlp *m, const float *x, const f
 	jn_status s = load(m, x, t, n);
 	size_t smem;
 	int grid;
-	unsigned int failed = 0;
+	unsigned int status[2] = { 0, 0 };
+	const int64_t t0 = m->t;
 	fused_kernel f = fused_for(m, n, &smem, &grid);
 	if (!s && f) {
-		s = fused_run(m, f, smem, grid, n, 0, 0.0f, 1, 1);
+		s = fused_run(m, f, smem, grid, n, 0, 0, 0.0f, 1, 1);
 		if (!s) mlp_loss_sum<<<1, 256, 0, m->stream>>>(m->d_loss, n, m->d_loss);
 	} else {
 		if (!s) s = forward(m, n);
@@ -787,9 +826,9 @@ extern "C" jn_status jn_mlp_loss_and_gradient(jn_mlp *m, const float *x, const f
 	if (s) return s;
 	if (loss) CUDA_TRY(cudaMemcpyAsync(loss, m->d_loss + n, sizeof(float), cudaMemcpyDeviceToHost, m->stream));
 	if (grad) CUDA_TRY(cudaMemcpyAsync(grad, m->d_g, m->np * sizeof(float), cudaMemcpyDeviceToHost, m->stream));
-	if (f) CUDA_TRY(cudaMemcpyAsync(&failed, m->d_corr + 2 * FUSED_STEPS, sizeof failed, cudaMemcpyDeviceToHost, m->stream));
+	if (f) CUDA_TRY(cudaMemcpyAsync(status, m->d_corr + 2 * FUSED_STEPS, sizeof status, cudaMemcpyDeviceToHost, m->stream));
 	CUDA_TRY(cudaStreamSynchronize(m->stream));
-	return fused_check(m, failed);
+	return fused_check(m, status, t0);
 }
 
 extern "C" jn_status jn_mlp_train(jn_mlp *m, const float *x, const float *t, int n, int steps, float lr, float *final_loss)
@@ -798,7 +837,8 @@ extern "C" jn_status jn_mlp_train(jn_mlp *m, const float *x, const float *t, int
 	jn_status s = load(m, x, t, n);
 	size_t smem;
 	int grid;
-	unsigned int failed = 0;
+	unsigned int status[2] = { 0, 0 };
+	const int64_t t0 = m->t;
 	fused_kernel f = fused_for(m, n, &smem, &grid);
 	if (!s && f) {
 		std::vector<float> corr(2 * FUSED_STEPS);
@@ -812,7 +852,7 @@ extern "C" jn_status jn_mlp_train(jn_mlp *m, const float *x, const float *t, int
 			/* pageable memory: the copy has left `corr` when the call returns */
 			if (run) CUDA_TRY(cudaMemcpyAsync(m->d_corr, corr.data(), 2 * run * sizeof(float), cudaMemcpyHostToDevice, m->stream));
 			/* the last launch also takes the loss of the final parameters */
-			s = fused_run(m, f, smem, grid, n, run, lr, 0, it + FUSED_STEPS >= steps);
+			s = fused_run(m, f, smem, grid, n, it, run, lr, 0, it + FUSED_STEPS >= steps);
 		}
 		if (!s) mlp_loss_sum<<<1, 256, 0, m->stream>>>(m->d_loss, n, m->d_loss);
 	} else {
@@ -830,10 +870,10 @@ extern "C" jn_status jn_mlp_train(jn_mlp *m, const float *x, const float *t, int
 	}
 	if (s) return s;
 	if (final_loss) CUDA_TRY(cudaMemcpyAsync(final_loss, m->d_loss + n, sizeof(float), cudaMemcpyDeviceToHost, m->stream));
-	if (f) CUDA_TRY(cudaMemcpyAsync(&failed, m->d_corr + 2 * FUSED_STEPS, sizeof failed, cudaMemcpyDeviceToHost, m->stream));
+	if (f) CUDA_TRY(cudaMemcpyAsync(status, m->d_corr + 2 * FUSED_STEPS, sizeof status, cudaMemcpyDeviceToHost, m->stream));
 	CUDA_TRY(cudaStreamSynchronize(m->stream));
 	CUDA_TRY(cudaGetLastError());
-	return fused_check(m, failed);
+	return fused_check(m, status, t0);
 }
 
 extern "C" jn_status jn_mlp_predict(jn_mlp *m, const float *x, int n, float *y)
@@ -842,14 +882,15 @@ extern "C" jn_status jn_mlp_predict(jn_mlp *m, const float *x, int n, float *y)
 	jn_status s = load(m, x, NULL, n);
 	size_t smem;
 	int grid;
-	unsigned int failed = 0;
+	unsigned int status[2] = { 0, 0 };
+	const int64_t t0 = m->t;
 	fused_kernel f = fused_for(m, n, &smem, &grid);
-	if (!s) s = f ? fused_run(m, f, smem, grid, n, 0, 0.0f, 0, 2) : forward(m, n);
+	if (!s) s = f ? fused_run(m, f, smem, grid, n, 0, 0, 0.0f, 0, 2) : forward(m, n);
 	if (s) return s;
 	CUDA_TRY(cudaMemcpyAsync(y, m->d_y, (size_t)n * m->nout * sizeof(float), cudaMemcpyDeviceToHost, m->stream));
-	if (f) CUDA_TRY(cudaMemcpyAsync(&failed, m->d_corr + 2 * FUSED_STEPS, sizeof failed, cudaMemcpyDeviceToHost, m->stream));
+	if (f) CUDA_TRY(cudaMemcpyAsync(status, m->d_corr + 2 * FUSED_STEPS, sizeof status, cudaMemcpyDeviceToHost, m->stream));
 	CUDA_TRY(cudaStreamSynchronize(m->stream));
-	return fused_check(m, failed);
+	return fused_check(m, status, t0);
 }
 
 
