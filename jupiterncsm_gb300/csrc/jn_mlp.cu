@@ -638,6 +638,23 @@ static fused_kernel fused_for(const jn_mlp *m, int n, size_t *smem, int *grid)
 	return f;
 }
 
+/* Whether the kernels of a pass take one forward pass (or one gradient) in less
+ * time than the cooperative launch, which costs about 20 us more to start and
+ * needs two grid barriers for a gradient; it wins where the passes' strided reads of the weights
+ * take longer than that.  Calls, kernels of a pass against cooperative, us:
+ * predict 2-8-8-4 on 1 / 1000 / 100 000 samples 19 / 21 / 119 against 37 / 41 / 199,
+ * 4-32-32-8 on 1 / 1000 / 10 000 21 / 31 / 87 against 37 / 41 / 69, 4-64-64-16 on 256 / 1000
+ * 30 / 44 against 39 / 40, 4-128-128-32 on 64 / 256 35 / 45 against 39 / 40,
+ * 8-160-160-40 on 1 / 64 41 / 43 against 39 / 39; gradient 4-16-16-8 on 1 / 16 / 64
+ * 45 / 47 / 58 against 55 / 53 / 54, 4-32-32-8 47 / 47 / 61 against 53 / 53 / 54,
+ * 4-64-64-16 on 1 58 against 55. */
+static int short_pass(const jn_mlp *m, int n, int gradient)
+{
+	const int64_t w = (int64_t)m->nh * (m->nin + m->nh + m->nout);
+	if (gradient) return w <= 2048 && n <= 32;
+	return w <= 512 || (w <= 24576 && n * w <= 1 << 21);
+}
+
 static const float ADAM_B1 = 0.9f, ADAM_B2 = 0.999f, ADAM_EPS = 1e-8f;
 
 static jn_status ensure_capacity(jn_mlp *m, int n)
@@ -815,7 +832,7 @@ extern "C" jn_status jn_mlp_loss_and_gradient(jn_mlp *m, const float *x, const f
 	int grid;
 	unsigned int status[2] = { 0, 0 };
 	const int64_t t0 = m->t;
-	fused_kernel f = fused_for(m, n, &smem, &grid);
+	fused_kernel f = short_pass(m, n, 1) ? NULL : fused_for(m, n, &smem, &grid);
 	if (!s && f) {
 		s = fused_run(m, f, smem, grid, n, 0, 0, 0.0f, 1, 1);
 		if (!s) mlp_loss_sum<<<1, 256, 0, m->stream>>>(m->d_loss, n, m->d_loss);
@@ -884,7 +901,7 @@ extern "C" jn_status jn_mlp_predict(jn_mlp *m, const float *x, int n, float *y)
 	int grid;
 	unsigned int status[2] = { 0, 0 };
 	const int64_t t0 = m->t;
-	fused_kernel f = fused_for(m, n, &smem, &grid);
+	fused_kernel f = short_pass(m, n, 0) ? NULL : fused_for(m, n, &smem, &grid);
 	if (!s) s = f ? fused_run(m, f, smem, grid, n, 0, 0, 0.0f, 0, 2) : forward(m, n);
 	if (s) return s;
 	CUDA_TRY(cudaMemcpyAsync(y, m->d_y, (size_t)n * m->nout * sizeof(float), cudaMemcpyDeviceToHost, m->stream));
