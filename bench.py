@@ -73,9 +73,6 @@ def measured_peaks():
 KERNELS = {(4, "f32"): "jn_panel_kernel_i32", (4, "i64"): "jn_panel_kernel_fp64", (4, "fp64"): "jn_panel_kernel_fp64",
            (3, "f32"): "jn_tile_kernel<float>", (3, "i64"): "jn_tile_kernel<double>", (3, "fp64"): "jn_tile_kernel<double>",
            (5, "i64"): "jn_walk_kernel<1>", (5, "fp64"): "jn_walk_kernel<64>", (5, "f32"): "jn_walk_kernel<32>"}
-# kernels launched per product: max|x| (and the copies of x), the product, the conversion into y; the walk
-# engine's integer path converts x in a kernel of its own above 12 288 states
-LAUNCHES = {(5, "i64"): lambda D: 4 if D > 12288 else 3}
 
 
 def max_over_ranks(v, dist, device):
@@ -887,6 +884,7 @@ def main():
     achieved = bytes_step / (main_r["kernel_ms"] / 1e3) / 1e9
     traffic = profile_traffic(args.workload, engine, args.arith)
     wstats = H.walk_stats() if engine == 5 else None
+    launches = H.product_kernels()
 
     def path_summary(r, a):
         return {"ms_per_step": r["ms_per_step"], "GB_per_s_fp64_bytes": bytes_step / (r["ms_per_step"] / 1e3) / 1e9,
@@ -919,7 +917,7 @@ def main():
                        "engine": engine, "open_seconds": open_s, "schedule": tuning, "walk_plan": wstats},
             "paths": {a: path_summary(runs[a], a) for a in order},
             "e2e": {"value": e2e_value, "unit": "GB/s", "h2d_bytes_per_step": 16 * D, "d2h_bytes_per_step": 8 * D},
-            "gpu_launches": LAUNCHES.get((engine, args.arith), lambda D: 3)(D) * args.steps,
+            "gpu_launches": launches * args.steps,
             "engine": engine,
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "traffic": traffic,

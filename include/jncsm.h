@@ -232,6 +232,12 @@ jn_status jn_set_panel_schedule(jn_ctx *ctx, int rows_per_lane, int ctas_per_sm)
  * accumulator does not fit), or -1 for a NULL context. */
 int jn_active_engine(const jn_ctx *ctx);
 
+/* The number of the library's kernels that one product of this context
+ * launches at its current engine, precision and arithmetic (copies and
+ * memsets not counted).  No reference counterpart (the benchmark's launch
+ * count). */
+jn_status jn_product_kernels(jn_ctx *ctx, int *count);
+
 /* Synchronise the context's stream. */
 jn_status jn_synchronize(jn_ctx *ctx);
 

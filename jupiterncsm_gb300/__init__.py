@@ -176,6 +176,8 @@ def gpu_lib():
     L.jn_set_panel_schedule.restype = ci
     L.jn_active_engine.argtypes = [vp]
     L.jn_active_engine.restype = ci
+    L.jn_product_kernels.argtypes = [vp, ctypes.POINTER(ci)]
+    L.jn_product_kernels.restype = ci
     L.jn_set_walk_arithmetic.argtypes = [vp, ci]
     L.jn_set_walk_arithmetic.restype = ci
     L.jn_walk_stats.argtypes = [vp, ctypes.POINTER(ctypes.c_double)]
@@ -408,6 +410,12 @@ class Hamiltonian:
     def active_engine(self):
         """The engine the next product runs (4 panels, 3 block tiles, 2 warp pieces)."""
         return gpu_lib().jn_active_engine(self._h)
+
+    def product_kernels(self):
+        """How many of the library's kernels one product launches at the current engine, precision and arithmetic."""
+        n = ctypes.c_int()
+        _check(gpu_lib().jn_product_kernels(self._h, ctypes.byref(n)))
+        return n.value
 
     def set_engine(self, engine):
         """4: panels (default where the accumulator fits in shared memory); 5: walks (default above that);

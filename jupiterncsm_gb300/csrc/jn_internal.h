@@ -138,6 +138,7 @@ jn_status jn_walk_setup(jn_ctx *c);
 void jn_walk_invalidate(jn_ctx *c);
 void jn_walk_release(jn_ctx *c);
 jn_status jn_enqueue_many(jn_ctx *c, const double *d_x, double *d_y, int n, cudaStream_t st);  /* Y = H X, any engine */
+int jn_walk_kernels(const jn_ctx *c);   /* kernels of a product (after jn_walk_setup) */
 jn_status jn_enqueue_walk(jn_ctx *c, const double *d_x, double *d_y, int accumulate, cudaStream_t st, cudaEvent_t pre,
 			  cudaEvent_t mid);
 

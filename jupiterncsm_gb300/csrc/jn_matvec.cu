@@ -806,6 +806,27 @@ extern "C" int jn_active_engine(const jn_ctx *c)
 	return c->engine;
 }
 
+extern "C" jn_status jn_product_kernels(jn_ctx *c, int *count)
+{
+	if (!c || !count) return fail(JN_ERR_INVALID, "null argument");
+	const jn_plan_t *p = &c->plan;
+	const int engine = jn_active_engine(c), dim = p->dim > 0;
+	if (engine == 5) {
+		jn_status s = jn_walk_setup(c);
+		if (s) return s;
+		*count = jn_walk_kernels(c);
+	} else if (engine == 4) {
+		jn_status s = jn_panels_setup(c);
+		if (s) return s;
+		*count = dim ? 2 + (p->nptasks > 0) : 0;
+	} else if (engine == 2) {
+		*count = (c->precision == 32 && dim) + (p->nunits > 0) + (p->ntiles > 0);
+	} else {
+		*count = 2 * dim + (p->nbtiles > 0);
+	}
+	return JN_OK;
+}
+
 jn_status jn_launch_matvec(jn_ctx *c, const double *d_x, double *d_y, int accumulate, cudaStream_t st)
 {
 	return enqueue(c, d_x, d_y, accumulate, st, NULL, NULL);

@@ -652,6 +652,15 @@ static jn_status walk_launch(jn_ctx *c, const double *d_x, double *d_y, int nvec
 	return JN_OK;
 }
 
+int jn_walk_kernels(const jn_ctx *c)
+{
+	const jn_plan_t *p = &c->plan;
+	if (!p->dim) return 0;
+	/* before the walk kernel: all in one, or max|x| and, where there is one to make, the converted copy of x */
+	const int views = p->dim <= WALK_SMALL_DIM ? 1 : p->wxt || walk_mode(c) != 64 ? 2 : 1;
+	return views + (p->nwtasks > 0) + 1;
+}
+
 /* y (+)= H x on the walk engine */
 jn_status jn_enqueue_walk(jn_ctx *c, const double *d_x, double *d_y, int accumulate, cudaStream_t st, cudaEvent_t pre,
 			  cudaEvent_t mid)
