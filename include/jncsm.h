@@ -327,6 +327,15 @@ typedef struct {
  * batched solvers. */
 jn_status jn_lanczos(jn_ctx *ctx, const jn_lanczos_options *options, jn_lanczos_result *result);
 
+/* The num_values lowest eigenvalues, ascending, of the symmetric tridiagonal
+ * matrix with diagonal a[0..n) and off-diagonal b[0..n-1), each to the last
+ * bits that its entries determine, and the unit eigenvectors of the num_vectors lowest (rows of
+ * n, first component >= 0, made orthogonal in order): the kernels that the
+ * solves use for their Ritz values (dsteqr in the reference,
+ * Bacchus/diagonalization/diagonalization.c:16-68).  Host memory. */
+jn_status jn_tridiagonal(const double *a, const double *b, int n, int num_values, double *values, int num_vectors,
+			 double *vectors);
+
 /* All Ritz values of the last solve in ascending order, as get_eigensystem +
  * print_eigensystem report them (lanczos.c:255-265, eigensystem.c:99-113). */
 jn_status jn_lanczos_ritz_values(jn_ctx *ctx, double *out, int capacity, int *count);

@@ -207,6 +207,8 @@ def gpu_lib():
                  "jn_mlp_train", "jn_mlp_predict", "jn_mlp_set_wait_limit", "jn_warm_start_fit", "jn_warm_start_vectors",
                  "jn_warm_start_basis"):
         getattr(L, name).restype = ci
+    L.jn_tridiagonal.argtypes = [vp, vp, ci, ci, vp, ci, vp]
+    L.jn_tridiagonal.restype = ci
     L.jn_subspace_matrices.argtypes = [vp, ci, vp, vp, vp]
     L.jn_subspace_matrices.restype = ci
     L.jn_ceres_files.argtypes = [vp, ci, vp, cp, cp]
@@ -556,6 +558,19 @@ class MLP:
     def set_wait_limit(self, polls):
         """Polls after which a kernel's wait for its copy of the weights gives up (JN_ERR_TIMEOUT)."""
         _check(gpu_lib().jn_mlp_set_wait_limit(self._h, int(polls)))
+
+
+def tridiagonal(a, b, num_values=None, num_vectors=0):
+    """The lowest eigenvalues of the symmetric tridiagonal matrix (a, b) and the unit eigenvectors of the num_vectors
+    lowest (rows), by the kernels of the Lanczos solves."""
+    a, b = (np.ascontiguousarray(v, dtype=np.float64) for v in (a, b))
+    n = len(a)
+    assert len(b) >= n - 1
+    values = np.zeros(n if num_values is None else num_values)
+    vectors = np.zeros((num_vectors, n))
+    _check(gpu_lib().jn_tridiagonal(a.ctypes.data, b.ctypes.data, n, len(values), values.ctypes.data, num_vectors,
+                                    vectors.ctypes.data))
+    return values, vectors
 
 
 def aurora(comb, anicre_dir, output_dir, Z, N, human_readable=False, skip_three_body=False):

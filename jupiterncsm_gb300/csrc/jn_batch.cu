@@ -223,12 +223,12 @@ __global__ void __launch_bounds__(BT) kb_normalize(const int2 *__restrict__ cta,
 /* eigenvalue i = blockIdx.x < want of each instance's T by two warps, and its
  * eigenvector (rows of Z, its bottom component in zlast when not NULL).
  * Scratch: shared memory, or `work` (JN_TRI_VECTOR_DOUBLES(ldz) a warp) when
- * the rows do not fit there.  The first `guesses` entries of theta hold an
+ * the rows do not fit there.  exact: to the last bit.  The first `guesses` entries of theta hold an
  * earlier check's eigenvalues. */
 __global__ void __launch_bounds__(64) kb_tri_pairs(const double *__restrict__ alpha, const double *__restrict__ beta, int64_t ldab,
 						    const int *__restrict__ n_arr, int want, double *__restrict__ theta, int ldt,
 						    double *__restrict__ Z, int ldz, double *__restrict__ work,
-						    double *__restrict__ zlast, int guesses, const int *__restrict__ active)
+						    double *__restrict__ zlast, int exact, int guesses, const int *__restrict__ active)
 {
 	SKIP_INACTIVE();
 	extern __shared__ double sbuf[];
@@ -244,7 +244,7 @@ __global__ void __launch_bounds__(64) kb_tri_pairs(const double *__restrict__ al
 	if (threadIdx.x < 32) jn_tri_stage(a, b, n, sc, as, b2);
 	const double old = i < guesses ? theta[(int64_t)inst * ldt + i] : 0.0;
 	__syncthreads();
-	const double x = jn_tri_multisect(as, b2, n, i, lo, hi, i < guesses, old * sc, &ex);
+	const double x = jn_tri_multisect(as, b2, n, i, lo, hi, exact, i < guesses, old * sc, &ex);
 	if (threadIdx.x >= 32) return;
 	jn_tri_vector_warp(as, b2, n, x, z, b2 + n);
 	if (threadIdx.x == 0) {
@@ -675,7 +675,7 @@ static jn_status batch_solve(cudaStream_t q, const jn_batch_options *o, const ba
 		cudaMemcpyAsync(s.narr, hn, B * sizeof(int), cudaMemcpyHostToDevice, q);
 		const int wk = want < k ? want : k;
 		kb_tri_pairs<<<dim3(wk, B), 64, tri_smem ? JN_TRI_SMEM(k) : 0, q>>>(
-			s.alpha, s.beta, ldab, s.narr, wk, s.theta, r + 1, s.Z, ldz, s.work, s.zlast, guesses, s.active);
+			s.alpha, s.beta, ldab, s.narr, wk, s.theta, r + 1, s.Z, ldz, s.work, s.zlast, 0, guesses, s.active);
 		guesses = wk;
 		kb_converged<<<(B + 127) / 128, 128, 0, q>>>(s.theta, s.zlast, r + 1, s.beta, ldab, s.narr, nev, o->tolerance,
 							     s.flag, s.active, B);
@@ -714,7 +714,7 @@ static jn_status batch_solve(cudaStream_t q, const jn_batch_options *o, const ba
 		cudaMemcpyAsync(s.narr, hn, B * sizeof(int), cudaMemcpyHostToDevice, q);
 		cudaMemcpyAsync(s.active, hact, B * sizeof(int), cudaMemcpyHostToDevice, q);
 		kb_tri_pairs<<<dim3(r, B), 64, tri_smem ? JN_TRI_SMEM(k) : 0, q>>>(
-			s.alpha, s.beta, ldab, s.narr, r, s.theta, r + 1, s.Z, ldz, s.work, NULL, guesses, NULL);
+			s.alpha, s.beta, ldab, s.narr, r, s.theta, r + 1, s.Z, ldz, s.work, NULL, 1, guesses, NULL);
 		kb_tri_mgs<<<g1, BT, 0, q>>>(s.Z, ldz, s.narr, r, NULL);
 		/* instances in waves of the grid's third dimension */
 		for (int i = 0; i < B; i += 65535)

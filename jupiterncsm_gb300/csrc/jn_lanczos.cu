@@ -373,6 +373,7 @@ __global__ void __launch_bounds__(512) k_rayleigh(const double *__restrict__ X, 
  * vectors orthogonal among themselves and packs the results for one copy to
  * the host: theta (want), the vectors' bottom components (nvec), beta_{n-1}.
  * The first `guesses` entries of theta hold an earlier check's eigenvalues.
+ * exact: to the last bit of each eigenvalue.
  * Scratch: shared memory, or `work` (JN_TRI_VECTOR_DOUBLES(n) a CTA) above
  * JN_TRI_SMEM_ROWS rows.  Bound by the FP64 chains of a warp (about five
  * rounds of 1.5 n instructions, then 2 n for the vector, 64 cycles each): 100
@@ -381,7 +382,7 @@ __global__ void __launch_bounds__(512) k_rayleigh(const double *__restrict__ X, 
 __global__ void __launch_bounds__(TRI_THREADS)
 	k_tri_check(const double *__restrict__ a, const double *__restrict__ b, int n, int want, int nvec,
 		    double *__restrict__ theta, double *Z, int ldz, double *work, unsigned int *__restrict__ done,
-		    double *__restrict__ pack, int first, int guesses)
+		    double *__restrict__ pack, int first, int exact, int guesses)
 {
 	extern __shared__ double sbuf[];
 	__shared__ jn_tri_exchange ex;
@@ -396,7 +397,7 @@ __global__ void __launch_bounds__(TRI_THREADS)
 	}
 	__syncthreads();
 	if (threadIdx.x < 64) {
-		const double x = jn_tri_multisect(as, b2, n, i, lo, hi, i < guesses, guess, &ex);
+		const double x = jn_tri_multisect(as, b2, n, i, lo, hi, exact, i < guesses, guess, &ex);
 		if (threadIdx.x == 0) theta[i] = x / sc;
 		if (i < nvec && threadIdx.x < 32) jn_tri_vector_warp(as, b2, n, x, Z + (int64_t)i * ldz, b2 + n);
 	}
@@ -490,27 +491,35 @@ static jn_status ensure_state(jn_ctx *c, int mmax, int nev)
 	return JN_OK;
 }
 
+/* k_tri_check for the `want` lowest eigenvalues of T_n */
+static void tri_launch(cudaStream_t st, const double *a, const double *b, int n, int want, int nvec, double *theta, double *Z,
+		       int ldz, double *work, unsigned int *done, double *pack, int exact, int guesses)
+{
+	const int in_smem = n <= JN_TRI_SMEM_ROWS;
+	/* TRI_WAVE at a time: all eigenvalues of a T_n whose rows do not fit shared memory */
+	for (int i = 0; i < want; i += TRI_WAVE)
+		if (in_smem || want <= TRI_WAVE) {
+			k_tri_check<<<want, TRI_THREADS, in_smem ? JN_TRI_SMEM(n) : 0, st>>>(a, b, n, want, nvec, theta, Z, ldz,
+											     in_smem ? NULL : work, done, pack, 0, exact, guesses);
+			break;
+		} else {
+			k_tri_check<<<want - i < TRI_WAVE ? want - i : TRI_WAVE, TRI_THREADS, 0, st>>>(
+				a, b, n, want, nvec, theta, Z, ldz, work, done, pack, i, exact, guesses);
+		}
+}
+
 /* Enqueue, behind the work now on the context's stream, the lowest `want`
  * eigenvalues of T_n and the eigenvectors of the lowest `nvec` (rows of d_Z)
- * on the checks' stream; h_pack[slot] receives theta (want), the bottom
+ * on the checks' stream.  exact: to the last bit, else to 2^-54 of the span.
+ * h_pack[slot] receives theta (want), the bottom
  * components (nvec) and beta_{n-1} once checked[slot] has happened. */
-static jn_status tri_enqueue(jn_ctx *c, int n, int want, int nvec, int slot)
+static jn_status tri_enqueue(jn_ctx *c, int n, int want, int nvec, int exact, int slot)
 {
 	struct jn_lanczos_state *s = c->lz;
 	CUDA_TRY(cudaEventRecord(s->stepped, c->stream));
 	CUDA_TRY(cudaStreamWaitEvent(s->check, s->stepped, 0));
-	const int in_smem = n <= JN_TRI_SMEM_ROWS;
-	if (in_smem || want <= TRI_WAVE) {
-		k_tri_check<<<want, TRI_THREADS, in_smem ? JN_TRI_SMEM(n) : 0, s->check>>>(
-			s->d_alpha, s->d_beta, n, want, nvec, s->d_theta, s->d_Z, s->mmax + 1, in_smem ? NULL : s->d_work, s->d_done,
-			s->d_pack, 0, s->guesses);
-	} else {
-		/* all eigenvalues of a T_n whose rows do not fit shared memory */
-		for (int i = 0; i < want; i += TRI_WAVE)
-			k_tri_check<<<want - i < TRI_WAVE ? want - i : TRI_WAVE, TRI_THREADS, 0, s->check>>>(
-				s->d_alpha, s->d_beta, n, want, nvec, s->d_theta, s->d_Z, s->mmax + 1, s->d_work, s->d_done,
-				s->d_pack, i, s->guesses);
-	}
+	tri_launch(s->check, s->d_alpha, s->d_beta, n, want, nvec, s->d_theta, s->d_Z, s->mmax + 1, s->d_work, s->d_done, s->d_pack,
+		   exact, s->guesses);
 	s->guesses = want;
 	CUDA_TRY(cudaGetLastError());
 	CUDA_TRY(cudaMemcpyAsync(s->h_pack[slot], s->d_pack, (size_t)(want + nvec + 1) * sizeof(double), cudaMemcpyDeviceToHost,
@@ -519,16 +528,69 @@ static jn_status tri_enqueue(jn_ctx *c, int n, int want, int nvec, int slot)
 	return JN_OK;
 }
 
-/* the same, waited for, into h_pack[0] */
+/* each eigenvalue is found by itself: those of a cluster may cross by a rounding */
+static void ascending(double *v, int n)
+{
+	for (int i = 1; i < n; i++)
+		if (v[i] < v[i - 1]) v[i] = v[i - 1];
+}
+
+/* the same, exact and waited for, into h_pack[0] */
 static jn_status tri_eig(jn_ctx *c, int n, int want, int nvec)
 {
 	struct jn_lanczos_state *s = c->lz;
-	jn_status st = tri_enqueue(c, n, want, nvec, 0);
+	jn_status st = tri_enqueue(c, n, want, nvec, 1, 0);
 	if (st) return st;
 	CUDA_TRY(cudaEventSynchronize(s->checked[0]));
-	/* each eigenvalue is found by itself: those of a cluster may cross by a rounding */
-	for (int i = 1; i < want; i++)
-		if (s->h_pack[0][i] < s->h_pack[0][i - 1]) s->h_pack[0][i] = s->h_pack[0][i - 1];
+	ascending(s->h_pack[0], want);
+	return JN_OK;
+}
+
+extern "C" jn_status jn_tridiagonal(const double *a, const double *b, int n, int num_values, double *values, int num_vectors,
+				    double *vectors)
+{
+	if (!a || (!b && n > 1) || !values || n < 1 || num_values < 1 || num_values > n || num_vectors < 0 || num_vectors > num_values ||
+	    (num_vectors && !vectors))
+		return jn_fail(JN_ERR_INVALID, "bad argument");
+	const size_t wave = num_values < TRI_WAVE ? num_values : TRI_WAVE;
+	const size_t nv = (size_t)num_vectors * n, nw = n > JN_TRI_SMEM_ROWS ? wave * JN_TRI_VECTOR_DOUBLES(n) : 0;
+	const size_t np = (size_t)num_values + num_vectors + 1;
+	double *d = NULL;
+	cudaStream_t st = NULL;
+	/* the matrix (2 n), the values, the vectors, the scratch, the packed results, the counter */
+	const size_t bytes = (2 * (size_t)n + num_values + nv + nw + np + 1) * sizeof(double);
+	cudaError_t e = cudaMalloc((void **)&d, bytes);
+	if (e != cudaSuccess) {
+		cudaGetLastError();
+		return jn_fail(JN_ERR_NOMEM, "tridiagonal matrix of %d rows: %s", n, cudaGetErrorString(e));
+	}
+	double *theta = d + 2 * (size_t)n, *Z = theta + num_values, *work = Z + nv, *pack = work + nw;
+	e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
+	if (e == cudaSuccess)
+		e = cudaFuncSetAttribute(k_tri_check, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)JN_TRI_SMEM(JN_TRI_SMEM_ROWS));
+	if (e == cudaSuccess) e = cudaMemsetAsync(d, 0, bytes, st);
+	if (e == cudaSuccess) e = cudaMemcpyAsync(d, a, n * sizeof(double), cudaMemcpyHostToDevice, st);
+	if (e == cudaSuccess && n > 1) e = cudaMemcpyAsync(d + n, b, (n - 1) * sizeof(double), cudaMemcpyHostToDevice, st);
+	if (e == cudaSuccess) {
+		tri_launch(st, d, d + n, n, num_values, num_vectors, theta, Z, n, work, (unsigned int *)(pack + np), pack, 1, 0);
+		e = cudaGetLastError();
+	}
+	if (e == cudaSuccess) e = cudaMemcpyAsync(values, pack, num_values * sizeof(double), cudaMemcpyDeviceToHost, st);
+	if (e == cudaSuccess && nv) e = cudaMemcpyAsync(vectors, Z, nv * sizeof(double), cudaMemcpyDeviceToHost, st);
+	if (st) {
+		const cudaError_t es = cudaStreamSynchronize(st);
+		if (e == cudaSuccess) e = es;
+		cudaStreamDestroy(st);
+	}
+	cudaFree(d);
+	if (e != cudaSuccess) return jn_fail(JN_ERR_CUDA, "tridiagonal matrix: %s", cudaGetErrorString(e));
+	ascending(values, num_values);
+	/* the kernels take couplings >= 0, as a recurrence makes them; the others' signs go into the components */
+	int negative = 0;
+	for (int i = 1; i < n; i++) {
+		negative ^= b[i - 1] < 0.0;
+		for (int k = 0; k < num_vectors && negative; k++) vectors[(size_t)k * n + i] = -vectors[(size_t)k * n + i];
+	}
 	return JN_OK;
 }
 
@@ -654,7 +716,7 @@ extern "C" jn_status jn_lanczos(jn_ctx *c, const jn_lanczos_options *opt, jn_lan
 		   converged has two steps too many in flight, which nothing reads */
 		if (check) {
 			const int wv = nev < n ? nev : n;
-			st = tri_enqueue(c, n, wv + (wv < n ? 1 : 0), wv, n % CHECKS);
+			st = tri_enqueue(c, n, wv + (wv < n ? 1 : 0), wv, 0, n % CHECKS);
 			if (st) return st;
 			pending[npending++] = n;
 		}

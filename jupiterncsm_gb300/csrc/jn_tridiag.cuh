@@ -76,14 +76,16 @@ __device__ __forceinline__ double jn_tri_scale(const double *a, const double *b,
 	return sc;
 }
 
-/* one warp: a sc into as, (b sc)^2 into b2; couplings below 2^-53 of the
- * span are raised to it (a change below the rounding of a), so that the
- * minors cannot stay at zero */
+/* one warp: a sc into as, (b sc)^2 into b2; couplings below 2^-110 of the
+ * span are raised to it, so that the minors cannot stay at zero (eight steps
+ * of such couplings keep a minor above 2^-880).  A floor at the rounding of
+ * the span, 2^-53, moves the small eigenvalues of a graded matrix: of
+ * diag(2^-5i) with couplings of 2^-(5i+8), n = 14, the smallest came out 10^4 times off. */
 __device__ __forceinline__ void jn_tri_stage(const double *a, const double *b, int n, double sc, double *as, double *b2)
 {
 	for (int j = threadIdx.x & 31; j < n; j += 32) {
 		as[j] = a[j] * sc;
-		const double v = j < n - 1 ? fmax(fabs(b[j]) * sc, 0x1p-53) : 0.0;
+		const double v = j < n - 1 ? fmax(fabs(b[j]) * sc, 0x1p-110) : 0.0;
 		b2[j] = v * v;
 	}
 	__syncwarp();
@@ -162,15 +164,19 @@ __device__ __forceinline__ int jn_sturm_count(const double *as, const double *b2
  * A guess (the same eigenvalue of an earlier, smaller T of the solve) takes
  * the estimate's place in the first round.  The counts alone decide the
  * bracket, so a poor estimate costs a round and nothing else.  It ends at
- * 2^-54 of the span.  Every lane returns the same value. */
+ * 2^-54 of the span or, `exact`, of the eigenvalue where that is smaller, two or three
+ * rounds later: a convergence check compares errors far above either.  Every lane returns the same value. */
 __device__ __forceinline__ double jn_tri_multisect(const double *as, const double *b2, int n, int i, double lo, double hi,
-						    bool guessed, double guess, jn_tri_exchange *ex)
+						    bool exact, bool guessed, double guess, jn_tri_exchange *ex)
 {
 	const int lane = threadIdx.x & 31;
 	int cl = 0, ch = n, el = 0, eh = 0, known = 0;          /* known: 1 det at lo, 2 det at hi */
 	double pl = 0.0, ph = 0.0;
 	int geo_ok = 1;
-	for (int round = 0; round < 96 && hi - lo > 0x1p-54; round++) {
+	for (int round = 0; round < 96; round++) {
+		/* 2^-54 to 2^-53 of the larger end, in integer work */
+		const int e2 = exact ? max(min(max(jn_expo(lo), jn_expo(hi)) - 53, 1023 - 54), 1) : 1023 - 54;
+		if (!(hi - lo > __hiloint2double(e2 << 20, 0))) break;
 		const double w = hi - lo;
 		const int first = guessed && round == 0;
 		const int geo = first || (geo_ok && known == 3 && cl == i && ch == i + 1 && pl != 0.0);
