@@ -714,7 +714,7 @@ static jn_status batch_solve(cudaStream_t q, const jn_batch_options *o, const ba
 		cudaMemcpyAsync(s.narr, hn, B * sizeof(int), cudaMemcpyHostToDevice, q);
 		cudaMemcpyAsync(s.active, hact, B * sizeof(int), cudaMemcpyHostToDevice, q);
 		kb_tri_pairs<<<dim3(r, B), 64, tri_smem ? JN_TRI_SMEM(k) : 0, q>>>(
-			s.alpha, s.beta, ldab, s.narr, r, s.theta, r + 1, s.Z, ldz, s.work, NULL, 1, guesses, NULL);
+			s.alpha, s.beta, ldab, s.narr, r, s.theta, r + 1, s.Z, ldz, s.work, NULL, 1, 0, NULL);
 		kb_tri_mgs<<<g1, BT, 0, q>>>(s.Z, ldz, s.narr, r, NULL);
 		/* instances in waves of the grid's third dimension */
 		for (int i = 0; i < B; i += 65535)

@@ -510,8 +510,9 @@ static void tri_launch(cudaStream_t st, const double *a, const double *b, int n,
 
 /* Enqueue, behind the work now on the context's stream, the lowest `want`
  * eigenvalues of T_n and the eigenvectors of the lowest `nvec` (rows of d_Z)
- * on the checks' stream.  exact: to the last bit, else to 2^-54 of the span.
- * h_pack[slot] receives theta (want), the bottom
+ * on the checks' stream.  exact: to the last bit and from T_n alone, whatever
+ * was checked before; else to 2^-54 of the span, from the last check's values
+ * on.  h_pack[slot] receives theta (want), the bottom
  * components (nvec) and beta_{n-1} once checked[slot] has happened. */
 static jn_status tri_enqueue(jn_ctx *c, int n, int want, int nvec, int exact, int slot)
 {
@@ -519,7 +520,7 @@ static jn_status tri_enqueue(jn_ctx *c, int n, int want, int nvec, int exact, in
 	CUDA_TRY(cudaEventRecord(s->stepped, c->stream));
 	CUDA_TRY(cudaStreamWaitEvent(s->check, s->stepped, 0));
 	tri_launch(s->check, s->d_alpha, s->d_beta, n, want, nvec, s->d_theta, s->d_Z, s->mmax + 1, s->d_work, s->d_done, s->d_pack,
-		   exact, s->guesses);
+		   exact, exact ? 0 : s->guesses);
 	s->guesses = want;
 	CUDA_TRY(cudaGetLastError());
 	CUDA_TRY(cudaMemcpyAsync(s->h_pack[slot], s->d_pack, (size_t)(want + nvec + 1) * sizeof(double), cudaMemcpyDeviceToHost,
@@ -779,7 +780,6 @@ extern "C" jn_status jn_lanczos_ritz_values(jn_ctx *c, double *out, int capacity
 {
 	if (!c || !c->lz || !out) return jn_fail(JN_ERR_INVALID, "no Lanczos solve on this context");
 	struct jn_lanczos_state *s = c->lz;
-	s->guesses = 0;         /* the same bits on every call */
 	jn_status st = tri_eig(c, s->k, s->k, 0);
 	if (st) return st;
 	int n = s->k < capacity ? s->k : capacity;
