@@ -81,7 +81,7 @@ struct jn_lanczos_state {
 	double *d_rr;           /* Rayleigh quotients, residual norms (2 nev_cap) */
 	double *h_pack[CHECKS]; /* pinned copies of d_pack: a check is read while the next ones run */
 	cudaStream_t check;     /* the checks' stream */
-	cudaEvent_t stepped, checked[CHECKS];
+	cudaEvent_t stepped, begun, checked[CHECKS];
 	int guesses;            /* entries of d_theta that hold eigenvalues of the last T of this solve */
 	int nev_cap;
 	int have_ritz;
@@ -100,6 +100,7 @@ void jn_lanczos_release(jn_ctx *c)
 		if (s->checked[i]) cudaEventDestroy(s->checked[i]);
 	}
 	if (s->stepped) cudaEventDestroy(s->stepped);
+	if (s->begun) cudaEventDestroy(s->begun);
 	if (s->check) cudaStreamDestroy(s->check);
 	free(s->h_rq); free(s->h_res);
 	free(s);
@@ -474,6 +475,7 @@ static jn_status ensure_state(jn_ctx *c, int mmax, int nev)
 		if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s->checked[i], cudaEventDisableTiming);
 	}
 	if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s->stepped, cudaEventDisableTiming);
+	if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s->begun, cudaEventDisableTiming);
 	/* the checks' few CTAs are scheduled before the product's thousands */
 	int least = 0, greatest = 0;
 	if (e == cudaSuccess) e = cudaDeviceGetStreamPriorityRange(&least, &greatest);
@@ -519,6 +521,7 @@ static jn_status tri_enqueue(jn_ctx *c, int n, int want, int nvec, int exact, in
 	struct jn_lanczos_state *s = c->lz;
 	CUDA_TRY(cudaEventRecord(s->stepped, c->stream));
 	CUDA_TRY(cudaStreamWaitEvent(s->check, s->stepped, 0));
+	if (exact) CUDA_TRY(cudaEventRecord(s->begun, s->check));
 	tri_launch(s->check, s->d_alpha, s->d_beta, n, want, nvec, s->d_theta, s->d_Z, s->mmax + 1, s->d_work, s->d_done, s->d_pack,
 		   exact, exact ? 0 : s->guesses);
 	s->guesses = want;
@@ -536,15 +539,20 @@ static void ascending(double *v, int n)
 		if (v[i] < v[i - 1]) v[i] = v[i - 1];
 }
 
-/* the same, exact and waited for, into h_pack[0] */
-static jn_status tri_eig(jn_ctx *c, int n, int want, int nvec)
+/* wait for the results in h_pack[0] */
+static jn_status tri_wait(jn_ctx *c, int want)
 {
 	struct jn_lanczos_state *s = c->lz;
-	jn_status st = tri_enqueue(c, n, want, nvec, 1, 0);
-	if (st) return st;
 	CUDA_TRY(cudaEventSynchronize(s->checked[0]));
 	ascending(s->h_pack[0], want);
 	return JN_OK;
+}
+
+/* the same, exact and waited for, into h_pack[0] */
+static jn_status tri_eig(jn_ctx *c, int n, int want, int nvec)
+{
+	jn_status st = tri_enqueue(c, n, want, nvec, 1, 0);
+	return st ? st : tri_wait(c, want);
 }
 
 extern "C" jn_status jn_tridiagonal(const double *a, const double *b, int n, int num_values, double *values, int num_vectors,
@@ -738,12 +746,16 @@ extern "C" jn_status jn_lanczos(jn_ctx *c, const jn_lanczos_options *opt, jn_lan
 	s->k = k;
 	res->iterations = k;
 	res->converged = converged;
-	const double t_final = seconds_now();      /* the loop ends on a convergence check, which is waited for */
-	res->iteration_seconds = t_final - t_loop;
 	/* final decomposition of T_k: the Ritz values and vectors of the lowest nev */
 	int want = nev < k ? nev : k;
 	res->num_ritz_values = k;
-	st = tri_eig(c, k, want, want);
+	st = tri_enqueue(c, k, want, want, 1, 0);
+	if (st) return st;
+	/* the steps and checks under way when convergence was read end before it begins */
+	CUDA_TRY(cudaEventSynchronize(s->begun));
+	const double t_final = seconds_now();
+	res->iteration_seconds = t_final - t_loop;
+	st = tri_wait(c, want);
 	if (st) return st;
 	/* Ritz vectors x_i = sum_j z_i[j] v_j and their FP64 refinement */
 	k_ritz_vectors<<<dim3((unsigned int)((D + 127) / 128), (want + RITZ_ROWS - 1) / RITZ_ROWS), 128, 0, q>>>(
