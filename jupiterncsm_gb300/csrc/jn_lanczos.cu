@@ -29,8 +29,8 @@
  * cooperative kernel (k_orthonormalize) takes w = H v_k to v_{k+1}.  The
  * convergence check (k_tri_check: eigenvalues of T by multisection and their
  * eigenvectors, jn_tridiag.cuh) runs on its own stream beside the next
- * steps' products: the host enqueues steps k + 1 and k + 2, then reads the check of
- * step k.  The final Ritz vectors are refined by FP64 products (Rayleigh
+ * steps' products: the host enqueues step k + 1 (and k + 2, where steps are
+ * short), then reads the check of step k.  The final Ritz vectors are refined by FP64 products (Rayleigh
  * quotient and residual norm).
  */
 #include <math.h>
@@ -52,13 +52,18 @@
 #define RED_BLOCKS 304      /* 2 x 152 SMs */
 #define RED_THREADS 256
 
-/* Checks in flight, one more than the steps by which the host reads them
- * behind: it enqueues steps k + 1 and k + 2, then reads check k.  A check
+/* Checks in flight at most, one more than the steps by which the host reads
+ * them behind: it enqueues steps k + 1 and k + 2, then reads check k.  A check
  * takes about as long as a small basis's product (83 against 96 us for 4He
  * Nmax 6), and one step behind left the host no time to enqueue the next
  * before the device ran out: 165 steps with a check each 23.1 -> 21.1 ms, where
- * a check every tenth takes 20.7. */
+ * a check every tenth takes 20.7.  The steps behind are run for nothing once a
+ * solve has converged, so where a step takes twice a check and more, from
+ * about 1.5e8 multiply-adds a product on (300 us), it is one: 6Li Nmax 6,
+ * 3.5 ms a step, ends a step sooner; 6Li Nmax 4 with 3NF (5.6e7, 190 us a
+ * step) stays at two. */
 #define CHECKS 3
+#define LONG_STEP 1.5e8
 
 struct jn_lanczos_state {
 	int64_t D;
@@ -643,6 +648,7 @@ extern "C" jn_status jn_lanczos(jn_ctx *c, const jn_lanczos_options *opt, jn_lan
 
 	double prev = 0.0;
 	int k, converged = 0;
+	const int behind = c->plan.visits >= LONG_STEP ? 1 : CHECKS - 1;
 	int pending[CHECKS], npending = 0;      /* rows of the checks that are still to be read, oldest first */
 	/* the eigenvector criterion keeps the previous step's vector (and the current one after it) */
 	const int by_vector = reference_mode && opt->criterion == JN_CONVERGE_EIGENVECTORS;
@@ -720,16 +726,16 @@ extern "C" jn_status jn_lanczos(jn_ctx *c, const jn_lanczos_options *opt, jn_lan
 			if (diff < opt->tolerance) { converged = 1; k++; break; }
 			continue;
 		}
-		/* full mode: this step's check is enqueued, then the one two steps
+		/* full mode: this step's check is enqueued, then the one `behind` steps
 		   before it is read, so the device always holds work; a solve that has
-		   converged has two steps too many in flight, which nothing reads */
+		   converged has as many steps too many in flight, which nothing reads */
 		if (check) {
 			const int wv = nev < n ? nev : n;
 			st = tri_enqueue(c, n, wv + (wv < n ? 1 : 0), wv, 0, n % CHECKS);
 			if (st) return st;
 			pending[npending++] = n;
 		}
-		if (npending && pending[0] <= n - (CHECKS - 1)) {
+		if (npending && pending[0] <= n - behind) {
 			const int t = test_full(pending[0]);
 			if (t < 0) return st;
 			if (t) { converged = 1; k = pending[0]; npending = 0; break; }

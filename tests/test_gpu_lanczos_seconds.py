@@ -25,3 +25,15 @@ def test_refinement_leaves_the_steps_out(problem):
     # two steps of 130 us are a quarter of the refinement's time
     assert after < 1.12 * alone
     H.close()
+
+
+@pytest.mark.slow
+def test_long_steps_past_convergence(problem):
+    d, Z, N, *_ = problem("li6_n6_3b")
+    H = jn.Hamiltonian.from_dir(d, Z, N)
+    for every in (1, 10):
+        t, _, k = _times(H, 3, max_iterations=300, tolerance=1e-4, check_every=every)
+        limit, _, same = _times(H, 3, max_iterations=k, tolerance=1e-300, check_every=every)
+        assert same == k
+        assert t - limit < 1.5 * limit / k
+    H.close()
