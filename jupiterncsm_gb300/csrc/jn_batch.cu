@@ -819,7 +819,7 @@ static jn_status elements_bound(jn_ctx *c, double *me, int64_t n, double *bound,
 
 /* HX = H_i X for the r vectors of B instances of one basis (X, HX: B x r
  * vectors Dp apart) on the block-tile engine in FP64: as many vectors at a
- * time as 512 MB of scratch and the grid take.  (One launch a vector, 56 for
+ * time as 512 MB of scratch, the memory left and the grid take.  (One launch a vector, 56 for
  * 14 vectors on four bases, took 19 ms, most of it launches too small to fill
  * the GPU.) */
 static jn_status refine_products(jn_ctx *c, int B, const double *me64, const double *X, int r, int64_t Dp, double *HX,
@@ -831,14 +831,17 @@ static jn_status refine_products(jn_ctx *c, int B, const double *me64, const dou
 	if (per > 65535 / B) per = 65535 / B;
 	if (per > r) per = r;
 	if (per < 1) per = 1;
+	/* V, X and HX are all there: with less memory left, fewer vectors at a time */
 	double *x64 = NULL;
-	unsigned long long *gacc = NULL;
-	unsigned int *ctrl = NULL;
+	while (cudaMalloc((void **)&x64, (size_t)B * per * (16 * D + 8)) != cudaSuccess) {
+		cudaGetLastError();
+		if (per == 1) return jn_fail(JN_ERR_NOMEM, "batched Lanczos: device allocation of a product's scratch failed");
+		per = (per + 1) / 2;
+	}
+	unsigned long long *gacc = (unsigned long long *)(x64 + (size_t)B * per * D);
+	unsigned int *ctrl = (unsigned int *)(gacc + (size_t)B * per * D);
 	jn_status st = JN_OK;
-	BALLOC(x64, (size_t)B * per * D);
-	BALLOC(gacc, (size_t)B * per * D);
-	BALLOC(ctrl, (size_t)2 * B * per);
-	if (!st && cudaMemsetAsync(gacc, 0, (size_t)B * per * D * sizeof(unsigned long long), q) != cudaSuccess)
+	if (cudaMemsetAsync(gacc, 0, (size_t)B * per * D * sizeof(unsigned long long), q) != cudaSuccess)
 		st = jn_fail(JN_ERR_CUDA, "accumulator clear");
 	for (int j = 0; j < r && !st; j += (int)per) {
 		const int nv = r - j < per ? r - j : (int)per;
@@ -846,7 +849,7 @@ static jn_status refine_products(jn_ctx *c, int B, const double *me64, const dou
 					HX + (size_t)j * Dp, (int64_t)r * Dp, x64, NULL, gacc, ctrl, NULL, abs_bound, q);
 	}
 	if (cudaStreamSynchronize(q) != cudaSuccess && !st) st = jn_fail(JN_ERR_CUDA, "refinement products");
-	cudaFree(x64); cudaFree(gacc); cudaFree(ctrl);
+	cudaFree(x64);
 	return st;
 }
 
