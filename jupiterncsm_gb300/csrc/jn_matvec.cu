@@ -573,10 +573,10 @@ extern "C" jn_status jn_open_files(const char *comb, const char *order, const ch
 	{
 		cudaError_t z = cudaMemset(c->d_gacc, 0, (p->dim ? p->dim : 1) * sizeof(unsigned long long));
 		size_t smem = (size_t)(p->max_tile_elems ? p->max_tile_elems : 1) * 2 * sizeof(unsigned int);
-		if (z == cudaSuccess)
-			z = cudaFuncSetAttribute(jn_tile_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-		if (z == cudaSuccess)
-			z = cudaFuncSetAttribute(jn_tile_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+		/* the limit is the kernel's, shared by every context of the process: the largest tile's, not this plan's */
+		const int limit = JN_TILE_SMEM_ELEMS * 2 * (int)sizeof(unsigned int);
+		if (z == cudaSuccess) z = cudaFuncSetAttribute(jn_tile_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, limit);
+		if (z == cudaSuccess) z = cudaFuncSetAttribute(jn_tile_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, limit);
 		int per_sm_f = 1, per_sm_d = 1;
 		if (z == cudaSuccess)
 			z = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_f, jn_tile_kernel<float>, TILE_THREADS, smem);

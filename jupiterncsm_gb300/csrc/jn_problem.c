@@ -586,8 +586,6 @@ static int cmp_cost_desc(const void *a, const void *b, void *cost)
 	return *(const int *)a - *(const int *)b;
 }
 
-/* shared-memory accumulator budget of one CTA, in 64-bit elements */
-#define TILE_SMEM_ELEMS 8192
 /* work of one lane in one task, at most (multiply-adds plus per-output cost) */
 #define LANE_VISITS 96
 /* fixed per-task cost in the work model, in multiply-add units */
@@ -681,7 +679,7 @@ static void tiles_block(int64_t bi, void *v)
 	}
 	for (size_t e = 0; e < E; e++) o->abs_bound = fmax(o->abs_bound, bound[e]);
 	free(bound);
-	if (stride > TILE_SMEM_ELEMS) { o->status = 2; return; }
+	if (stride > JN_TILE_SMEM_ELEMS) { o->status = 2; return; }
 	int64_t tcap = 0;
 	int rcap = 0;
 #define PUSH_TASK(TERM, KIND, COUNT, LANE_BASE, LOOP_BASE, LOOP_LEN, COST)                     \
@@ -699,7 +697,7 @@ static void tiles_block(int64_t bi, void *v)
 		q_->t.loop_len = (uint32_t)(LOOP_LEN);                                         \
 		q_->cost = TASK_OVERHEAD + (COST);                                             \
 	} while (0)
-	const int64_t R = TILE_SMEM_ELEMS / stride;
+	const int64_t R = JN_TILE_SMEM_ELEMS / stride;
 	for (int64_t r0 = 0; r0 < B->Np; r0 += R) {
 		const int64_t r1 = r0 + R < B->Np ? r0 + R : B->Np;
 		if (o->nranges == rcap) {
@@ -953,7 +951,7 @@ static int build_block_tiles(jn_plan_t *p, const int *term_dst, int target_units
 		p->btiles_off = 1;
 		snprintf(p->btiles_why, sizeof p->btiles_why,
 			 "basis block %d has %lld neutron states: more than one shared-memory row of the block-tile engine (%d)",
-			 p->blocks[wide].id, (long long)p->blocks[wide].Nn, TILE_SMEM_ELEMS - 1);
+			 p->blocks[wide].id, (long long)p->blocks[wide].Nn, JN_TILE_SMEM_ELEMS - 1);
 		return build_tterms(p, err, errlen);
 	}
 	tile_range_t *ranges = status ? NULL : malloc((nranges ? nranges : 1) * sizeof *ranges);

@@ -30,6 +30,9 @@ extern "C" {
 
 enum { JN_KIND_N = 1, JN_KIND_P = 2, JN_KIND_NP = 3 };
 
+/* the accumulator of a block tile at most, in 64-bit elements (shared memory) */
+#define JN_TILE_SMEM_ELEMS 8192
+
 typedef struct {
 	int Ep, Mp, En, Mn;
 	int64_t Np, Nn;
