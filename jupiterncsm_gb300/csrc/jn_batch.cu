@@ -568,10 +568,15 @@ static jn_status batch_solve(cudaStream_t q, const jn_batch_options *o, const ba
 	if (chunk < (Dp + 303) / 304) chunk = (Dp + 303) / 304;
 	if (chunk < 32) chunk = 32;
 	std::vector<int2> cta;
-	std::vector<int> first(B);
-	for (int i = 0; i < B; i++) {
-		first[i] = (int)cta.size();
-		for (int64_t b = 0; b * chunk < job.dims[i]; b++) cta.push_back(make_int2(i, (int)b));
+	std::vector<int> first;
+	try {
+		first.resize(B);
+		for (int i = 0; i < B; i++) {
+			first[i] = (int)cta.size();
+			for (int64_t b = 0; b * chunk < job.dims[i]; b++) cta.push_back(make_int2(i, (int)b));
+		}
+	} catch (const std::bad_alloc &) {
+		if (!st) st = jn_fail(JN_ERR_NOMEM, "out of host memory");
 	}
 	BALLOC(s.part, cta.size() * ncol);
 	BALLOC(s.h, (size_t)B * ncol);
@@ -922,15 +927,19 @@ extern "C" jn_status jn_lanczos_batch(jn_ctx *c, const jn_batch_options *o, jn_b
 		job.num_sms = c->num_sms;
 		job.Dp = D;
 		job.dims = dims;
-		job.product = [&](const double *V, int64_t ldV, const int *d_k, double *W, const int *act, cudaStream_t qs) {
+		/* as references to them: a function made of so large an object allocates */
+		auto product = [&](const double *V, int64_t ldV, const int *d_k, double *W, const int *act, cudaStream_t qs) {
 			return pb ? jn_panel_batch_enqueue(pb, V, ldV, d_k, D, W, D, act, D, qs)
 				  : jn_enqueue_batched(c, B, 1, f32, f32 ? (const void *)me32 : (const void *)me64, nme, V, ldV, 0, d_k, D, W,
 						       D, x64, x32, gacc, ctrl, act, abs_bound, qs);
 		};
-		job.product64 = [&](const double *X, int r, double *HX, cudaStream_t qs) {
+		auto product64 = [&](const double *X, int r, double *HX, cudaStream_t qs) {
 			return refine_products(c, B, me64, X, r, D, HX, abs_bound, qs);
 		};
-		if (pb) job.rebalance = [&](const int *act, int *changed) { return jn_panel_batch_rebalance(pb, act, changed); };
+		auto rebalance = [&](const int *act, int *changed) { return jn_panel_batch_rebalance(pb, act, changed); };
+		job.product = std::ref(product);
+		job.product64 = std::ref(product64);
+		if (pb) job.rebalance = std::ref(rebalance);
 		job.start_vectors = o->start_vectors;
 		job.eigenvectors = o->eigenvectors;
 		job.res = rp;
@@ -1026,12 +1035,13 @@ extern "C" jn_status jn_lanczos_batch_bases(jn_ctx *const *ctxs, int num_bases, 
 		job.num_sms = ctxs[0]->num_sms;
 		job.Dp = Dp;
 		job.dims = dims;
-		job.product = [&](const double *V, int64_t ldV, const int *d_k, double *W, const int *act, cudaStream_t qs) {
+		/* as references to them: a function made of so large an object allocates */
+		auto product = [&](const double *V, int64_t ldV, const int *d_k, double *W, const int *act, cudaStream_t qs) {
 			return pb ? jn_panel_batch_enqueue(pb, V, ldV, d_k, Dp, W, Dp, act, Dp, qs)
 				  : jn_walk_batch_enqueue(wb, mode, V, ldV, d_k, Dp, W, Dp, act, Dp, qs);
 		};
 		/* refinement, basis by basis, on the block-tile engine in FP64 */
-		job.product64 = [&](const double *X, int r, double *HX, cudaStream_t qs) {
+		auto product64 = [&](const double *X, int r, double *HX, cudaStream_t qs) {
 			for (int b = 0; b < num_bases; b++) {
 				const size_t at = (size_t)first[b] * r * Dp;
 				jn_status e = refine_products(ctxs[b], count[b], me64[b], X + at, r, Dp, HX + at, bound[b], qs);
@@ -1039,7 +1049,10 @@ extern "C" jn_status jn_lanczos_batch_bases(jn_ctx *const *ctxs, int num_bases, 
 			}
 			return JN_OK;
 		};
-		if (pb) job.rebalance = [&](const int *act, int *changed) { return jn_panel_batch_rebalance(pb, act, changed); };
+		auto rebalance = [&](const int *act, int *changed) { return jn_panel_batch_rebalance(pb, act, changed); };
+		job.product = std::ref(product);
+		job.product64 = std::ref(product64);
+		if (pb) job.rebalance = std::ref(rebalance);
 		job.start_vectors = sv;
 		job.eigenvectors = ev;
 		job.res = rp;

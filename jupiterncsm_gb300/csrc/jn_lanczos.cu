@@ -652,7 +652,12 @@ extern "C" jn_status jn_lanczos(jn_ctx *c, const jn_lanczos_options *opt, jn_lan
 	int pending[CHECKS], npending = 0;      /* rows of the checks that are still to be read, oldest first */
 	/* the eigenvector criterion keeps the previous step's vector (and the current one after it) */
 	const int by_vector = reference_mode && opt->criterion == JN_CONVERGE_EIGENVECTORS;
-	std::vector<double> zbuf(by_vector ? 2 * (size_t)(m + 1) : 0, 0.0);
+	std::vector<double> zbuf;
+	try {
+		zbuf.resize(by_vector ? 2 * (size_t)(m + 1) : 0);
+	} catch (const std::bad_alloc &) {
+		return jn_fail(JN_ERR_NOMEM, "out of host memory");
+	}
 	double *zprev = zbuf.data();
 	res->iterations = 0;
 	res->iteration_seconds = res->refinement_seconds = 0.0;

@@ -17,8 +17,6 @@
 #include <stdlib.h>
 #include <string.h>
 
-#include <vector>
-
 #include <cooperative_groups.h>
 
 #include "jn_internal.h"
@@ -858,7 +856,7 @@ extern "C" jn_status jn_mlp_train(jn_mlp *m, const float *x, const float *t, int
 	const int64_t t0 = m->t;
 	fused_kernel f = fused_for(m, n, &smem, &grid);
 	if (!s && f) {
-		std::vector<float> corr(2 * FUSED_STEPS);
+		float corr[2 * FUSED_STEPS];
 		for (int it = 0; (it < steps || it == 0) && !s; it += FUSED_STEPS) {
 			const int run = steps - it < FUSED_STEPS ? steps - it : FUSED_STEPS;
 			for (int i = 0; i < run; i++) {
@@ -867,7 +865,7 @@ extern "C" jn_status jn_mlp_train(jn_mlp *m, const float *x, const float *t, int
 				corr[2 * i + 1] = 1.0f - powf(ADAM_B2, (float)m->t);
 			}
 			/* pageable memory: the copy has left `corr` when the call returns */
-			if (run) CUDA_TRY(cudaMemcpyAsync(m->d_corr, corr.data(), 2 * run * sizeof(float), cudaMemcpyHostToDevice, m->stream));
+			if (run) CUDA_TRY(cudaMemcpyAsync(m->d_corr, corr, 2 * run * sizeof(float), cudaMemcpyHostToDevice, m->stream));
 			/* the last launch also takes the loss of the final parameters */
 			s = fused_run(m, f, smem, grid, n, it, run, lr, 0, it + FUSED_STEPS >= steps);
 		}

@@ -1303,7 +1303,7 @@ static void panel_batch_split(const std::vector<double> &cost, const std::vector
  * 1 024 threads.  One round of CTAs: two rounds clear and flush every
  * accumulator twice as often (+1.5 % of the whole solve, three +6 %).  The
  * result does not depend on the partition. */
-static jn_status panel_batch_partition(jn_panel_batch *pb, const int *act)
+static jn_status panel_batch_share_out(jn_panel_batch *pb, const int *act)
 {
 	const int sms = pb->ctxs[0]->num_sms;
 	std::vector<int> count(pb->nbases, 0), g(pb->nbases, 0);
@@ -1324,29 +1324,28 @@ static jn_status panel_batch_partition(jn_panel_batch *pb, const int *act)
 	int optin = 0, xs = 0;
 	CUDA_TRY(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, pb->ctxs[0]->device));
 	struct host_part {
-		uint32_t *cta, *fptr, *flush;
-		int64_t nf, words;
+		uint32_t *cta = NULL, *fptr = NULL, *flush = NULL;
+		int64_t nf = 0, words = 0;
+		void release()
+		{
+			free(cta); free(fptr); free(flush);
+			cta = fptr = flush = NULL;
+			nf = words = 0;
+		}
+		~host_part() { release(); }
 	};
 	std::vector<host_part> hp(pb->nbases);
-	auto release = [&]() {
-		for (auto &q : hp) {
-			free(q.cta); free(q.fptr); free(q.flush);
-			memset(&q, 0, sizeof q);
-		}
-	};
 	size_t smem = 0;
 	for (int shape = 0; shape < 2; shape++) {
 		const int per = shape == 0 ? 3 : 1;
 		size_t with = 0, without = 0;
-		release();
+		for (auto &q : hp) q.release();
 		panel_batch_split(cost, per_cta, count, per * sms, g);
 		for (int b = 0; b < pb->nbases; b++) {
 			if (!count[b]) continue;
 			const jn_plan_t *p = &pb->ctxs[b]->plan;
-			if (jn_panels_partition(p, g[b], &hp[b].cta, &hp[b].fptr, &hp[b].flush, &hp[b].nf, &hp[b].words)) {
-				release();
+			if (jn_panels_partition(p, g[b], &hp[b].cta, &hp[b].fptr, &hp[b].flush, &hp[b].nf, &hp[b].words))
 				return jn_fail(JN_ERR_NOMEM, "out of host memory");
-			}
 			with = std::max(with, panel_smem_words(p, hp[b].words, 1));
 			without = std::max(without, panel_smem_words(p, hp[b].words, 0));
 		}
@@ -1377,7 +1376,6 @@ static jn_status panel_batch_partition(jn_panel_batch *pb, const int *act)
 		pb->h[i].words = (int)hp[b].words;
 		for (int k = 0; k < g[b]; k++) cl.push_back({ cost[b] / g[b] + per_cta[b], make_int2(i, k) });
 	}
-	release();
 	if (s) return s;
 	std::stable_sort(cl.begin(), cl.end(), [](const std::pair<double, int2> &x, const std::pair<double, int2> &y) { return x.first > y.first; });
 	std::vector<int2> list;
@@ -1395,6 +1393,15 @@ static jn_status panel_batch_partition(jn_panel_batch *pb, const int *act)
 				      (int)std::max(smem, (size_t)optin - 1024)));
 	CUDA_TRY(cudaDeviceSynchronize());
 	return JN_OK;
+}
+
+static jn_status panel_batch_partition(jn_panel_batch *pb, const int *act)
+{
+	try {
+		return panel_batch_share_out(pb, act);
+	} catch (const std::bad_alloc &) {
+		return jn_fail(JN_ERR_NOMEM, "out of host memory");
+	}
 }
 
 jn_status jn_panel_batch_rebalance(jn_panel_batch *pb, const int *act, int *changed)
