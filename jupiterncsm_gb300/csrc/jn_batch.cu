@@ -721,11 +721,8 @@ static jn_status batch_solve(cudaStream_t q, const jn_batch_options *o, const ba
 		kb_tri_pairs<<<dim3(r, B), 64, tri_smem ? JN_TRI_SMEM(k) : 0, q>>>(
 			s.alpha, s.beta, ldab, s.narr, r, s.theta, r + 1, s.Z, ldz, s.work, NULL, 1, 0, NULL);
 		kb_tri_mgs<<<g1, BT, 0, q>>>(s.Z, ldz, s.narr, r, NULL);
-		/* instances in waves of the grid's third dimension */
-		for (int i = 0; i < B; i += 65535)
-			kb_ritz<<<dim3((unsigned int)((Dp + 127) / 128), (r + RITZ_ROWS - 1) / RITZ_ROWS, B - i < 65535 ? B - i : 65535), 128, 0,
-				  q>>>(s.V + (size_t)i * ldV, ldV, s.Z + (size_t)i * r * ldz, ldz, s.narr + i, r, Dp, dims + i,
-				       s.X + (size_t)i * r * Dp);
+		kb_ritz<<<dim3((unsigned int)((Dp + 127) / 128), (r + RITZ_ROWS - 1) / RITZ_ROWS, B), 128, 0, q>>>(
+			s.V, ldV, s.Z, ldz, s.narr, r, Dp, dims, s.X);
 		st = job.product64(s.X, r, s.HX, q);
 	}
 	if (!st) {

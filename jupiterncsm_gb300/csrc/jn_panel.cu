@@ -1115,7 +1115,7 @@ struct jn_panel_inst {
 	unsigned long long *gacc;
 	const unsigned long long *cmax; /* max|c| bits of the instance's coefficients */
 	int64_t dim;
-	int grid, words, nblocks;
+	int words, nblocks;
 	int owner;                      /* the first instance of a basis owns the basis's coefficient arrays */
 };
 static_assert(sizeof(jn_panel_inst) == 112, "one descriptor is 112 bytes");
@@ -1372,7 +1372,6 @@ static jn_status panel_batch_share_out(jn_panel_batch *pb, const int *act)
 		pb->h[i].cta = pb->parts[b].cta;
 		pb->h[i].flush_ptr = pb->parts[b].flush_ptr;
 		pb->h[i].flush = pb->parts[b].flush;
-		pb->h[i].grid = g[b];
 		pb->h[i].words = (int)hp[b].words;
 		for (int k = 0; k < g[b]; k++) cl.push_back({ cost[b] / g[b] + per_cta[b], make_int2(i, k) });
 	}

@@ -25,9 +25,8 @@
 
 #include <stdint.h>
 
-/* doubles of scratch one warp needs for n rows: the staged matrix, and with
- * it the work space of one vector */
-#define JN_TRI_VALUE_DOUBLES(n) (2 * (size_t)(n))
+/* doubles of scratch one warp needs for n rows: the staged matrix and the
+ * work space of one vector */
 #define JN_TRI_VECTOR_DOUBLES(n) (8 * (size_t)(n) + 8)
 /* rows up to which that scratch is taken in shared memory (204 KB) */
 #define JN_TRI_SMEM_ROWS 3192
