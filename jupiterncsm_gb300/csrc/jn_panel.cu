@@ -196,8 +196,8 @@ __device__ __forceinline__ PanelBlock panel_block(const uint32_t *__restrict__ f
  * and a word's block is found among them by shuffles.  The blocks' records
  * are so two dependent loads for 32 blocks; block by block, with the whole
  * CTA on each, a CTA paid about 830 cycles a block (4He Nmax 6: 6 blocks a
- * CTA on average, up to 44; the 32-bit product went from 76.5 to 65.5 us;
- * 3H Nmax 8 60.3 to 39.5 us). */
+ * CTA on average, up to 44; 32-bit products back to back went from 76.5 to
+ * 65.5 us, the call from 82 to 76; 3H Nmax 8 back to back 60.3 to 39.5 us). */
 template <typename Body>
 __device__ __forceinline__ void panel_words(const uint32_t *__restrict__ flush, const uint4 *__restrict__ blocks, uint32_t f0,
 					    uint32_t f1, PanelBlock b, Body body)
@@ -1312,8 +1312,9 @@ static jn_status panel_batch_share_out(jn_panel_batch *pb, const int *act)
 	double work = 0.0;
 	for (int b = 0; b < pb->nbases; b++) {
 		const jn_plan_t *p = &pb->ctxs[b]->plan;
-		/* clearing, staging and adding an accumulator of the whole vector, about 100 instructions a warp's words
-		   where a contribution takes 45, and the latencies at both ends */
+		/* in contributions of 45 instructions: 2.2 for clearing, staging and adding a warp's words of the
+		   accumulator (of the whole vector), about 100 instructions, and 300, taken and not fitted, for the
+		   latencies at both ends */
 		per_cta[b] = 300.0 + 2.2 / 32 * (double)p->psmem_words;
 	}
 	for (int i = 0; i < pb->B; i++)

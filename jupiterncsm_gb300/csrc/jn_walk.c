@@ -544,13 +544,15 @@ static void wdir_free(wdir_t *D)
  * Tasks differ by two orders of magnitude, and a long one taken last keeps
  * one warp busy while the others have nothing left.  So the last
  * WALK_TAIL_TASKS of the list (all of them for most bases) go by falling
- * cost, in classes of powers of two that keep the order inside a class; their
- * matrix elements fit L2 together, which the list's order otherwise serves.
- * Products back to back, list order -> by cost: 6Li Nmax 4 2NF (18 659 tasks)
- * 50.2 -> 42.3 us; with 3NF 7Li Nmax 4 (44 758) 117 -> 92, 4He Nmax 6 (51 432)
- * 129 -> 99, 6Li Nmax 4 (82 282) 174 -> 148 us (157 with the last 65 536 by
- * cost); 6Li Nmax 6 (1.4 million) 3498 -> 3488 us, but 3606 us with all of
- * them by cost.
+ * cost, in classes of powers of two that keep the order inside a class.  The
+ * list's order lets L2 serve the elements that neighbouring instructions
+ * share.  The smaller bases measured read blocks of 4 to 210 MB, of which L2
+ * holds all or most in any order; of 6Li Nmax 6 (blocks of 3.5 GB) these tasks
+ * are the last 5 % of the work.  Products back to back, list order -> by cost:
+ * 6Li Nmax 4 2NF (18 659 tasks) 47.2 -> 38.5 us; with 3NF 7Li Nmax 4 (44 870)
+ * 105 -> 82.4, 4He Nmax 6 (51 444) 123 -> 93.3, 6Li Nmax 4 (82 470) 163.5 ->
+ * 145.0 us (143.6 with the last 65 536 by cost); 6Li Nmax 6 (1.45 million)
+ * 3408 us either way, but 3560 us with all of them by cost.
  */
 #define WALK_TAIL_TASKS 131072
 
@@ -586,12 +588,12 @@ static int order_tail(jn_wtask_t *t, int64_t n, const jn_wpiece_t *pieces, int64
  * Rows of a piece.  A task's fixed cost (its records, its sums) asks for long
  * pieces, the end of the product for short ones: at most WALK_CAP rows, and
  * WALK_CAP_FEW where that leaves at most WALK_FEW_TASKS tasks, about as many
- * as the chip holds warps twice over, so that the longest task sets the time.
- * Products back to back with 64, 16, 8, 4 and 2 rows: 4He Nmax 2 (145 tasks)
- * 12.4, 12.4, 12.3, 10.3, 10.3 us; 6Li Nmax 2 (about 2000) 18.5, 18.5, 15.0,
- * 14.4, 14.4; 4He Nmax 4 (2396) 19.3, 19.3, 16.8, 16.4, 17.4; 6Li Nmax 4
- * (18 659) 42.0, 42.2, 41.9, 48.0, 63.5; 7Li Nmax 4 with 3NF (44 758) 88.8,
- * 92.2, 99.6, 116, 168.
+ * as the chip holds warps twice over (152 SMs of 28), so that the longest task
+ * sets the time.  Products back to back with 64, 16, 8, 4 and 2 rows: 4He Nmax 2
+ * (145 tasks at 64 rows) 8.5, 8.5, 8.5, 7.8, 7.5 us; 6Li Nmax 2 (1279) 13.9, 12.9,
+ * 12.0, 11.2, 11.9; 4He Nmax 4 (2396) 15.4, 15.3, 13.6, 13.5, 15.2; 6Li Nmax 4
+ * (18 659) 38.5, 37.8, 38.1, 45.1, 62.0; with 3NF 7Li Nmax 4 (44 870) 82.4, 85.4,
+ * 92.4, 112, 163; 4He Nmax 6 (51 444) 93.3, 95.2, 102, 118, 158.
  */
 #define WALK_CAP 64
 #define WALK_CAP_FEW 4

@@ -364,10 +364,10 @@ __global__ void jn_walk_xview_kernel(const double *__restrict__ x, const int32_t
  * counter ctrl[1] to zero.
  * Bound by latency; it stands for a memset and two kernels.  Up to 12 288
  * states reading x once per CTA costs less than those launches: products back
- * to back at D = 59 / 952 / 7916 / 10 817 / 15 764 take 12.4 / 21.3 / 128.3 /
- * 117.0 / 49.6 us with it and 15.4 / 23.0 / 129.4 / 118.3 / 49.6 us without
- * (a cluster of eight CTAs that meets over the maximum: 16.4 / 26.6 / 132.4 /
- * 121.3 / 52.8 us). */
+ * to back at D = 59 / 952 / 7916 / 10 817 take 7.8 / 13.5 / 93.3 / 82.4 us with
+ * it and 13.3 / 17.5 / 96.0 / 85.2 us without; at 15 764 the two took the same.
+ * (A cluster of eight CTAs that meets over the maximum was slower than either at
+ * all of these.) */
 #define WALK_SMALL_THREADS 256
 #define WALK_SMALL_DIM 12288
 template <int MODE>
